@@ -6,6 +6,7 @@ a RuntimeError is raised.  Nothing here computes anything on the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -69,6 +70,25 @@ def load():
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+HOST_PATH = os.path.join(HERE, "_mamba_b200_host.so")
+_host = None
+
+
+def host():
+    """The host-side extension (csrc/host), loaded on first use.  Raises if it was never built."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m mamba_b200.build` (needs g++)")
+        import torch  # noqa: F401  (the extension links against torch's libraries)
+        spec = importlib.util.spec_from_file_location("_mamba_b200_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def check(code: int, what: str) -> None:

@@ -1,0 +1,118 @@
+// Host side of the package in C++: argument checks, allocations, autograd nodes and kernel launches, so that a call
+// costs a few microseconds of host time instead of a few tens.  Device work goes through the C ABI of
+// libmamba_b200.so (include/mamba_b200.h) only.
+#pragma once
+#include <torch/extension.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/core/grad_mode.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <optional>
+#include "mamba_b200.h"
+
+namespace mb200_host {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// ---- checks and preparation ------------------------------------------------------------------------------
+inline const Tensor& undefined() {
+  static const Tensor t;
+  return t;
+}
+inline const Tensor& value(const OptTensor& t) { return t.has_value() ? *t : undefined(); }
+
+template <typename... Ts> void require_cuda(const Ts&... ts) {
+  for (const Tensor* t : {&ts...})
+    TORCH_CHECK(!t->defined() || t->is_cuda(), "mamba_b200 runs on CUDA tensors only (there is no CPU path)");
+}
+
+inline void check(int rc, const char* what) {
+  TORCH_CHECK(rc == MB200_OK, what, " failed: ", mb200_strerror(rc), " (code ", rc, ")");
+}
+
+// Activation dtype a kernel runs in: bfloat16 only when EVERY activation tensor is bfloat16, float32 as soon as one of
+// them is (under autocast the reference keeps delta in float32 while x, B and C are bfloat16,
+// mambapy/mamba.py:264-265; rounding delta to bfloat16 would change the decay).
+template <typename... Ts> at::ScalarType act_dtype(const Ts&... ts) {
+  bool all_bf16 = true;
+  for (const Tensor* t : {&ts...}) {
+    if (!t->defined()) continue;
+    const auto d = t->scalar_type();
+    TORCH_CHECK_TYPE(d == at::kFloat || d == at::kBFloat16, "mamba_b200 kernels take float32 or bfloat16 activations, got ", d);
+    all_bf16 = all_bf16 && d == at::kBFloat16;
+  }
+  return all_bf16 ? at::kBFloat16 : at::kFloat;
+}
+inline int dtype_code(at::ScalarType d) { return d == at::kBFloat16 ? MB200_BF16 : MB200_F32; }
+
+// Cast to the activation dtype and make the last dimension unit-stride (copies only if needed).
+inline Tensor rows(const Tensor& t, at::ScalarType dt) {
+  if (!t.defined()) return t;
+  Tensor r = t.scalar_type() == dt ? t : t.to(dt);
+  return r.stride(-1) == 1 ? r : r.contiguous();
+}
+inline Tensor f32(const Tensor& t) {
+  if (!t.defined()) return t;
+  return (t.scalar_type() == at::kFloat && t.is_contiguous()) ? t.detach() : t.detach().to(at::kFloat).contiguous();
+}
+inline Tensor like(const Tensor& grad, at::ScalarType dt) { return grad.scalar_type() == dt ? grad : grad.to(dt); }
+
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+inline int64_t st(const Tensor& t, int d) { return t.defined() ? t.stride(d) : 0; }
+inline Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& on) { return at::empty(shape, on.options().dtype(dt)); }
+inline void* cuda_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+
+// With MB200_CHECK_STATUS=1 in the environment every fused-scan launch is followed by a device synchronisation and a
+// read of the kernels' status word; a bounded wait that gave up then raises.
+void check_status(const char* what);
+
+// The library's own tensor operations record nothing: autograd sees the nodes below only.
+using BelowAutograd = at::AutoDispatchBelowADInplaceOrView;
+
+// ---- autograd plumbing ------------------------------------------------------------------------------------
+template <typename... Ts> bool wants_grad(const Ts&... ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : {&ts...})
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+template <typename N> std::shared_ptr<N> new_node() { return std::shared_ptr<N>(new N(), torch::autograd::deleteNode); }
+
+// A tensor kept for the backward; intermediates and inputs alike (version counters are checked on unpacking).
+struct Saved {
+  SavedVariable v;
+  bool defined = false;
+  void save(const Tensor& t, bool is_output = false) {
+    defined = t.defined();
+    if (defined) v = SavedVariable(t, is_output);
+  }
+  Tensor get(const std::shared_ptr<torch::autograd::Node>& self = nullptr) const { return defined ? v.unpack(self) : Tensor(); }
+  void reset() { v.reset_data(); }
+};
+
+// What a node remembers of an input whose gradient it returns.
+inline at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() : at::kFloat; }
+
+// ---- entry points -------------------------------------------------------------------------------------------
+py::object selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D,
+                          const OptTensor& z, const OptTensor& delta_bias, const OptTensor& h0, bool return_last_state, bool reverse,
+                          std::optional<int64_t> subshards);
+Tensor pscan(const Tensor& A, const Tensor& X);
+Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias);
+Tensor rms_norm(const Tensor& x, const OptTensor& weight, double eps);
+std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residual, const OptTensor& weight, double eps);
+std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const Tensor& delta, const Tensor& A, const Tensor& B,
+                                    const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& delta_bias, bool inplace);
+std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace);
+
+int64_t pick_subshards(int64_t batch, int64_t length, int64_t width);
+
+}  // namespace mb200_host

@@ -1,0 +1,262 @@
+// The per-layer operations around the scan: depthwise convolution + SiLU, RMSNorm with and without the residual add, and
+// the two kernels of a decode step.
+#include "host.h"
+
+namespace mb200_host {
+namespace {
+
+void zero_fill(const Tensor& t) { C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), at::cuda::getCurrentCUDAStream())); }
+
+Tensor filter(const Tensor& weight) { return f32(weight).view({weight.size(0), weight.size(-1)}); }
+
+struct ConvBackward : public torch::autograd::Node {
+  Saved x, w, b;
+  at::ScalarType tx, tw, tb;
+  std::vector<int64_t> w_shape;
+  std::string name() const override { return "CausalConv1dSiluBackward"; }
+  void release_variables() override { x.reset(); w.reset(); b.reset(); }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    const BelowAutograd guard_ad;
+    const Tensor xs = x.get(), w32 = w.get(), b32 = b.get();
+    const c10::cuda::CUDAGuard guard(xs.device());
+    const Tensor dy = rows(grads[0], xs.scalar_type());
+    const int64_t B = xs.size(0), L = xs.size(1), W = xs.size(2), K = w32.size(1);
+    const Tensor dx = empty({B, L, W}, xs.scalar_type(), xs), acc = empty({W * K + W}, at::kFloat, xs);
+    zero_fill(acc);
+    const Tensor dw = acc.narrow(0, 0, W * K).view({W, K}), db = b32.defined() ? acc.narrow(0, W * K, W) : Tensor();
+    check(mb200_conv1d_silu_bwd(ptr(xs), fptr(w32), fptr(b32), ptr(dy), ptr(dx), fptr(dw), fptr(db), B, L, W, int(K), st(xs, 0), st(xs, 1),
+                                st(dy, 0), st(dy, 1), st(dx, 0), st(dx, 1), dtype_code(xs.scalar_type()), cuda_stream()),
+          "mb200_conv1d_silu_bwd");
+    out[0] = like(dx, tx);
+    out[1] = like(dw, tw).view(w_shape);
+    if (db.defined()) out[2] = like(db, tb);
+    return out;
+  }
+};
+
+}  // namespace
+
+Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias_) {
+  const Tensor& bias = value(bias_);
+  require_cuda(x, weight, bias);
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor y, xs, w32, b32;
+  {
+    const BelowAutograd guard_ad;
+    xs = rows(x, act_dtype(x));
+    w32 = filter(weight);
+    b32 = f32(bias);
+    const int64_t B = xs.size(0), L = xs.size(1), W = xs.size(2), K = w32.size(1);
+    y = empty({B, L, W}, xs.scalar_type(), xs);
+    check(mb200_conv1d_silu_fwd(ptr(xs), fptr(w32), fptr(b32), ptr(y), B, L, W, int(K), st(xs, 0), st(xs, 1), st(y, 0), st(y, 1),
+                                dtype_code(xs.scalar_type()), cuda_stream()),
+          "mb200_conv1d_silu_fwd");
+  }
+  if (wants_grad(x, weight, bias)) {
+    auto node = new_node<ConvBackward>();
+    node->set_next_edges(torch::autograd::collect_next_edges(x, weight, bias));
+    node->x.save(xs); node->w.save(w32); node->b.save(b32);
+    node->tx = type_of(x); node->tw = type_of(weight); node->tb = type_of(bias);
+    node->w_shape = weight.sizes().vec();
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+// ------------------------------------------------------------------------------------------------------ norms
+namespace {
+
+// (rows, D) view of a tensor for the row-wise kernels.
+Tensor row_view(const Tensor& t, at::ScalarType dt) {
+  Tensor r = t.reshape({-1, t.size(-1)});
+  if (r.scalar_type() != dt) r = r.to(dt);
+  return r.stride(-1) == 1 ? r : r.contiguous();
+}
+
+struct RmsNormBackward : public torch::autograd::Node {
+  Saved x, w, rstd;
+  std::vector<int64_t> shape;
+  at::ScalarType tx, tw;
+  std::string name() const override { return "RMSNormBackward"; }
+  void release_variables() override { x.reset(); w.reset(); rstd.reset(); }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(2);
+    if (!grads[0].defined()) return out;
+    const BelowAutograd guard_ad;
+    const Tensor x2 = x.get(), w32 = w.get(), rs = rstd.get();
+    const c10::cuda::CUDAGuard guard(x2.device());
+    const int64_t n = x2.size(0), D = x2.size(1);
+    const Tensor dy = row_view(grads[0], x2.scalar_type()), dx = empty({n, D}, x2.scalar_type(), x2);
+    Tensor dw;
+    if (w32.defined()) {
+      dw = empty({D}, at::kFloat, x2);
+      zero_fill(dw);
+    }
+    check(mb200_rmsnorm_bwd(ptr(x2), fptr(w32), fptr(rs), ptr(dy), ptr(dx), fptr(dw), n, D, st(x2, 0), st(dy, 0), st(dx, 0),
+                            dtype_code(x2.scalar_type()), cuda_stream()),
+          "mb200_rmsnorm_bwd");
+    out[0] = like(dx.view(shape), tx);
+    if (dw.defined()) out[1] = like(dw, tw);
+    return out;
+  }
+};
+
+struct AddRmsNormBackward : public torch::autograd::Node {
+  Saved s, w, rstd;
+  std::vector<int64_t> shape;
+  at::ScalarType tx, tr, tw;
+  bool has_residual = false;
+  std::string name() const override { return "AddRMSNormBackward"; }
+  void release_variables() override { s.reset(); w.reset(); rstd.reset(); }
+  variable_list apply(variable_list&& grads) override {                    // d y, d s -> x, residual, weight
+    variable_list out(3);
+    const BelowAutograd guard_ad;
+    const Tensor sum = s.get(shared_from_this()), w32 = w.get(), rs = rstd.get();
+    const c10::cuda::CUDAGuard guard(sum.device());
+    const Tensor s2 = sum.view({-1, sum.size(-1)});
+    const int64_t n = s2.size(0), D = s2.size(1);
+    const auto ts = s2.scalar_type();
+    Tensor ds;
+    if (grads[0].defined()) {
+      auto ty = grads[0].scalar_type();
+      if (ty != at::kBFloat16 || ts == at::kBFloat16) ty = ts == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
+      const Tensor dy = row_view(grads[0], ty), dr = grads[1].defined() ? row_view(grads[1], ts) : Tensor();
+      ds = empty({n, D}, ts, s2);
+      Tensor dw;
+      if (w32.defined()) {
+        dw = empty({D}, at::kFloat, s2);
+        zero_fill(dw);
+      }
+      check(mb200_add_rmsnorm_bwd(ptr(s2), fptr(w32), fptr(rs), ptr(dy), ptr(dr), ptr(ds), fptr(dw), n, D, st(s2, 0), st(dy, 0), st(dr, 0),
+                                  st(ds, 0), dtype_code(ts), dtype_code(ty), cuda_stream()),
+            "mb200_add_rmsnorm_bwd");
+      if (dw.defined()) out[2] = like(dw, tw);
+      ds = ds.view(shape);
+    } else {
+      ds = grads[1];                                                       // only the sum was used further on
+      if (!ds.defined()) return out;
+    }
+    out[0] = like(ds, tx);
+    if (has_residual) out[1] = like(ds, tr);
+    return out;
+  }
+};
+
+constexpr const char* kNeedCuda = "mamba_b200 kernels need CUDA tensors; there is no CPU path";
+
+}  // namespace
+
+Tensor rms_norm(const Tensor& x, const OptTensor& weight_, double eps) {
+  const Tensor& weight = value(weight_);
+  TORCH_CHECK(x.is_cuda(), kNeedCuda);
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor y, x2, w32, rstd;
+  {
+    const BelowAutograd guard_ad;
+    const auto dt = act_dtype(x);
+    x2 = row_view(x, dt);
+    w32 = f32(weight);
+    const int64_t n = x2.size(0), D = x2.size(1);
+    y = empty(x.sizes(), dt, x);
+    rstd = empty({n}, at::kFloat, x);
+    check(mb200_rmsnorm_fwd(ptr(x2), fptr(w32), ptr(y), fptr(rstd), n, D, st(x2, 0), D, float(eps), dtype_code(dt), cuda_stream()),
+          "mb200_rmsnorm_fwd");
+  }
+  if (wants_grad(x, weight)) {
+    auto node = new_node<RmsNormBackward>();
+    node->set_next_edges(torch::autograd::collect_next_edges(x, weight));
+    node->x.save(x2); node->w.save(w32); node->rstd.save(rstd);
+    node->shape = x.sizes().vec();
+    node->tx = type_of(x); node->tw = type_of(weight);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residual_, const OptTensor& weight_, double eps) {
+  const Tensor &residual = value(residual_), &weight = value(weight_);
+  TORCH_CHECK(x.is_cuda(), kNeedCuda);
+  const c10::cuda::CUDAGuard guard(x.device());
+  // the sum has the type `x + residual` would give; under autocast y comes out in the autocast dtype, which is what the
+  // projection that consumes it would cast it to anyway
+  const auto ts = residual.defined() ? c10::promoteTypes(x.scalar_type(), residual.scalar_type()) : x.scalar_type();
+  auto ty = at::autocast::is_autocast_enabled(at::kCUDA) ? at::autocast::get_autocast_dtype(at::kCUDA) : ts;
+  if (ty != at::kBFloat16) ty = at::kFloat;
+  Tensor y, s, w32, rstd;
+  {
+    const BelowAutograd guard_ad;
+    act_dtype(x, residual);
+    const Tensor x2 = row_view(x, x.scalar_type()), r2 = residual.defined() ? row_view(residual, ts) : Tensor();
+    w32 = f32(weight);
+    const int64_t n = x2.size(0), D = x2.size(1);
+    s = empty(x.sizes(), ts, x);
+    y = empty(x.sizes(), ty, x);
+    rstd = empty({n}, at::kFloat, x);
+    check(mb200_add_rmsnorm_fwd(ptr(x2), ptr(r2), fptr(w32), ptr(s), ptr(y), fptr(rstd), n, D, st(x2, 0), st(r2, 0), D, D, float(eps),
+                                dtype_code(x2.scalar_type()), dtype_code(ts), dtype_code(ty), cuda_stream()),
+          "mb200_add_rmsnorm_fwd");
+  }
+  if (wants_grad(x, residual, weight)) {
+    auto node = new_node<AddRmsNormBackward>();
+    node->set_next_edges(torch::autograd::collect_next_edges(x, residual, weight));
+    node->shape = x.sizes().vec();
+    node->tx = type_of(x); node->tr = type_of(residual); node->tw = type_of(weight);
+    node->has_residual = residual.defined();
+    variable_list outs{y, s};
+    torch::autograd::set_history(outs, node);
+    node->s.save(s, true); node->w.save(w32); node->rstd.save(rstd);
+  }
+  return {y, s};
+}
+
+// ------------------------------------------------------------------------------------------------ decode step
+std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h_, const Tensor& delta, const Tensor& A, const Tensor& B,
+                                    const Tensor& C, const OptTensor& D_, const OptTensor& z_, const OptTensor& bias_, bool inplace) {
+  const Tensor &h = value(h_), &D = value(D_), &z = value(z_), &bias = value(bias_);
+  require_cuda(x, delta, A, B, C, D, z, bias, h);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const BelowAutograd guard_ad;
+  const auto dt = act_dtype(x, delta, z, B, C);
+  const Tensor xs = rows(x, dt), ds = rows(delta, dt), zs = rows(z, dt), Bs = rows(B, dt), Cs = rows(C, dt);
+  const Tensor A32 = f32(A), D32 = f32(D), b32 = f32(bias), h32 = f32(h);
+  const int64_t n = xs.size(0), W = xs.size(1), N = A32.size(1);
+  Tensor h_new;
+  if (inplace) {
+    TORCH_CHECK_VALUE(h.defined() && h32.data_ptr() == h.data_ptr(), "inplace=True needs a float32 contiguous state tensor");
+    h_new = h;
+  } else {
+    h_new = empty({n, W, N}, at::kFloat, xs);
+  }
+  const Tensor y = empty({n, W}, dt, xs);
+  check(mb200_ssm_step(ptr(xs), ptr(ds), ptr(zs), fptr(A32), ptr(Bs), ptr(Cs), fptr(D32), fptr(b32), fptr(h32), fptr(h_new), ptr(y), n, W,
+                       int(N), st(xs, 0), st(ds, 0), st(zs, 0), st(Bs, 0), st(Cs, 0), st(y, 0), dtype_code(dt),
+                       b32.defined() ? MB200_DELTA_SOFTPLUS : 0, cuda_stream()),
+        "mb200_ssm_step");
+  return {y, h_new};
+}
+
+std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias_, bool inplace) {
+  const Tensor& bias = value(bias_);
+  require_cuda(x, inputs, weight, bias);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const BelowAutograd guard_ad;
+  const auto dt = act_dtype(x);
+  const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), w32 = filter(weight), b32 = f32(bias);
+  const int64_t n = xs.size(0), W = xs.size(1);
+  const Tensor xc = empty({n, W}, dt, xs);
+  Tensor fresh;
+  if (inplace) {
+    TORCH_CHECK_VALUE(win.data_ptr() == inputs.data_ptr(), "inplace=True needs a contiguous window of the activation dtype");
+    fresh = inputs;
+  } else {
+    fresh = empty(win.sizes(), dt, xs);
+  }
+  check(mb200_conv_step(ptr(xs), ptr(win), fptr(w32), fptr(b32), ptr(xc), ptr(fresh), n, W, int(w32.size(1)), st(xs, 0), dtype_code(dt),
+                        cuda_stream()),
+        "mb200_conv_step");
+  return {xc, fresh};
+}
+
+}  // namespace mb200_host

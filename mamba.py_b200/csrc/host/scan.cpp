@@ -1,0 +1,323 @@
+// selective_scan_fn and pscan: forward launches and their autograd nodes.
+#include "host.h"
+#include <cstdlib>
+
+namespace mb200_host {
+
+void check_status(const char* what) {
+  static const bool on = [] {
+    const char* v = std::getenv("MB200_CHECK_STATUS");
+    return v && *v && std::string(v) != "0";
+  }();
+  if (!on) return;
+  const int s = mb200_device_status();
+  TORCH_CHECK(s == 0, what, ": a bounded wait inside the kernel gave up (device status ", s, "); its outputs are invalid");
+}
+
+namespace {
+
+constexpr int64_t kResidentCtas = 444;          // 148 SMs x 3 CTAs of the fused kernels
+
+// The tensors of a scan as the kernels take them.
+struct ScanArgs {
+  Tensor x, delta, A, B, C, D, z, bias, h0;
+  bool reverse = false;
+  int flags() const { return (bias.defined() ? MB200_DELTA_SOFTPLUS : 0) | (reverse ? MB200_REVERSE : 0); }
+  int code() const { return dtype_code(x.scalar_type()); }
+  int64_t batch() const { return x.size(0); }
+  int64_t length() const { return x.size(1); }
+  int64_t width() const { return x.size(2); }
+  int64_t states() const { return A.size(1); }
+};
+
+struct ScanOut {
+  Tensor y, hT, carries, P;
+};
+
+// 16-byte aligned base and byte strides: what a tiled tensor map of a (B, L, C) tensor needs.
+bool tensor_map_ok(const Tensor& t) {
+  const int64_t es = t.element_size();
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 && t.stride(1) * es % 16 == 0;
+}
+
+// (B, L, C) -> (B*S, L/S, C): every batch row cut into S consecutive pieces (a view when the strides allow it).
+Tensor cut(const Tensor& t, int64_t S) {
+  if (!t.defined() || S == 1) return t;
+  return t.unflatten(1, {S, t.size(1) / S}).flatten(0, 1);
+}
+Tensor join(const Tensor& t, int64_t S) {
+  if (!t.defined() || S == 1) return t;
+  return t.unflatten(0, {t.size(0) / S, S}).flatten(1, 2);
+}
+
+int launch_forward(const ScanArgs& a, ScanOut& o, bool want_last, bool want_carries) {
+  const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states(), chunk = mb200_sscan_chunk();
+  o.y = empty({B, L, W}, a.x.scalar_type(), a.x);
+  if (want_last) o.hT = empty({B, W, N}, at::kFloat, a.x);
+  if (want_carries) o.carries = empty({B, (L + chunk - 1) / chunk, W, N}, at::kFloat, a.x);
+  const int rc = mb200_sscan_fwd(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), fptr(a.h0),
+                                 ptr(o.y), fptr(o.hT), fptr(o.carries), B, L, W, int(N), st(a.x, 0), st(a.x, 1), st(a.delta, 0),
+                                 st(a.delta, 1), st(a.z, 0), st(a.z, 1), st(a.B, 0), st(a.B, 1), st(a.C, 0), st(a.C, 1), st(o.y, 0),
+                                 st(o.y, 1), a.code(), a.flags(), cuda_stream());
+  if (rc != MB200_EUNSUPPORTED) {
+    check(rc, "mb200_sscan_fwd");
+    check_status("mb200_sscan_fwd");
+  }
+  return rc;
+}
+
+// Rows cut into S pieces that run as extra batch rows: carry pass, fold, full pass (the protocol of split.py).
+ScanOut split_forward(const ScanArgs& a, int64_t S, bool want_carries) {
+  const int64_t B = a.batch(), W = a.width(), N = a.states();
+  ScanArgs s = a;
+  s.x = cut(a.x, S); s.delta = cut(a.delta, S); s.z = cut(a.z, S); s.B = cut(a.B, S); s.C = cut(a.C, S);
+  // one row: its last piece's carry feeds nothing, so that piece is left out of the pass
+  const int64_t skip = B == 1 ? 1 : 0, rows_all = B * S, n = rows_all - skip;
+  Tensor PS = empty({2, B, S, W, N}, at::kFloat, a.x);
+  if (skip) PS.view({2, rows_all, W, N}).slice(1, n, rows_all).zero_();
+  float *P = fptr(PS), *St = P + rows_all * W * N;
+  check(mb200_sscan_fwd_carry(ptr(s.x), ptr(s.delta), fptr(s.A), ptr(s.B), fptr(s.bias), St, P, n, s.length(), W, int(N), st(s.x, 0),
+                              st(s.x, 1), st(s.delta, 0), st(s.delta, 1), st(s.B, 0), st(s.B, 1), s.code(), s.flags(), cuda_stream()),
+        "mb200_sscan_fwd_carry");
+  check_status("mb200_sscan_fwd_carry");
+  s.h0 = empty({rows_all, W, N}, at::kFloat, a.x);
+  check(mb200_carry_fold_range(P, St, fptr(a.h0), fptr(s.h0), B, S, W * N, 0, int(S), 0, cuda_stream()), "mb200_carry_fold_range");
+  ScanOut o;
+  launch_forward(s, o, true, want_carries);
+  o.y = join(o.y, S);
+  o.hT = o.hT.unflatten(0, {B, S}).select(1, S - 1);
+  o.P = PS.select(0, 0);
+  return o;
+}
+
+struct ScanGrads {
+  Tensor dx, dd, dz, dB, dC, dA, dD, dbias, g_out;
+};
+
+ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out) {
+  const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states();
+  ScanGrads g;
+  const auto dt = a.x.scalar_type();
+  g.dx = empty({B, L, W}, dt, a.x);
+  g.dd = empty({B, L, W}, dt, a.x);
+  if (a.z.defined()) g.dz = empty({B, L, W}, dt, a.x);
+  // every buffer the kernel accumulates into comes out of ONE zero-filled allocation
+  const int64_t nBC = B * L * N, nA = W * N;
+  const Tensor acc = empty({2 * nBC + nA + 2 * W}, at::kFloat, a.x);
+  C10_CUDA_CHECK(cudaMemsetAsync(acc.data_ptr(), 0, acc.nbytes(), at::cuda::getCurrentCUDAStream()));
+  g.dB = acc.narrow(0, 0, nBC).view({B, L, N});
+  g.dC = acc.narrow(0, nBC, nBC).view({B, L, N});
+  g.dA = acc.narrow(0, 2 * nBC, nA).view({W, N});
+  g.dD = acc.narrow(0, 2 * nBC + nA, W);
+  if (a.bias.defined()) g.dbias = acc.narrow(0, 2 * nBC + nA + W, W);
+  if (want_g_out) g.g_out = empty({B, W, N}, at::kFloat, a.x);
+  check(mb200_sscan_bwd(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), ptr(dy), fptr(carries),
+                        fptr(g_in), ptr(g.dx), ptr(g.dd), ptr(g.dz), fptr(g.dB), fptr(g.dC), fptr(g.dA), fptr(g.dD), fptr(g.dbias),
+                        fptr(g.g_out), B, L, W, int(N), st(a.x, 0), st(a.x, 1), st(a.delta, 0), st(a.delta, 1), st(a.z, 0), st(a.z, 1),
+                        st(a.B, 0), st(a.B, 1), st(a.C, 0), st(a.C, 1), st(dy, 0), st(dy, 1), st(g.dx, 0), st(g.dx, 1), st(g.dd, 0),
+                        st(g.dd, 1), st(g.dz, 0), st(g.dz, 1), a.code(), a.flags(), cuda_stream()),
+        "mb200_sscan_bwd");
+  check_status("mb200_sscan_bwd");
+  return g;
+}
+
+ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P) {
+  const int64_t B = a.batch(), W = a.width(), N = a.states();
+  ScanArgs s = a;
+  s.x = cut(a.x, S); s.delta = cut(a.delta, S); s.z = cut(a.z, S); s.B = cut(a.B, S); s.C = cut(a.C, S);
+  const Tensor dys = cut(dy, S);
+  const int64_t skip = B == 1 ? 1 : 0, rows_all = B * S;              // the first piece's carry feeds nothing
+  Tensor G = empty({rows_all, W, N}, at::kFloat, a.x);
+  if (skip) G.slice(0, 0, 1).zero_();
+  auto from = [&](const Tensor& t) { return (skip && t.defined()) ? t.slice(0, skip) : t; };
+  const Tensor d1 = from(s.delta), z1 = from(s.z), y1 = from(dys), c1 = from(s.C);
+  check(mb200_sscan_bwd_carry(ptr(d1), ptr(z1), ptr(y1), ptr(c1), fptr(s.A), fptr(s.bias), fptr(G) + skip * W * N, rows_all - skip,
+                              s.length(), W, int(N), st(d1, 0), st(d1, 1), st(z1, 0), st(z1, 1), st(y1, 0), st(y1, 1), st(c1, 0),
+                              st(c1, 1), s.code(), s.flags(), cuda_stream()),
+        "mb200_sscan_bwd_carry");
+  check_status("mb200_sscan_bwd_carry");
+  const Tensor g_in = empty({rows_all, W, N}, at::kFloat, a.x);
+  check(mb200_carry_fold_range(fptr(P), fptr(G), nullptr, fptr(g_in), B, S, W * N, 0, int(S), 1, cuda_stream()), "mb200_carry_fold_range");
+  ScanGrads g = launch_backward(s, dys, carries, g_in, true);
+  for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC}) *t = join(*t, S);
+  g.g_out = g.g_out.unflatten(0, {B, S}).select(1, 0);
+  return g;
+}
+
+enum { kX, kDelta, kA, kB, kC, kD, kZ, kBias, kH0, kInputs };
+
+struct ScanBackward : public torch::autograd::Node {
+  Saved x, delta, A, B, C, D, z, bias, carries, P;
+  at::ScalarType types[kInputs];
+  bool given[kInputs];
+  bool reverse = false, flipped = false;
+  int64_t subshards = 1;
+
+  std::string name() const override { return "SelectiveScanBackward"; }
+  void release_variables() override {
+    for (Saved* s : {&x, &delta, &A, &B, &C, &D, &z, &bias, &carries, &P}) s->reset();
+  }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(kInputs);
+    if (!grads[0].defined()) return out;
+    const BelowAutograd guard_ad;
+    ScanArgs a{x.get(), delta.get(), A.get(), B.get(), C.get(), D.get(), z.get(), bias.get(), Tensor(), reverse};
+    const c10::cuda::CUDAGuard guard(a.x.device());
+    Tensor dy = rows(flipped ? grads[0].flip(1) : grads[0], a.x.scalar_type());
+    // the in-kernel reverse backward exists on the tensor-map path only; an upstream gradient that is an offset or
+    // narrow view of something wider is copied to a dense tensor first
+    if (reverse && !tensor_map_ok(dy)) dy = dy.contiguous();
+    ScanGrads g = subshards > 1 ? split_backward(a, subshards, dy, carries.get(), P.get())
+                                : launch_backward(a, dy, carries.get(), Tensor(), given[kH0]);
+    if (flipped)
+      for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC})
+        if (t->defined()) *t = t->flip(1);
+    Tensor all[kInputs] = {g.dx, g.dd, g.dA, g.dB, g.dC, g.dD, g.dz, g.dbias, g.g_out};
+    for (int i = 0; i < kInputs; ++i)
+      if (given[i] && all[i].defined() && task_should_compute_output(i)) out[i] = like(all[i], types[i]);
+    return out;
+  }
+};
+
+}  // namespace
+
+// How many pieces to cut each row into.  The fused kernels have batch * ceil(width / 32) independent work items (a CTA owns
+// one) and 148 SMs hold three CTAs each.  Measured on B200, forward + backward of one row (ms): width 2048, length 65536:
+// 12.0 uncut, 7.8 / 5.8 / 5.8 / 4.8 in 2 / 4 / 8 / 16 pieces; 2048 x 8192: 1.53 uncut, 0.68 in 16; 5120 x 131072: 35.5
+// uncut, 27.0 / 23.9 / 23.7 in 4 / 8 / 16.  So: cut until there are about two waves of CTAs (the pieces' tails then
+// overlap), keep pieces at least 512 timesteps long, and leave alone what already fills half the GPU (a cut costs two extra
+// carry passes) or is so short that the extra launches eat the gain.
+int64_t pick_subshards(int64_t batch, int64_t length, int64_t width) {
+  const int64_t items = batch * ((width + 31) / 32);
+  if (length < 4096 || 2 * items >= kResidentCtas) return 1;
+  int64_t best = 1;
+  for (int64_t S : {2, 4, 8, 16}) {
+    if (length % (16 * S) || length / S < 512) break;
+    best = S;
+    if (items * S >= 2 * kResidentCtas) break;
+  }
+  return best;
+}
+
+py::object selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const OptTensor& D_,
+                          const OptTensor& z_, const OptTensor& bias_, const OptTensor& h0_, bool return_last_state, bool reverse,
+                          std::optional<int64_t> subshards) {
+  const Tensor &D = value(D_), &z = value(z_), &bias = value(bias_), &h0 = value(h0_);
+  Tensor y, hT;
+  {
+    py::gil_scoped_release no_gil;
+    require_cuda(x, delta, A, B, C, D, z, bias, h0);
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto dt = act_dtype(x, delta, z, B, C);
+    const bool grad = wants_grad(x, delta, A, B, C, D, z, bias, h0);
+    ScanOut o;
+    ScanArgs a;
+    bool flipped = false;
+    int64_t S;
+    {
+      const BelowAutograd guard_ad;
+      a = ScanArgs{rows(x, dt), rows(delta, dt), f32(A), rows(B, dt), rows(C, dt), f32(D), rows(z, dt), f32(bias), f32(h0), reverse};
+      const int64_t L = a.length();
+      // Few batch rows: cut every row into S consecutive pieces that run side by side.
+      S = subshards.value_or(0) ? *subshards : pick_subshards(a.batch(), L, a.width());
+      if (reverse || S < 1 || L % (16 * S) || L == 0) S = 1;
+      if (S > 1) {
+        o = split_forward(a, S, grad);
+      } else {
+        // the reverse backward exists for d_state 16 on the tensor-map path; otherwise do what the reference does
+        // (mambapy/vim.py:228-261): scan the flipped sequence, flip back
+        flipped = reverse && grad && a.states() != 16;
+        if (!flipped && launch_forward(a, o, return_last_state, grad) == MB200_EUNSUPPORTED) flipped = true;
+        if (flipped) {
+          for (Tensor* t : {&a.x, &a.delta, &a.z, &a.B, &a.C})
+            if (t->defined()) *t = t->flip(1);
+          a.reverse = false;
+          launch_forward(a, o, return_last_state, grad);
+          o.y = o.y.flip(1);
+        }
+      }
+    }
+    y = o.y;
+    hT = o.hT;
+    if (grad) {
+      auto node = new_node<ScanBackward>();
+      const Tensor* in[kInputs] = {&x, &delta, &A, &B, &C, &D, &z, &bias, &h0};
+      for (int i = 0; i < kInputs; ++i) {
+        node->given[i] = in[i]->defined();
+        node->types[i] = type_of(*in[i]);
+      }
+      node->set_next_edges(torch::autograd::collect_next_edges(x, delta, A, B, C, D, z, bias, h0));
+      node->x.save(a.x); node->delta.save(a.delta); node->A.save(a.A); node->B.save(a.B); node->C.save(a.C); node->D.save(a.D);
+      node->z.save(a.z); node->bias.save(a.bias); node->carries.save(o.carries); node->P.save(o.P);
+      node->reverse = a.reverse; node->flipped = flipped; node->subshards = S;
+      torch::autograd::set_history(y, node);
+    }
+  }
+  if (return_last_state) return py::make_tuple(y, hT);
+  return py::cast(y);
+}
+
+// ------------------------------------------------------------------------------------------------------ pscan
+namespace {
+
+// (B, L, D, N) tensor whose (D, N) block is dense; copies only if it is not.
+Tensor dense_dn(const Tensor& t) {
+  return (t.stride(3) == 1 && (t.size(2) == 1 || t.stride(2) == t.size(3))) ? t : t.contiguous();
+}
+Tensor pscan_workspace(int64_t B, int64_t nseg, int64_t DN, const Tensor& on) {
+  return nseg > 1 ? empty({2 * B * nseg * DN}, at::kFloat, on) : Tensor();
+}
+
+struct PScanBackward : public torch::autograd::Node {
+  Saved A, H;
+  std::string name() const override { return "PScanBackward"; }
+  void release_variables() override { A.reset(); H.reset(); }
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(2);
+    const BelowAutograd guard_ad;
+    const Tensor h0 = H.get(shared_from_this());
+    const c10::cuda::CUDAGuard guard(h0.device());
+    const Tensor a = dense_dn(A.get()), h = dense_dn(h0), g = dense_dn(like(grads[0], h0.scalar_type()));
+    const int64_t B = h.size(0), L = h.size(1), DN = h.size(2) * h.size(3);
+    const Tensor gA = empty(h.sizes(), h.scalar_type(), h), gX = empty(h.sizes(), h.scalar_type(), h);
+    const int nseg = L > 0 ? mb200_pscan_segments(B, L, DN) : 1;
+    const Tensor ws = pscan_workspace(B, nseg, DN, h);
+    check(mb200_pscan_bwd(ptr(a), ptr(h), ptr(g), ptr(gA), ptr(gX), B, L, DN, a.stride(0), a.stride(1), h.stride(0), h.stride(1),
+                          g.stride(0), g.stride(1), gA.stride(0), gA.stride(1), gX.stride(0), gX.stride(1), nullptr, fptr(ws), nseg,
+                          dtype_code(h.scalar_type()), cuda_stream()),
+          "mb200_pscan_bwd");
+    return {gA, gX};
+  }
+};
+
+}  // namespace
+
+Tensor pscan(const Tensor& A, const Tensor& X) {
+  require_cuda(A, X);
+  TORCH_CHECK_VALUE(A.dim() == 4 && A.sizes() == X.sizes(), "pscan expects two (B, L, D, N) tensors, got ", A.sizes(), " and ", X.sizes());
+  TORCH_CHECK_TYPE(A.scalar_type() == X.scalar_type(), "A_in and X_in must have the same dtype");
+  act_dtype(X);
+  const c10::cuda::CUDAGuard guard(X.device());
+  const int64_t B = X.size(0), L = X.size(1), DN = X.size(2) * X.size(3);
+  Tensor H;
+  {
+    const BelowAutograd guard_ad;
+    const Tensor a = dense_dn(A), x = dense_dn(X);
+    H = empty(X.sizes(), X.scalar_type(), X);
+    const int nseg = L > 0 ? mb200_pscan_segments(B, L, DN) : 1;
+    const Tensor ws = pscan_workspace(B, nseg, DN, X);
+    check(mb200_pscan_fwd(ptr(a), ptr(x), ptr(H), B, L, DN, a.stride(0), a.stride(1), x.stride(0), x.stride(1), H.stride(0), H.stride(1),
+                          nullptr, nullptr, fptr(ws), nseg, dtype_code(X.scalar_type()), cuda_stream()),
+          "mb200_pscan_fwd");
+  }
+  if (wants_grad(A, X)) {
+    auto node = new_node<PScanBackward>();
+    node->set_next_edges(torch::autograd::collect_next_edges(A, X));
+    node->A.save(A);
+    torch::autograd::set_history(H, node);
+    node->H.save(H, true);
+  }
+  return H;
+}
+
+}  // namespace mb200_host

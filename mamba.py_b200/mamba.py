@@ -19,86 +19,8 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from . import _lib
-
-
-from .kernels import (_require_cuda, _rows, _act_dtype, _tensor_map_ok, _f32, sscan_fwd_raw, sscan_bwd_raw,
-                      sscan_fwd_carry_raw, sscan_bwd_carry_raw, carry_fold_range, conv1d_silu_fwd_raw,
-                      conv1d_silu_bwd_raw)
-from .split import CudaOps, pick_subshards, split_forward, split_backward
-
-
-class SelectiveScanFn(torch.autograd.Function):
-    """y (and optionally the last state) of the fused scan; gradients for every input."""
-
-    @staticmethod
-    def forward(ctx, x, delta, A, Bm, Cm, D, z, delta_bias, h0, return_last_state, reverse=False, subshards=None):
-        _require_cuda(x, delta, A, Bm, Cm, D, z, delta_bias, h0)
-        dt = _act_dtype(x, delta, z, Bm, Cm)
-        xs, ds, zs = _rows(x, dt), _rows(delta, dt), _rows(z, dt)
-        Bs, Cs = _rows(Bm, dt), _rows(Cm, dt)
-        A32, D32, b32, h032 = _f32(A), _f32(D), _f32(delta_bias), _f32(h0)
-        needs_grad = any(t is not None and t.requires_grad
-                         for t in (x, delta, A, Bm, Cm, D, z, delta_bias, h0))
-        out = None
-        ctx.flipped = False
-        P_all = None
-        # Few batch rows: cut every row into S consecutive pieces that run side by side (split.py); the
-        # reference's own published shapes are all batch 1, i.e. 64 work items for a 148-SM GPU.
-        S = subshards if subshards else pick_subshards(xs.shape[0], xs.shape[1], xs.shape[2], 1)
-        if reverse or S < 1 or xs.shape[1] % (16 * S) or xs.shape[1] == 0:
-            S = 1
-        if S > 1:
-            y, _, P_all, carries, hT = split_forward(CudaOps, None, xs, ds, A32, Bs, Cs, D32, zs, b32, h0=h032,
-                                                     want_carries=needs_grad, subshards=S)
-            out = (y, hT if return_last_state else None, carries)
-        if out is None and reverse and not (needs_grad and A32.shape[1] != 16):    # the reverse backward exists for d_state 16
-            out = sscan_fwd_raw(xs, ds, A32, Bs, Cs, D32, zs, b32, h032, want_last=return_last_state,
-                                want_carries=needs_grad, reverse=True)
-        if reverse and out is None:
-            # what the reference does (mambapy/vim.py:228-261): scan the flipped sequence, flip back
-            xs, ds, zs, Bs, Cs = (None if t is None else t.flip(1) for t in (xs, ds, zs, Bs, Cs))
-            ctx.flipped = True
-        if out is None:
-            out = sscan_fwd_raw(xs, ds, A32, Bs, Cs, D32, zs, b32, h032,
-                                want_last=return_last_state, want_carries=needs_grad)
-        y, hT, carries = out
-        if ctx.flipped:
-            y = y.flip(1)
-        ctx.reverse = reverse and not ctx.flipped
-        ctx.subshards = S
-        ctx.save_for_backward(xs, ds, A32, Bs, Cs, D32, zs, b32, carries, P_all)
-        ctx.in_dtypes = tuple(None if t is None else t.dtype
-                              for t in (x, delta, A, Bm, Cm, D, z, delta_bias, h0))
-        ctx.has_h0 = h0 is not None
-        if return_last_state:
-            ctx.mark_non_differentiable(hT)
-            return y, hT
-        return y
-
-    @staticmethod
-    def backward(ctx, dy, *unused):
-        xs, ds, A32, Bs, Cs, D32, zs, b32, carries, P_all = ctx.saved_tensors
-        dy = _rows(dy.flip(1) if ctx.flipped else dy, xs.dtype)
-        if ctx.subshards > 1:
-            dx, dd, dz, dB, dC, dA, dD, dbias, g_out = split_backward(
-                CudaOps, None, xs, ds, A32, Bs, Cs, D32, zs, b32, dy, carries, P_all, subshards=ctx.subshards)
-            tx, td, tA, tB, tC, tD, tz, tb, th = ctx.in_dtypes
-            cast = lambda g, t: None if (g is None or t is None) else g.to(t)
-            return (cast(dx, tx), cast(dd, td), cast(dA, tA), cast(dB, tB), cast(dC, tC), cast(dD, tD),
-                    cast(dz, tz), cast(dbias, tb), cast(g_out if ctx.has_h0 else None, th), None, None, None)
-        if ctx.reverse and not _tensor_map_ok(dy):
-            # the in-kernel reverse backward exists on the tensor-map path only; an upstream gradient
-            # that is an offset or narrow view of something wider is copied to a dense tensor first
-            dy = dy.contiguous()
-        dx, dd, dz, dB, dC, dA, dD, dbias, g_out = sscan_bwd_raw(
-            xs, ds, A32, Bs, Cs, D32, zs, b32, dy, carries, want_g_out=ctx.has_h0, reverse=ctx.reverse)
-        if ctx.flipped:
-            dx, dd, dz, dB, dC = (None if t is None else t.flip(1) for t in (dx, dd, dz, dB, dC))
-        tx, td, tA, tB, tC, tD, tz, tb, th = ctx.in_dtypes
-        cast = lambda g, t: None if (g is None or t is None) else g.to(t)
-        return (cast(dx, tx), cast(dd, td), cast(dA, tA), cast(dB, tB), cast(dC, tC),
-                cast(dD, tD), cast(dz, tz), cast(dbias, tb), cast(g_out, th), None, None, None)
+from ._lib import host as _host
+from .kernels import (_rows, _f32, sscan_fwd_raw, sscan_bwd_raw, conv1d_silu_fwd_raw, conv1d_silu_bwd_raw)
 
 
 def selective_scan_fn(x, delta, A, B, C, D=None, z=None, delta_bias=None, h0=None,
@@ -121,7 +43,7 @@ def selective_scan_fn(x, delta, A, B, C, D=None, z=None, delta_bias=None, h0=Non
     side (two extra carry passes, see split.py): None picks the number from the shape, 1 never cuts, any
     other value is used if L is a multiple of 16 * subshards.
     """
-    return SelectiveScanFn.apply(x, delta, A, B, C, D, z, delta_bias, h0, return_last_state, reverse, subshards)
+    return _host().selective_scan(x, delta, A, B, C, D, z, delta_bias, h0, return_last_state, reverse, subshards)
 
 
 # ----------------------------------------------------------------- MambaBlock method drop-ins
@@ -142,30 +64,7 @@ def ssm_step_fn(x, h, delta, A, B, C, D=None, z=None, delta_bias=None, inplace=F
     Returns (y, h_new); h_new is a fresh float32 tensor (the reference also returns a new one,
     mambapy/mamba.py:408).  `inplace=True` (opt-in, for decode loops that own their cache)
     overwrites a float32 contiguous `h` instead and returns it."""
-    _require_cuda(x, delta, A, B, C, D, z, delta_bias, h)
-    lib = _lib.load()
-    dt = _act_dtype(x, delta, z, B, C)
-    xs, ds, zs, Bs, Cs = (_rows(t, dt) for t in (x, delta, z, B, C))
-    A32, D32, b32 = _f32(A), _f32(D), _f32(delta_bias)
-    h32 = None if h is None else h.float().contiguous()
-    Bsz, ED = xs.shape
-    N = A32.shape[1]
-    if inplace:
-        if h is None or h32.data_ptr() != h.data_ptr():
-            raise ValueError("inplace=True needs a float32 contiguous state tensor")
-        h_new = h
-    else:
-        h_new = torch.empty((Bsz, ED, N), dtype=torch.float32, device=xs.device)
-    y = torch.empty((Bsz, ED), dtype=dt, device=xs.device)
-    flags = _lib.DELTA_SOFTPLUS if b32 is not None else 0
-    with torch.cuda.device(xs.device):
-        rc = lib.mb200_ssm_step(
-            xs.data_ptr(), ds.data_ptr(), _lib.ptr(zs), A32.data_ptr(), Bs.data_ptr(), Cs.data_ptr(),
-            _lib.ptr(D32), _lib.ptr(b32), _lib.ptr(h32), h_new.data_ptr(), y.data_ptr(), Bsz, ED, N,
-            xs.stride(0), ds.stride(0), zs.stride(0) if zs is not None else 0, Bs.stride(0),
-            Cs.stride(0), y.stride(0), _lib.dtype_code(dt), flags, _lib.current_stream(xs.device))
-    _lib.check(rc, "mb200_ssm_step")
-    return y, h_new
+    return _host().ssm_step(x, h, delta, A, B, C, D, z, delta_bias, inplace)
 
 
 def conv_step_fn(x, inputs, weight, bias, inplace=False):
@@ -175,194 +74,19 @@ def conv_step_fn(x, inputs, weight, bias, inplace=False):
     weight: (ED, 1, d_conv) depthwise filter; bias: (ED) or None.
     Returns (silu(conv(x)), new window).  The window is a fresh tensor unless `inplace=True`
     (opt-in), which shifts a contiguous window of the activation dtype in place."""
-    _require_cuda(x, inputs, weight, bias)
-    lib = _lib.load()
-    dt = _act_dtype(x)
-    xs = _rows(x, dt)
-    win = inputs.to(dt).contiguous()
-    Bsz, ED = xs.shape
-    K = weight.shape[-1]
-    w32 = weight.detach().reshape(ED, K).float().contiguous()
-    b32 = _f32(bias)
-    xc = torch.empty((Bsz, ED), dtype=dt, device=xs.device)
-    if inplace:
-        if win.data_ptr() != inputs.data_ptr():
-            raise ValueError("inplace=True needs a contiguous window of the activation dtype")
-        new_win = inputs
-    else:
-        new_win = torch.empty_like(win)
-    with torch.cuda.device(xs.device):
-        rc = lib.mb200_conv_step(xs.data_ptr(), win.data_ptr(), w32.data_ptr(), _lib.ptr(b32),
-                                 xc.data_ptr(), new_win.data_ptr(), Bsz, ED, K, xs.stride(0),
-                                 _lib.dtype_code(dt), _lib.current_stream(xs.device))
-    _lib.check(rc, "mb200_conv_step")
-    return xc, new_win
-
-
-class CausalConv1dSiluFn(torch.autograd.Function):
-    """silu(depthwise causal conv1d(x)) on (B, L, ED) tensors, d_conv = 4."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias):
-        _require_cuda(x, weight, bias)
-        lib = _lib.load()
-        dt = _act_dtype(x)
-        xs = _rows(x, dt)
-        Bsz, L, ED = xs.shape
-        K = weight.shape[-1]
-        w32 = weight.detach().reshape(ED, K).float().contiguous()
-        b32 = _f32(bias)
-        y = torch.empty((Bsz, L, ED), dtype=dt, device=xs.device)
-        with torch.cuda.device(xs.device):
-            rc = lib.mb200_conv1d_silu_fwd(xs.data_ptr(), w32.data_ptr(), _lib.ptr(b32), y.data_ptr(), Bsz, L, ED, K,
-                                           xs.stride(0), xs.stride(1), y.stride(0), y.stride(1),
-                                           _lib.dtype_code(dt), _lib.current_stream(xs.device))
-        _lib.check(rc, "mb200_conv1d_silu_fwd")
-        ctx.save_for_backward(xs, w32, b32)
-        ctx.meta = (x.dtype, weight.dtype, weight.shape, None if bias is None else bias.dtype)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        xs, w32, b32 = ctx.saved_tensors
-        lib = _lib.load()
-        dy = _rows(dy, xs.dtype)
-        Bsz, L, ED = xs.shape
-        K = w32.shape[1]
-        dx = torch.empty_like(xs)
-        dw = torch.zeros_like(w32)
-        db = torch.zeros(ED, dtype=torch.float32, device=xs.device) if b32 is not None else None
-        with torch.cuda.device(xs.device):
-            rc = lib.mb200_conv1d_silu_bwd(xs.data_ptr(), w32.data_ptr(), _lib.ptr(b32), dy.data_ptr(), dx.data_ptr(),
-                                           dw.data_ptr(), _lib.ptr(db), Bsz, L, ED, K, xs.stride(0), xs.stride(1),
-                                           dy.stride(0), dy.stride(1), dx.stride(0), dx.stride(1),
-                                           _lib.dtype_code(xs.dtype), _lib.current_stream(xs.device))
-        _lib.check(rc, "mb200_conv1d_silu_bwd")
-        tx, tw, wshape, tb = ctx.meta
-        return dx.to(tx), dw.to(tw).reshape(wshape), None if db is None else db.to(tb)
+    return _host().conv_step(x, inputs, weight, bias, inplace)
 
 
 def causal_conv1d_silu(x, weight, bias=None):
     """silu(conv1d(x)) of MambaBlock.forward (mambapy/mamba.py:217-221) without the transposes.
 
     x: (B, L, ED); weight: (ED, 1, 4) as nn.Conv1d(groups=ED) holds it; bias: (ED) or None."""
-    return CausalConv1dSiluFn.apply(x, weight, bias)
-
-
-class RMSNormFn(torch.autograd.Function):
-    """y = x * rsqrt(mean(x^2, -1) + eps) * weight in one pass over x (mambapy/mamba.py:416-433)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, eps):
-        lib = _lib.load()
-        dt = _act_dtype(x)
-        D = x.shape[-1]
-        x2 = x.reshape(-1, D)
-        if x2.dtype != dt or x2.stride(-1) != 1:
-            x2 = x2.to(dt).contiguous()
-        rows = x2.shape[0]
-        w32 = None if weight is None else _f32(weight)
-        y = torch.empty((rows, D), dtype=dt, device=x.device)
-        rstd = torch.empty((rows,), dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
-            rc = lib.mb200_rmsnorm_fwd(x2.data_ptr(), _lib.ptr(w32), y.data_ptr(), rstd.data_ptr(), rows, D,
-                                       x2.stride(0), y.stride(0), float(eps), _lib.dtype_code(dt),
-                                       _lib.current_stream(x.device))
-        _lib.check(rc, "mb200_rmsnorm_fwd")
-        ctx.save_for_backward(x2, w32, rstd)
-        ctx.meta = (x.shape, x.dtype, None if weight is None else weight.dtype)
-        return y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w32, rstd = ctx.saved_tensors
-        shape, tx, tw = ctx.meta
-        lib = _lib.load()
-        rows, D = x2.shape
-        dy2 = dy.reshape(rows, D)
-        if dy2.dtype != x2.dtype or dy2.stride(-1) != 1:
-            dy2 = dy2.to(x2.dtype).contiguous()
-        dx = torch.empty_like(x2)
-        dw = torch.zeros(D, dtype=torch.float32, device=x2.device) if w32 is not None else None
-        with torch.cuda.device(x2.device):
-            rc = lib.mb200_rmsnorm_bwd(x2.data_ptr(), _lib.ptr(w32), rstd.data_ptr(), dy2.data_ptr(), dx.data_ptr(),
-                                       _lib.ptr(dw), rows, D, x2.stride(0), dy2.stride(0), dx.stride(0),
-                                       _lib.dtype_code(x2.dtype), _lib.current_stream(x2.device))
-        _lib.check(rc, "mb200_rmsnorm_bwd")
-        return dx.view(shape).to(tx), None if dw is None else dw.to(tw), None
+    return _host().conv1d_silu(x, weight, bias)
 
 
 def rms_norm(x, weight=None, eps=1e-5):
     """RMSNorm over the last dimension; weight None is the reference's muP variant (no gain)."""
-    if not x.is_cuda:
-        raise RuntimeError("mamba_b200 kernels need CUDA tensors; there is no CPU path")
-    return RMSNormFn.apply(x, weight, eps)
-
-
-class AddRMSNormFn(torch.autograd.Function):
-    """(y, s) with s = x + residual and y = RMSNorm(s), one pass (mb200_add_rmsnorm_fwd)."""
-
-    @staticmethod
-    def forward(ctx, x, residual, weight, eps, y_dtype):
-        lib = _lib.load()
-        D = x.shape[-1]
-        x2 = x.reshape(-1, D)
-        if x2.stride(-1) != 1:
-            x2 = x2.contiguous()
-        r2 = None
-        res_dtype = x.dtype
-        if residual is not None:
-            r2 = residual.reshape(-1, D)
-            if r2.stride(-1) != 1:
-                r2 = r2.contiguous()
-            res_dtype = torch.promote_types(x.dtype, residual.dtype)       # what `x + residual` would give
-            if r2.dtype != res_dtype:
-                r2 = r2.to(res_dtype)
-        rows = x2.shape[0]
-        w32 = None if weight is None else _f32(weight)
-        s = torch.empty((rows, D), dtype=res_dtype, device=x.device)
-        y = torch.empty((rows, D), dtype=y_dtype, device=x.device)
-        rstd = torch.empty((rows,), dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
-            rc = lib.mb200_add_rmsnorm_fwd(x2.data_ptr(), _lib.ptr(r2), _lib.ptr(w32), s.data_ptr(), y.data_ptr(),
-                                           rstd.data_ptr(), rows, D, x2.stride(0), 0 if r2 is None else r2.stride(0),
-                                           s.stride(0), y.stride(0), float(eps), _lib.dtype_code(x2.dtype),
-                                           _lib.dtype_code(res_dtype), _lib.dtype_code(y_dtype),
-                                           _lib.current_stream(x.device))
-        _lib.check(rc, "mb200_add_rmsnorm_fwd")
-        ctx.save_for_backward(s, w32, rstd)
-        ctx.meta = (x.shape, x.dtype, None if residual is None else residual.dtype,
-                    None if weight is None else weight.dtype)
-        return y.view(x.shape), s.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy, ds_out):
-        s, w32, rstd = ctx.saved_tensors
-        shape, tx, tr, tw = ctx.meta
-        lib = _lib.load()
-        rows, D = s.shape
-        y_dtype = dy.dtype if dy.dtype in (torch.float32, torch.bfloat16) else torch.float32
-        dy2 = dy.reshape(rows, D)
-        if dy2.dtype != y_dtype or dy2.stride(-1) != 1:
-            dy2 = dy2.to(y_dtype).contiguous()
-        if s.dtype == torch.bfloat16 and y_dtype != torch.bfloat16:
-            dy2, y_dtype = dy2.to(torch.bfloat16), torch.bfloat16
-        dr2 = None
-        if ds_out is not None:
-            dr2 = ds_out.reshape(rows, D)
-            if dr2.dtype != s.dtype or dr2.stride(-1) != 1:
-                dr2 = dr2.to(s.dtype).contiguous()
-        ds = torch.empty_like(s)
-        dw = torch.zeros(D, dtype=torch.float32, device=s.device) if w32 is not None else None
-        with torch.cuda.device(s.device):
-            rc = lib.mb200_add_rmsnorm_bwd(s.data_ptr(), _lib.ptr(w32), rstd.data_ptr(), dy2.data_ptr(), _lib.ptr(dr2),
-                                           ds.data_ptr(), _lib.ptr(dw), rows, D, s.stride(0), dy2.stride(0),
-                                           0 if dr2 is None else dr2.stride(0), ds.stride(0),
-                                           _lib.dtype_code(s.dtype), _lib.dtype_code(y_dtype),
-                                           _lib.current_stream(s.device))
-        _lib.check(rc, "mb200_add_rmsnorm_bwd")
-        ds = ds.view(shape)
-        return ds.to(tx), None if tr is None else ds.to(tr), None if dw is None else dw.to(tw), None, None
+    return _host().rms_norm(x, weight, eps)
 
 
 def add_rms_norm(x, residual=None, weight=None, eps=1e-5):
@@ -370,14 +94,7 @@ def add_rms_norm(x, residual=None, weight=None, eps=1e-5):
     the residual add of one layer fused with the normalisation in front of the next
     (mambapy/mamba.py:106-112).  Under autocast y comes out in the autocast dtype, which is what the
     projection that consumes it would cast it to anyway."""
-    if not x.is_cuda:
-        raise RuntimeError("mamba_b200 kernels need CUDA tensors; there is no CPU path")
-    y_dtype = x.dtype if residual is None else torch.promote_types(x.dtype, residual.dtype)
-    if torch.is_autocast_enabled():
-        y_dtype = torch.get_autocast_gpu_dtype()
-    if y_dtype not in (torch.float32, torch.bfloat16):
-        y_dtype = torch.float32
-    return AddRMSNormFn.apply(x, residual, weight, eps, y_dtype)
+    return _host().add_rms_norm(x, residual, weight, eps)
 
 
 def stack_forward(self, x):

@@ -90,7 +90,10 @@ def pscan_bwd_raw(A, H, G, h0=None):
 
 
 class PScan(torch.autograd.Function):
-    """Same call contract as mambapy/pscan.py:35-224 (`PScan.apply(A_in, X_in)`)."""
+    """Same call contract as mambapy/pscan.py:35-224 (`PScan.apply(A_in, X_in)`).
+
+    `apply` is the native implementation (its autograd node is C++, csrc/host/scan.cpp); forward and backward
+    are the two halves as plain functions of tensors."""
 
     @staticmethod
     def forward(ctx, A_in, X_in):
@@ -109,8 +112,11 @@ class PScan(torch.autograd.Function):
     def backward(ctx, grad_output_in):
         """Returns gradA, gradX, both (B, L, D, N) (mambapy/pscan.py:188-224)."""
         A_in, H = ctx.saved_tensors
-        gA, gX = pscan_bwd_raw(A_in, H, grad_output_in)
-        return gA, gX
+        return pscan_bwd_raw(A_in, H, grad_output_in)
+
+    @staticmethod
+    def apply(A_in, X_in):
+        return _lib.host().pscan(A_in, X_in)
 
 
 pscan = PScan.apply
