@@ -309,6 +309,19 @@ int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const float* rstd,
                           int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, int dtype_res,
                           int dtype_y, void* stream);
 
+/* Element-wise jobs, up to 12 in one launch.  Job: dst[r, c] = op(src[r, c]) for r < rows, c < cols, both with unit
+ * stride along c and their own row strides; columns src_cols .. cols-1 (all of them if src is NULL) count as zero.
+ * MB200_CONVERT_NEG_EXP: dst = -exp(src).  MB200_CONVERT_MUL: dst = src * factor, factor dense float32 (rows, cols). */
+enum { MB200_CONVERT_COPY = 0, MB200_CONVERT_NEG_EXP = 1, MB200_CONVERT_MUL = 2 };
+typedef struct {
+  const void* src;
+  void* dst;
+  const float* factor;
+  int64_t rows, cols, src_cols, src_stride, dst_stride;
+  int src_dtype, dst_dtype, op;
+} mb200_convert_job;
+int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

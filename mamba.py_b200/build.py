@@ -73,7 +73,8 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
             cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-c", s, "-o", o]
             jobs.append(cmd)
 
-    host_headers = [os.path.join(HOST_SRC, "host.h"), os.path.join(INCLUDE, "mamba_b200.h")]
+    host_headers = [os.path.join(HOST_SRC, f) for f in os.listdir(HOST_SRC) if f.endswith(".h")]
+    host_headers.append(os.path.join(INCLUDE, "mamba_b200.h"))
     host_flags = None
     for src in sorted(f for f in os.listdir(HOST_SRC) if f.endswith(".cpp")):
         s, o = os.path.join(HOST_SRC, src), os.path.join(OBJDIR, "host_" + src[:-4] + ".o")

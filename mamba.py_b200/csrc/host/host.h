@@ -113,6 +113,10 @@ std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const T
                                     const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& delta_bias, bool inplace);
 std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace);
 
+Tensor inner(const Tensor& xz, const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w, const Tensor& dt_b,
+             const Tensor& A_log, const Tensor& D, int64_t dt_rank, int64_t d_state, bool reverse);
+bool inner_reversible(const Tensor& xz, int64_t d_state);
+
 int64_t pick_subshards(int64_t batch, int64_t length, int64_t width);
 
 }  // namespace mb200_host

@@ -18,5 +18,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_rms_norm", &add_rms_norm, NoGil());
   m.def("ssm_step", &ssm_step, NoGil());
   m.def("conv_step", &conv_step, NoGil());
+  m.def("inner", &inner, NoGil());
+  m.def("inner_reversible", &inner_reversible);
   m.def("pick_subshards", &pick_subshards);
 }

@@ -1,5 +1,5 @@
 // selective_scan_fn and pscan: forward launches and their autograd nodes.
-#include "host.h"
+#include "scan.h"
 #include <cstdlib>
 
 namespace mb200_host {
@@ -17,28 +17,6 @@ void check_status(const char* what) {
 namespace {
 
 constexpr int64_t kResidentCtas = 444;          // 148 SMs x 3 CTAs of the fused kernels
-
-// The tensors of a scan as the kernels take them.
-struct ScanArgs {
-  Tensor x, delta, A, B, C, D, z, bias, h0;
-  bool reverse = false;
-  int flags() const { return (bias.defined() ? MB200_DELTA_SOFTPLUS : 0) | (reverse ? MB200_REVERSE : 0); }
-  int code() const { return dtype_code(x.scalar_type()); }
-  int64_t batch() const { return x.size(0); }
-  int64_t length() const { return x.size(1); }
-  int64_t width() const { return x.size(2); }
-  int64_t states() const { return A.size(1); }
-};
-
-struct ScanOut {
-  Tensor y, hT, carries, P;
-};
-
-// 16-byte aligned base and byte strides: what a tiled tensor map of a (B, L, C) tensor needs.
-bool tensor_map_ok(const Tensor& t) {
-  const int64_t es = t.element_size();
-  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 && t.stride(1) * es % 16 == 0;
-}
 
 // (B, L, C) -> (B*S, L/S, C): every batch row cut into S consecutive pieces (a view when the strides allow it).
 Tensor cut(const Tensor& t, int64_t S) {
@@ -90,26 +68,24 @@ ScanOut split_forward(const ScanArgs& a, int64_t S, bool want_carries) {
   return o;
 }
 
-struct ScanGrads {
-  Tensor dx, dd, dz, dB, dC, dA, dD, dbias, g_out;
-};
-
-ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out) {
+ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out, const Tensor& dz,
+                          int64_t extra) {
   const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states();
   ScanGrads g;
   const auto dt = a.x.scalar_type();
   g.dx = empty({B, L, W}, dt, a.x);
   g.dd = empty({B, L, W}, dt, a.x);
-  if (a.z.defined()) g.dz = empty({B, L, W}, dt, a.x);
+  if (a.z.defined()) g.dz = dz.defined() ? dz : empty({B, L, W}, dt, a.x);
   // every buffer the kernel accumulates into comes out of ONE zero-filled allocation
   const int64_t nBC = B * L * N, nA = W * N;
-  const Tensor acc = empty({2 * nBC + nA + 2 * W}, at::kFloat, a.x);
+  const Tensor acc = empty({2 * nBC + nA + 2 * W + extra}, at::kFloat, a.x);
   C10_CUDA_CHECK(cudaMemsetAsync(acc.data_ptr(), 0, acc.nbytes(), at::cuda::getCurrentCUDAStream()));
   g.dB = acc.narrow(0, 0, nBC).view({B, L, N});
   g.dC = acc.narrow(0, nBC, nBC).view({B, L, N});
   g.dA = acc.narrow(0, 2 * nBC, nA).view({W, N});
   g.dD = acc.narrow(0, 2 * nBC + nA, W);
   if (a.bias.defined()) g.dbias = acc.narrow(0, 2 * nBC + nA + W, W);
+  if (extra) g.extra = acc.narrow(0, 2 * nBC + nA + 2 * W, extra);
   if (want_g_out) g.g_out = empty({B, W, N}, at::kFloat, a.x);
   check(mb200_sscan_bwd(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), ptr(dy), fptr(carries),
                         fptr(g_in), ptr(g.dx), ptr(g.dd), ptr(g.dz), fptr(g.dB), fptr(g.dC), fptr(g.dA), fptr(g.dD), fptr(g.dbias),
@@ -121,7 +97,8 @@ ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& car
   return g;
 }
 
-ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P) {
+ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, const Tensor& dz,
+                         int64_t extra) {
   const int64_t B = a.batch(), W = a.width(), N = a.states();
   ScanArgs s = a;
   s.x = cut(a.x, S); s.delta = cut(a.delta, S); s.z = cut(a.z, S); s.B = cut(a.B, S); s.C = cut(a.C, S);
@@ -138,10 +115,54 @@ ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const T
   check_status("mb200_sscan_bwd_carry");
   const Tensor g_in = empty({rows_all, W, N}, at::kFloat, a.x);
   check(mb200_carry_fold_range(fptr(P), fptr(G), nullptr, fptr(g_in), B, S, W * N, 0, int(S), 1, cuda_stream()), "mb200_carry_fold_range");
-  ScanGrads g = launch_backward(s, dys, carries, g_in, true);
+  ScanGrads g = launch_backward(s, dys, carries, g_in, true, cut(dz, S), extra);
   for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC}) *t = join(*t, S);
   g.g_out = g.g_out.unflatten(0, {B, S}).select(1, 0);
   return g;
+}
+
+}  // namespace
+
+bool tensor_map_ok(const Tensor& t) {
+  const int64_t es = t.element_size();
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 && t.stride(1) * es % 16 == 0;
+}
+bool tensor_maps_ok(const ScanArgs& a) {
+  for (const Tensor* t : {&a.x, &a.delta, &a.z})
+    if (t->defined() && !tensor_map_ok(*t)) return false;
+  return a.width() * a.x.element_size() % 16 == 0;
+}
+
+bool scan_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carries, ScanOut& o) {
+  if (S > 1) {
+    o = split_forward(a, S, want_carries);
+    return true;
+  }
+  return launch_forward(a, o, want_last, want_carries) == MB200_OK;
+}
+ScanGrads scan_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
+                        const Tensor& dz, int64_t extra) {
+  return S > 1 ? split_backward(a, S, dy, carries, P, dz, extra) : launch_backward(a, dy, carries, Tensor(), want_g_out, dz, extra);
+}
+
+namespace {
+
+// B and C are slices of the x_proj output, whose width dt_rank + 2 N often leaves them off the 16-byte grid a tensor map
+// needs.  They are 2 N values a token: copying them onto the grid costs a few microseconds and keeps the fused kernels'
+// tensor-map path, which is two to three times faster than the path for arbitrary alignment.
+void align_bc(ScanArgs& a) {
+  if (a.length() == 0 || a.batch() == 0 || !tensor_maps_ok(a) || (tensor_map_ok(a.B) && tensor_map_ok(a.C))) return;
+  const int64_t N = a.B.size(2), es = a.B.element_size();
+  const bool side_by_side = a.B.strides() == a.C.strides() &&
+                            static_cast<char*>(a.C.data_ptr()) - static_cast<char*>(a.B.data_ptr()) == N * es && a.B.stride(1) >= 2 * N;
+  if (side_by_side) {                                                   // one copy for both
+    const Tensor bc = a.B.as_strided({a.B.size(0), a.B.size(1), 2 * N}, a.B.strides()).contiguous();
+    a.B = bc.narrow(2, 0, N);
+    a.C = bc.narrow(2, N, N);
+  } else {
+    a.B = a.B.clone(at::MemoryFormat::Contiguous);
+    a.C = a.C.clone(at::MemoryFormat::Contiguous);
+  }
 }
 
 enum { kX, kDelta, kA, kB, kC, kD, kZ, kBias, kH0, kInputs };
@@ -167,8 +188,7 @@ struct ScanBackward : public torch::autograd::Node {
     // the in-kernel reverse backward exists on the tensor-map path only; an upstream gradient that is an offset or
     // narrow view of something wider is copied to a dense tensor first
     if (reverse && !tensor_map_ok(dy)) dy = dy.contiguous();
-    ScanGrads g = subshards > 1 ? split_backward(a, subshards, dy, carries.get(), P.get())
-                                : launch_backward(a, dy, carries.get(), Tensor(), given[kH0]);
+    ScanGrads g = scan_backward(a, subshards, dy, carries.get(), P.get(), given[kH0]);
     if (flipped)
       for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC})
         if (t->defined()) *t = t->flip(1);
@@ -221,20 +241,17 @@ py::object selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A,
       // Few batch rows: cut every row into S consecutive pieces that run side by side.
       S = subshards.value_or(0) ? *subshards : pick_subshards(a.batch(), L, a.width());
       if (reverse || S < 1 || L % (16 * S) || L == 0) S = 1;
-      if (S > 1) {
-        o = split_forward(a, S, grad);
-      } else {
-        // the reverse backward exists for d_state 16 on the tensor-map path; otherwise do what the reference does
-        // (mambapy/vim.py:228-261): scan the flipped sequence, flip back
-        flipped = reverse && grad && a.states() != 16;
-        if (!flipped && launch_forward(a, o, return_last_state, grad) == MB200_EUNSUPPORTED) flipped = true;
-        if (flipped) {
-          for (Tensor* t : {&a.x, &a.delta, &a.z, &a.B, &a.C})
-            if (t->defined()) *t = t->flip(1);
-          a.reverse = false;
-          launch_forward(a, o, return_last_state, grad);
-          o.y = o.y.flip(1);
-        }
+      align_bc(a);
+      // the reverse backward exists for d_state 16 on the tensor-map path; otherwise do what the reference does
+      // (mambapy/vim.py:228-261): scan the flipped sequence, flip back
+      flipped = reverse && grad && a.states() != 16;
+      if (!flipped && !scan_forward(a, S, return_last_state, grad, o)) flipped = true;
+      if (flipped) {
+        for (Tensor* t : {&a.x, &a.delta, &a.z, &a.B, &a.C})
+          if (t->defined()) *t = t->flip(1);
+        a.reverse = false;
+        scan_forward(a, 1, return_last_state, grad, o);
+        o.y = o.y.flip(1);
       }
     }
     y = o.y;

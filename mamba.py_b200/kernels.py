@@ -192,33 +192,3 @@ def carry_fold_range(P_all, S_all, init, first, num, reverse):
                                         first, num, int(reverse), _lib.current_stream(P_all.device))
     _lib.check(rc, "mb200_carry_fold_range")
     return out
-
-
-def conv1d_silu_fwd_raw(xs, w32, b32):
-    """silu(depthwise causal conv1d(x)), d_conv 4, on (B, L, ED) with any batch / row strides."""
-    lib = _lib.load()
-    Bsz, L, ED = xs.shape
-    y = torch.empty((Bsz, L, ED), dtype=xs.dtype, device=xs.device)
-    with torch.cuda.device(xs.device):
-        rc = lib.mb200_conv1d_silu_fwd(xs.data_ptr(), w32.data_ptr(), _lib.ptr(b32), y.data_ptr(), Bsz, L, ED,
-                                       w32.shape[1], xs.stride(0), xs.stride(1), y.stride(0), y.stride(1),
-                                       _lib.dtype_code(xs.dtype), _lib.current_stream(xs.device))
-    _lib.check(rc, "mb200_conv1d_silu_fwd")
-    return y
-
-
-def conv1d_silu_bwd_raw(xs, w32, b32, dy, out_dx=None):
-    """Backward of conv1d_silu_fwd_raw.  Returns (dx, dw (ED, K) float32, db (ED) float32 or None); dx may be a
-    caller's (strided) view."""
-    lib = _lib.load()
-    Bsz, L, ED = xs.shape
-    dx = out_dx if out_dx is not None else torch.empty_like(xs)
-    dw = torch.zeros_like(w32)
-    db = torch.zeros(ED, dtype=torch.float32, device=xs.device) if b32 is not None else None
-    with torch.cuda.device(xs.device):
-        rc = lib.mb200_conv1d_silu_bwd(xs.data_ptr(), w32.data_ptr(), _lib.ptr(b32), dy.data_ptr(), dx.data_ptr(),
-                                       dw.data_ptr(), _lib.ptr(db), Bsz, L, ED, w32.shape[1], xs.stride(0), xs.stride(1),
-                                       dy.stride(0), dy.stride(1), dx.stride(0), dx.stride(1),
-                                       _lib.dtype_code(xs.dtype), _lib.current_stream(xs.device))
-    _lib.check(rc, "mb200_conv1d_silu_bwd")
-    return dx, dw, db

@@ -20,7 +20,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import host as _host
-from .kernels import (_rows, _f32, sscan_fwd_raw, sscan_bwd_raw, conv1d_silu_fwd_raw, conv1d_silu_bwd_raw)
+from .kernels import sscan_fwd_raw, sscan_bwd_raw  # noqa: F401  (re-exported)
 
 
 def selective_scan_fn(x, delta, A, B, C, D=None, z=None, delta_bias=None, h0=None,
@@ -146,62 +146,6 @@ def step(self, x, cache):
     return self.out_proj(y), (h, inputs)
 
 
-class FusedInnerFn(torch.autograd.Function):
-    """Everything between in_proj and out_proj of MambaBlock.forward (mambapy/mamba.py:214-231) as ONE autograd
-    node: conv1d + SiLU, x_proj, dt_proj, and the fused scan with softplus(delta + bias) and the gate inside.
-
-    Written as separate nodes, autograd glues the backward together with copies: a `cat` of the gradients of
-    the two halves of xz (the whole (B, L, 2*ED) tensor again), a `cat` for the split of the x_proj output, an
-    add of the two gradients that reach the conv output, and casts of dB, dC.  Here the backward writes dz and
-    the conv's dx straight into the two halves of d(xz), dB and dC straight into d(x_proj output), and adds
-    the second gradient of the conv output in the epilogue of the GEMM that produces it."""
-
-    @staticmethod
-    def forward(ctx, xz, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D, dt_rank, d_state):
-        dt = xz.dtype
-        ED = xz.shape[-1] // 2
-        R, N = dt_rank, d_state
-        xs, z = xz[..., :ED], xz[..., ED:]
-        cw32 = conv_w.detach().reshape(ED, conv_w.shape[-1]).float().contiguous()
-        cb32 = _f32(conv_b)
-        xc = conv1d_silu_fwd_raw(xs, cw32, cb32)
-        Wx, Wdt = xproj_w.detach().to(dt), dt_w.detach().to(dt)
-        dbc = F.linear(xc, Wx)                                   # (B, L, R + 2N)
-        delta_r = F.linear(dbc[..., :R], Wdt)                    # (B, L, ED); bias and softplus happen in the kernel
-        A = -torch.exp(A_log.detach().float())
-        D32, b32 = _f32(D), _f32(dt_b)
-        needs_grad = any(ctx.needs_input_grad)
-        y, _, carries = sscan_fwd_raw(xc, delta_r, A, dbc[..., R:R + N], dbc[..., R + N:], D32, z, b32,
-                                      want_carries=needs_grad)
-        ctx.save_for_backward(xz, xc, dbc, delta_r, A, D32, b32, carries, cw32, cb32, Wx, Wdt)
-        ctx.meta = (R, N, conv_w.shape, conv_w.dtype, None if conv_b is None else conv_b.dtype, xproj_w.dtype,
-                    dt_w.dtype, dt_b.dtype, A_log.dtype, D.dtype)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        xz, xc, dbc, delta_r, A, D32, b32, carries, cw32, cb32, Wx, Wdt = ctx.saved_tensors
-        R, N, cw_shape, t_cw, t_cb, t_wx, t_wdt, t_bdt, t_A, t_D = ctx.meta
-        ED = xc.shape[-1]
-        dy = _rows(dy, xc.dtype)
-        dxz = torch.empty_like(xz, memory_format=torch.contiguous_format)
-        dx_s, dd, _, dB, dC, dA, dD, dbias, _ = sscan_bwd_raw(
-            xc, delta_r, A, dbc[..., R:R + N], dbc[..., R + N:], D32, xz[..., ED:], b32, dy, carries,
-            out_dz=dxz[..., ED:])
-        d_dbc = torch.empty_like(dbc)
-        dd2 = dd.flatten(0, 1)
-        d_dbc[..., :R] = F.linear(dd, Wdt.t())                   # through dt_proj
-        d_dbc[..., R:R + N].copy_(dB)                            # float32 accumulators -> activation dtype, in place
-        d_dbc[..., R + N:].copy_(dC)
-        d2 = d_dbc.flatten(0, 1)
-        dWdt = dd2.t() @ dbc[..., :R].flatten(0, 1)              # (ED, R)
-        dWx = d2.t() @ xc.flatten(0, 1)                          # (R + 2N, ED)
-        dx_s.flatten(0, 1).addmm_(d2, Wx)                        # + gradient through x_proj, in the GEMM's epilogue
-        _, dcw, dcb = conv1d_silu_bwd_raw(xz[..., :ED], cw32, cb32, dx_s, out_dx=dxz[..., :ED])
-        return (dxz, dcw.reshape(cw_shape).to(t_cw), None if dcb is None else dcb.to(t_cb), dWx.to(t_wx), dWdt.to(t_wdt),
-                dbias.to(t_bdt), (dA * A).to(t_A), dD.to(t_D), None, None)
-
-
 def _fusable(self, xz):
     cfg = self.config
     return (xz.is_cuda and xz.dtype in (torch.float32, torch.bfloat16) and self.conv1d.weight.shape[-1] == 4
@@ -226,8 +170,8 @@ def forward(self, x):
     xz = self.in_proj(x)
     if _fusable(self, xz):
         cfg = self.config
-        y = FusedInnerFn.apply(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight,
-                               self.dt_proj.bias, self.A_log, self.D, cfg.dt_rank, cfg.d_state)
+        y = _host().inner(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight,
+                          self.dt_proj.bias, self.A_log, self.D, cfg.dt_rank, cfg.d_state, False)
         return self.out_proj(y)
     xs, z = xz.chunk(2, dim=-1)
     if self.conv1d.weight.shape[-1] == 4:

@@ -2,15 +2,17 @@
 
 The reference runs its second direction as flip(xz) -> conv -> projections -> scan -> flip(y).  Here
 the second scan walks the ORIGINAL sequence from its last timestep to its first inside the kernels
-(`selective_scan_fn(..., reverse=True)`), gated by the un-flipped z, so only the convolution input is
-flipped (the convolution kernel is causal); delta, B, C, z and y are never flipped or copied.
+(`selective_scan_fn(..., reverse=True)`), gated by the un-flipped z, and the convolution kernel takes the rows
+backwards through a negative stride; nothing is flipped or copied.  Blocks the fused interior cannot take (other
+d_state, activations off the 16-byte grid) flip the convolution input as the reference does.
 """
 from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
 
-from .mamba import causal_conv1d_silu, selective_scan_fn
+from ._lib import host as _host
+from .mamba import _fusable, causal_conv1d_silu, selective_scan_fn
 
 
 def _conv_silu(conv, xs, L):
@@ -32,14 +34,24 @@ def _ssm(self, x, z, A_log, D, x_proj, dt_proj, reverse):
 def forward(self, x):
     """mambapy/vim.py:205-261; x: (B, L, D) -> (B, L, D)."""
     _, L, _ = x.shape
+    cfg = self.config
     xz = self.in_proj(x)
     xs, z = xz.chunk(2, dim=-1)
-    y = _ssm(self, _conv_silu(self.conv1d, xs, L), z, self.A_log, self.D, self.x_proj, self.dt_proj, False)
-    if not self.config.bidirectional:
+    fused = _fusable(self, xz)
+    if fused:
+        y = _host().inner(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight, self.dt_proj.bias,
+                          self.A_log, self.D, cfg.dt_rank, cfg.d_state, False)
+    else:
+        y = _ssm(self, _conv_silu(self.conv1d, xs, L), z, self.A_log, self.D, self.x_proj, self.dt_proj, False)
+    if not cfg.bidirectional:
         return self.out_proj(y)
     # second direction: the reference convolves the flipped sequence; in original time order that is
     # flip(conv(flip(x))).  Everything after it is per-timestep, and the scan runs right to left.
-    xb = _conv_silu(self.conv1d_b, xs.flip(1), L).flip(1)
-    yb = _ssm(self, xb, z, self.A_log_b, self.D_b, self.x_proj_b, self.dt_proj_b, True)
+    if fused and _host().inner_reversible(xz, cfg.d_state):
+        yb = _host().inner(xz, self.conv1d_b.weight, self.conv1d_b.bias, self.x_proj_b.weight, self.dt_proj_b.weight, self.dt_proj_b.bias,
+                           self.A_log_b, self.D_b, cfg.dt_rank, cfg.d_state, True)
+    else:
+        xb = _conv_silu(self.conv1d_b, xs.flip(1), L).flip(1)
+        yb = _ssm(self, xb, z, self.A_log_b, self.D_b, self.x_proj_b, self.dt_proj_b, True)
     s = y + yb
-    return self.out_proj(s / 2 if self.config.divide_output else s)
+    return self.out_proj(s / 2 if cfg.divide_output else s)
