@@ -180,24 +180,6 @@ int mb200_sscan_bwd(const void* x, const void* delta, const void* z,
                     int64_t dz_sb, int64_t dz_sl,
                     int dtype, int flags, void* stream);
 
-/* The same with every row cut into `pieces` spans of piece_len timesteps (a multiple of 8; the last may be shorter) that are
- * walked side by side, for problems with few rows: a carry pass over all spans but one comes first.  ws: 2*B*pieces*ED*N floats,
- * 16-byte aligned.  pieces = 1 (ws NULL) is mb200_sscan_bwd; tensors that need the generic kernel are walked in one span. */
-int mb200_sscan_bwd_split(const void* x, const void* delta, const void* z,
-                          const float* A, const void* Bm, const void* Cm, const float* D,
-                          const float* delta_bias, const void* dy, const float* carries,
-                          const float* g_in,
-                          void* dx, void* ddelta, void* dz,
-                          float* dB, float* dC, float* dA, float* dD, float* ddelta_bias,
-                          float* g_out,
-                          int64_t B, int64_t L, int64_t ED, int N,
-                          int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
-                          int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
-                          int64_t c_sb, int64_t c_sl, int64_t dy_sb, int64_t dy_sl,
-                          int64_t dx_sb, int64_t dx_sl, int64_t dd_sb, int64_t dd_sl,
-                          int64_t dz_sb, int64_t dz_sl,
-                          int dtype, int flags, int64_t pieces, int64_t piece_len, float* ws, void* stream);
-
 /* ---- Reverse carry pass of the sequence-sharded backward (no reference counterpart; the
  * reference is single-device).  For one shard of the sequence it returns, in g_out (B, ED, N)
  * float32, the gradient carry a[0]*g[0] that leaves the shard's first timestep when NO carry

@@ -103,19 +103,7 @@ struct SscanBwdParams {
   int64_t x_sb, x_sl, d_sb, d_sl, z_sb, z_sl, b_sb, b_sl, c_sb, c_sl, dy_sb, dy_sl;
   int64_t dx_sb, dx_sl, dd_sb, dd_sl, dz_sb, dz_sl;
   int flags;
-  // A sequence cut into `pieces` spans of piece_len timesteps (a multiple of 8; the last may be shorter) that are walked side
-  // by side: piece_P, piece_G (B, pieces, ED, N) hold every piece's decay product and the carry that leaves it when none
-  // enters it.  A launch covers launch_pieces of them from piece0.
-  int64_t pieces = 1, piece_len = int64_t(1) << 40, piece0 = 0, launch_pieces = 1;
-  float *piece_P = nullptr, *piece_G = nullptr;
 };
-
-// Backward for d_state 16 on tensors that a tensor map can describe (sscan_bwd16.cuh): 0 = launched, 1 = these tensors need the
-// generic kernel, negative = error.  carry_only: fill piece_P and piece_G.
-int bwd16_launch_f32(const SscanBwdParams& p, bool carry_only, cudaStream_t st);
-int bwd16_launch_bf16(const SscanBwdParams& p, bool carry_only, cudaStream_t st);
-int bwd16_status_f32();
-int bwd16_status_bf16();
 
 }  // namespace mb200
 

@@ -87,10 +87,8 @@ def sscan_fwd_raw(x, delta, A, Bm, Cm, D, z=None, delta_bias=None, h0=None,
 
 
 def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None, want_g_out=False,
-                  reverse=False, general_decay=False, out_dz=None, pieces=1):
+                  reverse=False, general_decay=False, out_dz=None):
     """Launch the fused backward.  Returns (dx, ddelta, dz, dB, dC, dA, dD, dbias, g_out).
-
-    `pieces` cuts every row into that many spans that are walked side by side (one extra carry pass).
 
     `reverse` must be what the forward that produced `carries` ran with."""
     lib = _lib.load()
@@ -114,10 +112,8 @@ def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None,
              | (_lib.GENERAL_DECAY if general_decay else 0))
     zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
     dzs = (dz.stride(0), dz.stride(1)) if dz is not None else (0, 0)
-    piece_len = -(-L // (8 * pieces)) * 8
-    ws = torch.empty(2 * Bsz * pieces * ED * N, dtype=torch.float32, device=dev) if pieces > 1 else None
     with torch.cuda.device(dev):
-        rc = lib.mb200_sscan_bwd_split(
+        rc = lib.mb200_sscan_bwd(
             x.data_ptr(), delta.data_ptr(), _lib.ptr(z), A.data_ptr(), Bm.data_ptr(), Cm.data_ptr(),
             _lib.ptr(D), _lib.ptr(delta_bias), dy.data_ptr(), carries.data_ptr(), _lib.ptr(g_in),
             dx.data_ptr(), dd.data_ptr(), _lib.ptr(dz), dB.data_ptr(), dC.data_ptr(), dA.data_ptr(),
@@ -125,7 +121,7 @@ def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None,
             x.stride(0), x.stride(1), delta.stride(0), delta.stride(1), zs[0], zs[1],
             Bm.stride(0), Bm.stride(1), Cm.stride(0), Cm.stride(1), dy.stride(0), dy.stride(1),
             dx.stride(0), dx.stride(1), dd.stride(0), dd.stride(1), dzs[0], dzs[1],
-            _lib.dtype_code(x.dtype), flags, pieces, piece_len, _lib.ptr(ws), _lib.current_stream(dev))
+            _lib.dtype_code(x.dtype), flags, _lib.current_stream(dev))
     _lib.check(rc, "mb200_sscan_bwd")
     _lib.check_status(dev, "mb200_sscan_bwd")
     return dx, dd, dz, dB, dC, dA, dD, dbias, g_out
