@@ -322,6 +322,36 @@ typedef struct {
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
+/* mb200_ssm_step and mb200_conv_step with the small parameters in the model's own types (float32 or bfloat16 each); with A_is_log
+ * A holds A_log and the decay rate is -exp(A_log). */
+int mb200_ssm_step_params(const void* x, const void* delta, const void* z, const void* A, int A_dtype, int A_is_log,
+                          const void* Bm, const void* Cm, const void* D, int D_dtype, const void* delta_bias, int bias_dtype,
+                          const float* h_in, float* h_out, void* y, int64_t B, int64_t ED, int N,
+                          int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb, int64_t c_sb, int64_t y_sb,
+                          int dtype, int flags, void* stream);
+int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype, const void* bias, int bias_dtype,
+                           void* xc, void* conv_out, int64_t B, int64_t ED, int K, int64_t x_sb, int dtype, void* stream);
+
+/* One decode step of a whole block for up to 8 tokens in one cooperative launch: in_proj, conv window and SiLU, x_proj,
+ * dt_proj, state update with softplus(delta + dt_b), gate, out_proj (mambapy/mamba.py:351-414).  x (B, D_model) with row stride
+ * x_sb, out (B, D_model), conv_in / conv_out (B, W, d_conv-1), h_in (NULL: zeros) / h_out (B, W, N) float32; the weights in_w
+ * (2W, D_model), xproj_w (R+2N, W), dt_w (W, R), out_w (D_model, W) and in_b, out_b (or NULL) have type `dtype`, the small
+ * parameters conv_w (W, d_conv), conv_b (W, or NULL), dt_b (W), A_log (W, N), D (W) a type each.  conv_out may be conv_in, h_out
+ * may be h_in.  scratch: mb200_block_step_scratch_floats floats; barriers: mb200_block_step_barrier_bytes bytes that are zero
+ * before the first launch, left zero by every launch for the next, and used by one launch at a time.
+ * MB200_EUNSUPPORTED: weight rows off the 16-byte grid.  MB200_ETOOBIG: more than 8 tokens, or activations beyond 200 KB. */
+typedef struct {
+  const void *x, *in_w, *in_b, *conv_in, *conv_w, *conv_b, *xproj_w, *dt_w, *dt_b, *A_log, *D, *out_w, *out_b;
+  const float* h_in;
+  void *conv_out, *out;
+  float* h_out;
+  int64_t B, D_model, W, R, x_sb;
+  int N, d_conv, dtype, conv_w_dtype, conv_b_dtype, dt_b_dtype, A_log_dtype, D_dtype;
+} mb200_block_step_args;
+int64_t mb200_block_step_scratch_floats(int64_t B, int64_t W, int64_t R, int N);
+int mb200_block_step_barrier_bytes(void);
+int mb200_block_step(const mb200_block_step_args* args, float* scratch, void* barriers, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

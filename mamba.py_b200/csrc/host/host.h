@@ -117,6 +117,11 @@ Tensor inner(const Tensor& xz, const Tensor& conv_w, const OptTensor& conv_b, co
              const Tensor& A_log, const Tensor& D, int64_t dt_rank, int64_t d_state, bool reverse);
 bool inner_reversible(const Tensor& xz, int64_t d_state);
 
+std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& h, const Tensor& inputs, const Tensor& in_w, const OptTensor& in_b,
+                                              const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w,
+                                              const Tensor& dt_b, const Tensor& A_log, const Tensor& D, const Tensor& out_w,
+                                              const OptTensor& out_b, int64_t dt_rank, int64_t d_state);
+
 int64_t pick_subshards(int64_t batch, int64_t length, int64_t width);
 
 }  // namespace mb200_host

@@ -211,52 +211,4 @@ std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residu
   return {y, s};
 }
 
-// ------------------------------------------------------------------------------------------------ decode step
-std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h_, const Tensor& delta, const Tensor& A, const Tensor& B,
-                                    const Tensor& C, const OptTensor& D_, const OptTensor& z_, const OptTensor& bias_, bool inplace) {
-  const Tensor &h = value(h_), &D = value(D_), &z = value(z_), &bias = value(bias_);
-  require_cuda(x, delta, A, B, C, D, z, bias, h);
-  const c10::cuda::CUDAGuard guard(x.device());
-  const BelowAutograd guard_ad;
-  const auto dt = act_dtype(x, delta, z, B, C);
-  const Tensor xs = rows(x, dt), ds = rows(delta, dt), zs = rows(z, dt), Bs = rows(B, dt), Cs = rows(C, dt);
-  const Tensor A32 = f32(A), D32 = f32(D), b32 = f32(bias), h32 = f32(h);
-  const int64_t n = xs.size(0), W = xs.size(1), N = A32.size(1);
-  Tensor h_new;
-  if (inplace) {
-    TORCH_CHECK_VALUE(h.defined() && h32.data_ptr() == h.data_ptr(), "inplace=True needs a float32 contiguous state tensor");
-    h_new = h;
-  } else {
-    h_new = empty({n, W, N}, at::kFloat, xs);
-  }
-  const Tensor y = empty({n, W}, dt, xs);
-  check(mb200_ssm_step(ptr(xs), ptr(ds), ptr(zs), fptr(A32), ptr(Bs), ptr(Cs), fptr(D32), fptr(b32), fptr(h32), fptr(h_new), ptr(y), n, W,
-                       int(N), st(xs, 0), st(ds, 0), st(zs, 0), st(Bs, 0), st(Cs, 0), st(y, 0), dtype_code(dt),
-                       b32.defined() ? MB200_DELTA_SOFTPLUS : 0, cuda_stream()),
-        "mb200_ssm_step");
-  return {y, h_new};
-}
-
-std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias_, bool inplace) {
-  const Tensor& bias = value(bias_);
-  require_cuda(x, inputs, weight, bias);
-  const c10::cuda::CUDAGuard guard(x.device());
-  const BelowAutograd guard_ad;
-  const auto dt = act_dtype(x);
-  const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), w32 = filter(weight), b32 = f32(bias);
-  const int64_t n = xs.size(0), W = xs.size(1);
-  const Tensor xc = empty({n, W}, dt, xs);
-  Tensor fresh;
-  if (inplace) {
-    TORCH_CHECK_VALUE(win.data_ptr() == inputs.data_ptr(), "inplace=True needs a contiguous window of the activation dtype");
-    fresh = inputs;
-  } else {
-    fresh = empty(win.sizes(), dt, xs);
-  }
-  check(mb200_conv_step(ptr(xs), ptr(win), fptr(w32), fptr(b32), ptr(xc), ptr(fresh), n, W, int(w32.size(1)), st(xs, 0), dtype_code(dt),
-                        cuda_stream()),
-        "mb200_conv_step");
-  return {xc, fresh};
-}
-
 }  // namespace mb200_host

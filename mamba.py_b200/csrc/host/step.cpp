@@ -1,0 +1,162 @@
+// Decode steps: the state update, the conv window, and the whole block.
+#include <mutex>
+#include <unordered_map>
+#include "host.h"
+
+namespace mb200_host {
+namespace {
+
+bool small_type(const Tensor& t) { return t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16; }
+
+// A small parameter as the kernels read it: contiguous, float32 or bfloat16 as the model has it.
+Tensor small_param(const Tensor& t) {
+  if (!t.defined()) return t;
+  const Tensor r = small_type(t) ? t : t.to(at::kFloat);
+  return r.is_contiguous() ? r : r.contiguous();
+}
+int code_of(const Tensor& t) { return t.defined() ? dtype_code(t.scalar_type()) : MB200_F32; }
+
+struct StateStep {
+  Tensor y, h;
+};
+
+StateStep state_step(const Tensor& x, const Tensor& h, const Tensor& delta, const Tensor& A_, bool log_A, const Tensor& B, const Tensor& C,
+                     const Tensor& D_, const Tensor& z, const Tensor& bias_, bool inplace) {
+  const auto dt = act_dtype(x, delta, z, B, C);
+  const Tensor xs = rows(x, dt), ds = rows(delta, dt), zs = rows(z, dt), Bs = rows(B, dt), Cs = rows(C, dt);
+  const Tensor A = small_param(A_), D = small_param(D_), bias = small_param(bias_), h32 = f32(h);
+  const int64_t n = xs.size(0), W = xs.size(1), N = A.size(1);
+  StateStep o;
+  if (inplace) {
+    TORCH_CHECK_VALUE(h.defined() && h32.data_ptr() == h.data_ptr(), "inplace=True needs a float32 contiguous state tensor");
+    o.h = h;
+  } else {
+    o.h = empty({n, W, N}, at::kFloat, xs);
+  }
+  o.y = empty({n, W}, dt, xs);
+  check(mb200_ssm_step_params(ptr(xs), ptr(ds), ptr(zs), ptr(A), code_of(A), log_A, ptr(Bs), ptr(Cs), ptr(D), code_of(D), ptr(bias),
+                              code_of(bias), fptr(h32), fptr(o.h), ptr(o.y), n, W, int(N), st(xs, 0), st(ds, 0), st(zs, 0), st(Bs, 0),
+                              st(Cs, 0), st(o.y, 0), dtype_code(dt), bias.defined() ? MB200_DELTA_SOFTPLUS : 0, cuda_stream()),
+        "mb200_ssm_step");
+  return o;
+}
+
+struct WindowStep {
+  Tensor xc, window;
+};
+
+WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const Tensor& bias_, bool inplace) {
+  const auto dt = act_dtype(x);
+  const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), w = small_param(weight), bias = small_param(bias_);
+  const int64_t n = xs.size(0), W = xs.size(1);
+  WindowStep o;
+  o.xc = empty({n, W}, dt, xs);
+  if (inplace) {
+    TORCH_CHECK_VALUE(win.data_ptr() == inputs.data_ptr(), "inplace=True needs a contiguous window of the activation dtype");
+    o.window = inputs;
+  } else {
+    o.window = empty(win.sizes(), dt, xs);
+  }
+  check(mb200_conv_step_params(ptr(xs), ptr(win), ptr(w), code_of(w), ptr(bias), code_of(bias), ptr(o.xc), ptr(o.window), n, W,
+                               int(w.size(-1)), st(xs, 0), dtype_code(dt), cuda_stream()),
+        "mb200_conv_step");
+  return o;
+}
+
+// ---- barrier counters of the one-launch step -----------------------------------------------------------------------
+// A launch leaves its counters zero for the next one on the same stream, so a stream keeps its own.  At most kMaxStreams are
+// kept; a stream beyond them, and a stream that is being captured into a graph (whose replays may run anywhere), gets
+// counters of its own for the one call, cleared on the stream.
+constexpr size_t kMaxStreams = 64;
+
+Tensor barrier_counters(const Tensor& on) {
+  static std::mutex mutex;
+  static std::unordered_map<uint64_t, Tensor> kept;
+  const auto s = at::cuda::getCurrentCUDAStream();
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(s, &capturing));
+  const uint64_t key = (uint64_t(s.device_index()) << 56) ^ uint64_t(s.id());
+  std::lock_guard<std::mutex> lock(mutex);
+  const bool keep = capturing == cudaStreamCaptureStatusNone;
+  if (keep) {
+    const auto it = kept.find(key);
+    if (it != kept.end()) return it->second;
+  }
+  const Tensor t = at::empty({mb200_block_step_barrier_bytes()}, on.options().dtype(at::kByte));
+  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), s));
+  if (keep && kept.size() < kMaxStreams) kept.emplace(key, t);
+  return t;
+}
+
+}  // namespace
+
+std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const Tensor& delta, const Tensor& A, const Tensor& B,
+                                    const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& bias, bool inplace) {
+  require_cuda(x, delta, A, B, C, value(D), value(z), value(bias), value(h));
+  const c10::cuda::CUDAGuard guard(x.device());
+  const BelowAutograd guard_ad;
+  const StateStep o = state_step(x, value(h), delta, A, false, B, C, value(D), value(z), value(bias), inplace);
+  return {o.y, o.h};
+}
+
+std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace) {
+  require_cuda(x, inputs, weight, value(bias));
+  const c10::cuda::CUDAGuard guard(x.device());
+  const BelowAutograd guard_ad;
+  const WindowStep o = window_step(x, inputs, weight, value(bias), inplace);
+  return {o.xc, o.window};
+}
+
+// One decode step of a block (mambapy/mamba.py:351-414) -> (output (B, D), state, window), with fresh cache tensors.
+// Up to 8 tokens go through one cooperative launch (block_step.cu) when every weight has the activations' type and nothing wants
+// a gradient; otherwise the projections are library GEMMs with the two step kernels between them.  Beyond 8 tokens the
+// projections are real matrix products and the library's kernels are the better ones.
+std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& h_, const Tensor& inputs, const Tensor& in_w,
+                                              const OptTensor& in_b_, const Tensor& conv_w, const OptTensor& conv_b_, const Tensor& xproj_w,
+                                              const Tensor& dt_w, const Tensor& dt_b, const Tensor& A_log, const Tensor& D,
+                                              const Tensor& out_w, const OptTensor& out_b_, int64_t R, int64_t N) {
+  const Tensor &h = value(h_), &in_b = value(in_b_), &conv_b = value(conv_b_), &out_b = value(out_b_);
+  require_cuda(x, h, inputs, in_w, in_b, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D, out_w, out_b);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto dt = x.scalar_type();
+  const int64_t B = x.size(0), Dm = x.size(1), W = dt_w.size(0);
+  bool one = B >= 1 && B <= 8 && (dt == at::kFloat || dt == at::kBFloat16) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+             !wants_grad(x, in_w, in_b, out_w, out_b);
+  for (const Tensor* t : {&in_w, &in_b, &xproj_w, &dt_w, &out_w, &out_b})
+    one = one && (!t->defined() || (t->scalar_type() == dt && t->is_contiguous()));
+  if (one) {
+    const BelowAutograd guard_ad;
+    const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), h32 = f32(h);
+    const Tensor cw = small_param(conv_w), cb = small_param(conv_b), db = small_param(dt_b), al = small_param(A_log), d = small_param(D);
+    const Tensor out = empty({B, Dm}, dt, xs), h_new = empty({B, W, N}, at::kFloat, xs), fresh = empty(win.sizes(), dt, xs);
+    mb200_block_step_args a{};
+    a.x = ptr(xs); a.in_w = ptr(in_w); a.in_b = ptr(in_b); a.conv_in = ptr(win); a.conv_w = ptr(cw); a.conv_b = ptr(cb);
+    a.xproj_w = ptr(xproj_w); a.dt_w = ptr(dt_w); a.dt_b = ptr(db); a.A_log = ptr(al); a.D = ptr(d); a.out_w = ptr(out_w); a.out_b = ptr(out_b);
+    a.h_in = fptr(h32); a.conv_out = ptr(fresh); a.out = ptr(out); a.h_out = fptr(h_new);
+    a.B = B; a.D_model = Dm; a.W = W; a.R = R; a.x_sb = st(xs, 0);
+    a.N = int(N); a.d_conv = int(cw.size(-1)); a.dtype = dtype_code(dt);
+    a.conv_w_dtype = code_of(cw); a.conv_b_dtype = code_of(cb); a.dt_b_dtype = code_of(db); a.A_log_dtype = code_of(al); a.D_dtype = code_of(d);
+    const Tensor scratch = empty({mb200_block_step_scratch_floats(B, W, R, int(N))}, at::kFloat, xs), bars = barrier_counters(xs);
+    const int rc = mb200_block_step(&a, fptr(scratch), ptr(bars), cuda_stream());
+    if (rc != MB200_EUNSUPPORTED && rc != MB200_ETOOBIG) {
+      check(rc, "mb200_block_step");
+      return {out, h_new, fresh};
+    }
+  }
+  const Tensor xz = at::linear(x, in_w, in_b_);
+  WindowStep w;
+  {
+    const BelowAutograd guard_ad;
+    w = window_step(xz.narrow(1, 0, W), inputs, conv_w, conv_b, false);
+  }
+  const Tensor dbc = at::linear(w.xc, xproj_w);
+  const Tensor delta = at::linear(dbc.narrow(1, 0, R), dt_w);                // bias and softplus happen in the kernel
+  StateStep s;
+  {
+    const BelowAutograd guard_ad;
+    s = state_step(w.xc, h, delta, A_log, true, dbc.narrow(1, R, N), dbc.narrow(1, R + N, N), D, xz.narrow(1, W, W), dt_b, false);
+  }
+  return {at::linear(s.y, out_w, out_b_), s.h, w.window};
+}
+
+}  // namespace mb200_host

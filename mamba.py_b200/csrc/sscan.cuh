@@ -115,3 +115,4 @@ int mb200_fwd_tma_try(const mb200::SscanFwdParams& p, int N, int dtype, cudaStre
 // and clears its kernel's word, synchronising the device).
 int mb200_fwd_device_status();
 int mb200_bwd_device_status();
+int mb200_block_step_device_status();

@@ -5,6 +5,7 @@
 // Mapping for the state update: N/4 lanes share a channel, each lane moves one float4 of the
 // state (so a warp reads 512 contiguous bytes of h), computes its four decays and partial
 // C-contraction, and the lanes of a channel combine with warp shuffles.
+#include <initializer_list>
 #include "common.cuh"
 #include "sscan.cuh"
 
@@ -20,14 +21,26 @@ constexpr int kStepThreads = 256;
 #define MB200_STEP_SPL 8
 #endif
 
-template <typename T, int N, bool kVecBC>
+// A small parameter of the model in whatever type the model has.
+struct Param {
+  const void* p;
+  int dtype;
+  __device__ __forceinline__ float at(int64_t i) const {
+    return dtype == MB200_F32 ? __ldg(static_cast<const float*>(p) + i)
+                              : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p) + i));
+  }
+};
+
+// kLogA: A holds A_log and the decay rate is -exp(A_log).  A CTA takes `rows` consecutive batch rows of its channels, so
+// that the parameters (and those exponentials) are fetched once for all of them.
+template <typename T, int N, bool kVecBC, bool kLogA>
 __global__ void __launch_bounds__(kStepThreads)
 ssm_step_kernel(const T* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ z,
-                const float* __restrict__ A, const T* __restrict__ Bm, const T* __restrict__ Cm,
-                const float* __restrict__ D, const float* __restrict__ delta_bias,
+                const Param A, const T* __restrict__ Bm, const T* __restrict__ Cm,
+                const Param D, const Param delta_bias,
                 const float* __restrict__ h_in, float* __restrict__ h_out, T* __restrict__ y,
-                int64_t ED, int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb,
-                int64_t c_sb, int64_t y_sb, int flags) {
+                int64_t B, int64_t ED, int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb,
+                int64_t c_sb, int64_t y_sb, int flags, int rows) {
   constexpr int kSPL = MB200_STEP_SPL < N ? MB200_STEP_SPL : N;   // states per lane
   constexpr int kV = kSPL / 4;                                    // float4 per lane
   constexpr int kLPE = N / kSPL;                                  // lanes per channel
@@ -35,70 +48,86 @@ ssm_step_kernel(const T* __restrict__ x, const T* __restrict__ delta, const T* _
   const int tid = threadIdx.x;
   const int q = tid % kLPE;
   const int64_t e = int64_t(blockIdx.x) * kEPB + tid / kLPE;
-  const int64_t b = blockIdx.y;
   const bool ok = e < ED;
-  float yv = 0.f, xv = 0.f;
+  float Av[kSPL], bias = 0.f, Dv = 0.f;
   if (ok) {
-    // the state is the only large stream: get it moving first, everything else is small
-    float4 hv[kV];
-    const float4* hp = reinterpret_cast<const float4*>(h_in + (b * ED + e) * N + kSPL * q);
+    if (A.dtype == MB200_F32) {
 #pragma unroll
-    for (int v = 0; v < kV; ++v) hv[v] = h_in ? __ldcs(hp + v) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 Av[kV];
-#pragma unroll
-    for (int v = 0; v < kV; ++v) Av[v] = *reinterpret_cast<const float4*>(A + e * N + kSPL * q + 4 * v);
-    float b4[kSPL], c4[kSPL];
-    if constexpr (kVecBC) {
-#pragma unroll
-      for (int v = 0; v < kV; ++v) {
-        const Vec4<T> bv = *reinterpret_cast<const Vec4<T>*>(Bm + b * b_sb + kSPL * q + 4 * v);
-        const Vec4<T> cv = *reinterpret_cast<const Vec4<T>*>(Cm + b * c_sb + kSPL * q + 4 * v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { b4[4 * v + j] = Elem<T>::to_f(bv.v[j]); c4[4 * v + j] = Elem<T>::to_f(cv.v[j]); }
-      }
+      for (int v = 0; v < kV; ++v)
+        *reinterpret_cast<float4*>(Av + 4 * v) = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(A.p) + e * N + kSPL * q + 4 * v));
     } else {
 #pragma unroll
-      for (int j = 0; j < kSPL; ++j) {
-        b4[j] = Elem<T>::to_f(Bm[b * b_sb + kSPL * q + j]);
-        c4[j] = Elem<T>::to_f(Cm[b * c_sb + kSPL * q + j]);
-      }
+      for (int j = 0; j < kSPL; ++j) Av[j] = A.at(e * N + kSPL * q + j);
     }
-    xv = Elem<T>::to_f(x[b * x_sb + e]);
-    float dv = Elem<T>::to_f(delta[b * d_sb + e]);
-    if (flags & MB200_DELTA_SOFTPLUS) dv = softplus_fast(dv + delta_bias[e]);
-    const float dxs = dv * xv, d2s = dv * kLog2e;
-    const float2 dx = make_float2(dxs, dxs), d2 = make_float2(d2s, d2s);
-    float2 y2 = make_float2(0.f, 0.f);
-    float4* op = reinterpret_cast<float4*>(h_out + (b * ED + e) * N + kSPL * q);
+    if constexpr (kLogA) {
 #pragma unroll
-    for (int v = 0; v < kV; ++v) {
-      // packed f32x2 arithmetic: two states per instruction (the decays stay scalar ex2)
-      const float2 e01 = __fmul2_rn(d2, make_float2(Av[v].x, Av[v].y)), e23 = __fmul2_rn(d2, make_float2(Av[v].z, Av[v].w));
-      const float2 a01 = make_float2(ex2f(e01.x), ex2f(e01.y)), a23 = make_float2(ex2f(e23.x), ex2f(e23.y));
-      const float2 h01 = __ffma2_rn(a01, make_float2(hv[v].x, hv[v].y), __fmul2_rn(dx, make_float2(b4[4 * v], b4[4 * v + 1])));
-      const float2 h23 = __ffma2_rn(a23, make_float2(hv[v].z, hv[v].w), __fmul2_rn(dx, make_float2(b4[4 * v + 2], b4[4 * v + 3])));
-      y2 = __ffma2_rn(h01, make_float2(c4[4 * v], c4[4 * v + 1]), y2);
-      y2 = __ffma2_rn(h23, make_float2(c4[4 * v + 2], c4[4 * v + 3]), y2);
-      __stcs(op + v, make_float4(h01.x, h01.y, h23.x, h23.y));
+      for (int j = 0; j < kSPL; ++j) Av[j] = -expf(Av[j]);
     }
-    yv = y2.x + y2.y;
+    if (flags & MB200_DELTA_SOFTPLUS) bias = delta_bias.at(e);
+    if (D.p && q == 0) Dv = D.at(e);
   }
+  const int64_t b1 = min64(B, (int64_t(blockIdx.y) + 1) * rows);
+  for (int64_t b = int64_t(blockIdx.y) * rows; b < b1; ++b) {
+    float yv = 0.f, xv = 0.f;
+    if (ok) {
+      // the state is the only large stream: get it moving first, everything else is small
+      float4 hv[kV];
+      const float4* hp = reinterpret_cast<const float4*>(h_in + (b * ED + e) * N + kSPL * q);
 #pragma unroll
-  for (int s = kLPE / 2; s >= 1; s >>= 1) yv += __shfl_xor_sync(0xffffffffu, yv, s);
-  if (ok && q == 0) {
-    yv = fmaf(D ? D[e] : 0.f, xv, yv);
-    if (z) {
-      const float zv = Elem<T>::to_f(z[b * z_sb + e]);
-      yv *= zv * sigmoid_fast(zv);
+      for (int v = 0; v < kV; ++v) hv[v] = h_in ? __ldcs(hp + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float b4[kSPL], c4[kSPL];
+      if constexpr (kVecBC) {
+#pragma unroll
+        for (int v = 0; v < kV; ++v) {
+          const Vec4<T> bv = *reinterpret_cast<const Vec4<T>*>(Bm + b * b_sb + kSPL * q + 4 * v);
+          const Vec4<T> cv = *reinterpret_cast<const Vec4<T>*>(Cm + b * c_sb + kSPL * q + 4 * v);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) { b4[4 * v + j] = Elem<T>::to_f(bv.v[j]); c4[4 * v + j] = Elem<T>::to_f(cv.v[j]); }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kSPL; ++j) {
+          b4[j] = Elem<T>::to_f(Bm[b * b_sb + kSPL * q + j]);
+          c4[j] = Elem<T>::to_f(Cm[b * c_sb + kSPL * q + j]);
+        }
+      }
+      xv = Elem<T>::to_f(x[b * x_sb + e]);
+      float dv = Elem<T>::to_f(delta[b * d_sb + e]);
+      if (flags & MB200_DELTA_SOFTPLUS) dv = softplus_fast(dv + bias);
+      const float dxs = dv * xv, d2s = dv * kLog2e;
+      const float2 dx = make_float2(dxs, dxs), d2 = make_float2(d2s, d2s);
+      float2 y2 = make_float2(0.f, 0.f);
+      float4* op = reinterpret_cast<float4*>(h_out + (b * ED + e) * N + kSPL * q);
+#pragma unroll
+      for (int v = 0; v < kV; ++v) {
+        // packed f32x2 arithmetic: two states per instruction (the decays stay scalar ex2)
+        const float2 e01 = __fmul2_rn(d2, make_float2(Av[4 * v], Av[4 * v + 1])), e23 = __fmul2_rn(d2, make_float2(Av[4 * v + 2], Av[4 * v + 3]));
+        const float2 a01 = make_float2(ex2f(e01.x), ex2f(e01.y)), a23 = make_float2(ex2f(e23.x), ex2f(e23.y));
+        const float2 h01 = __ffma2_rn(a01, make_float2(hv[v].x, hv[v].y), __fmul2_rn(dx, make_float2(b4[4 * v], b4[4 * v + 1])));
+        const float2 h23 = __ffma2_rn(a23, make_float2(hv[v].z, hv[v].w), __fmul2_rn(dx, make_float2(b4[4 * v + 2], b4[4 * v + 3])));
+        y2 = __ffma2_rn(h01, make_float2(c4[4 * v], c4[4 * v + 1]), y2);
+        y2 = __ffma2_rn(h23, make_float2(c4[4 * v + 2], c4[4 * v + 3]), y2);
+        __stcs(op + v, make_float4(h01.x, h01.y, h23.x, h23.y));
+      }
+      yv = y2.x + y2.y;
     }
-    y[b * y_sb + e] = Elem<T>::from_f(yv);
+#pragma unroll
+    for (int s = kLPE / 2; s >= 1; s >>= 1) yv += __shfl_xor_sync(0xffffffffu, yv, s);
+    if (ok && q == 0) {
+      yv = fmaf(Dv, xv, yv);
+      if (z) {
+        const float zv = Elem<T>::to_f(z[b * z_sb + e]);
+        yv *= zv * sigmoid_fast(zv);
+      }
+      y[b * y_sb + e] = Elem<T>::from_f(yv);
+    }
   }
 }
 
 // xc = silu(sum_k w[e,k]*win[k] + bias[e]) with win = [conv_in[b,e,:], xin[b,e]]; conv_out = win[1:].
 template <typename T>
 __global__ void conv_step_kernel(const T* __restrict__ xin, const T* __restrict__ conv_in,
-                                 const float* __restrict__ w, const float* __restrict__ bias,
+                                 const Param w, const Param bias,
                                  T* __restrict__ xc, T* __restrict__ conv_out,
                                  int64_t ED, int K, int64_t x_sb) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -107,11 +136,11 @@ __global__ void conv_step_kernel(const T* __restrict__ xin, const T* __restrict_
   const T* ci = conv_in + (b * ED + e) * (K - 1);
   T* co = conv_out + (b * ED + e) * (K - 1);
   const float xn = Elem<T>::to_f(xin[b * x_sb + e]);
-  float acc = bias ? bias[e] : 0.f;
+  float acc = bias.p ? bias.at(e) : 0.f;
   float win[8];
   for (int k = 0; k < K - 1; ++k) win[k] = Elem<T>::to_f(ci[k]);
   win[K - 1] = xn;
-  for (int k = 0; k < K; ++k) acc = fmaf(w[e * K + k], win[k], acc);
+  for (int k = 0; k < K; ++k) acc = fmaf(w.at(e * K + k), win[k], acc);
   for (int k = 0; k < K - 1; ++k) co[k] = Elem<T>::from_f(win[k + 1]);
   xc[b * ED + e] = Elem<T>::from_f(acc * sigmoidf(acc));
 }
@@ -120,8 +149,8 @@ __global__ void conv_step_kernel(const T* __restrict__ xin, const T* __restrict_
 // those channels (12 contiguous elements) and the new inputs move as 8- or 16-byte vectors.
 template <typename T>
 __global__ void __launch_bounds__(256)
-conv_step_k4_kernel(const T* __restrict__ xin, const T* __restrict__ conv_in, const float* __restrict__ w,
-                    const float* __restrict__ bias, T* __restrict__ xc, T* __restrict__ conv_out,
+conv_step_k4_kernel(const T* __restrict__ xin, const T* __restrict__ conv_in, const Param w,
+                    const Param bias, T* __restrict__ xc, T* __restrict__ conv_out,
                     int64_t ED, int64_t x_sb) {
   const int64_t e = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   const int64_t b = blockIdx.y;
@@ -136,8 +165,14 @@ conv_step_k4_kernel(const T* __restrict__ xin, const T* __restrict__ conv_in, co
   Vec4<T> xo;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    const float4 wf = *reinterpret_cast<const float4*>(w + (e + c) * 4);
-    float acc = bias ? bias[e + c] : 0.f;
+    float4 wf;
+    if (w.dtype == MB200_F32) {
+      wf = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(w.p) + (e + c) * 4));
+    } else {
+      const Vec4<__nv_bfloat16> wb = *reinterpret_cast<const Vec4<__nv_bfloat16>*>(static_cast<const __nv_bfloat16*>(w.p) + (e + c) * 4);
+      wf = make_float4(__bfloat162float(wb.v[0]), __bfloat162float(wb.v[1]), __bfloat162float(wb.v[2]), __bfloat162float(wb.v[3]));
+    }
+    float acc = bias.p ? bias.at(e + c) : 0.f;
     acc = fmaf(wf.x, Elem<T>::to_f(win[3 * c]), acc);
     acc = fmaf(wf.y, Elem<T>::to_f(win[3 * c + 1]), acc);
     acc = fmaf(wf.z, Elem<T>::to_f(win[3 * c + 2]), acc);
@@ -230,25 +265,25 @@ __global__ void decay_prod_kernel(const T* __restrict__ delta, const float* __re
 using namespace mb200;
 
 template <typename T>
-static int ssm_step_t(const void* x, const void* delta, const void* z, const float* A,
-                      const void* Bm, const void* Cm, const float* D, const float* delta_bias,
-                      const float* h_in, float* h_out, void* y, int64_t B, int64_t ED, int N,
+static int ssm_step_t(const void* x, const void* delta, const void* z, Param A, const void* Bm, const void* Cm, Param D,
+                      Param delta_bias, const float* h_in, float* h_out, void* y, int64_t B, int64_t ED, int N,
                       int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb, int64_t c_sb,
-                      int64_t y_sb, int flags, cudaStream_t st) {
+                      int64_t y_sb, int flags, bool log_A, cudaStream_t st) {
   const bool vec_bc = (reinterpret_cast<uintptr_t>(Bm) % (4 * sizeof(T)) == 0) &&
                       (reinterpret_cast<uintptr_t>(Cm) % (4 * sizeof(T)) == 0) && b_sb % 4 == 0 && c_sb % 4 == 0;
+#define MB200_STEP_LAUNCH(NN, V, LOGA)                                                          \
+  ssm_step_kernel<T, NN, V, LOGA><<<grid, kStepThreads, 0, st>>>(                               \
+      (const T*)x, (const T*)delta, (const T*)z, A, (const T*)Bm, (const T*)Cm, D, delta_bias, \
+      h_in, h_out, (T*)y, B, ED, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags, rows)
 #define MB200_STEP(NN)                                                                          \
   {                                                                                             \
     constexpr int epb = kStepThreads / (NN / (MB200_STEP_SPL < NN ? MB200_STEP_SPL : NN));      \
-    dim3 grid(unsigned((ED + epb - 1) / epb), unsigned(B));                                     \
-    if (vec_bc)                                                                                 \
-      ssm_step_kernel<T, NN, true><<<grid, kStepThreads, 0, st>>>(                              \
-          (const T*)x, (const T*)delta, (const T*)z, A, (const T*)Bm, (const T*)Cm, D, delta_bias, \
-          h_in, h_out, (T*)y, ED, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags);                   \
-    else                                                                                        \
-      ssm_step_kernel<T, NN, false><<<grid, kStepThreads, 0, st>>>(                             \
-          (const T*)x, (const T*)delta, (const T*)z, A, (const T*)Bm, (const T*)Cm, D, delta_bias, \
-          h_in, h_out, (T*)y, ED, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags);                   \
+    const int64_t cols = (ED + epb - 1) / epb;                                                  \
+    /* rows per CTA: up to 4 while at least four CTAs per SM remain */                          \
+    const int rows = cols * B >= 4 * 592 ? 4 : cols * B >= 2 * 592 ? 2 : 1;                     \
+    dim3 grid(unsigned(cols), unsigned((B + rows - 1) / rows));                                 \
+    if (vec_bc) { if (log_A) MB200_STEP_LAUNCH(NN, true, true); else MB200_STEP_LAUNCH(NN, true, false); }    \
+    else { if (log_A) MB200_STEP_LAUNCH(NN, false, true); else MB200_STEP_LAUNCH(NN, false, false); }         \
     return check_launch();                                                                      \
   }
   switch (N) {
@@ -259,6 +294,32 @@ static int ssm_step_t(const void* x, const void* delta, const void* z, const flo
     default: return MB200_ENSTATE;
   }
 #undef MB200_STEP
+#undef MB200_STEP_LAUNCH
+}
+
+extern "C" int mb200_ssm_step_params(const void* x, const void* delta, const void* z, const void* A, int A_dtype, int A_is_log,
+                                     const void* Bm, const void* Cm, const void* D, int D_dtype, const void* delta_bias,
+                                     int bias_dtype, const float* h_in, float* h_out, void* y,
+                                     int64_t B, int64_t ED, int N, int64_t x_sb, int64_t d_sb,
+                                     int64_t z_sb, int64_t b_sb, int64_t c_sb, int64_t y_sb, int dtype,
+                                     int flags, void* stream) {
+  if (B < 0 || ED < 0) return MB200_EINVAL;
+  if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
+  for (int d : {A_dtype, D_dtype, bias_dtype})
+    if (d != MB200_F32 && d != MB200_BF16) return MB200_EDTYPE;
+  if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
+  if (B == 0 || ED == 0) return MB200_OK;
+  if (!x || !delta || !A || !Bm || !Cm || !h_out || !y) return MB200_EINVAL;
+  if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
+  if (B > 65535) return MB200_ETOOBIG;
+  if (!aligned16(h_in) || !aligned16(h_out) || (A_dtype == MB200_F32 && !aligned16(A))) return MB200_EALIGN;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const Param pA{A, A_dtype}, pD{D, D_dtype}, pb{delta_bias, bias_dtype};
+  return dtype == MB200_F32
+             ? ssm_step_t<float>(x, delta, z, pA, Bm, Cm, pD, pb, h_in, h_out, y, B, ED, N, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags,
+                                 A_is_log != 0, st)
+             : ssm_step_t<__nv_bfloat16>(x, delta, z, pA, Bm, Cm, pD, pb, h_in, h_out, y, B, ED, N, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb,
+                                         flags, A_is_log != 0, st);
 }
 
 extern "C" int mb200_ssm_step(const void* x, const void* delta, const void* z, const float* A,
@@ -267,54 +328,50 @@ extern "C" int mb200_ssm_step(const void* x, const void* delta, const void* z, c
                               int64_t B, int64_t ED, int N, int64_t x_sb, int64_t d_sb,
                               int64_t z_sb, int64_t b_sb, int64_t c_sb, int64_t y_sb, int dtype,
                               int flags, void* stream) {
-  if (B < 0 || ED < 0) return MB200_EINVAL;
-  if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
-  if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
-  if (B == 0 || ED == 0) return MB200_OK;
-  if (!x || !delta || !A || !Bm || !Cm || !h_out || !y) return MB200_EINVAL;
-  if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
-  if (B > 65535) return MB200_ETOOBIG;
-  if (!aligned16(h_in) || !aligned16(h_out) || !aligned16(A)) return MB200_EALIGN;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  return dtype == MB200_F32
-             ? ssm_step_t<float>(x, delta, z, A, Bm, Cm, D, delta_bias, h_in, h_out, y, B, ED, N,
-                                 x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags, st)
-             : ssm_step_t<__nv_bfloat16>(x, delta, z, A, Bm, Cm, D, delta_bias, h_in, h_out, y, B,
-                                         ED, N, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags, st);
+  return mb200_ssm_step_params(x, delta, z, A, MB200_F32, 0, Bm, Cm, D, MB200_F32, delta_bias, MB200_F32, h_in, h_out, y, B, ED, N, x_sb,
+                               d_sb, z_sb, b_sb, c_sb, y_sb, dtype, flags, stream);
 }
 
-extern "C" int mb200_conv_step(const void* xin, const void* conv_in, const float* w,
-                               const float* bias, void* xc, void* conv_out, int64_t B, int64_t ED,
-                               int K, int64_t x_sb, int dtype, void* stream) {
+extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype,
+                                      const void* bias, int bias_dtype, void* xc, void* conv_out, int64_t B, int64_t ED,
+                                      int K, int64_t x_sb, int dtype, void* stream) {
   if (B < 0 || ED < 0 || K < 1) return MB200_EINVAL;
   if (K > 8) return MB200_ETOOBIG;
-  if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
+  for (int d : {dtype, w_dtype, bias_dtype})
+    if (d != MB200_F32 && d != MB200_BF16) return MB200_EDTYPE;
   if (B == 0 || ED == 0) return MB200_OK;
   if (!xin || !w || !xc || (K > 1 && (!conv_in || !conv_out))) return MB200_EINVAL;
   if (B > 65535) return MB200_ETOOBIG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int es = dtype == MB200_F32 ? 4 : 2;
+  const Param pw{w, w_dtype}, pb{bias, bias_dtype};
   if (K == 4 && ED % 4 == 0 && aligned16(xin) && aligned16(conv_in) && aligned16(conv_out) && aligned16(xc) &&
       aligned16(w) && (x_sb * es) % 16 == 0) {
     dim3 g4(unsigned((ED / 4 + 255) / 256), unsigned(B));
     if (dtype == MB200_F32)
-      conv_step_k4_kernel<float><<<g4, 256, 0, st>>>((const float*)xin, (const float*)conv_in, w, bias,
+      conv_step_k4_kernel<float><<<g4, 256, 0, st>>>((const float*)xin, (const float*)conv_in, pw, pb,
                                                      (float*)xc, (float*)conv_out, ED, x_sb);
     else
       conv_step_k4_kernel<__nv_bfloat16><<<g4, 256, 0, st>>>(
-          (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, w, bias, (__nv_bfloat16*)xc,
+          (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, pw, pb, (__nv_bfloat16*)xc,
           (__nv_bfloat16*)conv_out, ED, x_sb);
     return check_launch();
   }
   dim3 grid(unsigned((ED + 255) / 256), unsigned(B));
   if (dtype == MB200_F32)
-    conv_step_kernel<float><<<grid, 256, 0, st>>>((const float*)xin, (const float*)conv_in, w, bias,
+    conv_step_kernel<float><<<grid, 256, 0, st>>>((const float*)xin, (const float*)conv_in, pw, pb,
                                                   (float*)xc, (float*)conv_out, ED, K, x_sb);
   else
     conv_step_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-        (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, w, bias, (__nv_bfloat16*)xc,
+        (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, pw, pb, (__nv_bfloat16*)xc,
         (__nv_bfloat16*)conv_out, ED, K, x_sb);
   return check_launch();
+}
+
+extern "C" int mb200_conv_step(const void* xin, const void* conv_in, const float* w,
+                               const float* bias, void* xc, void* conv_out, int64_t B, int64_t ED,
+                               int K, int64_t x_sb, int dtype, void* stream) {
+  return mb200_conv_step_params(xin, conv_in, w, MB200_F32, bias, MB200_F32, xc, conv_out, B, ED, K, x_sb, dtype, stream);
 }
 
 extern "C" int mb200_carry_fold(const float* P, const float* S, float* out, int64_t R, int64_t M,
@@ -410,9 +467,9 @@ extern "C" int mb200_selftest_wait_timeout(int polls, void* stream) {
 }
 
 extern "C" int mb200_device_status(void) {
-  const int f = mb200_fwd_device_status(), b = mb200_bwd_device_status();
+  const int f = mb200_fwd_device_status(), b = mb200_bwd_device_status(), k = mb200_block_step_device_status();
   int s = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&s, g_selftest_status, sizeof(int)) != cudaSuccess) return -1;
   if (s) cudaMemcpyToSymbol(g_selftest_status, &zero, sizeof(int));
-  return (f < 0 || b < 0) ? -1 : (f | b | s);
+  return (f < 0 || b < 0 || k < 0) ? -1 : (f | b | k | s);
 }

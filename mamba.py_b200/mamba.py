@@ -18,6 +18,8 @@ from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
+from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from ._lib import host as _host
 from .kernels import sscan_fwd_raw, sscan_bwd_raw  # noqa: F401  (re-exported)
@@ -136,6 +138,11 @@ def step(self, x, cache):
 
     Returns (output (B, D), (h, inputs)) with fresh cache tensors."""
     h, inputs = cache
+    p = _plain_block(self)
+    if p is not None:
+        cfg = self.config
+        out, h, inputs = _host().block_step(x, h, inputs, *p, cfg.dt_rank, cfg.d_state)
+        return out, (h, inputs)
     xz = self.in_proj(x)
     xs, z = xz.chunk(2, dim=1)
     xc, inputs = conv_step_fn(xs, inputs, self.conv1d.weight, self.conv1d.bias)
@@ -144,6 +151,31 @@ def step(self, x, cache):
     delta = F.linear(delta, self.dt_proj.weight)
     y, h = ssm_step_fn(xc, h, delta, A, B, C, self.D, z=z, delta_bias=self.dt_proj.bias)
     return self.out_proj(y), (h, inputs)
+
+
+def _plain_linear(m):
+    """(weight, bias) of a projection that is an ordinary nn.Linear and nothing else (no hooks, no subclass)."""
+    if type(m) is not nn.Linear or m._forward_hooks or m._forward_pre_hooks:
+        return None
+    p = m._parameters
+    return p["weight"], p["bias"]
+
+
+def _plain_block(self):
+    """The block's tensors in the order the native step takes them, or None if any part of it has been replaced, hooked or
+    extended (layer norms on dt, B, C) and has to be called as the module it is."""
+    d = self.__dict__
+    mods, pars = d.get("_modules"), d.get("_parameters")
+    if not mods or _has_any_global_hook() or any(mods.get(k) is not None for k in ("dt_layernorm", "B_layernorm", "C_layernorm")):
+        return None
+    lin = [_plain_linear(mods.get(k)) for k in ("in_proj", "x_proj", "dt_proj", "out_proj")]
+    conv, A_log, D = mods.get("conv1d"), pars.get("A_log"), pars.get("D")
+    if any(p is None for p in lin) or conv is None or A_log is None or D is None or lin[1][1] is not None or lin[2][1] is None:
+        return None
+    if self.config.d_state not in (8, 16, 32, 64):
+        return None
+    conv = conv._parameters
+    return (*lin[0], conv.get("weight"), conv.get("bias"), lin[1][0], *lin[2], A_log, D, *lin[3]) if "weight" in conv else None
 
 
 def _fusable(self, xz):
