@@ -322,6 +322,11 @@ typedef struct {
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
+/* mb200_rmsnorm_fwd with a weight of either type (MB200_EUNSUPPORTED for a bfloat16 weight on rows off the vector grid or wider
+ * than 8192). */
+int mb200_rmsnorm_fwd_typed(const void* x, const void* weight, int w_dtype, void* y, float* rstd, int64_t rows, int64_t D,
+                            int64_t x_rs, int64_t y_rs, float eps, int dtype, void* stream);
+
 /* mb200_ssm_step and mb200_conv_step with the small parameters in the model's own types (float32 or bfloat16 each); with A_is_log
  * A holds A_log and the decay rate is -exp(A_log). */
 int mb200_ssm_step_params(const void* x, const void* delta, const void* z, const void* A, int A_dtype, int A_is_log,

@@ -23,7 +23,7 @@ HOST_SRC = os.path.join(CSRC, "host")
 HOST_LIB = os.path.join(HERE, "_mamba_b200_host.so")
 
 NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++20",
     "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC,
 ]
 

@@ -27,13 +27,20 @@ __global__ void __launch_bounds__(kConvertThreads) convert_kernel(const __grid_c
   const mb200_convert_job& j = jobs.job[k];
   const int64_t total = j.rows * j.cols;
   const int64_t base = int64_t(int(blockIdx.x) - jobs.first_block[k]) * kConvertThreads * kPerThread + threadIdx.x;
+  const bool small = total < (int64_t(1) << 31);               // 32-bit division is several times cheaper
+  auto row_col = [&](int64_t i, int64_t& r, int64_t& c) {
+    if (j.rows == 1) { r = 0; c = i; }
+    else if (small) { const unsigned q = unsigned(i) / unsigned(j.cols); r = q; c = i - int64_t(q) * j.cols; }
+    else { r = i / j.cols; c = i - r * j.cols; }
+  };
   float v[kPerThread];
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {
     const int64_t i = base + u * kConvertThreads;
     v[u] = 0.f;
     if (i >= total) continue;
-    const int64_t r = i / j.cols, c = i - r * j.cols;
+    int64_t r, c;
+    row_col(i, r, c);
     if (j.src && c < j.src_cols) v[u] = load_as_float(j.src, j.src_dtype, r * j.src_stride + c);
     if (j.op == MB200_CONVERT_NEG_EXP) v[u] = -expf(v[u]);
     if (j.op == MB200_CONVERT_MUL) v[u] *= j.factor[i];
@@ -42,7 +49,9 @@ __global__ void __launch_bounds__(kConvertThreads) convert_kernel(const __grid_c
   for (int u = 0; u < kPerThread; ++u) {
     const int64_t i = base + u * kConvertThreads;
     if (i >= total) continue;
-    const int64_t r = i / j.cols, c = i - r * j.cols, o = r * j.dst_stride + c;
+    int64_t r, c;
+    row_col(i, r, c);
+    const int64_t o = r * j.dst_stride + c;
     if (j.dst_dtype == MB200_F32) static_cast<float*>(j.dst)[o] = v[u];
     else static_cast<__nv_bfloat16*>(j.dst)[o] = __float2bfloat16_rn(v[u]);
   }

@@ -152,19 +152,25 @@ Tensor rms_norm(const Tensor& x, const OptTensor& weight_, double eps) {
   const Tensor& weight = value(weight_);
   TORCH_CHECK(x.is_cuda(), kNeedCuda);
   const c10::cuda::CUDAGuard guard(x.device());
+  const bool grad = wants_grad(x, weight);
   Tensor y, x2, w32, rstd;
   {
     const BelowAutograd guard_ad;
     const auto dt = act_dtype(x);
     x2 = row_view(x, dt);
-    w32 = f32(weight);
     const int64_t n = x2.size(0), D = x2.size(1);
     y = empty(x.sizes(), dt, x);
-    rstd = empty({n}, at::kFloat, x);
-    check(mb200_rmsnorm_fwd(ptr(x2), fptr(w32), ptr(y), fptr(rstd), n, D, st(x2, 0), D, float(eps), dtype_code(dt), cuda_stream()),
-          "mb200_rmsnorm_fwd");
+    if (grad) rstd = empty({n}, at::kFloat, x);
+    int rc = MB200_EUNSUPPORTED;
+    if (!grad && weight.defined() && weight.scalar_type() == at::kBFloat16 && weight.is_contiguous())
+      rc = mb200_rmsnorm_fwd_typed(ptr(x2), ptr(weight), MB200_BF16, ptr(y), nullptr, n, D, st(x2, 0), D, float(eps), dtype_code(dt), cuda_stream());
+    if (rc == MB200_EUNSUPPORTED) {
+      w32 = f32(weight);
+      rc = mb200_rmsnorm_fwd(ptr(x2), fptr(w32), ptr(y), fptr(rstd), n, D, st(x2, 0), D, float(eps), dtype_code(dt), cuda_stream());
+    }
+    check(rc, "mb200_rmsnorm_fwd");
   }
-  if (wants_grad(x, weight)) {
+  if (grad) {
     auto node = new_node<RmsNormBackward>();
     node->set_next_edges(torch::autograd::collect_next_edges(x, weight));
     node->x.save(x2); node->w.save(w32); node->rstd.save(rstd);

@@ -154,7 +154,25 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
   StateStep s;
   {
     const BelowAutograd guard_ad;
-    s = state_step(w.xc, h, delta, A_log, true, dbc.narrow(1, R, N), dbc.narrow(1, R + N, N), D, xz.narrow(1, W, W), dt_b, false);
+    // the exponentials of A_log and the casts are worth a launch of their own once enough rows share them
+    const bool once = B >= 32 && small_type(A_log) && small_type(D) && small_type(dt_b) && A_log.is_contiguous() && D.is_contiguous() &&
+                      dt_b.is_contiguous();
+    Tensor A = A_log, Df = D, bf = dt_b;
+    if (once) {
+      mb200_convert_job jobs[3];
+      int n_jobs = 0;
+      auto add = [&](const Tensor& src, int op) {
+        const Tensor dst = empty(src.sizes(), at::kFloat, src);
+        const int64_t n = src.numel();
+        jobs[n_jobs++] = mb200_convert_job{ptr(src), ptr(dst), nullptr, 1, n, n, n, n, code_of(src), MB200_F32, op};
+        return dst;
+      };
+      A = add(A_log, MB200_CONVERT_NEG_EXP);
+      if (D.scalar_type() != at::kFloat) Df = add(D, MB200_CONVERT_COPY);
+      if (dt_b.scalar_type() != at::kFloat) bf = add(dt_b, MB200_CONVERT_COPY);
+      check(mb200_convert(jobs, n_jobs, cuda_stream()), "mb200_convert");
+    }
+    s = state_step(w.xc, h, delta, A, !once, dbc.narrow(1, R, N), dbc.narrow(1, R + N, N), Df, xz.narrow(1, W, W), bf, false);
   }
   return {at::linear(s.y, out_w, out_b_), s.h, w.window};
 }

@@ -31,96 +31,96 @@ struct Param {
   }
 };
 
-// kLogA: A holds A_log and the decay rate is -exp(A_log).  A CTA takes `rows` consecutive batch rows of its channels, so
-// that the parameters (and those exponentials) are fetched once for all of them.
-template <typename T, int N, bool kVecBC, bool kLogA>
+// kLogA: A holds A_log and the decay rate is -exp(A_log), which every batch row evaluates for itself; callers with many rows
+// do better with A.  (Several rows per CTA, parameters fetched once for all of them, measured slower: 34.2 us for two rows
+// and 35.6 for four against 31.5 at B 256, ED 5120: the registers cost more resident CTAs than the loads do.)
+// kF32: every parameter is float32 (the type test costs the streaming kernel registers and 4 us of 32).
+template <typename T, int N, bool kVecBC, bool kLogA, bool kF32>
 __global__ void __launch_bounds__(kStepThreads)
 ssm_step_kernel(const T* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ z,
-                const Param A, const T* __restrict__ Bm, const T* __restrict__ Cm,
-                const Param D, const Param delta_bias,
+                const Param A_, const T* __restrict__ Bm, const T* __restrict__ Cm,
+                const Param D_, const Param delta_bias_,
                 const float* __restrict__ h_in, float* __restrict__ h_out, T* __restrict__ y,
-                int64_t B, int64_t ED, int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb,
-                int64_t c_sb, int64_t y_sb, int flags, int rows) {
+                int64_t ED, int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb,
+                int64_t c_sb, int64_t y_sb, int flags) {
   constexpr int kSPL = MB200_STEP_SPL < N ? MB200_STEP_SPL : N;   // states per lane
   constexpr int kV = kSPL / 4;                                    // float4 per lane
   constexpr int kLPE = N / kSPL;                                  // lanes per channel
   constexpr int kEPB = kStepThreads / kLPE;                       // channels per CTA
+  const float* __restrict__ A = static_cast<const float*>(A_.p);
+  const float* __restrict__ D = static_cast<const float*>(D_.p);
+  const float* __restrict__ delta_bias = static_cast<const float*>(delta_bias_.p);
   const int tid = threadIdx.x;
   const int q = tid % kLPE;
   const int64_t e = int64_t(blockIdx.x) * kEPB + tid / kLPE;
   const bool ok = e < ED;
-  float Av[kSPL], bias = 0.f, Dv = 0.f;
+  const int64_t b = blockIdx.y;
+  float yv = 0.f, xv = 0.f;
   if (ok) {
-    if (A.dtype == MB200_F32) {
+    // the state is the only large stream: get it moving first, everything else is small
+    float4 hv[kV];
+    const float4* hp = reinterpret_cast<const float4*>(h_in + (b * ED + e) * N + kSPL * q);
 #pragma unroll
-      for (int v = 0; v < kV; ++v)
-        *reinterpret_cast<float4*>(Av + 4 * v) = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(A.p) + e * N + kSPL * q + 4 * v));
+    for (int v = 0; v < kV; ++v) hv[v] = h_in ? __ldcs(hp + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float Av[kSPL];
+    if (kF32 || A_.dtype == MB200_F32) {
+#pragma unroll
+      for (int v = 0; v < kV; ++v) *reinterpret_cast<float4*>(Av + 4 * v) = *reinterpret_cast<const float4*>(A + e * N + kSPL * q + 4 * v);
     } else {
+      static_assert(kSPL == 8, "one 16-byte vector of bfloat16 a lane");
+      const Vec16<__nv_bfloat16> w = ldg16(static_cast<const __nv_bfloat16*>(A_.p) + e * N + kSPL * q);
 #pragma unroll
-      for (int j = 0; j < kSPL; ++j) Av[j] = A.at(e * N + kSPL * q + j);
+      for (int j = 0; j < kSPL; ++j) Av[j] = __bfloat162float(w.v[j]);
     }
     if constexpr (kLogA) {
 #pragma unroll
       for (int j = 0; j < kSPL; ++j) Av[j] = -expf(Av[j]);
     }
-    if (flags & MB200_DELTA_SOFTPLUS) bias = delta_bias.at(e);
-    if (D.p && q == 0) Dv = D.at(e);
-  }
-  const int64_t b1 = min64(B, (int64_t(blockIdx.y) + 1) * rows);
-  for (int64_t b = int64_t(blockIdx.y) * rows; b < b1; ++b) {
-    float yv = 0.f, xv = 0.f;
-    if (ok) {
-      // the state is the only large stream: get it moving first, everything else is small
-      float4 hv[kV];
-      const float4* hp = reinterpret_cast<const float4*>(h_in + (b * ED + e) * N + kSPL * q);
-#pragma unroll
-      for (int v = 0; v < kV; ++v) hv[v] = h_in ? __ldcs(hp + v) : make_float4(0.f, 0.f, 0.f, 0.f);
-      float b4[kSPL], c4[kSPL];
-      if constexpr (kVecBC) {
-#pragma unroll
-        for (int v = 0; v < kV; ++v) {
-          const Vec4<T> bv = *reinterpret_cast<const Vec4<T>*>(Bm + b * b_sb + kSPL * q + 4 * v);
-          const Vec4<T> cv = *reinterpret_cast<const Vec4<T>*>(Cm + b * c_sb + kSPL * q + 4 * v);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) { b4[4 * v + j] = Elem<T>::to_f(bv.v[j]); c4[4 * v + j] = Elem<T>::to_f(cv.v[j]); }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < kSPL; ++j) {
-          b4[j] = Elem<T>::to_f(Bm[b * b_sb + kSPL * q + j]);
-          c4[j] = Elem<T>::to_f(Cm[b * c_sb + kSPL * q + j]);
-        }
-      }
-      xv = Elem<T>::to_f(x[b * x_sb + e]);
-      float dv = Elem<T>::to_f(delta[b * d_sb + e]);
-      if (flags & MB200_DELTA_SOFTPLUS) dv = softplus_fast(dv + bias);
-      const float dxs = dv * xv, d2s = dv * kLog2e;
-      const float2 dx = make_float2(dxs, dxs), d2 = make_float2(d2s, d2s);
-      float2 y2 = make_float2(0.f, 0.f);
-      float4* op = reinterpret_cast<float4*>(h_out + (b * ED + e) * N + kSPL * q);
+    float b4[kSPL], c4[kSPL];
+    if constexpr (kVecBC) {
 #pragma unroll
       for (int v = 0; v < kV; ++v) {
-        // packed f32x2 arithmetic: two states per instruction (the decays stay scalar ex2)
-        const float2 e01 = __fmul2_rn(d2, make_float2(Av[4 * v], Av[4 * v + 1])), e23 = __fmul2_rn(d2, make_float2(Av[4 * v + 2], Av[4 * v + 3]));
-        const float2 a01 = make_float2(ex2f(e01.x), ex2f(e01.y)), a23 = make_float2(ex2f(e23.x), ex2f(e23.y));
-        const float2 h01 = __ffma2_rn(a01, make_float2(hv[v].x, hv[v].y), __fmul2_rn(dx, make_float2(b4[4 * v], b4[4 * v + 1])));
-        const float2 h23 = __ffma2_rn(a23, make_float2(hv[v].z, hv[v].w), __fmul2_rn(dx, make_float2(b4[4 * v + 2], b4[4 * v + 3])));
-        y2 = __ffma2_rn(h01, make_float2(c4[4 * v], c4[4 * v + 1]), y2);
-        y2 = __ffma2_rn(h23, make_float2(c4[4 * v + 2], c4[4 * v + 3]), y2);
-        __stcs(op + v, make_float4(h01.x, h01.y, h23.x, h23.y));
-      }
-      yv = y2.x + y2.y;
-    }
+        const Vec4<T> bv = *reinterpret_cast<const Vec4<T>*>(Bm + b * b_sb + kSPL * q + 4 * v);
+        const Vec4<T> cv = *reinterpret_cast<const Vec4<T>*>(Cm + b * c_sb + kSPL * q + 4 * v);
 #pragma unroll
-    for (int s = kLPE / 2; s >= 1; s >>= 1) yv += __shfl_xor_sync(0xffffffffu, yv, s);
-    if (ok && q == 0) {
-      yv = fmaf(Dv, xv, yv);
-      if (z) {
-        const float zv = Elem<T>::to_f(z[b * z_sb + e]);
-        yv *= zv * sigmoid_fast(zv);
+        for (int j = 0; j < 4; ++j) { b4[4 * v + j] = Elem<T>::to_f(bv.v[j]); c4[4 * v + j] = Elem<T>::to_f(cv.v[j]); }
       }
-      y[b * y_sb + e] = Elem<T>::from_f(yv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kSPL; ++j) {
+        b4[j] = Elem<T>::to_f(Bm[b * b_sb + kSPL * q + j]);
+        c4[j] = Elem<T>::to_f(Cm[b * c_sb + kSPL * q + j]);
+      }
     }
+    xv = Elem<T>::to_f(x[b * x_sb + e]);
+    float dv = Elem<T>::to_f(delta[b * d_sb + e]);
+    if (flags & MB200_DELTA_SOFTPLUS) dv = softplus_fast(dv + (kF32 ? delta_bias[e] : delta_bias_.at(e)));
+    const float dxs = dv * xv, d2s = dv * kLog2e;
+    const float2 dx = make_float2(dxs, dxs), d2 = make_float2(d2s, d2s);
+    float2 y2 = make_float2(0.f, 0.f);
+    float4* op = reinterpret_cast<float4*>(h_out + (b * ED + e) * N + kSPL * q);
+#pragma unroll
+    for (int v = 0; v < kV; ++v) {
+      // packed f32x2 arithmetic: two states per instruction (the decays stay scalar ex2)
+      const float2 e01 = __fmul2_rn(d2, make_float2(Av[4 * v], Av[4 * v + 1])), e23 = __fmul2_rn(d2, make_float2(Av[4 * v + 2], Av[4 * v + 3]));
+      const float2 a01 = make_float2(ex2f(e01.x), ex2f(e01.y)), a23 = make_float2(ex2f(e23.x), ex2f(e23.y));
+      const float2 h01 = __ffma2_rn(a01, make_float2(hv[v].x, hv[v].y), __fmul2_rn(dx, make_float2(b4[4 * v], b4[4 * v + 1])));
+      const float2 h23 = __ffma2_rn(a23, make_float2(hv[v].z, hv[v].w), __fmul2_rn(dx, make_float2(b4[4 * v + 2], b4[4 * v + 3])));
+      y2 = __ffma2_rn(h01, make_float2(c4[4 * v], c4[4 * v + 1]), y2);
+      y2 = __ffma2_rn(h23, make_float2(c4[4 * v + 2], c4[4 * v + 3]), y2);
+      __stcs(op + v, make_float4(h01.x, h01.y, h23.x, h23.y));
+    }
+    yv = y2.x + y2.y;
+  }
+#pragma unroll
+  for (int s = kLPE / 2; s >= 1; s >>= 1) yv += __shfl_xor_sync(0xffffffffu, yv, s);
+  if (ok && q == 0) {
+    yv = fmaf(D ? (kF32 ? D[e] : D_.at(e)) : 0.f, xv, yv);
+    if (z) {
+      const float zv = Elem<T>::to_f(z[b * z_sb + e]);
+      yv *= zv * sigmoid_fast(zv);
+    }
+    y[b * y_sb + e] = Elem<T>::from_f(yv);
   }
 }
 
@@ -271,19 +271,20 @@ static int ssm_step_t(const void* x, const void* delta, const void* z, Param A, 
                       int64_t y_sb, int flags, bool log_A, cudaStream_t st) {
   const bool vec_bc = (reinterpret_cast<uintptr_t>(Bm) % (4 * sizeof(T)) == 0) &&
                       (reinterpret_cast<uintptr_t>(Cm) % (4 * sizeof(T)) == 0) && b_sb % 4 == 0 && c_sb % 4 == 0;
-#define MB200_STEP_LAUNCH(NN, V, LOGA)                                                          \
-  ssm_step_kernel<T, NN, V, LOGA><<<grid, kStepThreads, 0, st>>>(                               \
+  const bool all_f32 = A.dtype == MB200_F32 && D.dtype == MB200_F32 && delta_bias.dtype == MB200_F32;
+#define MB200_STEP_LAUNCH(NN, V, LOGA, F)                                                       \
+  ssm_step_kernel<T, NN, V, LOGA, F><<<grid, kStepThreads, 0, st>>>(                            \
       (const T*)x, (const T*)delta, (const T*)z, A, (const T*)Bm, (const T*)Cm, D, delta_bias, \
-      h_in, h_out, (T*)y, B, ED, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags, rows)
+      h_in, h_out, (T*)y, ED, x_sb, d_sb, z_sb, b_sb, c_sb, y_sb, flags)
 #define MB200_STEP(NN)                                                                          \
   {                                                                                             \
     constexpr int epb = kStepThreads / (NN / (MB200_STEP_SPL < NN ? MB200_STEP_SPL : NN));      \
-    const int64_t cols = (ED + epb - 1) / epb;                                                  \
-    /* rows per CTA: up to 4 while at least four CTAs per SM remain */                          \
-    const int rows = cols * B >= 4 * 592 ? 4 : cols * B >= 2 * 592 ? 2 : 1;                     \
-    dim3 grid(unsigned(cols), unsigned((B + rows - 1) / rows));                                 \
-    if (vec_bc) { if (log_A) MB200_STEP_LAUNCH(NN, true, true); else MB200_STEP_LAUNCH(NN, true, false); }    \
-    else { if (log_A) MB200_STEP_LAUNCH(NN, false, true); else MB200_STEP_LAUNCH(NN, false, false); }         \
+    dim3 grid(unsigned((ED + epb - 1) / epb), unsigned(B));                                     \
+    if (vec_bc && !log_A && all_f32) MB200_STEP_LAUNCH(NN, true, false, true);                  \
+    else if (vec_bc && log_A) MB200_STEP_LAUNCH(NN, true, true, false);                         \
+    else if (vec_bc) MB200_STEP_LAUNCH(NN, true, false, false);                                 \
+    else if (log_A) MB200_STEP_LAUNCH(NN, false, true, false);                                  \
+    else MB200_STEP_LAUNCH(NN, false, false, false);                                            \
     return check_launch();                                                                      \
   }
   switch (N) {
@@ -312,7 +313,7 @@ extern "C" int mb200_ssm_step_params(const void* x, const void* delta, const voi
   if (!x || !delta || !A || !Bm || !Cm || !h_out || !y) return MB200_EINVAL;
   if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
   if (B > 65535) return MB200_ETOOBIG;
-  if (!aligned16(h_in) || !aligned16(h_out) || (A_dtype == MB200_F32 && !aligned16(A))) return MB200_EALIGN;
+  if (!aligned16(h_in) || !aligned16(h_out) || !aligned16(A)) return MB200_EALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const Param pA{A, A_dtype}, pD{D, D_dtype}, pb{delta_bias, bias_dtype};
   return dtype == MB200_F32
