@@ -11,8 +11,8 @@
 // 3-step halo each chunk re-reads comes out of L2.  For the backward the host picks the chunk length
 // (a multiple of 4) so that the warps fill the GPU in whole waves.  Loads of a group of timesteps
 // are issued together, ahead of the arithmetic.
-// The backward walks a chunk in reverse with two windows (x behind, d(pre) ahead), recomputing the
-// pre-activation; the 8 warps of a CTA take 8 consecutive chunks of the same channels and add their
+// The backward walks a chunk with two windows (x and d(pre), both behind), recomputing the
+// pre-activation; the 4 warps of a CTA take 4 consecutive chunks of the same channels and add their
 // sums for dw and dbias in shared memory first, so global memory sees one atomic per CTA and value.
 #include <initializer_list>
 #include "common.cuh"
@@ -23,7 +23,13 @@ namespace {
 constexpr int kConvK = 4;
 constexpr int kConvThreads = 256;
 constexpr int kConvChunkFwd = 32;             // forward chunk (compile time: its loop is fully unrolled)
-constexpr int kConvGroup = 4;                 // timesteps whose loads are in flight together (forward)
+// Timesteps whose loads are in flight together.  Forward 8 (with 3 CTAs of 256 threads per SM): 29.5 us on the 130m layer
+// against 33.8 for 4.  Backward 4 (with 4 CTAs of 128 threads): 60 us; 6 and 8 need more registers than 16 warps per SM leave
+// and measured 71 and 75, walking backwards with CTAs of 256 threads 69.
+constexpr int kConvGroup = 8, kConvGroupBwd = 4;
+constexpr int kConvBwdThreads = 128;
+
+static_assert(kConvChunkFwd % kConvGroup == 0, "a chunk is a whole number of groups");
 
 template <typename T, int V> struct alignas(sizeof(T) * V) CVec {
   T v[V];
@@ -104,7 +110,7 @@ __device__ __forceinline__ CVec<T, V> pack(const Pk<W> (&o)[V / W]) {
 
 // grid: x = ceil(nvec / 32) channel groups, y = ceil(nchunk / 8), z = batch; warp w of a CTA takes chunk 8*y + w
 template <typename T, int V>
-__global__ void __launch_bounds__(kConvThreads, 4)
+__global__ void __launch_bounds__(kConvThreads, 3)
 conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                        T* __restrict__ y, int64_t L, int64_t ED, int64_t x_sb, int64_t x_sl,
                        int64_t y_sb, int64_t y_sl) {
@@ -163,17 +169,17 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
 // dx[t] = sum_k w[k] * dpre[t+3-k];  dw[k] = sum_{b,t} dpre[t] * x[t-3+k];  dbias = sum dpre;
 // dpre[t] = dy[t] * silu'(pre[t]),  pre recomputed from x.
 template <typename T, int V>
-__global__ void __launch_bounds__(kConvThreads, 2)
+__global__ void __launch_bounds__(kConvBwdThreads, 4)
 conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                        const T* __restrict__ dy, T* __restrict__ dx, float* __restrict__ dw,
                        float* __restrict__ dbias, int64_t L, int64_t ED, int64_t x_sb, int64_t x_sl,
                        int64_t dy_sb, int64_t dy_sl, int64_t dx_sb, int64_t dx_sl, int chunk) {
   __shared__ float s_acc[32 * V * (kConvK + 1)];          // per channel of the CTA: dw[0..3], dbias
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < 32 * V * (kConvK + 1); i += kConvThreads) s_acc[i] = 0.f;
+  for (int i = threadIdx.x; i < 32 * V * (kConvK + 1); i += kConvBwdThreads) s_acc[i] = 0.f;
   __syncthreads();
   const int64_t e = (int64_t(blockIdx.x) * 32 + lane) * V;
-  const int64_t t0 = (int64_t(blockIdx.y) * (kConvThreads / 32) + warp) * chunk;
+  const int64_t t0 = (int64_t(blockIdx.y) * (kConvBwdThreads / 32) + warp) * chunk;
   const int64_t t1 = min64(L, t0 + chunk);
   const int64_t b = blockIdx.z;
   if (e < ED && t0 < L) {
@@ -189,71 +195,79 @@ conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     const T* xp = x + b * x_sb + e;
     const T* gp = dy + b * dy_sb + e;
     T* op = dx + b * dx_sb + e;
-    // Both windows are circular buffers of 4 slots indexed by (steps taken) mod 4, and 4 steps are
-    // unrolled per loop iteration, so every slot index is a compile-time constant and nothing is moved:
-    // x[tau] and dpre[tau] live in slot (ts - tau) mod 4, ts = t1 + 2 being the first timestep processed.
-    F xr[P][kConvK], dr[P][kConvK], dwacc[P][kConvK], dbacc[P];
+    // Time is walked forwards in groups of kConvGroupBwd steps whose loads go out together; dx trails by three steps, because
+    // dx[t-3] needs dpre[t-3 .. t].  Slots 0..2 of the two windows are the last three steps of the group before.
+    constexpr int kG = kConvGroupBwd, kH = kConvK - 1;
+    F xw[P][kG + kH], dw_[P][kG + kH], dwacc[P][kConvK], dbacc[P];
 #pragma unroll
     for (int i = 0; i < P; ++i) {
       dbacc[i] = F::splat(0.f);
 #pragma unroll
-      for (int k = 0; k < kConvK; ++k) { dwacc[i][k] = F::splat(0.f); dr[i][k] = F::splat(0.f); }
-    }
-    const int64_t ts = t1 + kConvK - 2;
+      for (int k = 0; k < kConvK; ++k) dwacc[i][k] = F::splat(0.f);
 #pragma unroll
-    for (int k = 0; k < kConvK; ++k) {                     // x[ts-3 .. ts] -> slots 3-k
-      const int64_t t = ts - (kConvK - 1) + k;
+      for (int k = 0; k < kH; ++k) dw_[i][k] = F::splat(0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kH; ++k) {                         // x[t0-3 .. t0-1]
+      const int64_t t = t0 - kH + k;
       F xv[P];
-      unpack<T, V, W>(cload<T, V>(xp + t * x_sl, t >= 0 && t < L), xv);
+      unpack<T, V, W>(cload<T, V>(xp + t * x_sl, t >= 0), xv);
 #pragma unroll
-      for (int i = 0; i < P; ++i) xr[i][kConvK - 1 - k] = xv[i];
+      for (int i = 0; i < P; ++i) xw[i][k] = xv[i];
     }
-    // steps c = 0, 1, 2 (t >= t1) only produce dpre for the chunk's last outputs: their dx, dw belong
-    // to the next chunk.  Steps below t0 (a short last chunk, padding of the last group) do nothing.
-    const int nsteps = int(ts - t0) + 1;
+    // steps t1 .. t1+2 only produce dpre for the chunk's last outputs: their own dx, dw belong to the next chunk
     const F one = F::splat(1.f), mone = F::splat(-1.f);
 #pragma unroll 1
-    for (int c0 = 0; c0 < nsteps; c0 += kConvK) {
-      CVec<T, V> gv[kConvK], xv[kConvK];
+    for (int64_t tg = t0; tg < t1 + kH; tg += kG) {
+      CVec<T, V> gv[kG], xv[kG];
+      const T* xg = xp + tg * x_sl;
+      const T* gg = gp + tg * dy_sl;
 #pragma unroll
-      for (int j = 0; j < kConvK; ++j) {
-        const int64_t t = ts - (c0 + j);
-        gv[j] = cload<T, V>(gp + t * dy_sl, t >= t0 && t < L);
-        xv[j] = cload<T, V>(xp + (t - kConvK) * x_sl, t >= t0 && t - kConvK >= 0);
+      for (int j = 0; j < kG; ++j) {
+        const bool ok = tg + j < L && tg + j < t1 + kH;
+        xv[j] = cload<T, V>(xg, ok);
+        gv[j] = cload<T, V>(gg, ok);
+        xg += x_sl; gg += dy_sl;
       }
+      T* og = op + (tg - kH) * dx_sl;
 #pragma unroll
-      for (int j = 0; j < kConvK; ++j) {
-        const int c = c0 + j;
-        const int64_t t = ts - c;
-        const bool own = c >= kConvK - 1 && t >= t0;
+      for (int j = 0; j < kG; ++j) {
+        const int64_t t = tg + j;
+        const bool own = t < t1;
         F g[P], xn[P], o[P];
         unpack<T, V, W>(gv[j], g);
         unpack<T, V, W>(xv[j], xn);
 #pragma unroll
         for (int i = 0; i < P; ++i) {
-          // window of step t: x[t-3+k] is in slot (j + 3 - k) mod 4
+          xw[i][j + kH] = xn[i];
           F pre = bv[i];
 #pragma unroll
-          for (int k = 0; k < kConvK; ++k) pre = pfma(wk[i][k], xr[i][(j + 3 - k) & 3], pre);
+          for (int k = 0; k < kConvK; ++k) pre = pfma(wk[i][k], xw[i][j + k], pre);
           const F sg = psigmoid(pre);
-          // dpre = dy * s * (1 + pre * (1 - s));  dy is 0 outside [t0, L)
+          // dpre = dy * s * (1 + pre * (1 - s));  dy is 0 past the end
           const F dp = pmul(pmul(g[i], sg), pfma(pre, pfma(sg, mone, one), one));
-          // dx[t] = w3*dpre[t] + w2*dpre[t+1] + w1*dpre[t+2] + w0*dpre[t+3]; dpre[t+m] is in slot (j - m) mod 4
-          F acc = pmul(wk[i][3], dp);
-          acc = pfma(wk[i][2], dr[i][(j + 3) & 3], acc);
-          acc = pfma(wk[i][1], dr[i][(j + 2) & 3], acc);
-          acc = pfma(wk[i][0], dr[i][(j + 1) & 3], acc);
+          dw_[i][j + kH] = dp;
+          // dx[t-3] = w3*dpre[t-3] + w2*dpre[t-2] + w1*dpre[t-1] + w0*dpre[t]
+          F acc = pmul(wk[i][0], dp);
+#pragma unroll
+          for (int k = 1; k < kConvK; ++k) acc = pfma(wk[i][k], dw_[i][j + kH - k], acc);
           o[i] = acc;
           if (own) {
             dbacc[i] = padd(dbacc[i], dp);
 #pragma unroll
-            for (int k = 0; k < kConvK; ++k) dwacc[i][k] = pfma(dp, xr[i][(j + 3 - k) & 3], dwacc[i][k]);
+            for (int k = 0; k < kConvK; ++k) dwacc[i][k] = pfma(dp, xw[i][j + k], dwacc[i][k]);
           }
-          dr[i][j] = dp;
-          xr[i][j] = xn[i];                                  // x[t-4] takes the slot of x[t]
         }
-        if (own) cstore<T, V>(op + t * dx_sl, pack<T, V, W>(o));
+        if (t - kH >= t0 && t - kH < t1) cstore<T, V>(og, pack<T, V, W>(o));
+        og += dx_sl;
       }
+#pragma unroll
+      for (int i = 0; i < P; ++i)
+#pragma unroll
+        for (int k = 0; k < kH; ++k) {
+          xw[i][k] = xw[i][kG + k];
+          dw_[i][k] = dw_[i][kG + k];
+        }
     }
 #pragma unroll
     for (int i = 0; i < P; ++i) {
@@ -273,7 +287,7 @@ conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 32 * V * (kConvK + 1); i += kConvThreads) {
+  for (int i = threadIdx.x; i < 32 * V * (kConvK + 1); i += kConvBwdThreads) {
     const int64_t ch = int64_t(blockIdx.x) * 32 * V + i / (kConvK + 1);
     const int k = i % (kConvK + 1);
     if (ch >= ED) continue;
@@ -356,11 +370,11 @@ extern "C" int mb200_conv1d_silu_bwd(const void* x, const float* w, const float*
   const int64_t cols = (ED + 32 * int64_t(v) - 1) / (32 * int64_t(v));
   const int chunk = pick_conv_chunk(B, L, cols, 16);
   const int64_t nchunk = (L + chunk - 1) / chunk;
-  const int64_t ngroup = (nchunk + kConvThreads / 32 - 1) / (kConvThreads / 32);
+  const int64_t ngroup = (nchunk + kConvBwdThreads / 32 - 1) / (kConvBwdThreads / 32);
   if (B > 65535 || ngroup > 65535) return MB200_ETOOBIG;
   const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(ngroup), static_cast<unsigned>(B));
 #define MB200_CONV_BWD(TT, VV)                                                                          \
-  conv1d_silu_bwd_kernel<TT, VV><<<grid, kConvThreads, 0, st>>>((const TT*)x, w, bias, (const TT*)dy, \
+  conv1d_silu_bwd_kernel<TT, VV><<<grid, kConvBwdThreads, 0, st>>>((const TT*)x, w, bias, (const TT*)dy, \
       (TT*)dx, dw, dbias, L, ED, x_sb, x_sl, dy_sb, dy_sl, dx_sb, dx_sl, chunk)
   if (dtype == MB200_F32) { if (vec) MB200_CONV_BWD(float, 4); else MB200_CONV_BWD(float, 1); }
   else { if (vec) MB200_CONV_BWD(__nv_bfloat16, 4); else MB200_CONV_BWD(__nv_bfloat16, 1); }
