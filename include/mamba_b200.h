@@ -322,6 +322,48 @@ typedef struct {
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
+/* A sequence cut into `pieces` consecutive spans of piece_len timesteps (a multiple of 16; the last may be shorter) that are
+ * scanned side by side, for problems with few batch rows.  Per-token tensors and saved states keep their layouts; what belongs
+ * to a piece is (B, pieces, ED, N): the states entering the pieces (h0), the carry pass's states and decay products (the scan's
+ * last piece, whose carry feeds nothing, is left out of it), the gradient carries entering them from the right (g_in) and
+ * leaving them (g_out of the reverse carry pass, which leaves out the first).  hT and the backward's g_out stay (B, ED, N).
+ * mb200_carry_fold_range turns the carries into what enters each piece.  Forward direction only for the carry passes.
+ * MB200_EUNSUPPORTED: tensors no tensor map describes that cannot be read as B * pieces rows either. */
+int mb200_sscan_fwd_pieces(const void* x, const void* delta, const void* z,
+                    const float* A, const void* Bm, const void* Cm, const float* D,
+                    const float* delta_bias, const float* h0,
+                    void* y, float* hT, float* carries,
+                    int64_t B, int64_t L, int64_t ED, int N,
+                    int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                    int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
+                    int64_t c_sb, int64_t c_sl, int64_t y_sb, int64_t y_sl,
+                    int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream);
+int mb200_sscan_fwd_carry_pieces(const void* x, const void* delta, const float* A, const void* Bm,
+                          const float* delta_bias, float* h_out, float* p_out,
+                          int64_t B, int64_t L, int64_t ED, int N,
+                          int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                          int64_t b_sb, int64_t b_sl, int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream);
+int mb200_sscan_bwd_pieces(const void* x, const void* delta, const void* z,
+                    const float* A, const void* Bm, const void* Cm, const float* D,
+                    const float* delta_bias, const void* dy, const float* carries,
+                    const float* g_in,
+                    void* dx, void* ddelta, void* dz,
+                    float* dB, float* dC, float* dA, float* dD, float* ddelta_bias,
+                    float* g_out,
+                    int64_t B, int64_t L, int64_t ED, int N,
+                    int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                    int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
+                    int64_t c_sb, int64_t c_sl, int64_t dy_sb, int64_t dy_sl,
+                    int64_t dx_sb, int64_t dx_sl, int64_t dd_sb, int64_t dd_sl,
+                    int64_t dz_sb, int64_t dz_sl,
+                    int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream);
+int mb200_sscan_bwd_carry_pieces(const void* delta, const void* z, const void* dy, const void* Cm,
+                          const float* A, const float* delta_bias, float* g_out,
+                          int64_t B, int64_t L, int64_t ED, int N,
+                          int64_t d_sb, int64_t d_sl, int64_t z_sb, int64_t z_sl,
+                          int64_t dy_sb, int64_t dy_sl, int64_t c_sb, int64_t c_sl,
+                          int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream);
+
 /* mb200_rmsnorm_fwd with a weight of either type (MB200_EUNSUPPORTED for a bfloat16 weight on rows off the vector grid or wider
  * than 8192). */
 int mb200_rmsnorm_fwd_typed(const void* x, const void* weight, int w_dtype, void* y, float* rstd, int64_t rows, int64_t D,

@@ -89,18 +89,17 @@ struct InnerBackward : public torch::autograd::Node {
     const auto dt = xc_.scalar_type();
     const int64_t B = xc_.size(0), L = xc_.size(1), W = xc_.size(2), T = B * L, cols = Rp + 2 * N, K = cw_.size(1);
     Tensor dy = rows(grads[0], dt);
-    if (reverse && !tensor_map_ok(dy)) dy = dy.contiguous();
+    if ((reverse || S > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
     const Tensor dxz = empty({B, L, 2 * W}, dt, xz_);
     const ScanArgs a{xc_, delta.get(), A_, dbc_.narrow(2, Rp, N), dbc_.narrow(2, Rp + N, N), D.get(), xz_.narrow(2, W, W), bias.get(),
                      Tensor(), reverse};
     ScanGrads g = scan_backward(a, S, dy, carries.get(), P.get(), false, dxz.narrow(2, W, W), W * K + W);
     Convert conv;
-    const Tensor d_dbc = empty({T, cols}, dt, xz_), dd2 = g.dd.reshape({T, W}), xc2 = xc_.view({T, W}), dx2 = g.dx.reshape({T, W});
+    const Tensor d_dbc = empty({T, cols}, dt, xz_), dd2 = g.dd.view({T, W}), xc2 = xc_.view({T, W}), dx2 = g.dx.view({T, W});
     const int64_t es = d_dbc.element_size();
     auto col = [&](int64_t c) { return static_cast<char*>(d_dbc.data_ptr()) + c * es; };
-    const Tensor dB = g.dB.contiguous(), dC = g.dC.contiguous();
-    conv.add(ptr(dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);         // float32 accumulators -> activation dtype, in place
-    conv.add(ptr(dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
+    conv.add(ptr(g.dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);         // float32 accumulators -> activation dtype, in place
+    conv.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
     conv.run();
     Tensor d_dt = d_dbc.narrow(1, 0, Rp);
     at::mm_out(d_dt, dd2, Wdt_);                                            // through dt_proj
@@ -201,8 +200,12 @@ Tensor inner(const Tensor& xz, const Tensor& conv_w, const OptTensor& conv_b_, c
     a.B = dbc.narrow(2, Rp, N);
     a.C = dbc.narrow(2, Rp + N, N);
     a.reverse = reverse;
-    S = reverse ? 1 : pick_subshards(B, L, W);
-    TORCH_CHECK(scan_forward(a, S, false, grad, o), "mamba_b200: these tensors cannot be scanned in reverse");
+    S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
+    if (!scan_forward(a, S, false, grad, o)) {
+      TORCH_CHECK(!reverse, "mamba_b200: these tensors cannot be scanned in reverse");
+      S = 1;
+      scan_forward(a, 1, false, grad, o);
+    }
   }
   if (grad) {
     auto node = new_node<InnerBackward>();

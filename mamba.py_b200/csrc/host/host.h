@@ -122,6 +122,6 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
                                               const Tensor& dt_b, const Tensor& A_log, const Tensor& D, const Tensor& out_w,
                                               const OptTensor& out_b, int64_t dt_rank, int64_t d_state);
 
-int64_t pick_subshards(int64_t batch, int64_t length, int64_t width);
+int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad);
 
 }  // namespace mb200_host

@@ -21,5 +21,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("inner", &inner, NoGil());
   m.def("inner_reversible", &inner_reversible);
   m.def("block_step", &block_step, NoGil());
-  m.def("pick_subshards", &pick_subshards);
+  m.def("pick_pieces", &pick_pieces);
 }

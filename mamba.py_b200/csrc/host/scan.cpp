@@ -1,5 +1,6 @@
 // selective_scan_fn and pscan: forward launches and their autograd nodes.
 #include "scan.h"
+#include <cmath>
 #include <cstdlib>
 
 namespace mb200_host {
@@ -16,27 +17,16 @@ void check_status(const char* what) {
 
 namespace {
 
-constexpr int64_t kResidentCtas = 444;          // 148 SMs x 3 CTAs of the fused kernels
-
-// (B, L, C) -> (B*S, L/S, C): every batch row cut into S consecutive pieces (a view when the strides allow it).
-Tensor cut(const Tensor& t, int64_t S) {
-  if (!t.defined() || S == 1) return t;
-  return t.unflatten(1, {S, t.size(1) / S}).flatten(0, 1);
-}
-Tensor join(const Tensor& t, int64_t S) {
-  if (!t.defined() || S == 1) return t;
-  return t.unflatten(0, {t.size(0) / S, S}).flatten(1, 2);
-}
-
-int launch_forward(const ScanArgs& a, ScanOut& o, bool want_last, bool want_carries) {
+// What enters the pieces of a cut sequence (a.h0, the gradient carries) has one entry a piece.
+int launch_forward(const ScanArgs& a, ScanOut& o, bool want_last, bool want_carries, int64_t pieces = 1, int64_t piece_len = 0) {
   const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states(), chunk = mb200_sscan_chunk();
   o.y = empty({B, L, W}, a.x.scalar_type(), a.x);
   if (want_last) o.hT = empty({B, W, N}, at::kFloat, a.x);
   if (want_carries) o.carries = empty({B, (L + chunk - 1) / chunk, W, N}, at::kFloat, a.x);
-  const int rc = mb200_sscan_fwd(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), fptr(a.h0),
+  const int rc = mb200_sscan_fwd_pieces(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), fptr(a.h0),
                                  ptr(o.y), fptr(o.hT), fptr(o.carries), B, L, W, int(N), st(a.x, 0), st(a.x, 1), st(a.delta, 0),
                                  st(a.delta, 1), st(a.z, 0), st(a.z, 1), st(a.B, 0), st(a.B, 1), st(a.C, 0), st(a.C, 1), st(o.y, 0),
-                                 st(o.y, 1), a.code(), a.flags(), cuda_stream());
+                                 st(o.y, 1), a.code(), a.flags(), pieces, piece_len, cuda_stream());
   if (rc != MB200_EUNSUPPORTED) {
     check(rc, "mb200_sscan_fwd");
     check_status("mb200_sscan_fwd");
@@ -44,32 +34,29 @@ int launch_forward(const ScanArgs& a, ScanOut& o, bool want_last, bool want_carr
   return rc;
 }
 
-// Rows cut into S pieces that run as extra batch rows: carry pass, fold, full pass (the protocol of split.py).
-ScanOut split_forward(const ScanArgs& a, int64_t S, bool want_carries) {
-  const int64_t B = a.batch(), W = a.width(), N = a.states();
-  ScanArgs s = a;
-  s.x = cut(a.x, S); s.delta = cut(a.delta, S); s.z = cut(a.z, S); s.B = cut(a.B, S); s.C = cut(a.C, S);
-  // one row: its last piece's carry feeds nothing, so that piece is left out of the pass
-  const int64_t skip = B == 1 ? 1 : 0, rows_all = B * S, n = rows_all - skip;
-  Tensor PS = empty({2, B, S, W, N}, at::kFloat, a.x);
-  if (skip) PS.view({2, rows_all, W, N}).slice(1, n, rows_all).zero_();
-  float *P = fptr(PS), *St = P + rows_all * W * N;
-  check(mb200_sscan_fwd_carry(ptr(s.x), ptr(s.delta), fptr(s.A), ptr(s.B), fptr(s.bias), St, P, n, s.length(), W, int(N), st(s.x, 0),
-                              st(s.x, 1), st(s.delta, 0), st(s.delta, 1), st(s.B, 0), st(s.B, 1), s.code(), s.flags(), cuda_stream()),
-        "mb200_sscan_fwd_carry");
+int64_t piece_length(int64_t L, int64_t S) { return (L + 16 * S - 1) / (16 * S) * 16; }
+
+// Rows cut into S pieces: carry pass, fold, full pass (the protocol of split.py).  False when these tensors cannot be cut.
+bool split_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carries, ScanOut& o) {
+  const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states(), len = piece_length(L, S);
+  const Tensor PS = empty({2, B, S, W, N}, at::kFloat, a.x);
+  float *P = fptr(PS), *St = P + B * S * W * N;
+  const int rc = mb200_sscan_fwd_carry_pieces(ptr(a.x), ptr(a.delta), fptr(a.A), ptr(a.B), fptr(a.bias), St, P, B, L, W, int(N), st(a.x, 0),
+                                              st(a.x, 1), st(a.delta, 0), st(a.delta, 1), st(a.B, 0), st(a.B, 1), a.code(), a.flags(), S, len,
+                                              cuda_stream());
+  if (rc == MB200_EUNSUPPORTED) return false;
+  check(rc, "mb200_sscan_fwd_carry");
   check_status("mb200_sscan_fwd_carry");
-  s.h0 = empty({rows_all, W, N}, at::kFloat, a.x);
+  ScanArgs s = a;
+  s.h0 = empty({B, S, W, N}, at::kFloat, a.x);
   check(mb200_carry_fold_range(P, St, fptr(a.h0), fptr(s.h0), B, S, W * N, 0, int(S), 0, cuda_stream()), "mb200_carry_fold_range");
-  ScanOut o;
-  launch_forward(s, o, true, want_carries);
-  o.y = join(o.y, S);
-  o.hT = o.hT.unflatten(0, {B, S}).select(1, S - 1);
+  if (launch_forward(s, o, want_last, want_carries, S, len) == MB200_EUNSUPPORTED) return false;
   o.P = PS.select(0, 0);
-  return o;
+  return true;
 }
 
 ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out, const Tensor& dz,
-                          int64_t extra) {
+                          int64_t extra, int64_t pieces = 1, int64_t piece_len = 0) {
   const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states();
   ScanGrads g;
   const auto dt = a.x.scalar_type();
@@ -87,38 +74,27 @@ ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& car
   if (a.bias.defined()) g.dbias = acc.narrow(0, 2 * nBC + nA + W, W);
   if (extra) g.extra = acc.narrow(0, 2 * nBC + nA + 2 * W, extra);
   if (want_g_out) g.g_out = empty({B, W, N}, at::kFloat, a.x);
-  check(mb200_sscan_bwd(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), ptr(dy), fptr(carries),
+  check(mb200_sscan_bwd_pieces(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), ptr(dy), fptr(carries),
                         fptr(g_in), ptr(g.dx), ptr(g.dd), ptr(g.dz), fptr(g.dB), fptr(g.dC), fptr(g.dA), fptr(g.dD), fptr(g.dbias),
                         fptr(g.g_out), B, L, W, int(N), st(a.x, 0), st(a.x, 1), st(a.delta, 0), st(a.delta, 1), st(a.z, 0), st(a.z, 1),
                         st(a.B, 0), st(a.B, 1), st(a.C, 0), st(a.C, 1), st(dy, 0), st(dy, 1), st(g.dx, 0), st(g.dx, 1), st(g.dd, 0),
-                        st(g.dd, 1), st(g.dz, 0), st(g.dz, 1), a.code(), a.flags(), cuda_stream()),
+                        st(g.dd, 1), st(g.dz, 0), st(g.dz, 1), a.code(), a.flags(), pieces, piece_len, cuda_stream()),
         "mb200_sscan_bwd");
   check_status("mb200_sscan_bwd");
   return g;
 }
 
-ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, const Tensor& dz,
-                         int64_t extra) {
-  const int64_t B = a.batch(), W = a.width(), N = a.states();
-  ScanArgs s = a;
-  s.x = cut(a.x, S); s.delta = cut(a.delta, S); s.z = cut(a.z, S); s.B = cut(a.B, S); s.C = cut(a.C, S);
-  const Tensor dys = cut(dy, S);
-  const int64_t skip = B == 1 ? 1 : 0, rows_all = B * S;              // the first piece's carry feeds nothing
-  Tensor G = empty({rows_all, W, N}, at::kFloat, a.x);
-  if (skip) G.slice(0, 0, 1).zero_();
-  auto from = [&](const Tensor& t) { return (skip && t.defined()) ? t.slice(0, skip) : t; };
-  const Tensor d1 = from(s.delta), z1 = from(s.z), y1 = from(dys), c1 = from(s.C);
-  check(mb200_sscan_bwd_carry(ptr(d1), ptr(z1), ptr(y1), ptr(c1), fptr(s.A), fptr(s.bias), fptr(G) + skip * W * N, rows_all - skip,
-                              s.length(), W, int(N), st(d1, 0), st(d1, 1), st(z1, 0), st(z1, 1), st(y1, 0), st(y1, 1), st(c1, 0),
-                              st(c1, 1), s.code(), s.flags(), cuda_stream()),
+ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
+                         const Tensor& dz, int64_t extra) {
+  const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states(), len = piece_length(L, S);
+  const Tensor G = empty({B, S, W, N}, at::kFloat, a.x), g_in = empty({B, S, W, N}, at::kFloat, a.x);
+  check(mb200_sscan_bwd_carry_pieces(ptr(a.delta), ptr(a.z), ptr(dy), ptr(a.C), fptr(a.A), fptr(a.bias), fptr(G), B, L, W, int(N),
+                                     st(a.delta, 0), st(a.delta, 1), st(a.z, 0), st(a.z, 1), st(dy, 0), st(dy, 1), st(a.C, 0), st(a.C, 1),
+                                     a.code(), a.flags(), S, len, cuda_stream()),
         "mb200_sscan_bwd_carry");
   check_status("mb200_sscan_bwd_carry");
-  const Tensor g_in = empty({rows_all, W, N}, at::kFloat, a.x);
   check(mb200_carry_fold_range(fptr(P), fptr(G), nullptr, fptr(g_in), B, S, W * N, 0, int(S), 1, cuda_stream()), "mb200_carry_fold_range");
-  ScanGrads g = launch_backward(s, dys, carries, g_in, true, cut(dz, S), extra);
-  for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC}) *t = join(*t, S);
-  g.g_out = g.g_out.unflatten(0, {B, S}).select(1, 0);
-  return g;
+  return launch_backward(a, dy, carries, g_in, want_g_out, dz, extra, S, len);
 }
 
 }  // namespace
@@ -133,16 +109,22 @@ bool tensor_maps_ok(const ScanArgs& a) {
   return a.width() * a.x.element_size() % 16 == 0;
 }
 
+int64_t cuttable(const ScanArgs& a, int64_t S, bool grad, bool want_last) {
+  if (S == 1 || (tensor_maps_ok(a) && tensor_map_ok(a.B) && tensor_map_ok(a.C) && (!grad || a.states() == 16))) return S;
+  if (a.h0.defined() || want_last) return 1;
+  int64_t even = 1;
+  while (2 * even <= S && a.length() % (32 * even) == 0) even *= 2;
+  for (const Tensor* t : {&a.x, &a.delta, &a.z, &a.B, &a.C})
+    if (t->defined() && a.batch() > 1 && t->stride(0) != a.length() * t->stride(1)) return 1;
+  return even;
+}
+
 bool scan_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carries, ScanOut& o) {
-  if (S > 1) {
-    o = split_forward(a, S, want_carries);
-    return true;
-  }
-  return launch_forward(a, o, want_last, want_carries) == MB200_OK;
+  return S > 1 ? split_forward(a, S, want_last, want_carries, o) : launch_forward(a, o, want_last, want_carries) == MB200_OK;
 }
 ScanGrads scan_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
                         const Tensor& dz, int64_t extra) {
-  return S > 1 ? split_backward(a, S, dy, carries, P, dz, extra) : launch_backward(a, dy, carries, Tensor(), want_g_out, dz, extra);
+  return S > 1 ? split_backward(a, S, dy, carries, P, want_g_out, dz, extra) : launch_backward(a, dy, carries, Tensor(), want_g_out, dz, extra);
 }
 
 namespace {
@@ -185,9 +167,9 @@ struct ScanBackward : public torch::autograd::Node {
     ScanArgs a{x.get(), delta.get(), A.get(), B.get(), C.get(), D.get(), z.get(), bias.get(), Tensor(), reverse};
     const c10::cuda::CUDAGuard guard(a.x.device());
     Tensor dy = rows(flipped ? grads[0].flip(1) : grads[0], a.x.scalar_type());
-    // the in-kernel reverse backward exists on the tensor-map path only; an upstream gradient that is an offset or
-    // narrow view of something wider is copied to a dense tensor first
-    if (reverse && !tensor_map_ok(dy)) dy = dy.contiguous();
+    // the in-kernel reverse backward and uneven pieces exist on the tensor-map path only; an upstream gradient that is an
+    // offset or narrow view of something wider is copied to a dense tensor first
+    if ((reverse || subshards > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
     ScanGrads g = scan_backward(a, subshards, dy, carries.get(), P.get(), given[kH0]);
     if (flipped)
       for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC})
@@ -201,20 +183,28 @@ struct ScanBackward : public torch::autograd::Node {
 
 }  // namespace
 
-// How many pieces to cut each row into.  The fused kernels have batch * ceil(width / 32) independent work items (a CTA owns
-// one) and 148 SMs hold three CTAs each.  Measured on B200, forward + backward of one row (ms): width 2048, length 65536:
-// 12.0 uncut, 7.8 / 5.8 / 5.8 / 4.8 in 2 / 4 / 8 / 16 pieces; 2048 x 8192: 1.53 uncut, 0.68 in 16; 5120 x 131072: 35.5
-// uncut, 27.0 / 23.9 / 23.7 in 4 / 8 / 16.  So: cut until there are about two waves of CTAs (the pieces' tails then
-// overlap), keep pieces at least 512 timesteps long, and leave alone what already fills half the GPU (a cut costs two extra
-// carry passes) or is so short that the extra launches eat the gain.
-int64_t pick_subshards(int64_t batch, int64_t length, int64_t width) {
-  const int64_t items = batch * ((width + 31) / 32);
-  if (length < 4096 || 2 * items >= kResidentCtas) return 1;
+// How many pieces to cut each row into, from a model of the time: the fused kernels have batch * ceil(width / 32) independent
+// work items a piece (a CTA owns one, three fit an SM), and one CTA alone on an SM runs much faster than one of three.
+// Measured on the 130m layer (2048 timesteps, bfloat16), us with 1 / 2 / 3 CTAs on every SM: forward 109 / 142 / 199, backward
+// 345 / 480 / 658; the carry passes take 0.55 of a forward.  Launches and the fold cost about 6 us a pass.
+int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
+  constexpr double kSms = 148, kFwd[] = {0, 109. / 2048, 142. / 2048, 199. / 2048}, kBwd[] = {0, 345. / 2048, 480. / 2048, 658. / 2048};
+  const double items = double(batch) * double((width + 31) / 32);
+  auto passes = [&](double ctas, const double (&t)[4]) {                 // us per timestep of the longest SM
+    const int per_sm = int(std::ceil(ctas / kSms)), full = per_sm / 3, rest = per_sm % 3;
+    return full * t[3] + t[rest];
+  };
   int64_t best = 1;
-  for (int64_t S : {2, 4, 8, 16}) {
-    if (length % (16 * S) || length / S < 512) break;
-    best = S;
-    if (items * S >= 2 * kResidentCtas) break;
+  double best_us = 0;
+  for (int64_t S = 1; S <= 24 && (S == 1 || length / S >= 64); ++S) {
+    const double len = double(S == 1 ? length : (length + 16 * S - 1) / (16 * S) * 16);
+    if (S > 1 && (S - 1) * len >= length) continue;
+    double us = len * (passes(items * S, kFwd) + (grad ? passes(items * S, kBwd) : 0));
+    if (S > 1) us += (len * 0.55 * passes(items * (S - 1), kFwd) + 12) * (grad ? 2 : 1);
+    if (S == 1 || us < 0.95 * best_us) {
+      best = S;
+      best_us = us;
+    }
   }
   return best;
 }
@@ -239,13 +229,18 @@ py::object selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A,
       a = ScanArgs{rows(x, dt), rows(delta, dt), f32(A), rows(B, dt), rows(C, dt), f32(D), rows(z, dt), f32(bias), f32(h0), reverse};
       const int64_t L = a.length();
       // Few batch rows: cut every row into S consecutive pieces that run side by side.
-      S = subshards.value_or(0) ? *subshards : pick_subshards(a.batch(), L, a.width());
-      if (reverse || S < 1 || L % (16 * S) || L == 0) S = 1;
       align_bc(a);
+      S = subshards.value_or(0) ? *subshards : pick_pieces(a.batch(), L, a.width(), grad);
+      if (reverse || S < 1 || (subshards.value_or(0) && L % (16 * S)) || L == 0) S = 1;
+      S = cuttable(a, S, grad, return_last_state);
       // the reverse backward exists for d_state 16 on the tensor-map path; otherwise do what the reference does
       // (mambapy/vim.py:228-261): scan the flipped sequence, flip back
       flipped = reverse && grad && a.states() != 16;
-      if (!flipped && !scan_forward(a, S, return_last_state, grad, o)) flipped = true;
+      if (!flipped && !scan_forward(a, S, return_last_state, grad, o)) {
+        flipped = reverse;
+        S = 1;
+        if (!reverse) scan_forward(a, 1, return_last_state, grad, o);
+      }
       if (flipped) {
         for (Tensor* t : {&a.x, &a.delta, &a.z, &a.B, &a.C})
           if (t->defined()) *t = t->flip(1);

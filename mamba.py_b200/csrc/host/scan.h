@@ -27,6 +27,10 @@ struct ScanGrads {
 bool tensor_map_ok(const Tensor& t);
 bool tensor_maps_ok(const ScanArgs& a);
 
+// The number of pieces these tensors can be cut into, at most S: any number when every pass takes the tensor-map path, a power of
+// two that divides the sequence when the pieces have to be read as extra batch rows.
+int64_t cuttable(const ScanArgs& a, int64_t S, bool grad, bool want_last);
+
 // S consecutive pieces per row; S = 1 is the single launch.  False (S = 1 only) when the kernels cannot scan these tensors
 // in reverse.
 bool scan_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carries, ScanOut& o);

@@ -1,5 +1,6 @@
 // Geometry and parameter blocks shared by the fused selective-scan kernels.
 #pragma once
+#include <initializer_list>
 #include "common.cuh"
 #include "tile.cuh"
 
@@ -92,6 +93,10 @@ struct SscanFwdParams {
   int64_t B, L, ED;
   int64_t x_sb, x_sl, d_sb, d_sl, z_sb, z_sl, b_sb, b_sl, c_sb, c_sl, y_sb, y_sl;
   int flags;
+  // A sequence cut into `pieces` spans of piece_len timesteps (a multiple of 16; the last may be shorter) that are scanned
+  // side by side: h0, and the state and decay product of the passes without y, are then (B, pieces, ED, N).  A launch
+  // covers launch_pieces of them from piece0.
+  int64_t pieces = 1, piece_len = int64_t(1) << 40, piece0 = 0, launch_pieces = 1;
 };
 
 struct SscanBwdParams {
@@ -103,8 +108,25 @@ struct SscanBwdParams {
   int64_t x_sb, x_sl, d_sb, d_sl, z_sb, z_sl, b_sb, b_sl, c_sb, c_sl, dy_sb, dy_sl;
   int64_t dx_sb, dx_sl, dd_sb, dd_sl, dz_sb, dz_sl;
   int flags;
+  int64_t pieces = 1, piece_len = int64_t(1) << 40;      // as in the forward; g_in is then (B, pieces, ED, N)
 };
 
+}  // namespace mb200
+
+// Pieces of a sequence: their length is a multiple of the kernels' 16-step tiles and each holds at least one timestep.
+namespace mb200 {
+inline bool pieces_ok(int64_t pieces, int64_t piece_len, int64_t L) {
+  return pieces == 1 || (pieces > 1 && piece_len > 0 && piece_len % 16 == 0 && (pieces - 1) * piece_len < L);
+}
+// Whether (B, pieces) can be read as one batch dimension: even pieces, and batch strides that continue the rows.
+inline bool pieces_as_rows(int64_t B, int64_t L, int64_t pieces, int64_t piece_len, std::initializer_list<int64_t> sb,
+                           std::initializer_list<int64_t> sl) {
+  if (pieces * piece_len != L || B * pieces > 65535) return false;
+  auto l = sl.begin();
+  for (int64_t s : sb)
+    if (B > 1 && s != L * *l++) return false;
+  return true;
+}
 }  // namespace mb200
 
 // Internal flag (never part of the public flags): run the forward kernel as the reverse carry pass.

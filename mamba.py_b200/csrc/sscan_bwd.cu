@@ -106,17 +106,19 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t e0 = int64_t(blockIdx.x) * kBTE;
+  // times fit 32 bits on this path; what is 64-bit in the loops costs the recurrence warps spills
   const int64_t b = blockIdx.y;
+  const int pc = int(blockIdx.z), t_lo = int(pc * p.piece_len), t_hi = int(min64(p.L, t_lo + p.piece_len));
   const int cols_ok = int(min64(kBTE, p.ED - e0));
   constexpr bool softplus = kSoftplus;
   constexpr bool has_z = kHasZ;
-  const int64_t ntiles = (p.L + kBTile - 1) / kBTile;
+  const int ntiles = (t_hi - t_lo + kBTile - 1) / kBTile;
   // Direction of the scan being differentiated (MB200_REVERSE: it ran from t = L-1 down to 0).  Tiles
   // are taken in the opposite order of that scan: iteration j works on the tile that starts at
   // tile_t0(j); step s of a tile in the scan's own order is its row `row(s)`.  Saved states are
   // indexed by time chunk: entry c is the state entering chunk c in the scan direction.
   constexpr bool rev = kRev;
-  auto tile_t0 = [&](int64_t j) { return (rev ? j : ntiles - 1 - j) * kBTile; };
+  auto tile_t0 = [&](int j) { return t_lo + (rev ? j : ntiles - 1 - j) * kBTile; };
   auto row = [](int s) { return rev ? kBTile - 1 - s : s; };
 
   if (tid == 0) {
@@ -155,7 +157,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         a4[j] = e_ok ? p.A[e * N + 4 * q + j] * kLog2e : 0.f;
-        g4[j] = (e_ok && p.g_in) ? p.g_in[(b * p.ED + e) * N + 4 * q + j] : 0.f;
+        g4[j] = (e_ok && p.g_in) ? p.g_in[((b * p.pieces + pc) * p.ED + e) * N + 4 * q + j] : 0.f;
       }
       A2[0] = make_float2(a4[0], a4[1]); A2[1] = make_float2(a4[2], a4[3]);
       gc[0] = make_float2(g4[0], g4[1]); gc[1] = make_float2(g4[2], g4[3]);
@@ -163,21 +165,22 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
     }
     const int op_off0 = op_index(0, e_l, kBTE), op_off1 = op_index(1, e_l, kBTE) - kBTE;
     const int npo = np_chan(e_l) * 4 + q;
-    const int64_t nchunks = (p.L + kHalf - 1) / kHalf;
+    const int nchunks = int((p.L + kHalf - 1) / kHalf);
     const float* carry_base = p.carries + (b * nchunks * p.ED + e) * N + 4 * q;
-    auto load_carry = [&](int64_t c) {
+    auto load_carry = [&](int c) {
       return (e_ok && c < nchunks) ? *reinterpret_cast<const float4*>(carry_base + c * p.ED * N)
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     // states entering the first / second half (in scan order) of iteration j's tile
     // (time chunk 2*tile + 1 is the first half in scan order when reversed, chunk 2*tile otherwise)
-    float4 carry_next = load_carry(rev ? 1 : 2 * (ntiles - 1)), carry_next_mid = load_carry(rev ? 0 : 2 * (ntiles - 1) + 1);
+    const int c_lo = t_lo / kHalf;
+    float4 carry_next = load_carry(c_lo + (rev ? 1 : 2 * (ntiles - 1))), carry_next_mid = load_carry(c_lo + (rev ? 0 : 2 * (ntiles - 1) + 1));
 
-    for (int64_t j = 0; j < ntiles; ++j) {
+    for (int j = 0; j < ntiles; ++j) {
       const int buf = int(j & 1);
       const float4 cv = carry_next, cm = carry_next_mid;
       if (j + 1 < ntiles) {                               // the next tile's two states, a tile ahead
-        const int64_t c = rev ? 2 * j + 2 : 2 * (ntiles - 2 - j);
+        const int c = c_lo + (rev ? 2 * j + 2 : 2 * (ntiles - 2 - j));
         carry_next = load_carry(rev ? c + 1 : c);
         carry_next_mid = load_carry(rev ? c : c + 1);
       }
@@ -229,7 +232,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
 #pragma unroll
         for (int wi = kHalf / kBWin - 1; wi >= 0; --wi) {
           // window sequence number: tiles in processing order, windows from the tile's end
-          const int64_t wseq = j * kWinsPerTile + (1 - half) * (kHalf / kBWin) + (kHalf / kBWin - 1 - wi);
+          const int wseq = j * kWinsPerTile + (1 - half) * (kHalf / kBWin) + (kHalf / kBWin - 1 - wi);
           const int wb = int(wseq & 1);
           // asked now, needed only before the first store of the window
           const bool slot_free = wseq < 2 || mbar_test(&win_empty[wb], int(((wseq - 2) >> 1) & 1));
@@ -281,20 +284,20 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       float* dA = p.dA + e * N + 4 * q;
       atomicAdd(dA + 0, dAacc[0].x); atomicAdd(dA + 1, dAacc[0].y);
       atomicAdd(dA + 2, dAacc[1].x); atomicAdd(dA + 3, dAacc[1].y);
-      if (p.g_out)
+      if (p.g_out && pc == (rev ? p.pieces - 1 : 0))       // the carry that leaves the scan's first timestep
         *reinterpret_cast<float4*>(p.g_out + (b * p.ED + e) * N + 4 * q) =
             make_float4(gc[0].x, gc[0].y, gc[1].x, gc[1].y);
     }
     return;
   }
-  auto stage_ptr = [&](int64_t j) { return smem_raw + S::kRaw + int(j % kStages) * S::kStageBytes; };
+  auto stage_ptr = [&](int j) { return smem_raw + S::kRaw + int(j % kStages) * S::kStageBytes; };
   // window wl (0..7, in processing order) of a tile covers timesteps win_t(wl) and win_t(wl) + 1
   auto win_t = [](int wl) { return (wl < 4 ? kHalf : 0) + 2 * (3 - (wl & 3)); };
 
   if (warp == 4) {
     // ================================================================== loader + converter
     const uint32_t stage_tx = uint32_t((has_z ? 4 : 3) * S::kActBytes + 2 * S::kBcBytes);
-    auto issue = [&](int64_t j) -> bool {                       // lane 0 only
+    auto issue = [&](int j) -> bool {                       // lane 0 only
       const int r = int(j % kStages);
       if (j >= kStages && !mbar_wait(&raw_free[r], int((j / kStages - 1) & 1))) return false;
       unsigned char* st = stage_ptr(j);
@@ -309,12 +312,12 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       return true;
     };
     if (lane == 0) {
-      for (int64_t j = 0; j < kAhead && j < ntiles; ++j)
+      for (int j = 0; j < kAhead && j < ntiles; ++j)
         if (!issue(j)) { fail(); return; }
     }
-    for (int64_t j = 0; j < ntiles; ++j) {
+    for (int j = 0; j < ntiles; ++j) {
       const int buf = int(j & 1);
-      const int rows_ok = int(min64(kBTile, p.L - tile_t0(j)));
+      const int rows_ok = min(kBTile, t_hi - tile_t0(j));
       if (j >= 2 && !mbar_wait(&op_empty[buf], int(((j - 2) >> 1) & 1))) { fail(); return; }
       if (!mbar_wait(&raw_full[j % kStages], int((j / kStages) & 1))) { fail(); return; }
       const unsigned char* st = stage_ptr(j);
@@ -386,9 +389,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
     const int hf = lane >> 4, r = lane & 15;
     const int ti = r >> 3, which = (r >> 2) & 1, qq = r & 3;       // r = (ti * 2 + which) * 4 + qq
     float* gbase = (which ? p.dC : p.dB) + b * p.L * N + 4 * qq;
-    const int nt = int(ntiles);
-    for (int j = 0; j < nt; ++j) {
-      const int64_t t0 = tile_t0(j);
+    for (int j = 0; j < ntiles; ++j) {
+      const int t0 = tile_t0(j);
 #pragma unroll 1
       for (int wl = 0; wl < kWinsPerTile; ++wl) {
         const int wseq = j * kWinsPerTile + wl;
@@ -405,8 +407,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
           acc1 = __fadd2_rn(acc1, make_float2(v.z, v.w));
         }
         mbar_arrive(&win_empty[wb]);
-        const int64_t t = t0 + row(win_t(wl) + ti);
-        if (t < p.L) red_add_v4(gbase + t * N, acc0.x, acc0.y, acc1.x, acc1.y);
+        const int t = t0 + row(win_t(wl) + ti);
+        if (t < t_hi) red_add_v4(gbase + int64_t(t) * N, acc0.x, acc0.y, acc1.x, acc1.y);
       }
     }
     return;
@@ -421,8 +423,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
     T* odz = has_z ? static_cast<T*>(p.dz) + b * p.dz_sb + e0 + c0 : nullptr;
     const float Dv[2] = {s_D[c0], s_D[c0 + 1]};
     float dDacc[2] = {0.f, 0.f}, dbacc[2] = {0.f, 0.f};
-    for (int64_t j = 0; j < ntiles; ++j) {
-      const int64_t t0 = tile_t0(j);
+    for (int j = 0; j < ntiles; ++j) {
+      const int t0 = tile_t0(j);
       if (!mbar_wait(&raw_full[j % kStages], int((j / kStages) & 1))) { fail(); return; }
       const unsigned char* st = stage_ptr(j);
       const T* rx = reinterpret_cast<const T*>(st);
@@ -435,7 +437,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       const float* dyt = s_dyp + buf * kBTile * kBTE;
 #pragma unroll 1
       for (int wl = par; wl < kWinsPerTile; wl += 2) {
-        const int64_t wseq = j * kWinsPerTile + wl;
+        const int wseq = j * kWinsPerTile + wl;
         if (!mbar_wait(&win_full[par], int((wseq >> 1) & 1))) { fail(); return; }
         const float4* np = reinterpret_cast<const float4*>(s_np + (par * kBWin + ti) * 3 * 128);
         float ys[2], gBs[2], wAs[2];
@@ -449,8 +451,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         }
         mbar_arrive(&win_empty[par]);
         const int tt = row(win_t(wl) + ti);              // row inside the tile
-        const int64_t t = t0 + tt;
-        if (t < p.L && c0 < cols_ok) {
+        const int t = t0 + tt;
+        if (t < t_hi && c0 < cols_ok) {
           const Vec2<T> xv = *reinterpret_cast<const Vec2<T>*>(rx + tt * kBTE + c0);
           const float4 o4 = *reinterpret_cast<const float4*>(opt + op_index(tt, c0, kBTE));   // {delta, delta*x} x 2
           const float2 dyg2 = *reinterpret_cast<const float2*>(dyt + tt * kBTE + c0);
@@ -535,7 +537,7 @@ int bwd_tma_launch(const SscanBwdParams& p, cudaStream_t st) {
 #undef MB200_BWD_PICK
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes) != cudaSuccess)
     return MB200_ELAUNCH;
-  dim3 grid(unsigned((p.ED + kBTE - 1) / kBTE), unsigned(p.B));
+  dim3 grid(unsigned((p.ED + kBTE - 1) / kBTE), unsigned(p.B), unsigned(p.pieces));
   k<<<grid, kBwdThreads, S::kBytes, st>>>(m, p);
   return check_launch();
 }
@@ -567,7 +569,7 @@ int mb200_bwd_device_status() {
   return v;
 }
 
-extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, const float* A,
+extern "C" int mb200_sscan_bwd_pieces(const void* x, const void* delta, const void* z, const float* A,
                                const void* Bm, const void* Cm, const float* D,
                                const float* delta_bias, const void* dy, const float* carries,
                                const float* g_in, void* dx, void* ddelta, void* dz, float* dB,
@@ -577,7 +579,8 @@ extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, 
                                int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
                                int64_t c_sb, int64_t c_sl, int64_t dy_sb, int64_t dy_sl,
                                int64_t dx_sb, int64_t dx_sl, int64_t dd_sb, int64_t dd_sl,
-                               int64_t dz_sb, int64_t dz_sl, int dtype, int flags, void* stream) {
+                               int64_t dz_sb, int64_t dz_sl, int dtype, int flags, int64_t pieces, int64_t piece_len,
+                               void* stream) {
   if (B < 0 || L < 0 || ED < 0) return MB200_EINVAL;
   if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
   if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
@@ -594,7 +597,8 @@ extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, 
     return MB200_EINVAL;
   if (z && !dz) return MB200_EINVAL;
   if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
-  if (B > 65535) return MB200_ETOOBIG;
+  if (B > 65535 || pieces > 65535) return MB200_ETOOBIG;
+  if (!pieces_ok(pieces, piece_len, L)) return MB200_EINVAL;
   if (!aligned16(carries) || !aligned16(g_in) || !aligned16(g_out)) return MB200_EALIGN;
   SscanBwdParams p;
   p.x = x; p.delta = delta; p.z = z; p.Bm = Bm; p.Cm = Cm; p.dy = dy; p.A = A; p.D = D;
@@ -606,10 +610,20 @@ extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, 
   p.b_sb = b_sb; p.b_sl = b_sl; p.c_sb = c_sb; p.c_sl = c_sl; p.dy_sb = dy_sb; p.dy_sl = dy_sl;
   p.dx_sb = dx_sb; p.dx_sl = dx_sl; p.dd_sb = dd_sb; p.dd_sl = dd_sl; p.dz_sb = dz_sb; p.dz_sl = dz_sl;
   p.flags = flags;
+  if (pieces > 1) { p.pieces = pieces; p.piece_len = piece_len; }
   const int es = dtype == MB200_F32 ? 4 : 2;
   if (bwd_tma_path_ok(p, N, es)) {
     const int rc = dtype == MB200_F32 ? bwd_tma_launch<float>(p, st) : bwd_tma_launch<__nv_bfloat16>(p, st);
     if (rc <= 0) return rc;
+  }
+  if (pieces > 1) {                                // as extra batch rows, where the strides allow it
+    if (g_out || !pieces_as_rows(B, L, pieces, piece_len, {x_sb, d_sb, z ? z_sb : L * z_sl, b_sb, c_sb, dy_sb, dx_sb, dd_sb, z ? dz_sb : L * dz_sl},
+                                 {x_sl, d_sl, z_sl, b_sl, c_sl, dy_sl, dx_sl, dd_sl, dz_sl}))
+      return MB200_EUNSUPPORTED;
+    const int64_t n = piece_len;
+    return mb200_sscan_bwd(x, delta, z, A, Bm, Cm, D, delta_bias, dy, carries, g_in, dx, ddelta, dz, dB, dC, dA, dD, ddelta_bias, nullptr,
+                           B * pieces, n, ED, N, n * x_sl, x_sl, n * d_sl, d_sl, n * z_sl, z_sl, n * b_sl, b_sl, n * c_sl, c_sl, n * dy_sl,
+                           dy_sl, n * dx_sl, dx_sl, n * dd_sl, dd_sl, n * dz_sl, dz_sl, dtype, flags, stream);
   }
   if (flags & MB200_REVERSE) return MB200_EUNSUPPORTED;   // the reverse direction exists on the tensor-map path only
   const int kv = dtype == MB200_F32 ? 4 : 8;
@@ -621,4 +635,20 @@ extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, 
   if (z) vec = vec && z_sb % kv == 0 && z_sl % kv == 0 && dz_sb % kv == 0 && dz_sl % kv == 0;
   return dtype == MB200_F32 ? bwd_generic_launch_t<float>(p, N, vec, st)
                             : bwd_generic_launch_t<__nv_bfloat16>(p, N, vec, st);
+}
+
+extern "C" int mb200_sscan_bwd(const void* x, const void* delta, const void* z, const float* A,
+                               const void* Bm, const void* Cm, const float* D,
+                               const float* delta_bias, const void* dy, const float* carries,
+                               const float* g_in, void* dx, void* ddelta, void* dz, float* dB,
+                               float* dC, float* dA, float* dD, float* ddelta_bias, float* g_out,
+                               int64_t B, int64_t L, int64_t ED, int N,
+                               int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                               int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
+                               int64_t c_sb, int64_t c_sl, int64_t dy_sb, int64_t dy_sl,
+                               int64_t dx_sb, int64_t dx_sl, int64_t dd_sb, int64_t dd_sl,
+                               int64_t dz_sb, int64_t dz_sl, int dtype, int flags, void* stream) {
+  return mb200_sscan_bwd_pieces(x, delta, z, A, Bm, Cm, D, delta_bias, dy, carries, g_in, dx, ddelta, dz, dB, dC, dA, dD, ddelta_bias, g_out,
+                                B, L, ED, N, x_sb, x_sl, d_sb, d_sl, z_sb, z_sl, b_sb, b_sl, c_sb, c_sl, dy_sb, dy_sl, dx_sb, dx_sl,
+                                dd_sb, dd_sl, dz_sb, dz_sl, dtype, flags, 1, 0, stream);
 }

@@ -139,12 +139,12 @@ int launch_t(const CarryParams& p, int N, bool vec, cudaStream_t st) {
 
 using namespace mb200;
 
-extern "C" int mb200_sscan_bwd_carry(const void* delta, const void* z, const void* dy, const void* Cm,
+extern "C" int mb200_sscan_bwd_carry_pieces(const void* delta, const void* z, const void* dy, const void* Cm,
                                      const float* A, const float* delta_bias, float* g_out,
                                      int64_t B, int64_t L, int64_t ED, int N,
                                      int64_t d_sb, int64_t d_sl, int64_t z_sb, int64_t z_sl,
                                      int64_t dy_sb, int64_t dy_sl, int64_t c_sb, int64_t c_sl,
-                                     int dtype, int flags, void* stream) {
+                                     int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream) {
   if (B < 0 || L < 0 || ED < 0) return MB200_EINVAL;
   if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
   if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
@@ -157,7 +157,8 @@ extern "C" int mb200_sscan_bwd_carry(const void* delta, const void* z, const voi
   }
   if (!delta || !dy || !Cm || !A) return MB200_EINVAL;
   if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
-  if (B > 65535) return MB200_ETOOBIG;
+  if (B > 65535 || pieces > 65535) return MB200_ETOOBIG;
+  if (!pieces_ok(pieces, piece_len, L)) return MB200_EINVAL;
   if (!aligned16(g_out)) return MB200_EALIGN;
   CarryParams p;
   p.delta = delta; p.z = z; p.dy = dy; p.Cm = Cm; p.A = A; p.delta_bias = delta_bias; p.g_out = g_out;
@@ -173,12 +174,30 @@ extern "C" int mb200_sscan_bwd_carry(const void* delta, const void* z, const voi
     f.x_sb = dy_sb; f.x_sl = dy_sl; f.d_sb = d_sb; f.d_sl = d_sl; f.z_sb = z_sb; f.z_sl = z_sl;
     f.b_sb = c_sb; f.b_sl = c_sl; f.c_sb = c_sb; f.c_sl = c_sl; f.y_sb = 0; f.y_sl = 0;
     f.flags = (flags & MB200_DELTA_SOFTPLUS) | MB200_REVERSE | kFlagCarryPass;
+    if (pieces > 1) {                                        // nothing precedes the first piece: its carry is never used
+      f.pieces = pieces; f.piece_len = piece_len; f.launch_pieces = pieces - 1; f.piece0 = 1;
+    }
     const int rc = mb200_fwd_tma_try(f, N, dtype, st);
     if (rc <= 0) return rc;                                  // launched, or failed hard
+  }
+  if (pieces > 1) {
+    if (!pieces_as_rows(B, L, pieces, piece_len, {d_sb, z ? z_sb : L * z_sl, dy_sb, c_sb}, {d_sl, z_sl, dy_sl, c_sl})) return MB200_EUNSUPPORTED;
+    return mb200_sscan_bwd_carry(delta, z, dy, Cm, A, delta_bias, g_out, B * pieces, piece_len, ED, N, piece_len * d_sl, d_sl, piece_len * z_sl,
+                                 z_sl, piece_len * dy_sl, dy_sl, piece_len * c_sl, c_sl, dtype, flags, stream);
   }
   const int kv = dtype == MB200_F32 ? 4 : 8;
   bool vec = ED % kv == 0 && aligned16(delta) && aligned16(z) && aligned16(dy) && aligned16(Cm);
   for (int64_t s : {d_sb, d_sl, dy_sb, dy_sl, c_sb, c_sl}) vec = vec && s % kv == 0;
   if (z) vec = vec && z_sb % kv == 0 && z_sl % kv == 0;
   return dtype == MB200_F32 ? launch_t<float>(p, N, vec, st) : launch_t<__nv_bfloat16>(p, N, vec, st);
+}
+
+extern "C" int mb200_sscan_bwd_carry(const void* delta, const void* z, const void* dy, const void* Cm,
+                                     const float* A, const float* delta_bias, float* g_out,
+                                     int64_t B, int64_t L, int64_t ED, int N,
+                                     int64_t d_sb, int64_t d_sl, int64_t z_sb, int64_t z_sl,
+                                     int64_t dy_sb, int64_t dy_sl, int64_t c_sb, int64_t c_sl,
+                                     int dtype, int flags, void* stream) {
+  return mb200_sscan_bwd_carry_pieces(delta, z, dy, Cm, A, delta_bias, g_out, B, L, ED, N, d_sb, d_sl, z_sb, z_sl, dy_sb, dy_sl, c_sb, c_sl,
+                                      dtype, flags, 1, 0, stream);
 }

@@ -173,17 +173,19 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
   const int tid = threadIdx.x;
   const int64_t e0 = int64_t(blockIdx.x) * kTE;
   const int64_t b = blockIdx.y;
+  const int pc = int(blockIdx.z + p.piece0), t_lo = int(pc * p.piece_len), t_hi = int(min64(p.L, t_lo + p.piece_len));
+  const int64_t slot = b * p.pieces + pc;
   const int cols_ok = int(min64(kTE, p.ED - e0));
   const bool softplus = (p.flags & MB200_DELTA_SOFTPLUS) != 0;
   constexpr bool has_y = kHasY;
   const bool has_z = p.z != nullptr;
-  const int64_t ntiles = (p.L + kTile - 1) / kTile;
+  const int ntiles = (t_hi - t_lo + kTile - 1) / kTile;
   // Direction.  With MB200_REVERSE time is walked from L-1 down to 0: processing tile kt is the
   // tile of timesteps starting at tile_t0(kt), and processing step s of a tile is its row 15 - s.
   // Saved states are indexed by TIME chunk either way: entry c is the state entering chunk c in the
   // scan direction.
   constexpr bool rev = kRev;
-  auto tile_t0 = [&](int64_t kt) { return (rev ? ntiles - 1 - kt : kt) * kTile; };
+  auto tile_t0 = [&](int kt) { return t_lo + (rev ? ntiles - 1 - kt : kt) * kTile; };
 
   if (tid == 0) {
 #pragma unroll
@@ -219,7 +221,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         a4[j] = e_ok[i] ? p.A[e * N + 4 * q + j] * kLog2e : 0.f;
-        h4[j] = (e_ok[i] && p.h0) ? p.h0[(b * p.ED + e) * N + 4 * q + j] : 0.f;
+        h4[j] = (e_ok[i] && p.h0) ? p.h0[(slot * p.ED + e) * N + 4 * q + j] : 0.f;
       }
       A0[i] = e_ok[i] ? p.A[e * N] * kLog2e : 0.f;
       structured = structured && s4d_structured(a4, A0[i], q);
@@ -250,13 +252,13 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     for (int i = 0; i < kCPT; ++i) dsum[i] = dcomp[i] = 0.f;
     auto run_tiles = [&](auto struct_tag) {
       constexpr bool kStruct = decltype(struct_tag)::value;
-      for (int64_t kt = 0; kt < ntiles; ++kt) {
+      for (int kt = 0; kt < ntiles; ++kt) {
         const int buf = int(kt & 1);
         if (!mbar_wait(&op_full[buf], int((kt >> 1) & 1))) {
           atomicExch(&g_fwd_status, MB200_DEV_WAIT_TIMEOUT);
           return false;
         }
-        const int64_t t0a = tile_t0(kt);
+        const int t0a = tile_t0(kt);
         const float2* op = s_op + buf * kTile * kTE;
         const float* sB = s_B + buf * kTile * N + 4 * q;
         const float* sC = s_C + buf * kTile * N + 4 * q;
@@ -371,11 +373,12 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     };
     const bool ok = structured ? run_tiles(std::true_type{}) : run_tiles(std::false_type{});
     if (!ok) return;
-    if (p.hT) {
+    // the scan itself returns the state that leaves its last piece, the carry passes every piece's
+    if (p.hT && (!kHasY || pc == (rev ? 0 : p.pieces - 1))) {
 #pragma unroll
       for (int i = 0; i < kCPT; ++i)
         if (e_ok[i])
-          *reinterpret_cast<float4*>(p.hT + (b * p.ED + e0 + e_l + i) * N + 4 * q) =
+          *reinterpret_cast<float4*>(p.hT + ((kHasY ? b : slot) * p.ED + e0 + e_l + i) * N + 4 * q) =
               make_float4(hlo[i].x, hlo[i].y, hhi[i].x, hhi[i].y);
     }
     if constexpr (kWantP) {
@@ -383,7 +386,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
 #pragma unroll
         for (int i = 0; i < kCPT; ++i)
           if (e_ok[i])
-            *reinterpret_cast<float4*>(p.pT + (b * p.ED + e0 + e_l + i) * N + 4 * q) =
+            *reinterpret_cast<float4*>(p.pT + (slot * p.ED + e0 + e_l + i) * N + 4 * q) =
                 make_float4(ex2f(A2lo[i].x * dsum[i]), ex2f(A2lo[i].y * dsum[i]), ex2f(A2hi[i].x * dsum[i]),
                             ex2f(A2hi[i].y * dsum[i]));
       }
@@ -395,7 +398,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     // as it used to be, that made its warp the last one to hand every tile to the recurrence warps.
     if (tid != kNC + kNP) return;
     const uint32_t stage_tx = uint32_t((has_z ? 3 : 2) * S::kActBytes + 2 * S::kBcBytes);
-    for (int64_t kt = 0; kt < ntiles; ++kt) {
+    for (int kt = 0; kt < ntiles; ++kt) {
       const int r = int(kt % kStages);
       if (kt >= kStages && !mbar_wait(&raw_free[r], int((kt / kStages - 1) & 1))) {
         atomicExch(&g_fwd_status, MB200_DEV_WAIT_TIMEOUT);
@@ -417,13 +420,13 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     constexpr int kVecPerRow = kTE / 4;
     T* gy = has_y ? static_cast<T*>(p.y) + b * p.y_sb + e0 : nullptr;
 
-    auto stage_ptr = [&](int64_t kt) { return smem_raw + S::kRaw + int(kt % kStages) * S::kStageBytes; };
+    auto stage_ptr = [&](int kt) { return smem_raw + S::kRaw + int(kt % kStages) * S::kStageBytes; };
     auto fail = [&]() { atomicExch(&g_fwd_status, MB200_DEV_WAIT_TIMEOUT); };
 
     // raw tile kt -> float32 operands in buffer kt & 1
-    auto convert = [&](int64_t kt) {
+    auto convert = [&](int kt) {
       const int buf = int(kt & 1);
-      const int rows_ok = int(min64(kTile, p.L - tile_t0(kt)));
+      const int rows_ok = min(kTile, t_hi - tile_t0(kt));
       const unsigned char* st = stage_ptr(kt);
       const T* rx = reinterpret_cast<const T*>(st);
       const T* rd = reinterpret_cast<const T*>(st + S::kActBytes);
@@ -468,10 +471,10 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
       }
     };
     // finish tile kt: partial sums -> y (the consumers of tile kt have been waited for)
-    auto epilogue = [&](int64_t kt) {
+    auto epilogue = [&](int kt) {
       const int buf = int(kt & 1);
-      const int64_t t0 = tile_t0(kt);
-      const int rows_ok = int(min64(kTile, p.L - t0));
+      const int t0 = tile_t0(kt);
+      const int rows_ok = min(kTile, t_hi - t0);
       const unsigned char* st = stage_ptr(kt);
       const T* rx = reinterpret_cast<const T*>(st);
       const T* rz = reinterpret_cast<const T*>(st + 2 * S::kActBytes);
@@ -516,7 +519,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
           }
           out.v[k] = Elem<T>::from_f(yv);
         }
-        T* dst = gy + (t0 + rr) * p.y_sl + cc;
+        T* dst = gy + int64_t(t0 + rr) * p.y_sl + cc;
         if (cc + 4 <= cols_ok) {
           *reinterpret_cast<Vec4<T>*>(dst) = out;
         } else {
@@ -527,7 +530,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
       }
     };
 
-    for (int64_t kt = 0; kt < ntiles; ++kt) {
+    for (int kt = 0; kt < ntiles; ++kt) {
       if (kt >= 2) {
         if (!mbar_wait(&op_empty[kt & 1], int(((kt - 2) >> 1) & 1))) { fail(); return; }
         if (has_y) epilogue(kt - 2);
@@ -537,7 +540,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
       convert(kt);
       mbar_arrive(&op_full[kt & 1]);
     }
-    for (int64_t kt = ntiles >= 2 ? ntiles - 2 : 0; kt < ntiles; ++kt) {
+    for (int kt = ntiles >= 2 ? ntiles - 2 : 0; kt < ntiles; ++kt) {
       if (!mbar_wait(&op_empty[kt & 1], int((kt >> 1) & 1))) { fail(); return; }
       if (has_y) epilogue(kt);
     }
@@ -563,7 +566,7 @@ int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
                 : (hy ? sscan_fwd_tma_kernel<T, N, false, false, true> : sscan_fwd_tma_kernel<T, N, false, false, false>);
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes) != cudaSuccess)
     return MB200_ELAUNCH;
-  dim3 grid(unsigned((p.ED + G::kTE - 1) / G::kTE), unsigned(p.B));
+  dim3 grid(unsigned((p.ED + G::kTE - 1) / G::kTE), unsigned(p.B), unsigned(p.launch_pieces));
   k<<<grid, G::kThreads, S::kBytes, st>>>(m, p);
   return check_launch();
 }
@@ -616,14 +619,14 @@ int mb200_fwd_device_status() {
   return v;
 }
 
-extern "C" int mb200_sscan_fwd(const void* x, const void* delta, const void* z, const float* A,
+extern "C" int mb200_sscan_fwd_pieces(const void* x, const void* delta, const void* z, const float* A,
                                const void* Bm, const void* Cm, const float* D,
                                const float* delta_bias, const float* h0, void* y, float* hT,
                                float* carries, int64_t B, int64_t L, int64_t ED, int N,
                                int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
                                int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
                                int64_t c_sb, int64_t c_sl, int64_t y_sb, int64_t y_sl,
-                               int dtype, int flags, void* stream) {
+                               int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream) {
   if (B < 0 || L < 0 || ED < 0) return MB200_EINVAL;
   if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
   if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
@@ -638,7 +641,8 @@ extern "C" int mb200_sscan_fwd(const void* x, const void* delta, const void* z, 
   }
   if (!x || !delta || !A || !Bm || !Cm) return MB200_EINVAL;
   if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
-  if (B > 65535) return MB200_ETOOBIG;
+  if (B > 65535 || pieces > 65535) return MB200_ETOOBIG;
+  if (!pieces_ok(pieces, piece_len, L)) return MB200_EINVAL;
   if (!aligned16(h0) || !aligned16(hT) || !aligned16(carries)) return MB200_EALIGN;
   SscanFwdParams p;
   p.x = x; p.delta = delta; p.z = z; p.A = A; p.Bm = Bm; p.Cm = Cm; p.D = D;
@@ -647,11 +651,19 @@ extern "C" int mb200_sscan_fwd(const void* x, const void* delta, const void* z, 
   p.x_sb = x_sb; p.x_sl = x_sl; p.d_sb = d_sb; p.d_sl = d_sl; p.z_sb = z_sb; p.z_sl = z_sl;
   p.b_sb = b_sb; p.b_sl = b_sl; p.c_sb = c_sb; p.c_sl = c_sl; p.y_sb = y_sb; p.y_sl = y_sl;
   p.flags = flags;
+  if (pieces > 1) { p.pieces = p.launch_pieces = pieces; p.piece_len = piece_len; }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int es = dtype == MB200_F32 ? 4 : 2;
   if (tma_path_ok(p, N, es)) {
     const int rc = dtype == MB200_F32 ? tma_launch_t<float>(p, N, st) : tma_launch_t<__nv_bfloat16>(p, N, st);
     if (rc <= 0) return rc;                        // launched (0) or failed hard (< 0)
+  }
+  if (pieces > 1) {                                // as extra batch rows, where the strides allow it; hT is then every row's
+    if (hT || !pieces_as_rows(B, L, pieces, piece_len, {x_sb, d_sb, z ? z_sb : L * z_sl, b_sb, c_sb, y ? y_sb : L * y_sl}, {x_sl, d_sl, z_sl, b_sl, c_sl, y_sl}))
+      return MB200_EUNSUPPORTED;
+    return mb200_sscan_fwd(x, delta, z, A, Bm, Cm, D, delta_bias, h0, y, nullptr, carries, B * pieces, piece_len, ED, N, piece_len * x_sl, x_sl,
+                           piece_len * d_sl, d_sl, piece_len * z_sl, z_sl, piece_len * b_sl, b_sl, piece_len * c_sl, c_sl, piece_len * y_sl,
+                           y_sl, dtype, flags, stream);
   }
   if (flags & MB200_REVERSE) return MB200_EUNSUPPORTED;   // the reverse direction exists on the tensor-map path only
   const int kv = dtype == MB200_F32 ? 4 : 8;
@@ -663,13 +675,26 @@ extern "C" int mb200_sscan_fwd(const void* x, const void* delta, const void* z, 
                             : generic_launch_t<__nv_bfloat16>(p, N, vec, st);
 }
 
+extern "C" int mb200_sscan_fwd(const void* x, const void* delta, const void* z, const float* A,
+                               const void* Bm, const void* Cm, const float* D,
+                               const float* delta_bias, const float* h0, void* y, float* hT,
+                               float* carries, int64_t B, int64_t L, int64_t ED, int N,
+                               int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                               int64_t z_sb, int64_t z_sl, int64_t b_sb, int64_t b_sl,
+                               int64_t c_sb, int64_t c_sl, int64_t y_sb, int64_t y_sl,
+                               int dtype, int flags, void* stream) {
+  return mb200_sscan_fwd_pieces(x, delta, z, A, Bm, Cm, D, delta_bias, h0, y, hT, carries, B, L, ED, N, x_sb, x_sl, d_sb, d_sl, z_sb, z_sl,
+                                b_sb, b_sl, c_sb, c_sl, y_sb, y_sl, dtype, flags, 1, 0, stream);
+}
+
 // Forward carry pass of a split sequence: the state a span reaches from a zero state, and the span's decay
 // product, in one pass over x, delta, B (no y, no C, no saved states).
-extern "C" int mb200_sscan_fwd_carry(const void* x, const void* delta, const float* A, const void* Bm,
+extern "C" int mb200_sscan_fwd_carry_pieces(const void* x, const void* delta, const float* A, const void* Bm,
                                      const float* delta_bias, float* h_out, float* p_out,
                                      int64_t B, int64_t L, int64_t ED, int N,
                                      int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
-                                     int64_t b_sb, int64_t b_sl, int dtype, int flags, void* stream) {
+                                     int64_t b_sb, int64_t b_sl, int dtype, int flags, int64_t pieces, int64_t piece_len,
+                                     void* stream) {
   if (B < 0 || L < 0 || ED < 0) return MB200_EINVAL;
   if (dtype != MB200_F32 && dtype != MB200_BF16) return MB200_EDTYPE;
   if (N != 8 && N != 16 && N != 32 && N != 64) return MB200_ENSTATE;
@@ -677,6 +702,7 @@ extern "C" int mb200_sscan_fwd_carry(const void* x, const void* delta, const flo
   if (!h_out || !p_out || !A) return MB200_EINVAL;
   if ((flags & MB200_DELTA_SOFTPLUS) && !delta_bias) return MB200_EINVAL;
   if (flags & MB200_REVERSE) return MB200_EUNSUPPORTED;
+  if (!pieces_ok(pieces, piece_len, L) || B > 65535 || pieces > 65535) return MB200_EINVAL;
   if (!aligned16(h_out) || !aligned16(p_out)) return MB200_EALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (L > 0 && (!x || !delta || !Bm)) return MB200_EINVAL;
@@ -688,8 +714,16 @@ extern "C" int mb200_sscan_fwd_carry(const void* x, const void* delta, const flo
     p.x_sb = x_sb; p.x_sl = x_sl; p.d_sb = d_sb; p.d_sl = d_sl; p.z_sb = 0; p.z_sl = 0;
     p.b_sb = b_sb; p.b_sl = b_sl; p.c_sb = b_sb; p.c_sl = b_sl; p.y_sb = 0; p.y_sl = 0;
     p.flags = flags & (MB200_DELTA_SOFTPLUS | MB200_GENERAL_DECAY);
+    if (pieces > 1) {                              // nothing follows the last piece: its carry is never used
+      p.pieces = pieces; p.piece_len = piece_len; p.launch_pieces = pieces - 1;
+    }
     const int rc = mb200_fwd_tma_try(p, N, dtype, st);
     if (rc <= 0) return rc;                        // launched (0) or failed hard (< 0)
+    if (pieces > 1) {
+      if (!pieces_as_rows(B, L, pieces, piece_len, {x_sb, d_sb, b_sb}, {x_sl, d_sl, b_sl})) return MB200_EUNSUPPORTED;
+      return mb200_sscan_fwd_carry(x, delta, A, Bm, delta_bias, h_out, p_out, B * pieces, piece_len, ED, N, piece_len * x_sl, x_sl,
+                                   piece_len * d_sl, d_sl, piece_len * b_sl, b_sl, dtype, flags, stream);
+    }
   }
   // tensors the tensor-map path cannot take (or an empty span): the two pieces as separate launches
   int rc = mb200_sscan_fwd(x, delta, nullptr, A, Bm, Bm, nullptr, delta_bias, nullptr, nullptr, h_out, nullptr, B, L, ED,
@@ -698,4 +732,13 @@ extern "C" int mb200_sscan_fwd_carry(const void* x, const void* delta, const flo
   if (rc != MB200_OK) return rc;
   return mb200_decay_prod(delta, A, delta_bias, p_out, B, L, ED, N, d_sb, d_sl, dtype, flags & MB200_DELTA_SOFTPLUS,
                           stream);
+}
+
+extern "C" int mb200_sscan_fwd_carry(const void* x, const void* delta, const float* A, const void* Bm,
+                                     const float* delta_bias, float* h_out, float* p_out,
+                                     int64_t B, int64_t L, int64_t ED, int N,
+                                     int64_t x_sb, int64_t x_sl, int64_t d_sb, int64_t d_sl,
+                                     int64_t b_sb, int64_t b_sl, int dtype, int flags, void* stream) {
+  return mb200_sscan_fwd_carry_pieces(x, delta, A, Bm, delta_bias, h_out, p_out, B, L, ED, N, x_sb, x_sl, d_sb, d_sl, b_sb, b_sl, dtype, flags,
+                                      1, 0, stream);
 }

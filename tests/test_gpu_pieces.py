@@ -1,0 +1,75 @@
+"""Sequences cut into uneven pieces inside the kernels (tensor-map path): last pieces of one timestep, one tile, ragged tiles;
+ragged channel tiles; pieces that are not whole saved-state chunks of the row; against the float64 oracle."""
+import pytest
+import torch
+
+from tests.helpers import scan_inputs, assert_close
+from tests.test_gpu_sscan import RTOL, ATOL, BF_RTOL, BF_ATOL, _oracle
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("Bsz,L,ED,pieces", [(1, 33, 32, 3), (1, 129, 40, 3), (2, 200, 96, 5), (1, 257, 64, 2), (3, 100, 8, 4), (1, 500, 36, 7)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_uneven_pieces_vs_oracle(Bsz, L, ED, pieces, dtype, monkeypatch):
+    """The entry points with pieces, called as the host code calls them."""
+    import ctypes
+    from mamba_b200 import _lib
+    if dtype == torch.bfloat16 and ED % 8:
+        pytest.skip("no tensor map for this width")
+    lib = _lib.load()
+    inp = scan_inputs(L + ED, Bsz, L, ED, 16, dtype=dtype, structured_A=False, big_delta=True)
+    yo, ho, go = _oracle(inp)
+    t = {k: v.to(DEV).to(dtype if k in ("x", "delta", "B", "C", "z", "gy") else torch.float32).contiguous() for k, v in inp.items()}
+    n = -(-L // (16 * pieces)) * 16
+    assert (pieces - 1) * n < L
+    new = lambda *s, dt=torch.float32: torch.zeros(*s, dtype=dt, device=DEV)
+    code, st = _lib.dtype_code(dtype), torch.cuda.current_stream().cuda_stream
+    p = lambda v: None if v is None else v.data_ptr()
+    ss = lambda *vs: [k for v in vs for k in (v.stride(0), v.stride(1))]
+    P, S, h_in, G, g_in = (new(Bsz, pieces, ED, 16) for _ in range(5))
+    y, hT, car = new(Bsz, L, ED, dt=dtype), new(Bsz, ED, 16), new(Bsz, -(-L // 8), ED, 16)
+    i64, i32, vp = ctypes.c_int64, ctypes.c_int, ctypes.c_void_p
+
+    def call(name, ptrs, strides, N=16):
+        fn = getattr(lib, name)
+        fn.argtypes = [vp] * len(ptrs) + [i64] * 3 + [i32] + [i64] * len(strides) + [i32, i32, i64, i64, vp]
+        rc = fn(*map(p, ptrs), Bsz, L, ED, N, *strides, code, 0, pieces, n, st)
+        assert rc == 0, (name, lib.mb200_strerror(rc))
+
+    x, d, z, Bm, Cm, gy, A, D = (t[k] for k in ("x", "delta", "z", "B", "C", "gy", "A", "D"))
+    call("mb200_sscan_fwd_carry_pieces", [x, d, A, Bm, None, S, P], ss(x, d, Bm))
+    fold = lambda a, b, o, rev: lib.mb200_carry_fold_range(p(a), p(b), None, p(o), Bsz, pieces, ED * 16, 0, pieces, rev, st)
+    assert fold(P, S, h_in, 0) == 0
+    call("mb200_sscan_fwd_pieces", [x, d, z, A, Bm, Cm, D, None, h_in, y, hT, car], ss(x, d, z, Bm, Cm, y))
+    call("mb200_sscan_bwd_carry_pieces", [d, z, gy, Cm, A, None, G], ss(d, z, gy, Cm))
+    assert fold(P, G, g_in, 1) == 0
+    dx, dd, dz = (new(Bsz, L, ED, dt=dtype) for _ in range(3))
+    dB, dC, dA, dD, g_out = new(Bsz, L, 16), new(Bsz, L, 16), new(ED, 16), new(ED), new(Bsz, ED, 16)
+    call("mb200_sscan_bwd_pieces", [x, d, z, A, Bm, Cm, D, None, gy, car, g_in, dx, dd, dz, dB, dC, dA, dD, None, g_out],
+         ss(x, d, z, Bm, Cm, gy, dx, dd, dz))
+    rt, at = (RTOL, ATOL) if dtype == torch.float32 else (BF_RTOL, BF_ATOL)
+    assert_close(y, yo.float(), rt, at * max(1.0, yo.abs().max().item()), "y")
+    assert_close(hT, ho.float(), RTOL, ATOL * max(1.0, ho.abs().max().item()), "state")
+    for k, g in {"x": dx, "delta": dd, "z": dz, "B": dB, "C": dC, "A": dA, "D": dD}.items():
+        assert_close(g, go[k].float(), rt, at * 4 * max(1.0, go[k].abs().max().item()), "grad " + k)
+
+
+def test_library_chooses_pieces_and_handles_awkward_gradients():
+    """A short problem the library cuts by itself, with a gradient that is a narrow view, an incoming state and the outgoing one."""
+    import mamba_b200
+    inp = scan_inputs(5, 1, 777, 160, 16, structured_A=False, big_delta=True)
+    h0 = torch.randn(1, 160, 16, generator=torch.Generator().manual_seed(1))
+    yo, ho, go = _oracle(inp, h0=h0)
+    lv = {k: inp[k].to(DEV).requires_grad_() for k in ("x", "delta", "A", "B", "C", "D", "z")}
+    hl = h0.to(DEV).requires_grad_()
+    y, hT = mamba_b200.selective_scan_fn(lv["x"], lv["delta"], lv["A"], lv["B"], lv["C"], lv["D"], z=lv["z"], h0=hl, return_last_state=True)
+    wide = torch.zeros(1, 777, 165, device=DEV)
+    wide[..., 3:163] = inp["gy"].to(DEV)
+    y.backward(wide[..., 3:163])
+    assert_close(y, yo.float(), RTOL, ATOL * yo.abs().max().item(), "y")
+    assert_close(hT, ho.float(), RTOL, ATOL * max(1.0, ho.abs().max().item()), "state")
+    for k in ("x", "delta", "A", "B", "C", "D", "z"):
+        assert_close(lv[k].grad, go[k].float(), RTOL, ATOL * 4 * max(1.0, go[k].abs().max().item()), "grad " + k)
+    assert_close(hl.grad, go["h0"].float(), RTOL, ATOL * 4 * max(1.0, go["h0"].abs().max().item()), "grad h0")
