@@ -309,10 +309,11 @@ int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const float* rstd,
                           int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, int dtype_res,
                           int dtype_y, void* stream);
 
-/* Element-wise jobs, up to 12 in one launch.  Job: dst[r, c] = op(src[r, c]) for r < rows, c < cols, both with unit
+/* Element-wise jobs, up to 24 in one launch.  Job: dst[r, c] = op(src[r, c]) for r < rows, c < cols, both with unit
  * stride along c and their own row strides; columns src_cols .. cols-1 (all of them if src is NULL) count as zero.
- * MB200_CONVERT_NEG_EXP: dst = -exp(src).  MB200_CONVERT_MUL: dst = src * factor, factor dense float32 (rows, cols). */
-enum { MB200_CONVERT_COPY = 0, MB200_CONVERT_NEG_EXP = 1, MB200_CONVERT_MUL = 2 };
+ * MB200_CONVERT_NEG_EXP: dst = -exp(src).  MB200_CONVERT_MUL, _ADD: dst = src * factor, src + factor; factor is dense float32
+ * (rows, cols). */
+enum { MB200_CONVERT_COPY = 0, MB200_CONVERT_NEG_EXP = 1, MB200_CONVERT_MUL = 2, MB200_CONVERT_ADD = 3 };
 typedef struct {
   const void* src;
   void* dst;
@@ -363,6 +364,12 @@ int mb200_sscan_bwd_carry_pieces(const void* delta, const void* z, const void* d
                           int64_t d_sb, int64_t d_sl, int64_t z_sb, int64_t z_sl,
                           int64_t dy_sb, int64_t dy_sl, int64_t c_sb, int64_t c_sl,
                           int dtype, int flags, int64_t pieces, int64_t piece_len, void* stream);
+
+/* mb200_add_rmsnorm_bwd that also writes ds rounded to bfloat16, dense (rows, D): the gradient of a bfloat16 x beside that of a
+ * float32 stream (MB200_EUNSUPPORTED on rows off the vector grid or wider than 8192). */
+int mb200_add_rmsnorm_bwd_both(const void* s, const float* weight, const float* rstd, const void* dy, const void* dres, void* ds,
+                               void* ds_bf16, float* dweight, int64_t rows, int64_t D, int64_t s_rs, int64_t dy_rs, int64_t dr_rs,
+                               int64_t ds_rs, int dtype_res, int dtype_y, void* stream);
 
 /* mb200_rmsnorm_fwd with a weight of either type (MB200_EUNSUPPORTED for a bfloat16 weight on rows off the vector grid or wider
  * than 8192). */

@@ -9,10 +9,13 @@ namespace {
 
 constexpr int kConvertThreads = 256;
 constexpr int kPerThread = 4;
-constexpr int kMaxJobs = 12;
+constexpr int kMaxJobs = 24;
 
+struct Job : mb200_convert_job {
+  bool vec;
+};
 struct Jobs {
-  mb200_convert_job job[kMaxJobs];
+  Job job[kMaxJobs];
   int first_block[kMaxJobs + 1];             // blocks first_block[i] .. first_block[i + 1] - 1 work on job i
   int n;
 };
@@ -24,9 +27,39 @@ __device__ __forceinline__ float load_as_float(const void* p, int dtype, int64_t
 __global__ void __launch_bounds__(kConvertThreads) convert_kernel(const __grid_constant__ Jobs jobs) {
   int k = 0;
   while (k + 1 < jobs.n && int(blockIdx.x) >= jobs.first_block[k + 1]) ++k;
-  const mb200_convert_job& j = jobs.job[k];
+  const Job& j = jobs.job[k];
   const int64_t total = j.rows * j.cols;
   const int64_t base = int64_t(int(blockIdx.x) - jobs.first_block[k]) * kConvertThreads * kPerThread + threadIdx.x;
+  // one long row on the vector grid: four neighbouring elements a thread
+  if (j.rows == 1 && j.vec) {
+    const int64_t i = (int64_t(int(blockIdx.x) - jobs.first_block[k]) * kConvertThreads + threadIdx.x) * 4;
+    if (i >= total) return;
+    alignas(16) float f[4];
+    if (j.src_dtype == MB200_F32) {
+      *reinterpret_cast<float4*>(f) = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(j.src) + i));
+    } else {
+      const uint2 w = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(j.src) + i));
+      f[0] = __uint_as_float(w.x << 16); f[1] = __uint_as_float(w.x & 0xffff0000u);
+      f[2] = __uint_as_float(w.y << 16); f[3] = __uint_as_float(w.y & 0xffff0000u);
+    }
+    if (j.op == MB200_CONVERT_NEG_EXP) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) f[u] = -expf(f[u]);
+    } else if (j.op != MB200_CONVERT_COPY) {
+      const float4 g = __ldg(reinterpret_cast<const float4*>(j.factor + i));
+      const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) f[u] = j.op == MB200_CONVERT_MUL ? f[u] * gv[u] : f[u] + gv[u];
+    }
+    if (j.dst_dtype == MB200_F32) {
+      *reinterpret_cast<float4*>(static_cast<float*>(j.dst) + i) = make_float4(f[0], f[1], f[2], f[3]);
+    } else {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+      *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(j.dst) + i) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+    return;
+  }
   const bool small = total < (int64_t(1) << 31);               // 32-bit division is several times cheaper
   auto row_col = [&](int64_t i, int64_t& r, int64_t& c) {
     if (j.rows == 1) { r = 0; c = i; }
@@ -44,6 +77,7 @@ __global__ void __launch_bounds__(kConvertThreads) convert_kernel(const __grid_c
     if (j.src && c < j.src_cols) v[u] = load_as_float(j.src, j.src_dtype, r * j.src_stride + c);
     if (j.op == MB200_CONVERT_NEG_EXP) v[u] = -expf(v[u]);
     if (j.op == MB200_CONVERT_MUL) v[u] *= j.factor[i];
+    if (j.op == MB200_CONVERT_ADD) v[u] += j.factor[i];
   }
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {
@@ -73,8 +107,9 @@ extern "C" int mb200_convert(const mb200_convert_job* jobs, int n, void* stream)
     if ((j.src && j.src_dtype != MB200_F32 && j.src_dtype != MB200_BF16) || (j.dst_dtype != MB200_F32 && j.dst_dtype != MB200_BF16))
       return MB200_EDTYPE;
     if (j.rows == 0 || j.cols == 0) continue;
-    if (!j.dst || (j.op == MB200_CONVERT_MUL && !j.factor)) return MB200_EINVAL;
-    all.job[all.n] = j;
+    if (!j.dst || ((j.op == MB200_CONVERT_MUL || j.op == MB200_CONVERT_ADD) && !j.factor)) return MB200_EINVAL;
+    static_cast<mb200_convert_job&>(all.job[all.n]) = j;
+    all.job[all.n].vec = j.rows == 1 && j.cols % 4 == 0 && j.src && j.src_cols == j.cols && aligned16(j.src) && aligned16(j.dst) && aligned16(j.factor);
     all.first_block[all.n++] = int(blocks);
     blocks += (j.rows * j.cols + kConvertThreads * kPerThread - 1) / (kConvertThreads * kPerThread);
     if (blocks > (int64_t(1) << 30)) return MB200_ETOOBIG;

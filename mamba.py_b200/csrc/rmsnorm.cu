@@ -309,11 +309,13 @@ norm_rows_fwd_kernel(const TX* __restrict__ x, const TR* __restrict__ res_in, co
   }
 }
 
-// ds = (g - shat * mean(g * shat)) * rstd (+ dres), g = dy * w, shat = s * rstd;  dw = sum over rows of dy * shat.
+// ds = (g - shat * mean(g * shat)) * rstd (+ dres), g = dy * w, shat = s * rstd;  dw = sum over rows of dy * shat.  ds_bf16, when
+// given, is ds once more, dense and rounded: the gradient of a bfloat16 mixer output beside that of the float32 stream.
 template <typename TR, typename TY, int kTPR, int kC>
 __global__ void __launch_bounds__(kNormThreads)
 norm_rows_bwd_kernel(const TR* __restrict__ s, const float* __restrict__ w, const float* __restrict__ rstd,
-                     const TY* __restrict__ dy, const TR* __restrict__ dres, TR* __restrict__ ds, float* __restrict__ dw,
+                     const TY* __restrict__ dy, const TR* __restrict__ dres, TR* __restrict__ ds,
+                     __nv_bfloat16* __restrict__ ds_bf16, float* __restrict__ dw,
                      int64_t rows, int64_t D, int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs) {
   constexpr int kRows = kNormThreads / kTPR;
   __shared__ float s_part[kNormWarps];
@@ -369,6 +371,7 @@ norm_rows_bwd_kernel(const TR* __restrict__ s, const float* __restrict__ w, cons
 #pragma unroll
       for (int i = 0; i < 4; ++i) o[i] = (gv[c][i] - sv[c][i] * m) * rs + (dres ? rv[c][i] : 0.f);
       store_vec<TR, 4>(ds + r * ds_rs + d, o);
+      if (ds_bf16) store_vec<__nv_bfloat16, 4>(ds_bf16 + r * D + d, o);
     }
   }
   if (!dw) return;
@@ -429,14 +432,14 @@ bool rows_fwd(const void* x, const void* res_in, NormWeight w, void* res_out, vo
   });
 }
 template <typename TR, typename TY>
-bool rows_bwd(const void* s, const float* w, const float* rstd, const void* dy, const void* dres, void* ds, float* dw, int64_t rows, int64_t D,
+bool rows_bwd(const void* s, const float* w, const float* rstd, const void* dy, const void* dres, void* ds, void* ds_bf16, float* dw, int64_t rows, int64_t D,
               int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, cudaStream_t st) {
   return with_row_layout(D, [&]<int kTPR, int kC>(RowLayout<kTPR, kC>) {
     constexpr int kRows = kNormThreads / kTPR;
     // 3 CTAs per SM keep enough rows in flight; more would only add dweight atomics
     const int64_t want = (rows + kRows - 1) / kRows, cap = int64_t(sm_count()) * 3;
     norm_rows_bwd_kernel<TR, TY, kTPR, kC><<<unsigned(want < cap ? want : cap), kNormThreads, 0, st>>>(
-        (const TR*)s, w, rstd, (const TY*)dy, (const TR*)dres, (TR*)ds, dw, rows, D, s_rs, dy_rs, dr_rs, ds_rs);
+        (const TR*)s, w, rstd, (const TY*)dy, (const TR*)dres, (TR*)ds, (__nv_bfloat16*)ds_bf16, dw, rows, D, s_rs, dy_rs, dr_rs, ds_rs);
   });
 }
 
@@ -511,8 +514,8 @@ extern "C" int mb200_rmsnorm_bwd(const void* x, const float* weight, const float
   const int es = dtype == MB200_F32 ? 4 : 2;
   if (rows_vec(D, {x, dy, (const void*)dx, weight}, {x_rs, dy_rs, dx_rs})) {
     using bf = __nv_bfloat16;
-    if (dtype == MB200_F32 ? rows_bwd<float, float>(x, weight, rstd, dy, nullptr, dx, dweight, rows, D, x_rs, dy_rs, 0, dx_rs, st)
-                           : rows_bwd<bf, bf>(x, weight, rstd, dy, nullptr, dx, dweight, rows, D, x_rs, dy_rs, 0, dx_rs, st))
+    if (dtype == MB200_F32 ? rows_bwd<float, float>(x, weight, rstd, dy, nullptr, dx, nullptr, dweight, rows, D, x_rs, dy_rs, 0, dx_rs, st)
+                           : rows_bwd<bf, bf>(x, weight, rstd, dy, nullptr, dx, nullptr, dweight, rows, D, x_rs, dy_rs, 0, dx_rs, st))
       return check_launch();
   }
   const int v = norm_vec(D, es, {x, dy, (const void*)dx}, {x_rs, dy_rs, dx_rs});
@@ -581,11 +584,12 @@ extern "C" int mb200_add_rmsnorm_fwd(const void* x, const void* res_in, const fl
 
 template <typename TR, typename TY>
 static int add_norm_bwd_launch(const void* s, const float* weight, const float* rstd, const void* dy, const void* dres,
-                               void* ds, float* dweight, int64_t rows, int64_t D, int64_t s_rs, int64_t dy_rs,
+                               void* ds, void* ds_bf16, float* dweight, int64_t rows, int64_t D, int64_t s_rs, int64_t dy_rs,
                                int64_t dr_rs, int64_t ds_rs, bool vec, cudaStream_t st) {
   if (vec && aligned16(weight) &&
-      rows_bwd<TR, TY>(s, weight, rstd, dy, dres, ds, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, st))
+      rows_bwd<TR, TY>(s, weight, rstd, dy, dres, ds, ds_bf16, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, st))
     return check_launch();
+  if (ds_bf16) return MB200_EUNSUPPORTED;
   const int grid = norm_grid(rows);
   const size_t smem = dweight ? size_t(D) * sizeof(float) : 0;
 #define MB200_GO(VV, ACC)                                                                                         \
@@ -597,8 +601,8 @@ static int add_norm_bwd_launch(const void* s, const float* weight, const float* 
   return check_launch();
 }
 
-extern "C" int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const float* rstd, const void* dy,
-                                     const void* dres, void* ds, float* dweight, int64_t rows, int64_t D,
+extern "C" int mb200_add_rmsnorm_bwd_both(const void* s, const float* weight, const float* rstd, const void* dy,
+                                     const void* dres, void* ds, void* ds_bf16, float* dweight, int64_t rows, int64_t D,
                                      int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, int dtype_res,
                                      int dtype_y, void* stream) {
   if (rows < 0 || D < 0) return MB200_EINVAL;
@@ -609,13 +613,21 @@ extern "C" int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const f
   if (dweight && D > 12288) return MB200_ETOOBIG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   bool vec = D % 4 == 0;
-  for (const void* q : {s, dy, dres, (const void*)ds}) vec = vec && aligned16(q);
+  for (const void* q : {s, dy, dres, (const void*)ds, (const void*)ds_bf16}) vec = vec && aligned16(q);
   for (int64_t sd : {s_rs, dy_rs, dr_rs, ds_rs}) vec = vec && sd % 8 == 0;
   if (dtype_res == MB200_F32 && dtype_y == MB200_F32)
-    return add_norm_bwd_launch<float, float>(s, weight, rstd, dy, dres, ds, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
+    return add_norm_bwd_launch<float, float>(s, weight, rstd, dy, dres, ds, ds_bf16, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
   if (dtype_res == MB200_F32 && dtype_y == MB200_BF16)
-    return add_norm_bwd_launch<float, __nv_bfloat16>(s, weight, rstd, dy, dres, ds, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
+    return add_norm_bwd_launch<float, __nv_bfloat16>(s, weight, rstd, dy, dres, ds, ds_bf16, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
   if (dtype_res == MB200_BF16 && dtype_y == MB200_BF16)
-    return add_norm_bwd_launch<__nv_bfloat16, __nv_bfloat16>(s, weight, rstd, dy, dres, ds, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
+    return add_norm_bwd_launch<__nv_bfloat16, __nv_bfloat16>(s, weight, rstd, dy, dres, ds, ds_bf16, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, vec, st);
   return MB200_EUNSUPPORTED;
+}
+
+extern "C" int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const float* rstd, const void* dy,
+                                     const void* dres, void* ds, float* dweight, int64_t rows, int64_t D,
+                                     int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, int dtype_res,
+                                     int dtype_y, void* stream) {
+  return mb200_add_rmsnorm_bwd_both(s, weight, rstd, dy, dres, ds, nullptr, dweight, rows, D, s_rs, dy_rs, dr_rs, ds_rs, dtype_res, dtype_y,
+                                    stream);
 }
