@@ -10,6 +10,7 @@
 #include <ATen/core/grad_mode.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <optional>
 #include "mamba_b200.h"
@@ -67,7 +68,20 @@ inline Tensor like(const Tensor& grad, at::ScalarType dt) { return grad.scalar_t
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 inline int64_t st(const Tensor& t, int d) { return t.defined() ? t.stride(d) : 0; }
-inline Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& on) { return at::empty(shape, on.options().dtype(dt)); }
+// Straight to the caching allocator: the dispatcher's way to the same place costs three times as much.
+inline Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& on) {
+  return at::detail::empty_cuda(shape, dt, on.device(), std::nullopt);
+}
+// `shape` dense elements of `base`'s storage from element `offset` of it on (a plain alias, not an autograd view).
+inline Tensor alias(const Tensor& base, int64_t offset, at::IntArrayRef shape) {
+  Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(base.storage()), base.key_set(), base.dtype());
+  t.unsafeGetTensorImpl()->set_storage_offset(base.storage_offset() + offset);
+  t.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
+  return t;
+}
+inline void zero_fill(const Tensor& t) {
+  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), at::cuda::getCurrentCUDAStream()));
+}
 inline void* cuda_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // With MB200_CHECK_STATUS=1 in the environment every fused-scan launch is followed by a device synchronisation and a
@@ -98,6 +112,31 @@ struct Saved {
   void reset() { v.reset_data(); }
 };
 
+// Up to 24 element-wise jobs in one launch (mb200_convert).
+struct Convert {
+  mb200_convert_job jobs[24];
+  int n = 0;
+  mb200_convert_job& add(const void* src, at::ScalarType st, void* dst, at::ScalarType dt, int64_t rows, int64_t cols, int64_t src_cols,
+                         int64_t src_stride, int64_t dst_stride, int op = MB200_CONVERT_COPY) {
+    mb200_convert_job& j = jobs[n++];
+    j = mb200_convert_job{src, dst, nullptr, rows, cols, src_cols, src_stride, dst_stride, dtype_code(st), dtype_code(dt), op};
+    return j;
+  }
+  // a dense tensor once more in another type; itself when it has that type already
+  Tensor cast(const Tensor& src, at::ScalarType dt) {
+    if (!src.defined() || src.scalar_type() == dt) return src;
+    const Tensor dst = empty(src.sizes(), dt, src);
+    const int64_t m = src.numel();
+    add(ptr(src), src.scalar_type(), ptr(dst), dt, 1, m, m, m, m);
+    return dst;
+  }
+  void run() {
+    if (n) check(mb200_convert(jobs, n, cuda_stream()), "mb200_convert");
+    n = 0;
+  }
+};
+inline bool convertible(at::ScalarType d) { return d == at::kFloat || d == at::kBFloat16; }
+
 // What a node remembers of an input whose gradient it returns.
 inline at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() : at::kFloat; }
 
@@ -109,6 +148,7 @@ Tensor pscan(const Tensor& A, const Tensor& X);
 Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias);
 Tensor rms_norm(const Tensor& x, const OptTensor& weight, double eps);
 std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residual, const OptTensor& weight, double eps);
+Tensor add_residual(const Tensor& x, const Tensor& residual);
 std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const Tensor& delta, const Tensor& A, const Tensor& B,
                                     const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& delta_bias, bool inplace);
 std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace);

@@ -5,8 +5,6 @@
 namespace mb200_host {
 namespace {
 
-void zero_fill(const Tensor& t) { C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), at::cuda::getCurrentCUDAStream())); }
-
 Tensor filter(const Tensor& weight) { return f32(weight).view({weight.size(0), weight.size(-1)}); }
 
 struct ConvBackward : public torch::autograd::Node {
@@ -25,12 +23,12 @@ struct ConvBackward : public torch::autograd::Node {
     const int64_t B = xs.size(0), L = xs.size(1), W = xs.size(2), K = w32.size(1);
     const Tensor dx = empty({B, L, W}, xs.scalar_type(), xs), acc = empty({W * K + W}, at::kFloat, xs);
     zero_fill(acc);
-    const Tensor dw = acc.narrow(0, 0, W * K).view({W, K}), db = b32.defined() ? acc.narrow(0, W * K, W) : Tensor();
+    const Tensor dw = alias(acc, 0, w_shape), db = b32.defined() ? alias(acc, W * K, {W}) : Tensor();
     check(mb200_conv1d_silu_bwd(ptr(xs), fptr(w32), fptr(b32), ptr(dy), ptr(dx), fptr(dw), fptr(db), B, L, W, int(K), st(xs, 0), st(xs, 1),
                                 st(dy, 0), st(dy, 1), st(dx, 0), st(dx, 1), dtype_code(xs.scalar_type()), cuda_stream()),
           "mb200_conv1d_silu_bwd");
     out[0] = like(dx, tx);
-    out[1] = like(dw, tw).view(w_shape);
+    out[1] = like(dw, tw);
     if (db.defined()) out[2] = like(db, tb);
     return out;
   }
@@ -129,16 +127,28 @@ struct AddRmsNormBackward : public torch::autograd::Node {
         dw = empty({D}, at::kFloat, s2);
         zero_fill(dw);
       }
-      check(mb200_add_rmsnorm_bwd(ptr(s2), fptr(w32), fptr(rs), ptr(dy), ptr(dr), ptr(ds), fptr(dw), n, D, st(s2, 0), st(dy, 0), st(dr, 0),
-                                  st(ds, 0), dtype_code(ts), dtype_code(ty), cuda_stream()),
-            "mb200_add_rmsnorm_bwd");
+      // a bfloat16 x beside a float32 stream: its gradient leaves the kernel rounded, without a cast of its own
+      Tensor dx;
+      int rc = MB200_EUNSUPPORTED;
+      if (ts == at::kFloat && tx == at::kBFloat16) {
+        dx = empty(shape, at::kBFloat16, s2);
+        rc = mb200_add_rmsnorm_bwd_both(ptr(s2), fptr(w32), fptr(rs), ptr(dy), ptr(dr), ptr(ds), ptr(dx), fptr(dw), n, D, st(s2, 0), st(dy, 0),
+                                        st(dr, 0), st(ds, 0), dtype_code(ts), dtype_code(ty), cuda_stream());
+      }
+      if (rc == MB200_EUNSUPPORTED) {
+        dx = Tensor();
+        rc = mb200_add_rmsnorm_bwd(ptr(s2), fptr(w32), fptr(rs), ptr(dy), ptr(dr), ptr(ds), fptr(dw), n, D, st(s2, 0), st(dy, 0), st(dr, 0),
+                                   st(ds, 0), dtype_code(ts), dtype_code(ty), cuda_stream());
+      }
+      check(rc, "mb200_add_rmsnorm_bwd");
+      out[0] = dx;
       if (dw.defined()) out[2] = like(dw, tw);
       ds = ds.view(shape);
     } else {
       ds = grads[1];                                                       // only the sum was used further on
       if (!ds.defined()) return out;
     }
-    out[0] = like(ds, tx);
+    if (!out[0].defined()) out[0] = like(ds, tx);
     if (has_residual) out[1] = like(ds, tr);
     return out;
   }
@@ -215,6 +225,50 @@ std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residu
     node->s.save(s, true); node->w.save(w32); node->rstd.save(rstd);
   }
   return {y, s};
+}
+
+// ---------------------------------------------------------------------------------------------- the last residual add
+namespace {
+
+struct AddResidualBackward : public torch::autograd::Node {
+  at::ScalarType tx;
+  std::string name() const override { return "AddResidualBackward"; }
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(2);
+    const BelowAutograd guard_ad;
+    const c10::cuda::CUDAGuard guard(grads[0].device());
+    Convert conv;
+    const Tensor g = grads[0].is_contiguous() ? grads[0] : grads[0].contiguous();
+    const Tensor dx = g.scalar_type() == at::kFloat ? conv.cast(g, tx) : like(g, tx);
+    conv.run();
+    return {dx, grads[0]};
+  }
+};
+
+}  // namespace
+
+// x + residual at the end of a stack: a bfloat16 mixer output on a float32 stream in one vectorised pass.
+Tensor add_residual(const Tensor& x, const Tensor& residual) {
+  const bool ours = x.is_cuda() && residual.is_cuda() && x.sizes() == residual.sizes() && x.is_contiguous() && residual.is_contiguous() &&
+                    x.scalar_type() == at::kBFloat16 && residual.scalar_type() == at::kFloat;
+  if (!ours) return at::add(x, residual);
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor s;
+  {
+    const BelowAutograd guard_ad;
+    s = empty(x.sizes(), at::kFloat, x);
+    const int64_t n = s.numel();
+    Convert conv;
+    conv.add(ptr(x), at::kBFloat16, ptr(s), at::kFloat, 1, n, n, n, n, MB200_CONVERT_ADD).factor = fptr(residual);
+    conv.run();
+  }
+  if (wants_grad(x, residual)) {
+    auto node = new_node<AddResidualBackward>();
+    node->set_next_edges(torch::autograd::collect_next_edges(x, residual));
+    node->tx = type_of(x);
+    torch::autograd::set_history(s, node);
+  }
+  return s;
 }
 
 }  // namespace mb200_host

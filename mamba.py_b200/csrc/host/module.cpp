@@ -16,6 +16,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("conv1d_silu", &conv1d_silu, NoGil());
   m.def("rms_norm", &rms_norm, NoGil());
   m.def("add_rms_norm", &add_rms_norm, NoGil());
+  m.def("add_residual", &add_residual, NoGil());
   m.def("ssm_step", &ssm_step, NoGil());
   m.def("conv_step", &conv_step, NoGil());
   m.def("inner", &inner, NoGil());

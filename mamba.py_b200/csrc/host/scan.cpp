@@ -51,7 +51,7 @@ bool split_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carri
   s.h0 = empty({B, S, W, N}, at::kFloat, a.x);
   check(mb200_carry_fold_range(P, St, fptr(a.h0), fptr(s.h0), B, S, W * N, 0, int(S), 0, cuda_stream()), "mb200_carry_fold_range");
   if (launch_forward(s, o, want_last, want_carries, S, len) == MB200_EUNSUPPORTED) return false;
-  o.P = PS.select(0, 0);
+  o.P = alias(PS, 0, {B, S, W, N});
   return true;
 }
 
@@ -66,13 +66,13 @@ ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& car
   // every buffer the kernel accumulates into comes out of ONE zero-filled allocation
   const int64_t nBC = B * L * N, nA = W * N;
   const Tensor acc = empty({2 * nBC + nA + 2 * W + extra}, at::kFloat, a.x);
-  C10_CUDA_CHECK(cudaMemsetAsync(acc.data_ptr(), 0, acc.nbytes(), at::cuda::getCurrentCUDAStream()));
-  g.dB = acc.narrow(0, 0, nBC).view({B, L, N});
-  g.dC = acc.narrow(0, nBC, nBC).view({B, L, N});
-  g.dA = acc.narrow(0, 2 * nBC, nA).view({W, N});
-  g.dD = acc.narrow(0, 2 * nBC + nA, W);
-  if (a.bias.defined()) g.dbias = acc.narrow(0, 2 * nBC + nA + W, W);
-  if (extra) g.extra = acc.narrow(0, 2 * nBC + nA + 2 * W, extra);
+  zero_fill(acc);
+  g.dB = alias(acc, 0, {B, L, N});
+  g.dC = alias(acc, nBC, {B, L, N});
+  g.dA = alias(acc, 2 * nBC, {W, N});
+  g.dD = alias(acc, 2 * nBC + nA, {W});
+  if (a.bias.defined()) g.dbias = alias(acc, 2 * nBC + nA + W, {W});
+  if (extra) g.extra = alias(acc, 2 * nBC + nA + 2 * W, {extra});
   if (want_g_out) g.g_out = empty({B, W, N}, at::kFloat, a.x);
   check(mb200_sscan_bwd_pieces(ptr(a.x), ptr(a.delta), ptr(a.z), fptr(a.A), ptr(a.B), ptr(a.C), fptr(a.D), fptr(a.bias), ptr(dy), fptr(carries),
                         fptr(g_in), ptr(g.dx), ptr(g.dd), ptr(g.dz), fptr(g.dB), fptr(g.dC), fptr(g.dA), fptr(g.dD), fptr(g.dbias),
@@ -175,8 +175,13 @@ struct ScanBackward : public torch::autograd::Node {
       for (Tensor* t : {&g.dx, &g.dd, &g.dz, &g.dB, &g.dC})
         if (t->defined()) *t = t->flip(1);
     Tensor all[kInputs] = {g.dx, g.dd, g.dA, g.dB, g.dC, g.dD, g.dz, g.dbias, g.g_out};
-    for (int i = 0; i < kInputs; ++i)
-      if (given[i] && all[i].defined() && task_should_compute_output(i)) out[i] = like(all[i], types[i]);
+    Convert conv;                                                      // casts to the inputs' types, all in one launch
+    for (int i = 0; i < kInputs; ++i) {
+      if (!given[i] || !all[i].defined() || !task_should_compute_output(i)) continue;
+      const bool ours = all[i].is_contiguous() && convertible(types[i]) && convertible(all[i].scalar_type());
+      out[i] = ours ? conv.cast(all[i], types[i]) : like(all[i], types[i]);
+    }
+    conv.run();
     return out;
   }
 };

@@ -102,13 +102,13 @@ def add_rms_norm(x, residual=None, weight=None, eps=1e-5):
 def stack_forward(self, x):
     """Drop-in for Mamba.forward (mambapy/mamba.py:77-85): the loop over ResidualBlocks
     (`x = mixer(norm(x)) + x`, mambapy/mamba.py:106-112) with each layer's residual add fused into the
-    next layer's RMSNorm; the last add stays an ordinary add."""
+    next layer's RMSNorm; the last add is an ordinary add."""
     h, res = x, None
     for layer in self.layers:
         norm = layer.norm
         normed, res = add_rms_norm(h, res, None if getattr(norm, "use_mup", False) else norm.weight, norm.eps)
         h = layer.mixer(normed)
-    return h + res if res is not None else h
+    return _host().add_residual(h, res) if res is not None else h
 
 
 def rmsnorm_forward(self, x):
