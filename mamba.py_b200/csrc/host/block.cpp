@@ -1,38 +1,16 @@
-// The inside of a Mamba block as ONE autograd node.
+// A Mamba block -- projections, and one or both directions between them -- as ONE autograd node.
 //
 // Written as separate nodes, autograd glues a block's backward together with copies: a `cat` of the gradients of the two halves
 // of xz (the whole (B, L, 2 ED) tensor again), a `cat` for the split of the x_proj output, an add of the two gradients that
 // reach the conv output, casts of every parameter and of its gradient.  Here the backward writes dz and the conv's dx straight
 // into the two halves of d(xz), dB and dC straight into d(x_proj output), adds the second gradient of the conv output in the
-// epilogue of the GEMM that produces it, and prepares all parameters (and finishes all their gradients) in one launch.
+// epilogue of the GEMM that produces it, and prepares all parameters (and finishes all their gradients) in one launch.  For a
+// small model the launches and the host work around them are all that counts: 57 launches and 1660 us of host time for a
+// training step of two 64-wide layers with one node per operation.
 #include "scan.h"
 
 namespace mb200_host {
 namespace {
-
-// Up to 12 element-wise jobs in one launch (mb200_convert).
-struct Convert {
-  mb200_convert_job jobs[12];
-  int n = 0;
-  mb200_convert_job& add(const void* src, at::ScalarType st, void* dst, at::ScalarType dt, int64_t rows, int64_t cols, int64_t src_cols,
-                         int64_t src_stride, int64_t dst_stride, int op = MB200_CONVERT_COPY) {
-    mb200_convert_job& j = jobs[n++];
-    j = mb200_convert_job{src, dst, nullptr, rows, cols, src_cols, src_stride, dst_stride, dtype_code(st), dtype_code(dt), op};
-    return j;
-  }
-  // a dense copy of `src` in another type
-  Tensor cast(const Tensor& src, at::ScalarType dt) {
-    const Tensor dst = empty(src.sizes(), dt, src);
-    add(ptr(src), src.scalar_type(), ptr(dst), dt, 1, src.numel(), src.numel(), src.numel(), src.numel());
-    return dst;
-  }
-  void run() {
-    if (n) check(mb200_convert(jobs, n, cuda_stream()), "mb200_convert");
-    n = 0;
-  }
-};
-
-bool convertible(at::ScalarType d) { return d == at::kFloat || d == at::kBFloat16; }
 
 // The GEMMs below run in the type their operands have.
 using NoAutocast = c10::impl::ExcludeDispatchKeyGuard;
@@ -65,75 +43,220 @@ void conv_backward(const Tensor& x, const Tensor& w, const Tensor& b, const Tens
         "mb200_conv1d_silu_bwd");
 }
 
-enum { kXz, kConvW, kConvB, kXproj, kDtW, kDtB, kALog, kD, kParams };
+enum { kConvW, kConvB, kXproj, kDtW, kDtB, kALog, kD, kDirParams };
 
-struct InnerBackward : public torch::autograd::Node {
-  Saved xz, xc, dbc, delta, A, D, bias, carries, P, cw, cb, Wx, Wdt;
-  int64_t R = 0, Rp = 0, N = 0, S = 1;
+int64_t padded_rank(int64_t R, at::ScalarType dt) {
+  // dt_rank rounded up to a multiple of 16 bytes: the dt, B and C columns of the x_proj output and the K of the dt_proj GEMM
+  // then sit on the grid that TMA and the tensor-core GEMMs want; the extra weights are zero
+  const int64_t v = dt == at::kFloat ? 4 : 8;
+  return (R + v - 1) / v * v;
+}
+
+// One direction of a block between the projections (mambapy/mamba.py:214-231): conv1d + SiLU, x_proj, dt_proj and the fused
+// scan with softplus(delta + bias) and the gate inside.  With `reverse`, the second direction of the bidirectional block
+// (mambapy/vim.py:228-261): the convolution and the scan walk the sequence from its end, everything else is per timestep.
+struct Direction {
   bool reverse = false;
-  at::ScalarType types[kParams];
-  std::vector<int64_t> cw_shape;
+  int64_t S = 1;
+  Tensor xc, dbc, delta, carries, P;                        // what the forward leaves for the backward
+  Tensor A, D, bias, cw, cb, Wx, Wdt;                       // the parameters as the kernels take them
+  Tensor y;
 
-  std::string name() const override { return "MambaInnerBackward"; }
+  // Queues the parameters' conversions; run them before `forward`.
+  void prepare(Convert& conv, const Tensor* p, at::ScalarType dt, int64_t W, int64_t R, int64_t N) {
+    const int64_t Rp = padded_rank(R, dt), K = p[kConvW].size(-1);
+    const Tensor wx = param(p[kXproj]), wdt = param(p[kDtW]), alog = param(p[kALog]);
+    keep = {wx, wdt, alog};
+    A = empty({W, N}, at::kFloat, wx);
+    conv.add(ptr(alog), alog.scalar_type(), ptr(A), at::kFloat, 1, W * N, W * N, W * N, W * N, MB200_CONVERT_NEG_EXP);
+    if (Rp != R) {
+      Wx = empty({Rp + 2 * N, W}, dt, wx);
+      char* d = static_cast<char*>(ptr(Wx));
+      const int64_t es = Wx.element_size();
+      conv.add(ptr(wx), wx.scalar_type(), d, dt, 1, R * W, R * W, R * W, R * W);
+      conv.add(nullptr, dt, d + R * W * es, dt, 1, (Rp - R) * W, 0, 0, 0);
+      conv.add(static_cast<char*>(ptr(wx)) + R * W * wx.element_size(), wx.scalar_type(), d + Rp * W * es, dt, 1, 2 * N * W, 2 * N * W, 2 * N * W,
+               2 * N * W);
+      Wdt = empty({W, Rp}, dt, wx);
+      conv.add(ptr(wdt), wdt.scalar_type(), ptr(Wdt), dt, W, Rp, R, R, Rp);
+    } else {
+      Wx = conv.cast(wx, dt);
+      Wdt = conv.cast(wdt, dt);
+    }
+    auto f32_param = [&](const Tensor& t) {
+      if (!t.defined()) return Tensor();
+      keep.push_back(param(t));
+      return conv.cast(keep.back(), at::kFloat);
+    };
+    cw = f32_param(p[kConvW]).view({W, K});
+    cb = f32_param(p[kConvB]);
+    D = f32_param(p[kD]);
+    bias = f32_param(p[kDtB]);
+  }
+
+  void forward(const Tensor& xz, int64_t R, int64_t N, bool grad) {
+    const int64_t B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, xz.scalar_type()), cols = Rp + 2 * N;
+    keep.clear();
+    xc = empty({B, L, W}, xz.scalar_type(), xz);
+    conv_forward(xz.narrow(2, 0, W), cw, cb, xc, reverse);
+    const Tensor dbc2 = at::mm(alias(xc, 0, {T, W}), Wx.t());
+    delta = at::mm(dbc2.narrow(1, 0, Rp), Wdt.t()).view({B, L, W});         // bias and softplus happen in the kernel
+    dbc = dbc2.view({B, L, cols});
+    ScanArgs a{xc, delta, A, dbc.narrow(2, Rp, N), dbc.narrow(2, Rp + N, N), D, xz.narrow(2, W, W), bias, Tensor(), reverse};
+    S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
+    ScanOut o;
+    if (!scan_forward(a, S, false, grad, o)) {
+      TORCH_CHECK(!reverse, "mamba_b200: these tensors cannot be scanned in reverse");
+      S = 1;
+      scan_forward(a, 1, false, grad, o);
+    }
+    y = o.y;
+    carries = o.carries;
+    P = o.P;
+  }
+
+  // d(xz) of this direction into dxz (B, L, 2 W); the parameters' gradients into out[kDirParams], of types kt, by way of the jobs
+  // queued in `finish`, whose sources stay alive in `alive`.
+  void backward(const Tensor& xz, Tensor dy, const Tensor& dxz, int64_t R, int64_t N, const at::ScalarType* kt, const std::vector<int64_t>& cw_shape,
+                Tensor* out, Convert& finish, std::vector<Tensor>& alive) const {
+    const auto dt = xc.scalar_type();
+    const int64_t B = xc.size(0), L = xc.size(1), W = xc.size(2), T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N, K = cw.size(1);
+    if ((reverse || S > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
+    const ScanArgs a{xc, delta, A, dbc.narrow(2, Rp, N), dbc.narrow(2, Rp + N, N), D, xz.narrow(2, W, W), bias, Tensor(), reverse};
+    ScanGrads g = scan_backward(a, S, dy, carries, P, false, dxz.narrow(2, W, W), W * K + W);
+    const Tensor d_dbc = empty({T, cols}, dt, xz), dd2 = alias(g.dd, 0, {T, W}), xc2 = alias(xc, 0, {T, W}), dx2 = alias(g.dx, 0, {T, W});
+    auto col = [&](int64_t c) { return static_cast<char*>(d_dbc.data_ptr()) + c * d_dbc.element_size(); };
+    Convert acc;
+    acc.add(ptr(g.dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);          // float32 accumulators -> activation dtype, in place
+    acc.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
+    acc.run();
+    Tensor d_dt = d_dbc.narrow(1, 0, Rp);
+    at::mm_out(d_dt, dd2, Wdt);                                              // through dt_proj
+    const Tensor dWdt = at::mm(dd2.t(), alias(dbc, 0, {T, cols}).narrow(1, 0, Rp));      // (W, Rp)
+    const Tensor dWx = at::mm(d_dbc.t(), xc2);                               // (Rp + 2 N, W)
+    Tensor dxc = dx2;
+    at::addmm_out(dxc, dx2, d_dbc, Wx);                                      // + the gradient through x_proj, in the GEMM's epilogue
+    float *dcw = fptr(g.extra), *dcb = dcw + W * K;
+    conv_backward(xz.narrow(2, 0, W), cw, cb, alias(dxc, 0, {B, L, W}), dxz.narrow(2, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
+
+    auto dense = [&](int i, const Tensor& src, int64_t offset, at::IntArrayRef shape) {
+      if (kt[i] == at::kFloat) {
+        out[i] = alias(src, offset, shape);
+        return;
+      }
+      out[i] = empty(shape, kt[i], xz);
+      const int64_t n = out[i].numel();
+      finish.add(fptr(src) + offset, at::kFloat, ptr(out[i]), kt[i], 1, n, n, n, n);
+    };
+    dense(kConvW, g.extra, 0, cw_shape);
+    if (cb.defined()) dense(kConvB, g.extra, W * K, {W});
+    dense(kDtB, g.dbias, 0, {W});
+    dense(kD, g.dD, 0, {W});
+    out[kALog] = empty({W, N}, kt[kALog], xz);                               // d A_log = dA * A
+    finish.add(ptr(g.dA), at::kFloat, ptr(out[kALog]), kt[kALog], 1, W * N, W * N, W * N, W * N, MB200_CONVERT_MUL).factor = fptr(A);
+    if (Rp == R) {
+      out[kXproj] = finish.cast(dWx, kt[kXproj]);
+      out[kDtW] = finish.cast(dWdt, kt[kDtW]);
+    } else {
+      out[kXproj] = empty({R + 2 * N, W}, kt[kXproj], xz);
+      char* wx = static_cast<char*>(ptr(out[kXproj]));
+      finish.add(ptr(dWx), dt, wx, kt[kXproj], 1, R * W, R * W, R * W, R * W);
+      finish.add(static_cast<char*>(ptr(dWx)) + Rp * W * dWx.element_size(), dt, wx + R * W * out[kXproj].element_size(), kt[kXproj], 1,
+                 2 * N * W, 2 * N * W, 2 * N * W, 2 * N * W);
+      out[kDtW] = empty({W, R}, kt[kDtW], xz);
+      finish.add(ptr(dWdt), dt, ptr(out[kDtW]), kt[kDtW], W, R, R, Rp, R);
+    }
+    alive.insert(alive.end(), {dWx, dWdt, g.dA, g.extra});
+  }
+
+ private:
+  std::vector<Tensor> keep;                                 // sources of the queued conversions
+};
+
+enum { kX, kInW, kOutW, kBlockInputs };                     // then kDirParams per direction
+
+struct BlockBackward : public torch::autograd::Node {
+  struct SavedDirection {
+    Saved xc, dbc, delta, carries, P, A, D, bias, cw, cb, Wx, Wdt;
+    bool reverse;
+    int64_t S;
+    std::vector<int64_t> cw_shape;
+    template <typename F> void each(F f) {
+      for (Saved* s : {&xc, &dbc, &delta, &carries, &P, &A, &D, &bias, &cw, &cb, &Wx, &Wdt}) f(*s);
+    }
+    void save(const Direction& d) {
+      xc.save(d.xc); dbc.save(d.dbc); delta.save(d.delta); carries.save(d.carries); P.save(d.P); A.save(d.A); D.save(d.D); bias.save(d.bias);
+      cw.save(d.cw); cb.save(d.cb); Wx.save(d.Wx); Wdt.save(d.Wdt);
+      reverse = d.reverse; S = d.S;
+    }
+    Direction get() const {
+      Direction d;
+      d.reverse = reverse; d.S = S;
+      d.xc = xc.get(); d.dbc = dbc.get(); d.delta = delta.get(); d.carries = carries.get(); d.P = P.get(); d.A = A.get(); d.D = D.get();
+      d.bias = bias.get(); d.cw = cw.get(); d.cb = cb.get(); d.Wx = Wx.get(); d.Wdt = Wdt.get();
+      return d;
+    }
+  };
+  Saved x, in_w, out_w, xz, y;
+  std::vector<SavedDirection> dirs;
+  std::vector<at::ScalarType> types;
+  std::vector<int64_t> x_shape;
+  int64_t R = 0, N = 0;
+  double scale = 1.0;
+
+  std::string name() const override { return "MambaBlockBackward"; }
   void release_variables() override {
-    for (Saved* s : {&xz, &xc, &dbc, &delta, &A, &D, &bias, &carries, &P, &cw, &cb, &Wx, &Wdt}) s->reset();
+    for (Saved* s : {&x, &in_w, &out_w, &xz, &y}) s->reset();
+    for (auto& d : dirs) d.each([](Saved& s) { s.reset(); });
   }
   variable_list apply(variable_list&& grads) override {
-    variable_list out(kParams);
+    variable_list out(types.size());
     if (!grads[0].defined()) return out;
     const BelowAutograd guard_ad;
     const NoAutocast no_autocast(c10::DispatchKey::AutocastCUDA);
-    const Tensor xz_ = xz.get(), xc_ = xc.get(), dbc_ = dbc.get(), A_ = A.get(), Wx_ = Wx.get(), Wdt_ = Wdt.get(), cw_ = cw.get(),
-                 cb_ = cb.get();
+    const Tensor xz_ = xz.get();
     const c10::cuda::CUDAGuard guard(xz_.device());
-    const auto dt = xc_.scalar_type();
-    const int64_t B = xc_.size(0), L = xc_.size(1), W = xc_.size(2), T = B * L, cols = Rp + 2 * N, K = cw_.size(1);
+    const auto dt = xz_.scalar_type();
+    const int64_t B = xz_.size(0), L = xz_.size(1), W = xz_.size(2) / 2, T = B * L;
+    std::vector<at::ScalarType> kt;                                        // what the conversion writes; anything else is cast after it
+    for (auto t : types) kt.push_back(convertible(t) ? t : at::kFloat);
+    Convert finish;
+    std::vector<Tensor> alive;
     Tensor dy = rows(grads[0], dt);
-    if ((reverse || S > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
+    if (out_w.defined) {
+      const Tensor w = out_w.get(), s2 = alias(y.get(), 0, {T, W}), d2 = dy.reshape({T, w.size(0)});
+      Tensor ds = empty({T, W}, dt, xz_);
+      at::addmm_out(ds, ds, d2, w, 0, scale);
+      dy = alias(ds, 0, {B, L, W});
+      if (task_should_compute_output(kOutW)) {
+        Tensor dw = empty(w.sizes(), dt, xz_);
+        at::addmm_out(dw, dw, d2.t(), s2, 0, scale);
+        out[kOutW] = finish.cast(dw, kt[kOutW]);
+        alive.push_back(dw);
+      }
+    }
     const Tensor dxz = empty({B, L, 2 * W}, dt, xz_);
-    const ScanArgs a{xc_, delta.get(), A_, dbc_.narrow(2, Rp, N), dbc_.narrow(2, Rp + N, N), D.get(), xz_.narrow(2, W, W), bias.get(),
-                     Tensor(), reverse};
-    ScanGrads g = scan_backward(a, S, dy, carries.get(), P.get(), false, dxz.narrow(2, W, W), W * K + W);
-    Convert conv;
-    const Tensor d_dbc = empty({T, cols}, dt, xz_), dd2 = g.dd.view({T, W}), xc2 = xc_.view({T, W}), dx2 = g.dx.view({T, W});
-    const int64_t es = d_dbc.element_size();
-    auto col = [&](int64_t c) { return static_cast<char*>(d_dbc.data_ptr()) + c * es; };
-    conv.add(ptr(g.dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);         // float32 accumulators -> activation dtype, in place
-    conv.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
-    conv.run();
-    Tensor d_dt = d_dbc.narrow(1, 0, Rp);
-    at::mm_out(d_dt, dd2, Wdt_);                                            // through dt_proj
-    const Tensor dWdt = at::mm(dd2.t(), dbc_.view({T, cols}).narrow(1, 0, Rp));          // (W, Rp)
-    const Tensor dWx = at::mm(d_dbc.t(), xc2);                              // (Rp + 2 N, W)
-    Tensor dxc = dx2;
-    at::addmm_out(dxc, dx2, d_dbc, Wx_);                                    // + the gradient through x_proj, in the GEMM's epilogue
-    float* dcw = fptr(g.extra);
-    float* dcb = dcw + W * K;
-    conv_backward(xz_.narrow(2, 0, W), cw_, cb_, dxc.view({B, L, W}), dxz.narrow(2, 0, W), dcw, cb_.defined() ? dcb : nullptr, reverse);
-
-    out[kXz] = dxz;
-    at::ScalarType kt[kParams];                                            // what the conversion writes; anything else is cast after it
-    for (int i = 0; i < kParams; ++i) kt[i] = convertible(types[i]) ? types[i] : at::kFloat;
-    auto dense = [&](int i, const float* src, at::IntArrayRef shape) {
-      out[i] = empty(shape, kt[i], xz_);
-      const int64_t n = out[i].numel();
-      conv.add(src, at::kFloat, ptr(out[i]), kt[i], 1, n, n, n, n);
-    };
-    dense(kConvW, dcw, cw_shape);
-    if (cb_.defined()) dense(kConvB, dcb, {W});
-    dense(kDtB, fptr(g.dbias), {W});
-    dense(kD, fptr(g.dD), {W});
-    out[kALog] = empty({W, N}, kt[kALog], xz_);                             // d A_log = dA * A
-    conv.add(ptr(g.dA), at::kFloat, ptr(out[kALog]), kt[kALog], 1, W * N, W * N, W * N, W * N, MB200_CONVERT_MUL).factor = fptr(A_);
-    out[kXproj] = empty({R + 2 * N, W}, kt[kXproj], xz_);
-    char* wx = static_cast<char*>(ptr(out[kXproj]));
-    conv.add(ptr(dWx), dt, wx, kt[kXproj], R, W, W, W, W);
-    conv.add(static_cast<char*>(ptr(dWx)) + Rp * W * dWx.element_size(), dt, wx + R * W * out[kXproj].element_size(), kt[kXproj], 2 * N, W,
-             W, W, W);
-    out[kDtW] = empty({W, R}, kt[kDtW], xz_);
-    conv.add(ptr(dWdt), dt, ptr(out[kDtW]), kt[kDtW], W, R, R, Rp, R);
-    conv.run();
-    for (int i = kConvW; i < kParams; ++i)
+    for (size_t i = 0; i < dirs.size(); ++i) {
+      const Tensor d = i == 0 ? dxz : empty({B, L, 2 * W}, dt, xz_);
+      const int first = kBlockInputs + int(i) * kDirParams;
+      dirs[i].get().backward(xz_, dy, d, R, N, kt.data() + first, dirs[i].cw_shape, out.data() + first, finish, alive);
+      if (i > 0) dxz.add_(d);
+    }
+    if (in_w.defined) {
+      const Tensor w = in_w.get(), x2 = x.get(), d2 = alias(dxz, 0, {T, 2 * W});
+      if (task_should_compute_output(kInW)) {
+        alive.push_back(at::mm(d2.t(), x2));
+        out[kInW] = finish.cast(alive.back(), kt[kInW]);
+      }
+      if (task_should_compute_output(kX)) {
+        alive.push_back(alias(at::mm(d2, w), 0, x_shape));
+        out[kX] = finish.cast(alive.back(), kt[kX]);
+      }
+    } else {
+      out[kX] = dxz;
+    }
+    finish.run();
+    for (size_t i = 0; i < out.size(); ++i)
       if (out[i].defined()) out[i] = like(out[i], types[i]);
     return out;
   }
@@ -141,91 +264,83 @@ struct InnerBackward : public torch::autograd::Node {
 
 }  // namespace
 
-// Everything between in_proj and out_proj of MambaBlock.forward (mambapy/mamba.py:214-231): conv1d + SiLU, x_proj, dt_proj and the
-// fused scan with softplus(delta + bias) and the gate inside.  With `reverse`, the second direction of the bidirectional block
-// (mambapy/vim.py:228-261): the convolution and the scan walk the sequence from its end, everything else is per timestep.
-Tensor inner(const Tensor& xz, const Tensor& conv_w, const OptTensor& conv_b_, const Tensor& xproj_w, const Tensor& dt_w, const Tensor& dt_b,
-             const Tensor& A_log, const Tensor& D, int64_t R, int64_t N, bool reverse) {
-  const Tensor& conv_b = value(conv_b_);
-  require_cuda(xz, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D);
-  const c10::cuda::CUDAGuard guard(xz.device());
-  const bool grad = wants_grad(xz, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D);
-  const auto dt = act_dtype(xz);
-  ScanArgs a;
-  ScanOut o;
-  Tensor cw, cb, dbc, Wx, Wdt, xzs;
-  int64_t S = 1, Rp = 0;
+// x: the block's input (B, L, d_model), or with in_w undefined its xz (B, L, 2 W).  params: conv weight, conv bias, x_proj weight,
+// dt_proj weight and bias, A_log, D of one direction or of both.  Returns out_proj of the (summed, with `halve` averaged) scans, or
+// with out_w undefined the scan itself.
+Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, const std::vector<OptTensor>& params, int64_t R, int64_t N,
+             bool reverse, bool halve) {
+  const Tensor &in_w = value(in_w_), &out_w = value(out_w_);
+  TORCH_CHECK_VALUE(params.size() == kDirParams || params.size() == 2 * kDirParams, "a block has 7 parameters per direction");
+  std::vector<Tensor> in{x, in_w, out_w};
+  for (const auto& p : params) in.push_back(value(p));
+  bool grad = false;
+  for (const Tensor& t : in) {
+    require_cuda(t);
+    grad = grad || wants_grad(t);
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const size_t nd = params.size() / kDirParams;
+  std::vector<Direction> dirs(nd);
+  Tensor x2, wi, wo, xz, s, out;
+  const double scale = halve ? 0.5 : 1.0;
   {
+    const auto dt = in_w.defined() && at::autocast::is_autocast_enabled(at::kCUDA) ? at::autocast::get_autocast_dtype(at::kCUDA) : x.scalar_type();
+    TORCH_CHECK_TYPE(convertible(dt), "mamba_b200 kernels take float32 or bfloat16 activations, got ", dt);
     const BelowAutograd guard_ad;
     const NoAutocast no_autocast(c10::DispatchKey::AutocastCUDA);
-    xzs = rows(xz, dt);
-    const int64_t B = xzs.size(0), L = xzs.size(1), W = xzs.size(2) / 2, K = conv_w.size(-1), T = B * L;
-    // dt_rank rounded up to a multiple of 16 bytes: the dt, B and C columns of the x_proj output and the K of the dt_proj GEMM
-    // then sit on the grid that TMA and the tensor-core GEMMs want; the extra weights are zero
-    const int64_t v = 16 / xzs.element_size();
-    Rp = (R + v - 1) / v * v;
-    const int64_t cols = Rp + 2 * N;
+    const int64_t B = x.size(0), L = x.size(1), T = B * L, W = in[kBlockInputs + kDtW].size(0);
     Convert conv;
-    const Tensor wx = param(xproj_w), wdt = param(dt_w), alog = param(A_log);
-    a.A = empty({W, N}, at::kFloat, xzs);
-    conv.add(ptr(alog), alog.scalar_type(), ptr(a.A), at::kFloat, 1, W * N, W * N, W * N, W * N, MB200_CONVERT_NEG_EXP);
-    Wx = wx;
-    Wdt = wdt;
-    if (Rp != R || wx.scalar_type() != dt) {
-      Wx = empty({cols, W}, dt, xzs);
-      char* d = static_cast<char*>(ptr(Wx));
-      conv.add(ptr(wx), wx.scalar_type(), d, dt, R, W, W, W, W);
-      if (Rp != R) conv.add(nullptr, dt, d + R * W * Wx.element_size(), dt, Rp - R, W, 0, W, W);
-      conv.add(static_cast<char*>(ptr(wx)) + R * W * wx.element_size(), wx.scalar_type(), d + Rp * W * Wx.element_size(), dt, 2 * N, W, W, W, W);
+    const Tensor pi = param(in_w), po = param(out_w), px = rows(x, x.scalar_type());
+    Tensor xr;                                                               // stays alive until the conversions have been launched
+    if (pi.defined()) {
+      xr = px.reshape({T, px.size(2)});
+      x2 = xr.is_contiguous() && convertible(xr.scalar_type()) ? conv.cast(xr, dt) : xr.to(dt);
+      wi = conv.cast(pi, dt);
+    } else {
+      xz = rows(px, dt);
+      if ((nd > 1 || reverse) && !tensor_map_ok(xz)) xz = xz.contiguous();
     }
-    if (Rp != R || wdt.scalar_type() != dt) {
-      Wdt = empty({W, Rp}, dt, xzs);
-      conv.add(ptr(wdt), wdt.scalar_type(), ptr(Wdt), dt, W, Rp, R, R, Rp);
+    wo = conv.cast(po, dt);
+    for (size_t i = 0; i < nd; ++i) {
+      dirs[i].reverse = reverse || i == 1;
+      dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N);
     }
-    auto f32_param = [&](const Tensor& t) {
-      const Tensor p = param(t);
-      return (!p.defined() || p.scalar_type() == at::kFloat) ? p.detach() : conv.cast(p, at::kFloat);
-    };
-    cw = f32_param(conv_w).view({W, K});
-    cb = conv_b.defined() ? f32_param(conv_b) : Tensor();
-    a.D = f32_param(D);
-    a.bias = f32_param(dt_b);
     conv.run();
-    a.z = xzs.narrow(2, W, W);
-    a.x = empty({B, L, W}, dt, xzs);
-    conv_forward(xzs.narrow(2, 0, W), cw, cb, a.x, reverse);
-    const Tensor dbc2 = at::mm(a.x.view({T, W}), Wx.t());
-    a.delta = at::mm(dbc2.narrow(1, 0, Rp), Wdt.t()).view({B, L, W});       // bias and softplus happen in the kernel
-    dbc = dbc2.view({B, L, cols});
-    a.B = dbc.narrow(2, Rp, N);
-    a.C = dbc.narrow(2, Rp + N, N);
-    a.reverse = reverse;
-    S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
-    if (!scan_forward(a, S, false, grad, o)) {
-      TORCH_CHECK(!reverse, "mamba_b200: these tensors cannot be scanned in reverse");
-      S = 1;
-      scan_forward(a, 1, false, grad, o);
+    if (wi.defined()) xz = at::mm(x2, wi.t()).view({B, L, 2 * W});
+    for (auto& d : dirs) d.forward(xz, R, N, grad);
+    s = nd == 1 ? dirs[0].y : dirs[0].y + dirs[1].y;
+    if (wo.defined()) {
+      Tensor o = empty({T, wo.size(0)}, dt, xz);
+      at::addmm_out(o, o, alias(s, 0, {T, W}), wo.t(), 0, scale);
+      out = alias(o, 0, {B, L, wo.size(0)});
+    } else {
+      out = s;
     }
   }
   if (grad) {
-    auto node = new_node<InnerBackward>();
-    const Tensor* in[kParams] = {&xz, &conv_w, &conv_b, &xproj_w, &dt_w, &dt_b, &A_log, &D};
-    for (int i = 0; i < kParams; ++i) node->types[i] = type_of(*in[i]);
-    node->set_next_edges(torch::autograd::collect_next_edges(xz, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D));
-    node->xz.save(xzs); node->xc.save(a.x); node->dbc.save(dbc); node->delta.save(a.delta); node->A.save(a.A); node->D.save(a.D);
-    node->bias.save(a.bias); node->carries.save(o.carries); node->P.save(o.P); node->cw.save(cw); node->cb.save(cb); node->Wx.save(Wx);
-    node->Wdt.save(Wdt);
-    node->R = R; node->Rp = Rp; node->N = N; node->S = S; node->reverse = reverse;
-    node->cw_shape = conv_w.sizes().vec();
-    torch::autograd::set_history(o.y, node);
+    auto node = new_node<BlockBackward>();
+    torch::autograd::edge_list edges;
+    for (const Tensor& t : in) {
+      node->types.push_back(type_of(t));
+      edges.push_back(t.defined() && t.requires_grad() ? torch::autograd::impl::gradient_edge(t) : torch::autograd::Edge());
+    }
+    node->set_next_edges(std::move(edges));
+    if (wi.defined()) { node->x.save(x2); node->in_w.save(wi); }
+    if (wo.defined()) { node->out_w.save(wo); node->y.save(s); }
+    node->xz.save(xz);
+    node->dirs.resize(nd);
+    for (size_t i = 0; i < nd; ++i) {
+      node->dirs[i].save(dirs[i]);
+      node->dirs[i].cw_shape = in[kBlockInputs + i * kDirParams + kConvW].sizes().vec();
+    }
+    node->x_shape = x.sizes().vec();
+    node->R = R; node->N = N; node->scale = scale;
+    torch::autograd::set_history(out, node);
   }
-  return o.y;
+  return out;
 }
 
-// Whether `inner` can scan in reverse: the kernels' reverse direction exists for d_state 16 and activations on the 16-byte grid.
-bool inner_reversible(const Tensor& xz, int64_t N) {
-  return N == 16 && xz.is_cuda() && convertible(xz.scalar_type()) && xz.is_contiguous() &&
-         reinterpret_cast<uintptr_t>(xz.data_ptr()) % 16 == 0 && xz.size(2) / 2 * xz.element_size() % 16 == 0;
-}
+// Whether a direction can run in reverse on these activations: the kernels' reverse exists for d_state 16 on the 16-byte grid.
+bool reversible(int64_t W, int64_t N, at::ScalarType dt) { return N == 16 && convertible(dt) && W * (dt == at::kFloat ? 4 : 2) % 16 == 0; }
 
 }  // namespace mb200_host

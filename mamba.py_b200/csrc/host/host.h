@@ -153,10 +153,9 @@ std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const T
                                     const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& delta_bias, bool inplace);
 std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace);
 
-Tensor inner(const Tensor& xz, const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w, const Tensor& dt_b,
-             const Tensor& A_log, const Tensor& D, int64_t dt_rank, int64_t d_state, bool reverse);
-bool inner_reversible(const Tensor& xz, int64_t d_state);
-
+Tensor block(const Tensor& x, const OptTensor& in_w, const OptTensor& out_w, const std::vector<OptTensor>& params, int64_t dt_rank,
+             int64_t d_state, bool reverse, bool halve);
+bool reversible(int64_t width, int64_t d_state, at::ScalarType dt);
 std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& h, const Tensor& inputs, const Tensor& in_w, const OptTensor& in_b,
                                               const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w,
                                               const Tensor& dt_b, const Tensor& A_log, const Tensor& D, const Tensor& out_w,

@@ -19,8 +19,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_residual", &add_residual, NoGil());
   m.def("ssm_step", &ssm_step, NoGil());
   m.def("conv_step", &conv_step, NoGil());
-  m.def("inner", &inner, NoGil());
-  m.def("inner_reversible", &inner_reversible);
+  m.def("block", &block, NoGil());
+  m.def("reversible", &reversible);
   m.def("block_step", &block_step, NoGil());
   m.def("pick_pieces", &pick_pieces);
 }

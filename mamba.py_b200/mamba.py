@@ -178,11 +178,42 @@ def _plain_block(self):
     return (*lin[0], conv.get("weight"), conv.get("bias"), lin[1][0], *lin[2], A_log, D, *lin[3]) if "weight" in conv else None
 
 
-def _fusable(self, xz):
+def _fusable(self, x, dtype):
+    """Whether the native block takes this module on activations of `dtype` made from x."""
     cfg = self.config
-    return (xz.is_cuda and xz.dtype in (torch.float32, torch.bfloat16) and self.conv1d.weight.shape[-1] == 4
+    return (x.is_cuda and dtype in (torch.float32, torch.bfloat16) and self.conv1d.weight.shape[-1] == 4
             and getattr(self, "dt_layernorm", None) is None and getattr(self, "B_layernorm", None) is None
             and getattr(self, "C_layernorm", None) is None and cfg.d_state in (8, 16, 32, 64))
+
+
+def _native_linear(m, dtype):
+    """The weight of a projection the native block can run itself on activations of `dtype`: an ordinary nn.Linear without
+    a bias, of the activations' type or cast to it by autocast.  None for any other, which is called as the module it is."""
+    p = _plain_linear(m)
+    if p is None or p[1] is not None or _has_any_global_hook():
+        return None
+    ours = p[0].is_cuda and (p[0].dtype == dtype or (torch.is_autocast_enabled("cuda") and p[0].dtype in (torch.float32, torch.bfloat16)))
+    return p[0] if ours else None
+
+
+def run_block(self, x, directions, halve=False):
+    """in_proj, the scans of `directions` (lists of seven parameters) and out_proj as one native call, with those projections
+    called as modules that are not ordinary ones.  None if the block does not take the native path; the second value is
+    in_proj(x) if that has been computed on the way."""
+    dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+    in_w = _native_linear(self.in_proj, dtype) if x.dim() == 3 and x.dtype in (torch.float32, torch.bfloat16) else None
+    if in_w is None or not _fusable(self, x, dtype):
+        x, in_w = self.in_proj(x), None
+        dtype = x.dtype
+        if not _fusable(self, x, dtype):
+            return None, x
+    cfg = self.config
+    params = [p for d in directions for p in d]
+    out_w = _native_linear(self.out_proj, dtype)
+    if out_w is not None:
+        return _host().block(x, in_w, out_w, params, cfg.dt_rank, cfg.d_state, False, halve), None
+    y = _host().block(x, in_w, None, params, cfg.dt_rank, cfg.d_state, False, False)
+    return self.out_proj(y / 2 if halve else y), None
 
 
 def ssm(self, x, z):
@@ -199,12 +230,10 @@ def ssm(self, x, z):
 def forward(self, x):
     """mambapy/mamba.py:205-234 with the scan path fused; x: (B, L, D) -> (B, L, D)."""
     _, L, _ = x.shape
-    xz = self.in_proj(x)
-    if _fusable(self, xz):
-        cfg = self.config
-        y = _host().inner(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight,
-                          self.dt_proj.bias, self.A_log, self.D, cfg.dt_rank, cfg.d_state, False)
-        return self.out_proj(y)
+    out, xz = run_block(self, x, [[self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight,
+                                   self.dt_proj.bias, self.A_log, self.D]])
+    if out is not None:
+        return out
     xs, z = xz.chunk(2, dim=-1)
     if self.conv1d.weight.shape[-1] == 4:
         xs = causal_conv1d_silu(xs, self.conv1d.weight, self.conv1d.bias)

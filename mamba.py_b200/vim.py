@@ -12,7 +12,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import host as _host
-from .mamba import _fusable, causal_conv1d_silu, selective_scan_fn
+from .mamba import causal_conv1d_silu, run_block, selective_scan_fn
 
 
 def _conv_silu(conv, xs, L):
@@ -35,23 +35,26 @@ def forward(self, x):
     """mambapy/vim.py:205-261; x: (B, L, D) -> (B, L, D)."""
     _, L, _ = x.shape
     cfg = self.config
-    xz = self.in_proj(x)
-    xs, z = xz.chunk(2, dim=-1)
-    fused = _fusable(self, xz)
-    if fused:
-        y = _host().inner(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight, self.dt_proj.bias,
-                          self.A_log, self.D, cfg.dt_rank, cfg.d_state, False)
+    first = [self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight, self.dt_proj.bias, self.A_log, self.D]
+    dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+    native = not cfg.bidirectional
+    if cfg.bidirectional and _host().reversible(self.D.shape[0], cfg.d_state, dtype):
+        second = [self.conv1d_b.weight, self.conv1d_b.bias, self.x_proj_b.weight, self.dt_proj_b.weight, self.dt_proj_b.bias,
+                  self.A_log_b, self.D_b]
+        native = self.conv1d_b.weight.shape[-1] == 4
+    if native:
+        out, xz = run_block(self, x, [first, second] if cfg.bidirectional else [first], cfg.bidirectional and cfg.divide_output)
+        if out is not None:
+            return out
     else:
-        y = _ssm(self, _conv_silu(self.conv1d, xs, L), z, self.A_log, self.D, self.x_proj, self.dt_proj, False)
+        xz = self.in_proj(x)
+    xs, z = xz.chunk(2, dim=-1)
+    y = _ssm(self, _conv_silu(self.conv1d, xs, L), z, self.A_log, self.D, self.x_proj, self.dt_proj, False)
     if not cfg.bidirectional:
         return self.out_proj(y)
     # second direction: the reference convolves the flipped sequence; in original time order that is
     # flip(conv(flip(x))).  Everything after it is per-timestep, and the scan runs right to left.
-    if fused and _host().inner_reversible(xz, cfg.d_state):
-        yb = _host().inner(xz, self.conv1d_b.weight, self.conv1d_b.bias, self.x_proj_b.weight, self.dt_proj_b.weight, self.dt_proj_b.bias,
-                           self.A_log_b, self.D_b, cfg.dt_rank, cfg.d_state, True)
-    else:
-        xb = _conv_silu(self.conv1d_b, xs.flip(1), L).flip(1)
-        yb = _ssm(self, xb, z, self.A_log_b, self.D_b, self.x_proj_b, self.dt_proj_b, True)
+    xb = _conv_silu(self.conv1d_b, xs.flip(1), L).flip(1)
+    yb = _ssm(self, xb, z, self.A_log_b, self.D_b, self.x_proj_b, self.dt_proj_b, True)
     s = y + yb
     return self.out_proj(s / 2 if cfg.divide_output else s)
