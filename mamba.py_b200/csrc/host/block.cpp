@@ -88,7 +88,7 @@ struct Direction {
       keep.push_back(param(t));
       return conv.cast(keep.back(), at::kFloat);
     };
-    cw = f32_param(p[kConvW]).view({W, K});
+    cw = alias(f32_param(p[kConvW]), 0, {W, K});
     cb = f32_param(p[kConvB]);
     D = f32_param(p[kD]);
     bias = f32_param(p[kDtB]);
@@ -98,11 +98,11 @@ struct Direction {
     const int64_t B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, xz.scalar_type()), cols = Rp + 2 * N;
     keep.clear();
     xc = empty({B, L, W}, xz.scalar_type(), xz);
-    conv_forward(xz.narrow(2, 0, W), cw, cb, xc, reverse);
-    const Tensor dbc2 = at::mm(alias(xc, 0, {T, W}), Wx.t());
-    delta = at::mm(dbc2.narrow(1, 0, Rp), Wdt.t()).view({B, L, W});         // bias and softplus happen in the kernel
-    dbc = dbc2.view({B, L, cols});
-    ScanArgs a{xc, delta, A, dbc.narrow(2, Rp, N), dbc.narrow(2, Rp + N, N), D, xz.narrow(2, W, W), bias, Tensor(), reverse};
+    conv_forward(columns(xz, 0, W), cw, cb, xc, reverse);
+    const Tensor dbc2 = product(alias(xc, 0, {T, W}), transposed(Wx));
+    delta = alias(product(columns(dbc2, 0, Rp), transposed(Wdt)), 0, {B, L, W});  // bias and softplus happen in the kernel
+    dbc = alias(dbc2, 0, {B, L, cols});
+    ScanArgs a{xc, delta, A, columns(dbc, Rp, N), columns(dbc, Rp + N, N), D, columns(xz, W, W), bias, Tensor(), reverse};
     S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
     ScanOut o;
     if (!scan_forward(a, S, false, grad, o)) {
@@ -122,22 +122,21 @@ struct Direction {
     const auto dt = xc.scalar_type();
     const int64_t B = xc.size(0), L = xc.size(1), W = xc.size(2), T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N, K = cw.size(1);
     if ((reverse || S > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
-    const ScanArgs a{xc, delta, A, dbc.narrow(2, Rp, N), dbc.narrow(2, Rp + N, N), D, xz.narrow(2, W, W), bias, Tensor(), reverse};
-    ScanGrads g = scan_backward(a, S, dy, carries, P, false, dxz.narrow(2, W, W), W * K + W);
+    const ScanArgs a{xc, delta, A, columns(dbc, Rp, N), columns(dbc, Rp + N, N), D, columns(xz, W, W), bias, Tensor(), reverse};
+    ScanGrads g = scan_backward(a, S, dy, carries, P, false, columns(dxz, W, W), W * K + W);
     const Tensor d_dbc = empty({T, cols}, dt, xz), dd2 = alias(g.dd, 0, {T, W}), xc2 = alias(xc, 0, {T, W}), dx2 = alias(g.dx, 0, {T, W});
     auto col = [&](int64_t c) { return static_cast<char*>(d_dbc.data_ptr()) + c * d_dbc.element_size(); };
     Convert acc;
     acc.add(ptr(g.dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);          // float32 accumulators -> activation dtype, in place
     acc.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
     acc.run();
-    Tensor d_dt = d_dbc.narrow(1, 0, Rp);
-    at::mm_out(d_dt, dd2, Wdt);                                              // through dt_proj
-    const Tensor dWdt = at::mm(dd2.t(), alias(dbc, 0, {T, cols}).narrow(1, 0, Rp));      // (W, Rp)
-    const Tensor dWx = at::mm(d_dbc.t(), xc2);                               // (Rp + 2 N, W)
-    Tensor dxc = dx2;
-    at::addmm_out(dxc, dx2, d_dbc, Wx);                                      // + the gradient through x_proj, in the GEMM's epilogue
+    const Tensor d_dt = columns(d_dbc, 0, Rp);
+    product_into(d_dt, dd2, Wdt, 1.f, 0.f);                                           // through dt_proj
+    const Tensor dWdt = product(transposed(dd2), columns(alias(dbc, 0, {T, cols}), 0, Rp));      // (W, Rp)
+    const Tensor dWx = product(transposed(d_dbc), xc2);                               // (Rp + 2 N, W)
+    product_into(dx2, d_dbc, Wx, 1.f, 1.f);                                       // + the gradient through x_proj, in the GEMM's epilogue
     float *dcw = fptr(g.extra), *dcb = dcw + W * K;
-    conv_backward(xz.narrow(2, 0, W), cw, cb, alias(dxc, 0, {B, L, W}), dxz.narrow(2, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
+    conv_backward(columns(xz, 0, W), cw, cb, g.dx, columns(dxz, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
 
     auto dense = [&](int i, const Tensor& src, int64_t offset, at::IntArrayRef shape) {
       if (kt[i] == at::kFloat) {
@@ -202,7 +201,7 @@ struct BlockBackward : public torch::autograd::Node {
   std::vector<at::ScalarType> types;
   std::vector<int64_t> x_shape;
   int64_t R = 0, N = 0;
-  double scale = 1.0;
+  float scale = 1.f;
 
   std::string name() const override { return "MambaBlockBackward"; }
   void release_variables() override {
@@ -225,12 +224,12 @@ struct BlockBackward : public torch::autograd::Node {
     Tensor dy = rows(grads[0], dt);
     if (out_w.defined) {
       const Tensor w = out_w.get(), s2 = alias(y.get(), 0, {T, W}), d2 = dy.reshape({T, w.size(0)});
-      Tensor ds = empty({T, W}, dt, xz_);
-      at::addmm_out(ds, ds, d2, w, 0, scale);
+      const Tensor ds = empty({T, W}, dt, xz_);
+      product_into(ds, d2, w, scale, 0.f);
       dy = alias(ds, 0, {B, L, W});
       if (task_should_compute_output(kOutW)) {
-        Tensor dw = empty(w.sizes(), dt, xz_);
-        at::addmm_out(dw, dw, d2.t(), s2, 0, scale);
+        const Tensor dw = empty(w.sizes(), dt, xz_);
+        product_into(dw, transposed(d2), s2, scale, 0.f);
         out[kOutW] = finish.cast(dw, kt[kOutW]);
         alive.push_back(dw);
       }
@@ -245,11 +244,11 @@ struct BlockBackward : public torch::autograd::Node {
     if (in_w.defined) {
       const Tensor w = in_w.get(), x2 = x.get(), d2 = alias(dxz, 0, {T, 2 * W});
       if (task_should_compute_output(kInW)) {
-        alive.push_back(at::mm(d2.t(), x2));
+        alive.push_back(product(transposed(d2), x2));
         out[kInW] = finish.cast(alive.back(), kt[kInW]);
       }
       if (task_should_compute_output(kX)) {
-        alive.push_back(alias(at::mm(d2, w), 0, x_shape));
+        alive.push_back(alias(product(d2, w), 0, x_shape));
         out[kX] = finish.cast(alive.back(), kt[kX]);
       }
     } else {
@@ -282,7 +281,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
   const size_t nd = params.size() / kDirParams;
   std::vector<Direction> dirs(nd);
   Tensor x2, wi, wo, xz, s, out;
-  const double scale = halve ? 0.5 : 1.0;
+  const float scale = halve ? 0.5f : 1.f;
   {
     const auto dt = in_w.defined() && at::autocast::is_autocast_enabled(at::kCUDA) ? at::autocast::get_autocast_dtype(at::kCUDA) : x.scalar_type();
     TORCH_CHECK_TYPE(convertible(dt), "mamba_b200 kernels take float32 or bfloat16 activations, got ", dt);
@@ -306,12 +305,12 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
       dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N);
     }
     conv.run();
-    if (wi.defined()) xz = at::mm(x2, wi.t()).view({B, L, 2 * W});
+    if (wi.defined()) xz = alias(product(x2, transposed(wi)), 0, {B, L, 2 * W});
     for (auto& d : dirs) d.forward(xz, R, N, grad);
     s = nd == 1 ? dirs[0].y : dirs[0].y + dirs[1].y;
     if (wo.defined()) {
-      Tensor o = empty({T, wo.size(0)}, dt, xz);
-      at::addmm_out(o, o, alias(s, 0, {T, W}), wo.t(), 0, scale);
+      const Tensor o = empty({T, wo.size(0)}, dt, xz);
+      product_into(o, alias(s, 0, {T, W}), transposed(wo), scale, 0.f);
       out = alias(o, 0, {B, L, wo.size(0)});
     } else {
       out = s;

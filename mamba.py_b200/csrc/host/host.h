@@ -75,10 +75,24 @@ inline Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& on) 
 // `shape` dense elements of `base`'s storage from element `offset` of it on (a plain alias, not an autograd view).
 inline Tensor alias(const Tensor& base, int64_t offset, at::IntArrayRef shape) {
   Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(base.storage()), base.key_set(), base.dtype());
+  t.unsafeGetTensorImpl()->set_version_counter(base.unsafeGetTensorImpl()->version_counter());
   t.unsafeGetTensorImpl()->set_storage_offset(base.storage_offset() + offset);
   t.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
   return t;
 }
+// The same storage under other sizes and strides, the columns [first, first + n) of the last dimension, and a matrix transposed.
+inline Tensor strided(const Tensor& base, int64_t offset, at::IntArrayRef shape, at::IntArrayRef strides) {
+  Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(base.storage()), base.key_set(), base.dtype());
+  t.unsafeGetTensorImpl()->set_version_counter(base.unsafeGetTensorImpl()->version_counter());
+  t.unsafeGetTensorImpl()->set_sizes_and_strides(shape, strides, base.storage_offset() + offset);
+  return t;
+}
+inline Tensor columns(const Tensor& t, int64_t first, int64_t n) {
+  c10::SmallVector<int64_t, 4> shape(t.sizes().begin(), t.sizes().end());
+  shape.back() = n;
+  return strided(t, first * t.stride(-1), shape, t.strides());
+}
+inline Tensor transposed(const Tensor& t) { return strided(t, 0, {t.size(1), t.size(0)}, {t.stride(1), t.stride(0)}); }
 inline void zero_fill(const Tensor& t) {
   C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), at::cuda::getCurrentCUDAStream()));
 }
@@ -148,6 +162,9 @@ Tensor pscan(const Tensor& A, const Tensor& X);
 Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias);
 Tensor rms_norm(const Tensor& x, const OptTensor& weight, double eps);
 std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residual, const OptTensor& weight, double eps);
+// out = alpha * a b + beta * out, and a b (gemm.cpp)
+void product_into(const Tensor& out, const Tensor& a, const Tensor& b, float alpha, float beta);
+Tensor product(const Tensor& a, const Tensor& b);
 Tensor add_residual(const Tensor& x, const Tensor& residual);
 std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const Tensor& delta, const Tensor& A, const Tensor& B,
                                     const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& delta_bias, bool inplace);

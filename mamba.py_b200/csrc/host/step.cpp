@@ -143,14 +143,22 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
       return {out, h_new, fresh};
     }
   }
-  const Tensor xz = at::linear(x, in_w, in_b_);
+  // outside autograd and autocast the projections need nothing of at::linear but the product
+  bool direct = convertible(dt) && !at::autocast::is_autocast_enabled(at::kCUDA) && !wants_grad(x, in_w, in_b, out_w, out_b, xproj_w, dt_w);
+  for (const Tensor* t : {&in_w, &xproj_w, &dt_w, &out_w}) direct = direct && t->scalar_type() == dt;
+  auto project = [&](const Tensor& v, const Tensor& weight, const OptTensor& bias) {
+    if (!direct || value(bias).defined()) return at::linear(v, weight, bias);
+    const BelowAutograd guard_ad;
+    return product(v, transposed(weight));
+  };
+  const Tensor xz = project(x, in_w, in_b_);
   WindowStep w;
   {
     const BelowAutograd guard_ad;
     w = window_step(xz.narrow(1, 0, W), inputs, conv_w, conv_b, false);
   }
-  const Tensor dbc = at::linear(w.xc, xproj_w);
-  const Tensor delta = at::linear(dbc.narrow(1, 0, R), dt_w);                // bias and softplus happen in the kernel
+  const Tensor dbc = project(w.xc, xproj_w, {});
+  const Tensor delta = project(dbc.narrow(1, 0, R), dt_w, {});               // bias and softplus happen in the kernel
   StateStep s;
   {
     const BelowAutograd guard_ad;
@@ -174,7 +182,7 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
     }
     s = state_step(w.xc, h, delta, A, !once, dbc.narrow(1, R, N), dbc.narrow(1, R + N, N), Df, xz.narrow(1, W, W), bf, false);
   }
-  return {at::linear(s.y, out_w, out_b_), s.h, w.window};
+  return {project(s.y, out_w, out_b_), s.h, w.window};
 }
 
 }  // namespace mb200_host

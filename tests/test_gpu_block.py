@@ -1,0 +1,88 @@
+"""The native Mamba block (projections, one or both directions, one autograd node) against a float64 restatement of it: ranks off
+the 16-byte grid, a projection the native call leaves to its module, frozen inputs, both directions with the halving."""
+import math
+
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from tests.helpers import RefShapedBlock
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _build(d_model, d_state, both):
+    torch.manual_seed(d_model + d_state)
+    m = RefShapedBlock(d_model, d_state)
+    m.config.bidirectional, m.config.divide_output = both, True
+    with torch.no_grad():
+        m.dt_proj.bias.fill_(-3.0)
+        m.A_log.add_(0.2 * torch.randn_like(m.A_log))
+    if both:
+        other = RefShapedBlock(d_model, d_state)
+        for k in ("conv1d", "x_proj", "dt_proj", "A_log", "D"):
+            setattr(m, k + "_b", getattr(other, k))
+    return m.to(DEV)
+
+
+def _direction(p, xz, R, N):
+    w, b, wx, wdt, bdt, A_log, D = p
+    L, W = xz.shape[1], xz.shape[2] // 2
+    x = F.silu(F.conv1d(xz[..., :W].transpose(1, 2), w, b, groups=W, padding=3)[..., :L]).transpose(1, 2)
+    dt, B, C = torch.split(x @ wx.t(), [R, N, N], -1)
+    delta, A = F.softplus(dt @ wdt.t() + bdt), -torch.exp(A_log)
+    h, ys = 0.0, []
+    for t in range(L):
+        h = torch.exp(delta[:, t, :, None] * A) * h + (delta[:, t] * x[:, t])[..., None] * B[:, t, None]
+        ys.append((h * C[:, t, None]).sum(-1) + D * x[:, t])
+    return torch.stack(ys, 1) * F.silu(xz[..., W:])
+
+
+def _params(m, s):
+    conv, x_proj, dt_proj = (getattr(m, k + s) for k in ("conv1d", "x_proj", "dt_proj"))
+    return [conv.weight, conv.bias, x_proj.weight, dt_proj.weight, dt_proj.bias, getattr(m, "A_log" + s), getattr(m, "D" + s)]
+
+
+def _plain(m, x, both, leaves):
+    it = iter(leaves)
+    d = {id(p): next(it) for p in m.parameters()}
+    g = lambda s: [d[id(p)] for p in _params(m, s)]
+    R, N = m.config.dt_rank, m.config.d_state
+    xz = x @ d[id(m.in_proj.weight)].t()
+    y = _direction(g(""), xz, R, N)
+    if both:
+        y = (y + _direction(g("_b"), xz.flip(1), R, N).flip(1)) / 2
+    y = y @ d[id(m.out_proj.weight)].t()
+    return y if m.out_proj.bias is None else y + d[id(m.out_proj.bias)]
+
+
+@pytest.mark.parametrize("d_model,d_state,both,variant", [(32, 16, False, ""), (40, 16, False, "bias"), (24, 8, False, "hook"),
+                                                          (48, 16, True, ""), (64, 16, True, "bias"), (20, 16, False, "frozen")])
+@pytest.mark.parametrize("amp", [False, True])
+def test_block_against_float64(d_model, d_state, both, variant, amp):
+    from mamba_b200 import mamba, vim
+    m = _build(d_model, d_state, both)
+    if variant == "bias":
+        m.out_proj = nn.Linear(2 * d_model, d_model, bias=True, device=DEV)
+    if variant == "hook":
+        m.in_proj.register_forward_hook(lambda mod, i, o: o)
+    x = torch.randn(3, 37, d_model, device=DEV, requires_grad=variant != "frozen")
+    if variant == "frozen":
+        m.in_proj.weight.requires_grad_(False)
+    dy = torch.randn(3, 37, d_model, device=DEV)
+    run = vim.forward if both else mamba.forward
+    with torch.autocast("cuda", dtype=torch.bfloat16, enabled=amp):
+        y = run(m, x)
+    wanted = [t for t in [x, *m.parameters()] if t.requires_grad]
+    got = torch.autograd.grad(y, wanted, dy.to(y.dtype))
+    leaves = [p.detach().double().requires_grad_(p.requires_grad) for p in m.parameters()]
+    x64 = x.detach().double().requires_grad_(x.requires_grad)
+    want_y = _plain(m, x64, both, leaves)
+    want = torch.autograd.grad(want_y, [t for t in [x64, *leaves] if t.requires_grad], dy.double())
+    tol = 3e-2 if amp else 2e-5
+    for a, b, t in zip([y, *got], [want_y, *want], [y, *wanted]):
+        assert a.dtype == t.dtype and a.shape == b.shape
+        err = ((a.double() - b).norm() / b.norm().clamp_min(1e-12)).item()
+        assert err < tol and math.isfinite(err), (tuple(b.shape), err)
