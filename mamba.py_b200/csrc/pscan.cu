@@ -7,11 +7,11 @@
 // The loads of a block of kUnroll timesteps do not depend on the recurrence and are issued
 // together, which is what keeps enough bytes in flight to cover HBM latency.
 //
-// When B*D*N alone cannot fill the GPU, L is cut into segments handled by different CTAs:
+// When B*D*N alone cannot fill the GPU, the timesteps of a row are spread over one CTA's threads
+// (pscan_cta_*), and for long rows of few channels over several CTAs: L is cut into segments,
 // a first pass reduces every segment to (prod A, state reached from zero), a tiny fold
-// turns those into the state entering each segment, and the main pass starts from it.  That
-// costs one extra read of the inputs and is only chosen when the single pass would leave
-// most SMs idle.
+// turns those into the state entering each segment, and the main pass starts from it, at the
+// price of an extra read of the inputs.
 #include <initializer_list>
 #include "common.cuh"
 
@@ -45,6 +45,10 @@ template <typename T, int V>
 __device__ __forceinline__ void store_chan(T* p, const Chan<T, V>& r) {
   if constexpr (V == 1) {
     *p = r.v[0];
+  } else if constexpr (sizeof(T) * V == 8) {
+    __nv_bfloat162 w[2];
+    w[0].x = r.v[0]; w[0].y = r.v[1]; w[1].x = r.v[2]; w[1].y = r.v[3];
+    __stcs(reinterpret_cast<uint2*>(p), make_uint2(*reinterpret_cast<const uint32_t*>(&w[0]), *reinterpret_cast<const uint32_t*>(&w[1])));
   } else {
     __stcs(reinterpret_cast<uint4*>(p), *reinterpret_cast<const uint4*>(&r));
   }
@@ -268,16 +272,259 @@ pscan_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* __re
   }
 }
 
-int pick_segments(int64_t B, int64_t L, int64_t CH) {
+// ------------------------------------------------------- a row's timesteps spread over one CTA
+// Bound by latency: at (1, 1000, 128, 16) the tensors are 8 MB each way of a step and live in L2, and three launches with a
+// workspace between them cost more than the data.  A CTA owns 16 neighbouring channels of a row and spreads
+// 4 or 8 timesteps to a thread, up to 1024 to the CTA; a thread folds its steps into (product of A, state from zero), warps scan
+// these pairs by shuffles, the warps' totals go through shared memory, and the thread walks its steps again from the state
+// that enters them, out of registers.  Longer rows are a loop that carries the state.  Inputs are read once (the segmented
+// passes read them twice) and nothing is allocated.
+// Forward / backward, us, segmented passes before: 1 x 1000 x 2048 channels float32 26.4 / 28.9 -> 8.8 / 12.8, bfloat16 33 / 38 -> 8.8 / 8.8;
+// 4 x 1000 x 8192 float32 122 / 175 -> 76 / 121 (bytes 61 / 102); 1 x 16384 x 24576 1340 / 1850 -> 953 / 1609; 64 steps of 512 channels
+// 8.1 / 12.9 -> 4.7 / 4.7 (one serial thread per vector before).
+constexpr int kCtaVec = 4;                                        // channels of a vector: 8 of bfloat16 do not fit the registers
+template <typename T, int V, bool kBackward>
+constexpr int kStepsPerThread = sizeof(T) * V == 16 && kBackward ? 4 : 8;  // what registers hold
+constexpr int kMaxCtaThreads = 512;
+
+template <typename T, int V> struct CtaTile {
+  static constexpr int kVecs = 16 / V;                               // neighbouring vectors side by side in a warp
+  static constexpr int kSegs = 32 / kVecs;                       // segments of a warp
+};
+
+// V channels of one timestep as they wait in registers.  bfloat16 stays packed in whole words: as an array of 2-byte elements
+// the compiler keeps it on the stack.
+template <typename T, int V> struct Held {
+  float v[V];
+  __device__ __forceinline__ float f(int i) const { return v[i]; }
+};
+template <> struct Held<__nv_bfloat16, 4> {
+  uint32_t w[2];
+  __device__ __forceinline__ float f(int i) const { return __uint_as_float(i & 1 ? w[i / 2] & 0xffff0000u : w[i / 2] << 16); }
+};
+template <typename T, int V> __device__ __forceinline__ Held<T, V> hold(const T* p) {
+  Held<T, V> r;
+  if constexpr (V == 1) {
+    r.v[0] = Elem<T>::to_f(*p);
+  } else if constexpr (sizeof(T) == 2) {
+    const uint2 w = __ldcs(reinterpret_cast<const uint2*>(p));
+    r.w[0] = w.x; r.w[1] = w.y;
+  } else {
+    const float4 w = __ldcs(reinterpret_cast<const float4*>(p));
+    r.v[0] = w.x; r.v[1] = w.y; r.v[2] = w.z; r.v[3] = w.w;
+  }
+  return r;
+}
+
+template <int V> struct Span {                                   // a run of timesteps: h_out = P * h_in + S
+  float P[V], S[V];
+};
+
+// On entry `w` is the thread's own span.  On return it is the span of everything before the thread's segment in scan order
+// inside its warp, and the warp's total is in `total` of shared memory.  kReverse: scan order runs from the last segment to the first.
+template <typename T, int V, bool kReverse>
+__device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total) {
+  constexpr int kVecs = CtaTile<T, V>::kVecs, kSegs = CtaTile<T, V>::kSegs;
+  const int lane = threadIdx.x & 31, seg = kReverse ? kSegs - 1 - lane / kVecs : lane / kVecs;
+#pragma unroll
+  for (int d = 1; d < kSegs; d *= 2) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const float P = kReverse ? __shfl_down_sync(~0u, w.P[i], d * kVecs) : __shfl_up_sync(~0u, w.P[i], d * kVecs);
+      const float S = kReverse ? __shfl_down_sync(~0u, w.S[i], d * kVecs) : __shfl_up_sync(~0u, w.S[i], d * kVecs);
+      if (seg >= d) {
+        w.S[i] = fmaf(w.P[i], S, w.S[i]);
+        w.P[i] *= P;
+      }
+    }
+  }
+  if (seg == kSegs - 1) total[lane % kVecs] = w;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const float P = kReverse ? __shfl_down_sync(~0u, w.P[i], kVecs) : __shfl_up_sync(~0u, w.P[i], kVecs);
+    const float S = kReverse ? __shfl_down_sync(~0u, w.S[i], kVecs) : __shfl_up_sync(~0u, w.S[i], kVecs);
+    w.P[i] = seg ? P : 1.f;
+    w.S[i] = seg ? S : 0.f;
+  }
+}
+
+// The state entering this thread's segment, from the state `carry` entering the CTA's timesteps, which becomes the one leaving them.
+template <typename T, int V, bool kReverse>
+__device__ __forceinline__ void enter(const Span<V>& before, const Span<V>* totals, float (&carry)[V], float (&h)[V]) {
+  constexpr int kVecs = CtaTile<T, V>::kVecs;
+  const int warps = blockDim.x / 32, warp = threadIdx.x / 32, mine = kReverse ? warps - 1 - warp : warp, v = threadIdx.x % kVecs;
+#pragma unroll 1
+  for (int k = 0; k < warps; ++k) {
+    if (k == mine) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) h[i] = fmaf(before.P[i], carry[i], before.S[i]);
+    }
+    const Span<V>& t = totals[(kReverse ? warps - 1 - k : k) * kVecs + v];
+#pragma unroll
+    for (int i = 0; i < V; ++i) carry[i] = fmaf(t.P[i], carry[i], t.S[i]);
+  }
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(kMaxCtaThreads, 1)
+pscan_cta_fwd_kernel(const T* __restrict__ A, const T* __restrict__ X, T* __restrict__ H, int64_t L, int64_t CH, int64_t a_sb,
+                     int64_t a_sl, int64_t x_sb, int64_t x_sl, int64_t h_sb, int64_t h_sl, const float* __restrict__ h0,
+                     float* __restrict__ hT) {
+  constexpr int kVecs = CtaTile<T, V>::kVecs, U = kStepsPerThread<T, V, false>;
+  __shared__ Span<V> totals[2][kMaxCtaThreads / 32 * kVecs];
+  const int64_t c = (int64_t(blockIdx.x) * kVecs + threadIdx.x % kVecs) * V, b = blockIdx.y;
+  const bool live = c < CH;
+  const int64_t chunk = int64_t(blockDim.x / kVecs) * U;
+  float carry[V], h[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) carry[i] = h0 && live ? h0[b * CH + c + i] : 0.f;
+  A += b * a_sb + c; X += b * x_sb + c; H += b * h_sb + c;
+  int buf = 0;
+  for (int64_t first = 0; first < L; first += chunk, buf ^= 1) {
+    const int64_t t0 = first + int64_t(threadIdx.x / kVecs) * U;
+    const int n = !live || t0 >= L ? 0 : int(min(int64_t(U), L - t0));
+    const T *a = A + t0 * a_sl, *x = X + t0 * x_sl;
+    T* o = H + t0 * h_sl;
+    Held<T, V> av[U], xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < n) {
+        av[u] = hold<T, V>(a + u * a_sl);
+        xv[u] = hold<T, V>(x + u * x_sl);
+      }
+    Span<V> w;
+#pragma unroll
+    for (int i = 0; i < V; ++i) { w.P[i] = 1.f; w.S[i] = 0.f; }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < n)
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float af = av[u].f(i);
+          w.S[i] = fmaf(af, w.S[i], xv[u].f(i));
+          w.P[i] *= af;
+        }
+    warp_exclusive<T, V, false>(w, totals[buf] + threadIdx.x / 32 * kVecs);
+    __syncthreads();                                     // one per chunk: the next one writes the other buffer
+    enter<T, V, false>(w, totals[buf], carry, h);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < n) {
+        Chan<T, V> ov;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          h[i] = fmaf(av[u].f(i), h[i], xv[u].f(i));
+          ov.v[i] = Elem<T>::from_f(h[i]);
+        }
+        store_chan<T, V>(o + u * h_sl, ov);
+        if (hT && t0 + u == L - 1)
+#pragma unroll
+          for (int i = 0; i < V; ++i) hT[b * CH + c + i] = h[i];
+      }
+  }
+}
+
+// G[t] = gH[t] + carry;  gA[t] = H[t-1] * G[t];  carry = A[t] * G[t], from the last chunk to the first.
+template <typename T, int V>
+__global__ void __launch_bounds__(kMaxCtaThreads, 1)
+pscan_cta_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* __restrict__ GH, T* __restrict__ GA, T* __restrict__ GX,
+                     int64_t L, int64_t CH, int64_t a_sb, int64_t a_sl, int64_t h_sb, int64_t h_sl, int64_t g_sb, int64_t g_sl,
+                     int64_t ga_sb, int64_t ga_sl, int64_t gx_sb, int64_t gx_sl, const float* __restrict__ h0) {
+  constexpr int kVecs = CtaTile<T, V>::kVecs, U = kStepsPerThread<T, V, true>;
+  __shared__ Span<V> totals[2][kMaxCtaThreads / 32 * kVecs];
+  const int64_t c = (int64_t(blockIdx.x) * kVecs + threadIdx.x % kVecs) * V, b = blockIdx.y;
+  const bool live = c < CH;
+  const int64_t chunk = int64_t(blockDim.x / kVecs) * U;
+  float carry[V], cy[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) carry[i] = 0.f;
+  A += b * a_sb + c; H += b * h_sb + c; GH += b * g_sb + c; GA += b * ga_sb + c; GX += b * gx_sb + c;
+  int buf = 0;
+  for (int64_t first = (L - 1) / chunk * chunk; first >= 0; first -= chunk, buf ^= 1) {
+    const int64_t t0 = first + int64_t(threadIdx.x / kVecs) * U;
+    const int n = !live || t0 >= L ? 0 : int(min(int64_t(U), L - t0));
+    const T *a = A + t0 * a_sl, *g = GH + t0 * g_sl, *hp = H + (t0 - 1) * h_sl;
+    T *ga = GA + t0 * ga_sl, *gx = GX + t0 * gx_sl;
+    Held<T, V> av[U], gv[U], hv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < n) {
+        av[u] = hold<T, V>(a + u * a_sl);
+        gv[u] = hold<T, V>(g + u * g_sl);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < n && t0 + u > 0) hv[u] = hold<T, V>(hp + u * h_sl);
+    Span<V> w;
+#pragma unroll
+    for (int i = 0; i < V; ++i) { w.P[i] = 1.f; w.S[i] = 0.f; }
+#pragma unroll
+    for (int u = U - 1; u >= 0; --u)
+      if (u < n)
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float af = av[u].f(i);
+          w.S[i] = af * (gv[u].f(i) + w.S[i]);
+          w.P[i] *= af;
+        }
+    warp_exclusive<T, V, true>(w, totals[buf] + threadIdx.x / 32 * kVecs);
+    __syncthreads();
+    enter<T, V, true>(w, totals[buf], carry, cy);
+#pragma unroll
+    for (int u = U - 1; u >= 0; --u)
+      if (u < n) {
+        Chan<T, V> oa, ox;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float G = gv[u].f(i) + cy[i];
+          float before;
+          if (t0 + u > 0) before = hv[u].f(i);
+          else before = h0 ? h0[b * CH + c + i] : 0.f;
+          cy[i] = av[u].f(i) * G;
+          ox.v[i] = Elem<T>::from_f(G);
+          oa.v[i] = Elem<T>::from_f(before * G);
+        }
+        store_chan<T, V>(gx + u * gx_sl, ox);
+        store_chan<T, V>(ga + u * ga_sl, oa);
+      }
+  }
+}
+
+int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Serial threads when they fill the GPU by themselves (256 per SM: enough loads in flight).  Otherwise a CTA per 16 channels of a row,
+// as long as a row is a few rounds of such a CTA or there are CTAs enough for several on every SM (at 2 per SM, 1 x 8192 x 5120,
+// the backward lost 213 -> 230 us to the second wave); what is left, few channels and a long row, is cut into segments.
+bool serial_fills(int64_t B, int64_t CH, int sms) { return B * ((CH + 3) / 4) >= int64_t(sms) * 256; }
+bool rows_in_cta(int64_t B, int64_t L, int64_t CH) {
+  const int sms = sm_count();
+  return !serial_fills(B, CH, sms) && (L <= 2048 || B * ((CH + 15) / 16) >= 3 * sms);
+}
+
+int pick_segments(int64_t B, int64_t L, int64_t CH) {
+  const int sms = sm_count();
+  if (serial_fills(B, CH, sms) || rows_in_cta(B, L, CH)) return 1;
   const int64_t threads = B * ((CH + 3) / 4);
-  if (threads >= int64_t(sms) * 256 || L < 128) return 1;
-  int64_t want = (int64_t(sms) * 512 + threads - 1) / threads;
-  int64_t cap = L / 64;
-  int64_t s = want < cap ? want : cap;
+  const int64_t want = (int64_t(sms) * 512 + threads - 1) / threads, cap = L / 64, s = want < cap ? want : cap;
   return s < 1 ? 1 : int(s);
+}
+
+// 512 threads where all CTAs run at once and the row needs them, 256 (two CTAs per SM overlap) elsewhere; short rows fewer.
+template <typename T, int V> dim3 cta_grid(int64_t B, int64_t CH) {
+  constexpr int per = CtaTile<T, V>::kVecs * V;
+  return dim3(unsigned((CH + per - 1) / per), unsigned(B));
+}
+template <typename T, int V, int U> int cta_threads(int64_t B, int64_t L, int64_t CH) {
+  const dim3 g = cta_grid<T, V>(B, CH);
+  const int64_t most = int64_t(g.x) * g.y <= sm_count() ? kMaxCtaThreads : kMaxCtaThreads / 2;
+  const int64_t need = (L + U - 1) / U * CtaTile<T, V>::kVecs;
+  const int64_t rounds = (need + most - 1) / most;                // of equal size: a last round of few timesteps idles most threads
+  return int((need + rounds - 1) / rounds + 31) / 32 * 32;
 }
 
 template <typename T>
@@ -306,6 +553,14 @@ int fwd_impl(const void* A_, const void* X_, void* H_, int64_t B, int64_t L, int
   dim3 grid(unsigned((CH + int64_t(v) * kThreads - 1) / (int64_t(v) * kThreads)), unsigned(B),
             unsigned(nseg));
   const float* state_in = h0;
+  if (nseg == 1 && rows_in_cta(B, L, CH)) {
+#define MB200_CTA_FWD(VV)                                                                                                       \
+  pscan_cta_fwd_kernel<T, VV><<<cta_grid<T, VV>(B, CH), cta_threads<T, VV, kStepsPerThread<T, VV, false>>(B, L, CH), 0, st>>>(A, X, H, L, CH, a_sb, a_sl, x_sb, x_sl, h_sb, \
+                                                                                         h_sl, h0, hT)
+    if (vec) MB200_CTA_FWD(kCtaVec); else MB200_CTA_FWD(1);
+#undef MB200_CTA_FWD
+    return check_launch();
+  }
   if (nseg > 1) {
     if (vec) pscan_fwd_agg_kernel<T, V><<<grid, kThreads, 0, st>>>(A, X, d, a_sb, a_sl, x_sb, x_sl, wsP, wsS);
     else pscan_fwd_agg_kernel<T, 1><<<grid, kThreads, 0, st>>>(A, X, d, a_sb, a_sl, x_sb, x_sl, wsP, wsS);
@@ -339,6 +594,14 @@ int bwd_impl(const void* A_, const void* H_, const void* G_, void* GA_, void* GX
   dim3 grid(unsigned((CH + int64_t(v) * kThreads - 1) / (int64_t(v) * kThreads)), unsigned(B),
             unsigned(nseg));
   const float* carry_in = nullptr;
+  if (nseg == 1 && rows_in_cta(B, L, CH)) {
+#define MB200_CTA_BWD(VV)                                                                                                          \
+  pscan_cta_bwd_kernel<T, VV><<<cta_grid<T, VV>(B, CH), cta_threads<T, VV, kStepsPerThread<T, VV, true>>(B, L, CH), 0, st>>>(A, H, G, GA, GX, L, CH, a_sb, a_sl, h_sb, h_sl, \
+                                                                                         g_sb, g_sl, ga_sb, ga_sl, gx_sb, gx_sl, h0)
+    if (vec) MB200_CTA_BWD(kCtaVec); else MB200_CTA_BWD(1);
+#undef MB200_CTA_BWD
+    return check_launch();
+  }
 #define MB200_BWD_LAUNCH(VV, AGG)                                                              \
   pscan_bwd_kernel<T, VV, AGG><<<grid, kThreads, 0, st>>>(A, H, G, GA, GX, d, a_sb, a_sl, h_sb, \
       h_sl, g_sb, g_sl, ga_sb, ga_sl, gx_sb, gx_sl, carry_in, h0, wsP, wsS)
