@@ -320,6 +320,8 @@ typedef struct {
   const float* factor;
   int64_t rows, cols, src_cols, src_stride, dst_stride;
   int src_dtype, dst_dtype, op;
+  int slices;             /* > 1: src is the sum of that many matrices, slice_stride elements apart */
+  int64_t slice_stride;
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 

@@ -132,8 +132,9 @@ struct Direction {
     acc.run();
     const Tensor d_dt = columns(d_dbc, 0, Rp);
     product_into(d_dt, dd2, Wdt, 1.f, 0.f);                                           // through dt_proj
-    const Tensor dWdt = product(transposed(dd2), columns(alias(dbc, 0, {T, cols}), 0, Rp));      // (W, Rp)
-    const Tensor dWx = product(transposed(d_dbc), xc2);                               // (Rp + 2 N, W)
+    const int64_t Rw = R % 4 == 0 ? R : Rp;                                  // rows of dWdt on the 16-byte grid
+    const Partials dWdt = tall_product(dd2, columns(alias(dbc, 0, {T, cols}), 0, Rw), kt[kDtW], 1.f);        // (W, Rw)
+    const Partials dWx = tall_product(d_dbc, xc2, kt[kXproj], 1.f);                                          // (Rp + 2 N, W)
     product_into(dx2, d_dbc, Wx, 1.f, 1.f);                                       // + the gradient through x_proj, in the GEMM's epilogue
     float *dcw = fptr(g.extra), *dcb = dcw + W * K;
     conv_backward(columns(xz, 0, W), cw, cb, g.dx, columns(dxz, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
@@ -154,18 +155,22 @@ struct Direction {
     out[kALog] = empty({W, N}, kt[kALog], xz);                               // d A_log = dA * A
     finish.add(ptr(g.dA), at::kFloat, ptr(out[kALog]), kt[kALog], 1, W * N, W * N, W * N, W * N, MB200_CONVERT_MUL).factor = fptr(A);
     if (Rp == R) {
-      out[kXproj] = finish.cast(dWx, kt[kXproj]);
-      out[kDtW] = finish.cast(dWdt, kt[kDtW]);
+      out[kXproj] = finish.settle(dWx, kt[kXproj]);
     } else {
       out[kXproj] = empty({R + 2 * N, W}, kt[kXproj], xz);
       char* wx = static_cast<char*>(ptr(out[kXproj]));
-      finish.add(ptr(dWx), dt, wx, kt[kXproj], 1, R * W, R * W, R * W, R * W);
-      finish.add(static_cast<char*>(ptr(dWx)) + Rp * W * dWx.element_size(), dt, wx + R * W * out[kXproj].element_size(), kt[kXproj], 1,
-                 2 * N * W, 2 * N * W, 2 * N * W, 2 * N * W);
-      out[kDtW] = empty({W, R}, kt[kDtW], xz);
-      finish.add(ptr(dWdt), dt, ptr(out[kDtW]), kt[kDtW], W, R, R, Rp, R);
+      finish.rows_of(dWx, 0, R, wx, kt[kXproj]);
+      finish.rows_of(dWx, Rp, 2 * N, wx + R * W * out[kXproj].element_size(), kt[kXproj]);
     }
-    alive.insert(alive.end(), {dWx, dWdt, g.dA, g.extra});
+    if (Rw == R) {
+      out[kDtW] = finish.settle(dWdt, kt[kDtW]);
+    } else {
+      out[kDtW] = empty({W, R}, kt[kDtW], xz);
+      mb200_convert_job& j = finish.add(ptr(dWdt.t), dWdt.t.scalar_type(), ptr(out[kDtW]), kt[kDtW], W, R, R, Rw, R);
+      j.slices = dWdt.slices;
+      j.slice_stride = W * Rw;
+    }
+    alive.insert(alive.end(), {dWx.t, dWdt.t, g.dA, g.extra});
   }
 
  private:
@@ -228,10 +233,9 @@ struct BlockBackward : public torch::autograd::Node {
       product_into(ds, d2, w, scale, 0.f);
       dy = alias(ds, 0, {B, L, W});
       if (task_should_compute_output(kOutW)) {
-        const Tensor dw = empty(w.sizes(), dt, xz_);
-        product_into(dw, transposed(d2), s2, scale, 0.f);
-        out[kOutW] = finish.cast(dw, kt[kOutW]);
-        alive.push_back(dw);
+        const Partials dw = tall_product(d2, s2, kt[kOutW], scale);
+        out[kOutW] = finish.settle(dw, kt[kOutW]);
+        alive.push_back(dw.t);
       }
     }
     const Tensor dxz = empty({B, L, 2 * W}, dt, xz_);
@@ -244,8 +248,9 @@ struct BlockBackward : public torch::autograd::Node {
     if (in_w.defined) {
       const Tensor w = in_w.get(), x2 = x.get(), d2 = alias(dxz, 0, {T, 2 * W});
       if (task_should_compute_output(kInW)) {
-        alive.push_back(product(transposed(d2), x2));
-        out[kInW] = finish.cast(alive.back(), kt[kInW]);
+        const Partials dw = tall_product(d2, x2, kt[kInW], 1.f);
+        out[kInW] = finish.settle(dw, kt[kInW]);
+        alive.push_back(dw.t);
       }
       if (task_should_compute_output(kX)) {
         alive.push_back(alias(product(d2, w), 0, x_shape));

@@ -126,6 +126,15 @@ struct Saved {
   void reset() { v.reset_data(); }
 };
 
+// A matrix product as it leaves the GEMM: one (rows, cols) matrix, or `slices` float32 ones to be added up.
+struct Partials {
+  Tensor t;
+  int slices;
+  int64_t rows, cols;
+};
+// a^T b for two tall matrices of one type (gemm.cpp); `out` is the type wanted if nothing has to be added up.
+Partials tall_product(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha);
+
 // Up to 24 element-wise jobs in one launch (mb200_convert).
 struct Convert {
   mb200_convert_job jobs[24];
@@ -133,7 +142,7 @@ struct Convert {
   mb200_convert_job& add(const void* src, at::ScalarType st, void* dst, at::ScalarType dt, int64_t rows, int64_t cols, int64_t src_cols,
                          int64_t src_stride, int64_t dst_stride, int op = MB200_CONVERT_COPY) {
     mb200_convert_job& j = jobs[n++];
-    j = mb200_convert_job{src, dst, nullptr, rows, cols, src_cols, src_stride, dst_stride, dtype_code(st), dtype_code(dt), op};
+    j = mb200_convert_job{src, dst, nullptr, rows, cols, src_cols, src_stride, dst_stride, dtype_code(st), dtype_code(dt), op, 1, 0};
     return j;
   }
   // a dense tensor once more in another type; itself when it has that type already
@@ -144,11 +153,26 @@ struct Convert {
     add(ptr(src), src.scalar_type(), ptr(dst), dt, 1, m, m, m, m);
     return dst;
   }
+  // rows [first, first + rows) of a product into dst
+  void rows_of(const Partials& p, int64_t first, int64_t rows, void* dst, at::ScalarType dt);
+  Tensor settle(const Partials& p, at::ScalarType dt);
   void run() {
     if (n) check(mb200_convert(jobs, n, cuda_stream()), "mb200_convert");
     n = 0;
   }
 };
+inline void Convert::rows_of(const Partials& p, int64_t first, int64_t rows, void* dst, at::ScalarType dt) {
+  const int64_t n = rows * p.cols;
+  mb200_convert_job& j = add(static_cast<char*>(p.t.data_ptr()) + first * p.cols * p.t.element_size(), p.t.scalar_type(), dst, dt, 1, n, n, n, n);
+  j.slices = p.slices;
+  j.slice_stride = p.rows * p.cols;
+}
+inline Tensor Convert::settle(const Partials& p, at::ScalarType dt) {
+  if (p.slices == 1 && p.t.scalar_type() == dt) return p.t;
+  const Tensor dst = empty({p.rows, p.cols}, dt, p.t);
+  rows_of(p, 0, p.rows, ptr(dst), dt);
+  return dst;
+}
 inline bool convertible(at::ScalarType d) { return d == at::kFloat || d == at::kBFloat16; }
 
 // What a node remembers of an input whose gradient it returns.

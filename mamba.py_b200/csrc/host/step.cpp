@@ -172,7 +172,7 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
       auto add = [&](const Tensor& src, int op) {
         const Tensor dst = empty(src.sizes(), at::kFloat, src);
         const int64_t n = src.numel();
-        jobs[n_jobs++] = mb200_convert_job{ptr(src), ptr(dst), nullptr, 1, n, n, n, n, code_of(src), MB200_F32, op};
+        jobs[n_jobs++] = mb200_convert_job{ptr(src), ptr(dst), nullptr, 1, n, n, n, n, code_of(src), MB200_F32, op, 1, 0};
         return dst;
       };
       A = add(A_log, MB200_CONVERT_NEG_EXP);

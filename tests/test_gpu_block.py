@@ -58,7 +58,7 @@ def _plain(m, x, both, leaves):
     return y if m.out_proj.bias is None else y + d[id(m.out_proj.bias)]
 
 
-@pytest.mark.parametrize("d_model,d_state,both,variant", [(32, 16, False, ""), (40, 16, False, "bias"), (24, 8, False, "hook"),
+@pytest.mark.parametrize("d_model,d_state,both,variant", [(32, 16, False, ""), (40, 16, False, "many"), (32, 16, True, "ragged"), (40, 16, False, "bias"), (24, 8, False, "hook"),
                                                           (48, 16, True, ""), (64, 16, True, "bias"), (20, 16, False, "frozen")])
 @pytest.mark.parametrize("amp", [False, True])
 def test_block_against_float64(d_model, d_state, both, variant, amp):
@@ -68,10 +68,11 @@ def test_block_against_float64(d_model, d_state, both, variant, amp):
         m.out_proj = nn.Linear(2 * d_model, d_model, bias=True, device=DEV)
     if variant == "hook":
         m.in_proj.register_forward_hook(lambda mod, i, o: o)
-    x = torch.randn(3, 37, d_model, device=DEV, requires_grad=variant != "frozen")
+    rows = {"many": 40, "ragged": 83}.get(variant, 3)               # tokens enough to cut the weight gradients, evenly or not
+    x = torch.randn(rows, 37, d_model, device=DEV, requires_grad=variant != "frozen")
     if variant == "frozen":
         m.in_proj.weight.requires_grad_(False)
-    dy = torch.randn(3, 37, d_model, device=DEV)
+    dy = torch.randn(rows, 37, d_model, device=DEV)
     run = vim.forward if both else mamba.forward
     with torch.autocast("cuda", dtype=torch.bfloat16, enabled=amp):
         y = run(m, x)
