@@ -214,15 +214,20 @@ __global__ void carry_fold_range_kernel(const float* __restrict__ P, const float
   if (m >= M) return;
   P += bb * R * M; S += bb * R * M; out += bb * num * M;
   float cur = init ? init[bb * M + m] : 0.f;
+  // Nothing enters the first piece without `init`, and its P then need not have been written (a scan's last piece has no carry pass).
+  auto through = [&](int r, bool from_nothing) {
+    const float s = S[int64_t(r) * M + m];
+    cur = from_nothing ? s : fmaf(P[int64_t(r) * M + m], cur, s);
+  };
   if (!reverse) {
     for (int r = 0; r < first + num; ++r) {
       if (r >= first) out[int64_t(r - first) * M + m] = cur;
-      if (r + 1 < first + num) cur = fmaf(P[int64_t(r) * M + m], cur, S[int64_t(r) * M + m]);
+      if (r + 1 < first + num) through(r, r == 0 && !init);
     }
   } else {
     for (int r = R - 1; r >= first; --r) {
       if (r < first + num) out[int64_t(r - first) * M + m] = cur;
-      if (r > first) cur = fmaf(P[int64_t(r) * M + m], cur, S[int64_t(r) * M + m]);
+      if (r > first) through(r, r == R - 1 && !init);
     }
   }
 }

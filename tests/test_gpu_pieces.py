@@ -73,3 +73,22 @@ def test_library_chooses_pieces_and_handles_awkward_gradients():
     for k in ("x", "delta", "A", "B", "C", "D", "z"):
         assert_close(lv[k].grad, go[k].float(), RTOL, ATOL * 4 * max(1.0, go[k].abs().max().item()), "grad " + k)
     assert_close(hl.grad, go["h0"].float(), RTOL, ATOL * 4 * max(1.0, go["h0"].abs().max().item()), "grad h0")
+
+
+def test_carries_that_were_not_written_do_not_enter():
+    """The last piece of a row has no carry pass: whatever lies in its decay product must not reach the gradient carries."""
+    from mamba_b200.kernels import carry_fold_range
+    P, G = torch.rand(2, 3, 40, 16, device=DEV), torch.randn(2, 3, 40, 16, device=DEV)
+    P[:, -1] = float("nan")
+    got = carry_fold_range(P, G, None, 0, 3, True)
+    assert torch.equal(got[:, 2], torch.zeros_like(got[:, 2])) and torch.equal(got[:, 1], G[:, 2])
+    assert torch.allclose(got[:, 0], P[:, 1] * G[:, 2] + G[:, 1], atol=1e-5)
+    x = torch.full((1 << 24,), float("nan"), device=DEV)                    # garbage for the next allocations
+    del x
+    a = [torch.randn(1, 2048, 1536, device=DEV, dtype=torch.bfloat16, requires_grad=True) for _ in range(2)]
+    A = -torch.rand(1536, 16, device=DEV) - 0.5
+    BC = [torch.randn(1, 2048, 16, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    import mamba_b200
+    y = mamba_b200.selective_scan_fn(a[0], a[1], A, *BC, delta_bias=torch.zeros(1536, device=DEV))
+    for g in torch.autograd.grad(y, a, torch.ones_like(y)):
+        assert torch.isfinite(g).all()
