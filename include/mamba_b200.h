@@ -325,6 +325,18 @@ typedef struct {
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
+/* Up to 4 independent matrix products in one launch, out = alpha * a b + beta * out, for sizes that are all launch latency.
+ * a (M, K) and b (K, N) have any strides (elements; rm: of m, ck: of k, rk: of k, cn: of n) and type `dtype`; out has unit-stride rows.
+ * float32 accumulation. */
+typedef struct {
+  const void *a, *b;
+  void* out;
+  int64_t M, N, K, a_rm, a_ck, b_rk, b_cn, out_rm;
+  float alpha, beta;
+  int out_dtype;
+} mb200_product;
+int mb200_small_gemm(const mb200_product* products, int n, int dtype, void* stream);
+
 /* A sequence cut into `pieces` consecutive spans of piece_len timesteps (a multiple of 16; the last may be shorter) that are
  * scanned side by side, for problems with few batch rows.  Per-token tensors and saved states keep their layouts; what belongs
  * to a piece is (B, pieces, ED, N): the states entering the pieces (h0), the carry pass's states and decay products (the scan's

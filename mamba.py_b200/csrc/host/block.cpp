@@ -99,8 +99,11 @@ struct Direction {
     keep.clear();
     xc = empty({B, L, W}, xz.scalar_type(), xz);
     conv_forward(columns(xz, 0, W), cw, cb, xc, reverse);
-    const Tensor dbc2 = product(alias(xc, 0, {T, W}), transposed(Wx));
-    delta = alias(product(columns(dbc2, 0, Rp), transposed(Wdt)), 0, {B, L, W});  // bias and softplus happen in the kernel
+    Products mm;
+    const Tensor dbc2 = mm.of(alias(xc, 0, {T, W}), transposed(Wx));
+    mm.run();
+    delta = alias(mm.of(columns(dbc2, 0, Rp), transposed(Wdt)), 0, {B, L, W});
+    mm.run();                                                                // bias and softplus happen in the kernel
     dbc = alias(dbc2, 0, {B, L, cols});
     ScanArgs a{xc, delta, A, columns(dbc, Rp, N), columns(dbc, Rp + N, N), D, columns(xz, W, W), bias, Tensor(), reverse};
     S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
@@ -131,11 +134,14 @@ struct Direction {
     acc.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
     acc.run();
     const Tensor d_dt = columns(d_dbc, 0, Rp);
-    product_into(d_dt, dd2, Wdt, 1.f, 0.f);                                           // through dt_proj
+    Products mm;
+    mm.into(d_dt, dd2, Wdt, 1.f, 0.f);                                       // through dt_proj
     const int64_t Rw = R % 4 == 0 ? R : Rp;                                  // rows of dWdt on the 16-byte grid
-    const Partials dWdt = tall_product(dd2, columns(alias(dbc, 0, {T, cols}), 0, Rw), kt[kDtW], 1.f);        // (W, Rw)
-    const Partials dWx = tall_product(d_dbc, xc2, kt[kXproj], 1.f);                                          // (Rp + 2 N, W)
-    product_into(dx2, d_dbc, Wx, 1.f, 1.f);                                       // + the gradient through x_proj, in the GEMM's epilogue
+    const Partials dWdt = mm.tall(dd2, columns(alias(dbc, 0, {T, cols}), 0, Rw), kt[kDtW], 1.f);        // (W, Rw)
+    mm.run();
+    const Partials dWx = mm.tall(d_dbc, xc2, kt[kXproj], 1.f);                                          // (Rp + 2 N, W)
+    mm.into(dx2, d_dbc, Wx, 1.f, 1.f);                                       // + the gradient through x_proj, in the GEMM's epilogue
+    mm.run();
     float *dcw = fptr(g.extra), *dcb = dcw + W * K;
     conv_backward(columns(xz, 0, W), cw, cb, g.dx, columns(dxz, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
 
@@ -225,18 +231,20 @@ struct BlockBackward : public torch::autograd::Node {
     std::vector<at::ScalarType> kt;                                        // what the conversion writes; anything else is cast after it
     for (auto t : types) kt.push_back(convertible(t) ? t : at::kFloat);
     Convert finish;
+    Products mm;
     std::vector<Tensor> alive;
     Tensor dy = rows(grads[0], dt);
     if (out_w.defined) {
       const Tensor w = out_w.get(), s2 = alias(y.get(), 0, {T, W}), d2 = dy.reshape({T, w.size(0)});
       const Tensor ds = empty({T, W}, dt, xz_);
-      product_into(ds, d2, w, scale, 0.f);
+      mm.into(ds, d2, w, scale, 0.f);
       dy = alias(ds, 0, {B, L, W});
       if (task_should_compute_output(kOutW)) {
-        const Partials dw = tall_product(d2, s2, kt[kOutW], scale);
+        const Partials dw = mm.tall(d2, s2, kt[kOutW], scale);
         out[kOutW] = finish.settle(dw, kt[kOutW]);
         alive.push_back(dw.t);
       }
+      mm.run();
     }
     const Tensor dxz = empty({B, L, 2 * W}, dt, xz_);
     for (size_t i = 0; i < dirs.size(); ++i) {
@@ -248,17 +256,18 @@ struct BlockBackward : public torch::autograd::Node {
     if (in_w.defined) {
       const Tensor w = in_w.get(), x2 = x.get(), d2 = alias(dxz, 0, {T, 2 * W});
       if (task_should_compute_output(kInW)) {
-        const Partials dw = tall_product(d2, x2, kt[kInW], 1.f);
+        const Partials dw = mm.tall(d2, x2, kt[kInW], 1.f);
         out[kInW] = finish.settle(dw, kt[kInW]);
         alive.push_back(dw.t);
       }
       if (task_should_compute_output(kX)) {
-        alive.push_back(alias(product(d2, w), 0, x_shape));
+        alive.push_back(alias(mm.of(d2, w), 0, x_shape));
         out[kX] = finish.cast(alive.back(), kt[kX]);
       }
     } else {
       out[kX] = dxz;
     }
+    mm.run();
     finish.run();
     for (size_t i = 0; i < out.size(); ++i)
       if (out[i].defined()) out[i] = like(out[i], types[i]);
@@ -310,12 +319,15 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
       dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N);
     }
     conv.run();
-    if (wi.defined()) xz = alias(product(x2, transposed(wi)), 0, {B, L, 2 * W});
+    Products mm;
+    if (wi.defined()) xz = alias(mm.of(x2, transposed(wi)), 0, {B, L, 2 * W});
+    mm.run();
     for (auto& d : dirs) d.forward(xz, R, N, grad);
     s = nd == 1 ? dirs[0].y : dirs[0].y + dirs[1].y;
     if (wo.defined()) {
       const Tensor o = empty({T, wo.size(0)}, dt, xz);
-      product_into(o, alias(s, 0, {T, W}), transposed(wo), scale, 0.f);
+      mm.into(o, alias(s, 0, {T, W}), transposed(wo), scale, 0.f);
+      mm.run();
       out = alias(o, 0, {B, L, wo.size(0)});
     } else {
       out = s;

@@ -132,8 +132,18 @@ struct Partials {
   int slices;
   int64_t rows, cols;
 };
-// a^T b for two tall matrices of one type (gemm.cpp); `out` is the type wanted if nothing has to be added up.
-Partials tall_product(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha);
+// `tall` is a^T b for two tall matrices of one type (gemm.cpp); `out` is the type wanted if nothing has to be added up.
+// Independent products in one place: the small ones are collected and share a launch (run()), the others go to the library at once.
+struct Products {
+  mb200_product p[4];
+  int n = 0;
+  at::ScalarType dt;
+  bool add(const Tensor& out, const Tensor& a, const Tensor& b, float alpha, float beta);       // false: not a small one
+  void into(const Tensor& out, const Tensor& a, const Tensor& b, float alpha, float beta);      // out = alpha * a b + beta * out
+  Tensor of(const Tensor& a, const Tensor& b);
+  Partials tall(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha);
+  void run();
+};
 
 // Up to 24 element-wise jobs in one launch (mb200_convert).
 struct Convert {
