@@ -53,23 +53,38 @@ __device__ __forceinline__ float ex2f(float x) {       // 2^x on the MUFU pipe
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Reciprocal and base-2 logarithm straight from the MUFU pipe: __fdividef and __log2f add scaling for results below 2^-126 and
+// arguments below 2^-126, which 1 + e^x never has.  With the packed forms below in the element-wise warps of the fused scans this
+// took their backward from 652 to 605 us and their forward from 195 to 189 (8 x 2048 x 1536, bfloat16): those warps share the
+// issue slots with the recurrences.  (A softplus_fast without its early return costs ssm_step_kernel registers and 4 us of 30.)
+__device__ __forceinline__ float rcpf(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float lg2f(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+constexpr float kLn2 = 0.6931471805599453f;
 __device__ __forceinline__ float softplusf(float x) {   // torch semantics: threshold 20
   return x > 20.f ? x : log1pf(__expf(x));
 }
 __device__ __forceinline__ float sigmoidf(float x) { return 1.f / (1.f + __expf(-x)); }
 // Cheaper forms for the streaming kernels: approximate reciprocal / logarithm, with a short
 // series where 1 + e^x would lose the small term to rounding.  Relative error below 1e-5.
-__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+__device__ __forceinline__ float sigmoid_fast(float x) { return rcpf(1.f + ex2f(-kLog2e * x)); }
 __device__ __forceinline__ float softplus_fast(float x) {
   if (x > 20.f) return x;
-  const float e = __expf(x);
-  return e < 1e-2f ? e * (1.f - e * (0.5f - e * (1.f / 3.f))) : __logf(1.f + e);
+  const float e = ex2f(kLog2e * x);
+  return e < 1e-2f ? e * (1.f - e * (0.5f - e * (1.f / 3.f))) : lg2f(1.f + e) * kLn2;
 }
 
 // Two-lane versions of softplus_fast and x*sigmoid_fast(x) on the packed f32x2 instructions (the MUFU
 // calls stay scalar): the per-element warps of the fused kernels are bound by instruction issue.
 __device__ __forceinline__ float2 softplus_fast2(float2 x) {
-  const float2 m = __fmul2_rn(x, make_float2(1.4426950408889634f, 1.4426950408889634f));
+  const float2 m = __fmul2_rn(x, make_float2(kLog2e, kLog2e));
   const float2 e = make_float2(ex2f(m.x), ex2f(m.y));
   // e*(1 - e*(1/2 - e/3)) where 1 + e would lose the small term, log(1 + e) elsewhere
   const float2 third = make_float2(-1.f / 3.f, -1.f / 3.f), half = make_float2(0.5f, 0.5f), one = make_float2(1.f, 1.f);
@@ -77,17 +92,27 @@ __device__ __forceinline__ float2 softplus_fast2(float2 x) {
   const float2 inner = __ffma2_rn(e, third, half);                       // 1/2 - e/3
   const float2 poly = __fmul2_rn(e, __ffma2_rn(__fmul2_rn(e, inner), nh, one));
   const float2 s = __fadd2_rn(e, one);
-  const float ln2 = 0.6931471805599453f;
-  const float2 lg = make_float2(__log2f(s.x) * ln2, __log2f(s.y) * ln2);
+  const float2 lg = __fmul2_rn(make_float2(lg2f(s.x), lg2f(s.y)), make_float2(kLn2, kLn2));
   float2 r;
   r.x = x.x > 20.f ? x.x : (e.x < 1e-2f ? poly.x : lg.x);
   r.y = x.y > 20.f ? x.y : (e.y < 1e-2f ? poly.y : lg.y);
   return r;
 }
 __device__ __forceinline__ float2 sigmoid_fast2(float2 x) {
-  const float2 m = __fmul2_rn(x, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+  const float2 m = __fmul2_rn(x, make_float2(-kLog2e, -kLog2e));
   const float2 d = __fadd2_rn(make_float2(ex2f(m.x), ex2f(m.y)), make_float2(1.f, 1.f));
-  return make_float2(__fdividef(1.f, d.x), __fdividef(1.f, d.y));
+  return make_float2(rcpf(d.x), rcpf(d.y));
+}
+
+// Two neighbouring elements (4-byte aligned in a vector in registers) as floats, and back: whole words for bfloat16.
+__device__ __forceinline__ float2 pair_f(const float* v) { return make_float2(v[0], v[1]); }
+__device__ __forceinline__ float2 pair_f(const __nv_bfloat16* v) {
+  const uint32_t u = *reinterpret_cast<const uint32_t*>(v);
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+__device__ __forceinline__ void pair_to(float* v, float2 f) { v[0] = f.x; v[1] = f.y; }
+__device__ __forceinline__ void pair_to(__nv_bfloat16* v, float2 f) {
+  *reinterpret_cast<__nv_bfloat162*>(v) = __floats2bfloat162_rn(f.x, f.y);
 }
 
 // ---- packed float2 arithmetic (one issue slot for two lanes of FMA work) ------------

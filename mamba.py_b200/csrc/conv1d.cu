@@ -84,7 +84,7 @@ __device__ __forceinline__ Pk<2> padd(Pk<2> a, Pk<2> b) { return {__fadd2_rn(a.v
 __device__ __forceinline__ Pk<2> psigmoid(Pk<2> a) {
   const float2 m = __fmul2_rn(a.v, make_float2(-kLog2e, -kLog2e));
   const float2 d = __fadd2_rn(make_float2(ex2f(m.x), ex2f(m.y)), make_float2(1.f, 1.f));
-  return {make_float2(__fdividef(1.f, d.x), __fdividef(1.f, d.y))};
+  return {make_float2(rcpf(d.x), rcpf(d.y))};
 }
 // V raw elements <-> V/W packs
 template <typename T, int V, int W>
@@ -92,7 +92,7 @@ __device__ __forceinline__ void unpack(const CVec<T, V>& r, Pk<W> (&o)[V / W]) {
 #pragma unroll
   for (int i = 0; i < V / W; ++i) {
     if constexpr (W == 1) o[i].v = Elem<T>::to_f(r.v[i]);
-    else o[i].v = make_float2(Elem<T>::to_f(r.v[2 * i]), Elem<T>::to_f(r.v[2 * i + 1]));
+    else o[i].v = pair_f(&r.v[2 * i]);
   }
 }
 template <typename T, int V, int W>

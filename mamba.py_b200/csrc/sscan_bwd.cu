@@ -342,15 +342,15 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         float dyo[4];
 #pragma unroll
         for (int k = 0; k < 4; k += 2) {                   // two channels at a time (packed arithmetic)
-          float2 dv = make_float2(Elem<T>::to_f(dv4.v[k]), Elem<T>::to_f(dv4.v[k + 1]));
+          float2 dv = pair_f(&dv4.v[k]);
           if (softplus) dv = softplus_fast2(__fadd2_rn(dv, make_float2(bias4[k], bias4[k + 1])));
           if (rr >= rows_ok) dv = make_float2(0.f, 0.f);
-          const float2 dx2 = __fmul2_rn(dv, make_float2(Elem<T>::to_f(xv.v[k]), Elem<T>::to_f(xv.v[k + 1])));
+          const float2 dx2 = __fmul2_rn(dv, pair_f(&xv.v[k]));
           o[k] = make_float2(dv.x, dx2.x);
           o[k + 1] = make_float2(dv.y, dx2.y);
-          float2 g = make_float2(Elem<T>::to_f(yv4.v[k]), Elem<T>::to_f(yv4.v[k + 1]));
+          float2 g = pair_f(&yv4.v[k]);
           if (has_z) {
-            const float2 zf = make_float2(Elem<T>::to_f(zv4.v[k]), Elem<T>::to_f(zv4.v[k + 1]));
+            const float2 zf = pair_f(&zv4.v[k]);
             g = __fmul2_rn(g, __fmul2_rn(zf, sigmoid_fast2(zf)));
           }
           dyo[k] = g.x;
@@ -421,8 +421,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
     T* odx = static_cast<T*>(p.dx) + b * p.dx_sb + e0 + c0;
     T* odd = static_cast<T*>(p.ddelta) + b * p.dd_sb + e0 + c0;
     T* odz = has_z ? static_cast<T*>(p.dz) + b * p.dz_sb + e0 + c0 : nullptr;
-    const float Dv[2] = {s_D[c0], s_D[c0 + 1]};
-    float dDacc[2] = {0.f, 0.f}, dbacc[2] = {0.f, 0.f};
+    const float2 Dv = make_float2(s_D[c0], s_D[c0 + 1]);
+    float2 dDacc = make_float2(0.f, 0.f), dbacc = dDacc;
     for (int j = 0; j < ntiles; ++j) {
       const int t0 = tile_t0(j);
       if (!mbar_wait(&raw_full[j % kStages], int((j / kStages) & 1))) { fail(); return; }
@@ -456,34 +456,31 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
           const Vec2<T> xv = *reinterpret_cast<const Vec2<T>*>(rx + tt * kBTE + c0);
           const float4 o4 = *reinterpret_cast<const float4*>(opt + op_index(tt, c0, kBTE));   // {delta, delta*x} x 2
           const float2 dyg2 = *reinterpret_cast<const float2*>(dyt + tt * kBTE + c0);
-          const float dvs[2] = {o4.x, o4.z}, dygs[2] = {dyg2.x, dyg2.y};
           const Vec2<T> yv2 = *reinterpret_cast<const Vec2<T>*>(rdy + tt * kBTE + c0);
           Vec2<T> zv2 = yv2;
           if (has_z) zv2 = *reinterpret_cast<const Vec2<T>*>(rz + tt * kBTE + c0);
           Vec2<T> ox, od, oz;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const float xf = Elem<T>::to_f(xv.v[k]), dyf = Elem<T>::to_f(yv2.v[k]);
-            const float dv = dvs[k], dyg = dygs[k];
-            // d softplus = sigmoid(raw) = 1 - exp(-softplus(raw)); series where the difference cancels
-            float spg = 1.f;
-            if (softplus) spg = dv < 1e-2f ? dv * (1.f - dv * (0.5f - dv * (1.f / 6.f))) : 1.f - __expf(-dv);
-            float dzv = 0.f;
-            if (has_z) {
-              const float zf = Elem<T>::to_f(zv2.v[k]);
-              const float sg = sigmoid_fast(zf);
-              dzv = dyf * fmaf(Dv[k], xf, ys[k]) * sg * (1.f + zf * (1.f - sg));
-            }
-            const float dxv = fmaf(dyg, Dv[k], dv * gBs[k]);
-            const float ddv = fmaf(xf, gBs[k], wAs[k] * (1.f / kLog2e)) * spg;
-            if (c0 + k < cols_ok) {
-              dDacc[k] = fmaf(dyg, xf, dDacc[k]);
-              dbacc[k] += ddv;
-            }
-            ox.v[k] = Elem<T>::from_f(dxv);
-            od.v[k] = Elem<T>::from_f(ddv);
-            oz.v[k] = Elem<T>::from_f(dzv);
+          const float2 xf = pair_f(&xv.v[0]), dv = make_float2(o4.x, o4.z), gB = make_float2(gBs[0], gBs[1]);
+          const float2 one = make_float2(1.f, 1.f), mone = make_float2(-1.f, -1.f);
+          if (has_z) {
+            // dz = dy (y + D x) sg (1 + z (1 - sg))
+            const float2 zf = pair_f(&zv2.v[0]), sg = sigmoid_fast2(zf);
+            const float2 yd = __fmul2_rn(pair_f(&yv2.v[0]), __ffma2_rn(Dv, xf, make_float2(ys[0], ys[1])));
+            pair_to(&oz.v[0], __fmul2_rn(__fmul2_rn(yd, sg), __ffma2_rn(zf, __ffma2_rn(sg, mone, one), one)));
           }
+          pair_to(&ox.v[0], __ffma2_rn(dyg2, Dv, __fmul2_rn(dv, gB)));
+          float2 dd = __ffma2_rn(xf, gB, __fmul2_rn(make_float2(wAs[0], wAs[1]), make_float2(1.f / kLog2e, 1.f / kLog2e)));
+          if (softplus) {
+            // d softplus = sigmoid(raw) = 1 - exp(-softplus(raw)); series where the difference cancels
+            const float2 m = __fmul2_rn(dv, make_float2(-kLog2e, -kLog2e));
+            const float2 far = __ffma2_rn(make_float2(ex2f(m.x), ex2f(m.y)), mone, one);
+            const float2 inner = __ffma2_rn(dv, make_float2(-1.f / 6.f, -1.f / 6.f), make_float2(0.5f, 0.5f));
+            const float2 near = __fmul2_rn(dv, __ffma2_rn(__fmul2_rn(dv, inner), mone, one));
+            dd = __fmul2_rn(dd, make_float2(dv.x < 1e-2f ? near.x : far.x, dv.y < 1e-2f ? near.y : far.y));
+          }
+          dDacc = __ffma2_rn(dyg2, xf, dDacc);               // of channels past the end: never added up
+          dbacc = __fadd2_rn(dbacc, dd);
+          pair_to(&od.v[0], dd);
           if (c0 + 2 <= cols_ok) {
             *reinterpret_cast<Vec2<T>*>(odx + t * p.dx_sl) = ox;
             *reinterpret_cast<Vec2<T>*>(odd + t * p.dd_sl) = od;
@@ -501,8 +498,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       if (c0 + k < cols_ok) {
-        if (p.dD) atomicAdd(p.dD + e0 + c0 + k, dDacc[k]);
-        if (p.ddelta_bias) atomicAdd(p.ddelta_bias + e0 + c0 + k, dbacc[k]);
+        if (p.dD) atomicAdd(p.dD + e0 + c0 + k, k ? dDacc.y : dDacc.x);
+        if (p.ddelta_bias) atomicAdd(p.ddelta_bias + e0 + c0 + k, k ? dbacc.y : dbacc.x);
       }
     }
   }

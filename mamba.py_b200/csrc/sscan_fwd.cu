@@ -441,20 +441,21 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
         }
         float2 o[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float dv = Elem<T>::to_f(dv4.v[k]);
-          if (softplus) dv = softplus_fast(dv + s_bias[cc + k]);
-          if (rr >= rows_ok) dv = 0.f;                      // past the end of the sequence
+        for (int k = 0; k < 4; k += 2) {
+          float2 dv = pair_f(&dv4.v[k]);
+          if (softplus) dv = softplus_fast2(__fadd2_rn(dv, make_float2(s_bias[cc + k], s_bias[cc + k + 1])));
+          if (rr >= rows_ok) dv = make_float2(0.f, 0.f);    // past the end of the sequence
+          float2 g = pair_f(&xv.v[k]);                      // x, or dy in its place
           if constexpr (kCarry) {
-            float g = Elem<T>::to_f(xv.v[k]);               // dy in the place of x
             if (has_z) {
-              const float zf = Elem<T>::to_f(zv4.v[k]);
-              g *= zf * sigmoid_fast(zf);
+              const float2 zf = pair_f(&zv4.v[k]);
+              g = __fmul2_rn(g, __fmul2_rn(zf, sigmoid_fast2(zf)));
             }
-            o[k] = make_float2(dv, g);
           } else {
-            o[k] = make_float2(dv, dv * Elem<T>::to_f(xv.v[k]));
+            g = __fmul2_rn(dv, g);
           }
+          o[k] = make_float2(dv.x, g.x);
+          o[k + 1] = make_float2(dv.y, g.y);
         }
         *reinterpret_cast<float4*>(tile + op_index(rr, cc, kTE)) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
         *reinterpret_cast<float4*>(tile + op_index(rr, cc + 2, kTE)) = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
@@ -511,13 +512,14 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
         }
         Vec4<T> out;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          float yv = fmaf(s_D[cc + k], Elem<T>::to_f(xv.v[k]), s4[k]);
+        for (int k = 0; k < 4; k += 2) {
+          const float2 xf = pair_f(&xv.v[k]);
+          float2 yv = __ffma2_rn(make_float2(s_D[cc + k], s_D[cc + k + 1]), xf, make_float2(s4[k], s4[k + 1]));
           if (has_z) {
-            const float zf = Elem<T>::to_f(zv.v[k]);
-            yv *= zf * sigmoid_fast(zf);
+            const float2 zf = pair_f(&zv.v[k]);
+            yv = __fmul2_rn(yv, __fmul2_rn(zf, sigmoid_fast2(zf)));
           }
-          out.v[k] = Elem<T>::from_f(yv);
+          pair_to(&out.v[k], yv);
         }
         T* dst = gy + int64_t(t0 + rr) * p.y_sl + cc;
         if (cc + 4 <= cols_ok) {
