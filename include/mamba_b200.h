@@ -325,6 +325,11 @@ typedef struct {
 } mb200_convert_job;
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
+/* mb200_conv_step_params with up to 3 conversions in the same launch. */
+int mb200_conv_step_convert(const void* xin, const void* conv_in, const void* w, int w_dtype, const void* bias, int bias_dtype, void* xc,
+                            void* conv_out, int64_t B, int64_t ED, int K, int64_t x_sb, int dtype, const mb200_convert_job* jobs, int n_jobs,
+                            void* stream);
+
 /* Up to 4 independent matrix products in one launch, out = alpha * a b + beta * out, for sizes that are all launch latency.
  * a (M, K) and b (K, N) have any strides (elements; rm: of m, ck: of k, rk: of k, cn: of n) and type `dtype`; out has unit-stride rows.
  * float32 accumulation. */

@@ -45,7 +45,8 @@ struct WindowStep {
   Tensor xc, window;
 };
 
-WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const Tensor& bias_, bool inplace) {
+WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const Tensor& bias_, bool inplace,
+                       const mb200_convert_job* jobs = nullptr, int n_jobs = 0) {
   const auto dt = act_dtype(x);
   const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), w = small_param(weight), bias = small_param(bias_);
   const int64_t n = xs.size(0), W = xs.size(1);
@@ -57,8 +58,8 @@ WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weig
   } else {
     o.window = empty(win.sizes(), dt, xs);
   }
-  check(mb200_conv_step_params(ptr(xs), ptr(win), ptr(w), code_of(w), ptr(bias), code_of(bias), ptr(o.xc), ptr(o.window), n, W,
-                               int(w.size(-1)), st(xs, 0), dtype_code(dt), cuda_stream()),
+  check(mb200_conv_step_convert(ptr(xs), ptr(win), ptr(w), code_of(w), ptr(bias), code_of(bias), ptr(o.xc), ptr(o.window), n, W,
+                                int(w.size(-1)), st(xs, 0), dtype_code(dt), jobs, n_jobs, cuda_stream()),
         "mb200_conv_step");
   return o;
 }
@@ -153,34 +154,28 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
   };
   const Tensor xz = project(x, in_w, in_b_);
   WindowStep w;
+  // the exponentials of A_log and the casts are worth doing once as soon as enough rows share them
+  const bool once = B >= 32 && small_type(A_log) && small_type(D) && small_type(dt_b) && A_log.is_contiguous() && D.is_contiguous() &&
+                    dt_b.is_contiguous();
+  Tensor A = A_log, Df = D, bf = dt_b;
   {
     const BelowAutograd guard_ad;
-    w = window_step(xz.narrow(1, 0, W), inputs, conv_w, conv_b, false);
+    Convert conv;
+    if (once) {
+      A = empty(A_log.sizes(), at::kFloat, A_log);
+      const int64_t n = A.numel();
+      conv.add(ptr(A_log), A_log.scalar_type(), ptr(A), at::kFloat, 1, n, n, n, n, MB200_CONVERT_NEG_EXP);
+      Df = conv.cast(D, at::kFloat);
+      bf = conv.cast(dt_b, at::kFloat);
+    }
+    w = window_step(columns(xz, 0, W), inputs, conv_w, conv_b, false, conv.jobs, conv.n);
   }
   const Tensor dbc = project(w.xc, xproj_w, {});
-  const Tensor delta = project(dbc.narrow(1, 0, R), dt_w, {});               // bias and softplus happen in the kernel
+  const Tensor delta = project(direct ? columns(dbc, 0, R) : dbc.narrow(1, 0, R), dt_w, {});               // bias and softplus happen in the kernel
   StateStep s;
   {
     const BelowAutograd guard_ad;
-    // the exponentials of A_log and the casts are worth a launch of their own once enough rows share them
-    const bool once = B >= 32 && small_type(A_log) && small_type(D) && small_type(dt_b) && A_log.is_contiguous() && D.is_contiguous() &&
-                      dt_b.is_contiguous();
-    Tensor A = A_log, Df = D, bf = dt_b;
-    if (once) {
-      mb200_convert_job jobs[3];
-      int n_jobs = 0;
-      auto add = [&](const Tensor& src, int op) {
-        const Tensor dst = empty(src.sizes(), at::kFloat, src);
-        const int64_t n = src.numel();
-        jobs[n_jobs++] = mb200_convert_job{ptr(src), ptr(dst), nullptr, 1, n, n, n, n, code_of(src), MB200_F32, op, 1, 0};
-        return dst;
-      };
-      A = add(A_log, MB200_CONVERT_NEG_EXP);
-      if (D.scalar_type() != at::kFloat) Df = add(D, MB200_CONVERT_COPY);
-      if (dt_b.scalar_type() != at::kFloat) bf = add(dt_b, MB200_CONVERT_COPY);
-      check(mb200_convert(jobs, n_jobs, cuda_stream()), "mb200_convert");
-    }
-    s = state_step(w.xc, h, delta, A, !once, dbc.narrow(1, R, N), dbc.narrow(1, R + N, N), Df, xz.narrow(1, W, W), bf, false);
+    s = state_step(w.xc, h, delta, A, !once, columns(dbc, R, N), columns(dbc, R + N, N), Df, columns(xz, W, W), bf, false);
   }
   return {project(s.y, out_w, out_b_), s.h, w.window};
 }

@@ -6,13 +6,14 @@
 // state (so a warp reads 512 contiguous bytes of h), computes its four decays and partial
 // C-contraction, and the lanes of a channel combine with warp shuffles.
 #include <initializer_list>
-#include "common.cuh"
+#include "convert.cuh"
 #include "sscan.cuh"
 
 namespace mb200 {
 namespace {
 
 constexpr int kStepThreads = 256;
+constexpr int kStepJobs = 3;                  // conversions a conv step takes along
 
 // States per lane.  The work per (batch row, channel) - softplus, the gate, index arithmetic - is repeated
 // by every lane of the channel, and the kernel is bound as much by instruction issue as by memory, so
@@ -146,12 +147,18 @@ __global__ void conv_step_kernel(const T* __restrict__ xin, const T* __restrict_
 }
 
 // Same for the common d_conv = 4: a thread owns 4 neighbouring channels, so the 3-wide windows of
-// those channels (12 contiguous elements) and the new inputs move as 8- or 16-byte vectors.
+// those channels (12 contiguous elements) and the new inputs move as 8- or 16-byte vectors.  Rows of blocks past the batch
+// work on `jobs`, the parameter conversions of the state update that follows: a launch of their own cost 2.3 us and its gap.
 template <typename T>
 __global__ void __launch_bounds__(256)
 conv_step_k4_kernel(const T* __restrict__ xin, const T* __restrict__ conv_in, const Param w,
                     const Param bias, T* __restrict__ xc, T* __restrict__ conv_out,
-                    int64_t ED, int64_t x_sb) {
+                    int64_t B, int64_t ED, int64_t x_sb, const __grid_constant__ Jobs<kStepJobs> jobs) {
+  if (blockIdx.y >= B) {
+    const int block = int((blockIdx.y - B) * gridDim.x + blockIdx.x);
+    if (block < jobs.first_block[jobs.n]) convert_block(jobs, block);
+    return;
+  }
   const int64_t e = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   const int64_t b = blockIdx.y;
   if (e >= ED) return;
@@ -338,9 +345,9 @@ extern "C" int mb200_ssm_step(const void* x, const void* delta, const void* z, c
                                d_sb, z_sb, b_sb, c_sb, y_sb, dtype, flags, stream);
 }
 
-extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype,
-                                      const void* bias, int bias_dtype, void* xc, void* conv_out, int64_t B, int64_t ED,
-                                      int K, int64_t x_sb, int dtype, void* stream) {
+extern "C" int mb200_conv_step_convert(const void* xin, const void* conv_in, const void* w, int w_dtype,
+                                       const void* bias, int bias_dtype, void* xc, void* conv_out, int64_t B, int64_t ED,
+                                       int K, int64_t x_sb, int dtype, const mb200_convert_job* jobs, int n_jobs, void* stream) {
   if (B < 0 || ED < 0 || K < 1) return MB200_EINVAL;
   if (K > 8) return MB200_ETOOBIG;
   for (int d : {dtype, w_dtype, bias_dtype})
@@ -349,20 +356,28 @@ extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, cons
   if (!xin || !w || !xc || (K > 1 && (!conv_in || !conv_out))) return MB200_EINVAL;
   if (B > 65535) return MB200_ETOOBIG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  Jobs<kStepJobs> all;
+  int64_t blocks = 0;
+  if (const int rc = collect_jobs(jobs, n_jobs, all, blocks)) return rc;
   const int es = dtype == MB200_F32 ? 4 : 2;
   const Param pw{w, w_dtype}, pb{bias, bias_dtype};
   if (K == 4 && ED % 4 == 0 && aligned16(xin) && aligned16(conv_in) && aligned16(conv_out) && aligned16(xc) &&
       aligned16(w) && (x_sb * es) % 16 == 0) {
     dim3 g4(unsigned((ED / 4 + 255) / 256), unsigned(B));
+    const int64_t extra = (blocks + g4.x - 1) / g4.x;
+    const bool along = B + extra <= 65535;
+    if (along) g4.y += unsigned(extra);
+    else if (const int rc = mb200_convert(jobs, n_jobs, stream)) return rc;
     if (dtype == MB200_F32)
       conv_step_k4_kernel<float><<<g4, 256, 0, st>>>((const float*)xin, (const float*)conv_in, pw, pb,
-                                                     (float*)xc, (float*)conv_out, ED, x_sb);
+                                                     (float*)xc, (float*)conv_out, B, ED, x_sb, all);
     else
       conv_step_k4_kernel<__nv_bfloat16><<<g4, 256, 0, st>>>(
           (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, pw, pb, (__nv_bfloat16*)xc,
-          (__nv_bfloat16*)conv_out, ED, x_sb);
+          (__nv_bfloat16*)conv_out, B, ED, x_sb, all);
     return check_launch();
   }
+  if (const int rc = mb200_convert(jobs, n_jobs, stream)) return rc;
   dim3 grid(unsigned((ED + 255) / 256), unsigned(B));
   if (dtype == MB200_F32)
     conv_step_kernel<float><<<grid, 256, 0, st>>>((const float*)xin, (const float*)conv_in, pw, pb,
@@ -372,6 +387,12 @@ extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, cons
         (const __nv_bfloat16*)xin, (const __nv_bfloat16*)conv_in, pw, pb, (__nv_bfloat16*)xc,
         (__nv_bfloat16*)conv_out, ED, K, x_sb);
   return check_launch();
+}
+
+extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype,
+                                      const void* bias, int bias_dtype, void* xc, void* conv_out, int64_t B, int64_t ED,
+                                      int K, int64_t x_sb, int dtype, void* stream) {
+  return mb200_conv_step_convert(xin, conv_in, w, w_dtype, bias, bias_dtype, xc, conv_out, B, ED, K, x_sb, dtype, nullptr, 0, stream);
 }
 
 extern "C" int mb200_conv_step(const void* xin, const void* conv_in, const float* w,
