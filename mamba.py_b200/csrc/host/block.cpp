@@ -62,22 +62,22 @@ struct Direction {
   Tensor A, D, bias, cw, cb, Wx, Wdt;                       // the parameters as the kernels take them
   Tensor y;
 
-  // Queues the parameters' conversions; run them before `forward`.
-  void prepare(Convert& conv, const Tensor* p, at::ScalarType dt, int64_t W, int64_t R, int64_t N) {
+  // Queues the parameters' conversions, the projections' into the given places if there are any.
+  void prepare(Convert& conv, const Tensor* p, at::ScalarType dt, int64_t W, int64_t R, int64_t N, const Tensor& wx_at, const Tensor& wdt_at) {
     const int64_t Rp = padded_rank(R, dt), K = p[kConvW].size(-1);
     const Tensor wx = param(p[kXproj]), wdt = param(p[kDtW]), alog = param(p[kALog]);
     keep = {wx, wdt, alog};
     A = empty({W, N}, at::kFloat, wx);
     conv.add(ptr(alog), alog.scalar_type(), ptr(A), at::kFloat, 1, W * N, W * N, W * N, W * N, MB200_CONVERT_NEG_EXP);
-    if (Rp != R) {
-      Wx = empty({Rp + 2 * N, W}, dt, wx);
+    if (Rp != R || wx_at.defined()) {
+      Wx = wx_at.defined() ? wx_at : empty({Rp + 2 * N, W}, dt, wx);
       char* d = static_cast<char*>(ptr(Wx));
       const int64_t es = Wx.element_size();
       conv.add(ptr(wx), wx.scalar_type(), d, dt, 1, R * W, R * W, R * W, R * W);
       conv.add(nullptr, dt, d + R * W * es, dt, 1, (Rp - R) * W, 0, 0, 0);
       conv.add(static_cast<char*>(ptr(wx)) + R * W * wx.element_size(), wx.scalar_type(), d + Rp * W * es, dt, 1, 2 * N * W, 2 * N * W, 2 * N * W,
                2 * N * W);
-      Wdt = empty({W, Rp}, dt, wx);
+      Wdt = wdt_at.defined() ? wdt_at : empty({W, Rp}, dt, wx);
       conv.add(ptr(wdt), wdt.scalar_type(), ptr(Wdt), dt, W, Rp, R, R, Rp);
     } else {
       Wx = conv.cast(wx, dt);
@@ -94,17 +94,10 @@ struct Direction {
     bias = f32_param(p[kDtB]);
   }
 
-  void forward(const Tensor& xz, int64_t R, int64_t N, bool grad) {
-    const int64_t B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, xz.scalar_type()), cols = Rp + 2 * N;
-    keep.clear();
-    xc = empty({B, L, W}, xz.scalar_type(), xz);
-    conv_forward(columns(xz, 0, W), cw, cb, xc, reverse);
-    Products mm;
-    const Tensor dbc2 = mm.of(alias(xc, 0, {T, W}), transposed(Wx));
-    mm.run();
-    delta = alias(mm.of(columns(dbc2, 0, Rp), transposed(Wdt)), 0, {B, L, W});
-    mm.run();                                                                // bias and softplus happen in the kernel
-    dbc = alias(dbc2, 0, {B, L, cols});
+  void release() { keep.clear(); }                          // once the conversions have been launched
+  // The scan of xc, delta and dbc (B, L, Rp + 2 N), which the projections have filled.
+  void scan(const Tensor& xz, int64_t Rp, int64_t N, bool grad) {
+    const int64_t B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2;
     ScanArgs a{xc, delta, A, columns(dbc, Rp, N), columns(dbc, Rp + N, N), D, columns(xz, W, W), bias, Tensor(), reverse};
     S = reverse ? 1 : cuttable(a, pick_pieces(B, L, W, grad), grad, false);
     ScanOut o;
@@ -118,30 +111,18 @@ struct Direction {
     P = o.P;
   }
 
-  // d(xz) of this direction into dxz (B, L, 2 W); the parameters' gradients into out[kDirParams], of types kt, by way of the jobs
-  // queued in `finish`, whose sources stay alive in `alive`.
-  void backward(const Tensor& xz, Tensor dy, const Tensor& dxz, int64_t R, int64_t N, const at::ScalarType* kt, const std::vector<int64_t>& cw_shape,
-                Tensor* out, Convert& finish, std::vector<Tensor>& alive) const {
-    const auto dt = xc.scalar_type();
-    const int64_t B = xc.size(0), L = xc.size(1), W = xc.size(2), T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N, K = cw.size(1);
+  ScanGrads scan_back(const Tensor& xz, Tensor dy, const ScanSinks& to, int64_t Rp, int64_t N) const {
+    const int64_t W = xc.size(2);
     if ((reverse || S > 1) && !tensor_map_ok(dy)) dy = dy.contiguous();
     const ScanArgs a{xc, delta, A, columns(dbc, Rp, N), columns(dbc, Rp + N, N), D, columns(xz, W, W), bias, Tensor(), reverse};
-    ScanGrads g = scan_backward(a, S, dy, carries, P, false, columns(dxz, W, W), W * K + W);
-    const Tensor d_dbc = empty({T, cols}, dt, xz), dd2 = alias(g.dd, 0, {T, W}), xc2 = alias(xc, 0, {T, W}), dx2 = alias(g.dx, 0, {T, W});
-    auto col = [&](int64_t c) { return static_cast<char*>(d_dbc.data_ptr()) + c * d_dbc.element_size(); };
-    Convert acc;
-    acc.add(ptr(g.dB), at::kFloat, col(Rp), dt, T, N, N, N, cols);          // float32 accumulators -> activation dtype, in place
-    acc.add(ptr(g.dC), at::kFloat, col(Rp + N), dt, T, N, N, N, cols);
-    acc.run();
-    const Tensor d_dt = columns(d_dbc, 0, Rp);
-    Products mm;
-    mm.into(d_dt, dd2, Wdt, 1.f, 0.f);                                       // through dt_proj
-    const int64_t Rw = R % 4 == 0 ? R : Rp;                                  // rows of dWdt on the 16-byte grid
-    const Partials dWdt = mm.tall(dd2, columns(alias(dbc, 0, {T, cols}), 0, Rw), kt[kDtW], 1.f);        // (W, Rw)
-    mm.run();
-    const Partials dWx = mm.tall(d_dbc, xc2, kt[kXproj], 1.f);                                          // (Rp + 2 N, W)
-    mm.into(dx2, d_dbc, Wx, 1.f, 1.f);                                       // + the gradient through x_proj, in the GEMM's epilogue
-    mm.run();
+    return scan_backward(a, S, dy, carries, P, false, to);
+  }
+
+  // The convolution's backward into dxz (B, L, 2 W); the parameters' gradients into out[kDirParams], of types kt, by way of the jobs
+  // queued in `finish`, whose sources stay alive in `alive`.
+  void finish_back(const Tensor& xz, const ScanGrads& g, const Partials& dWx, const Partials& dWdt, const Tensor& dxz, int64_t R, int64_t N,
+                   const at::ScalarType* kt, const std::vector<int64_t>& cw_shape, Tensor* out, Convert& finish, std::vector<Tensor>& alive) const {
+    const int64_t W = xc.size(2), Rp = padded_rank(R, xc.scalar_type()), K = cw.size(1);
     float *dcw = fptr(g.extra), *dcb = dcw + W * K;
     conv_backward(columns(xz, 0, W), cw, cb, g.dx, columns(dxz, 0, W), dcw, cb.defined() ? dcb : nullptr, reverse);
 
@@ -162,19 +143,16 @@ struct Direction {
     finish.add(ptr(g.dA), at::kFloat, ptr(out[kALog]), kt[kALog], 1, W * N, W * N, W * N, W * N, MB200_CONVERT_MUL).factor = fptr(A);
     if (Rp == R) {
       out[kXproj] = finish.settle(dWx, kt[kXproj]);
+      out[kDtW] = finish.settle(dWdt, kt[kDtW]);
     } else {
       out[kXproj] = empty({R + 2 * N, W}, kt[kXproj], xz);
       char* wx = static_cast<char*>(ptr(out[kXproj]));
       finish.rows_of(dWx, 0, R, wx, kt[kXproj]);
       finish.rows_of(dWx, Rp, 2 * N, wx + R * W * out[kXproj].element_size(), kt[kXproj]);
-    }
-    if (Rw == R) {
-      out[kDtW] = finish.settle(dWdt, kt[kDtW]);
-    } else {
       out[kDtW] = empty({W, R}, kt[kDtW], xz);
-      mb200_convert_job& j = finish.add(ptr(dWdt.t), dWdt.t.scalar_type(), ptr(out[kDtW]), kt[kDtW], W, R, R, Rw, R);
+      mb200_convert_job& j = finish.add(ptr(dWdt.t), dWdt.t.scalar_type(), ptr(out[kDtW]), kt[kDtW], W, R, R, Rp, R);
       j.slices = dWdt.slices;
-      j.slice_stride = W * Rw;
+      j.slice_stride = W * Rp;
     }
     alive.insert(alive.end(), {dWx.t, dWdt.t, g.dA, g.extra});
   }
@@ -182,6 +160,58 @@ struct Direction {
  private:
   std::vector<Tensor> keep;                                 // sources of the queued conversions
 };
+
+// Both directions go through every projection together: their operands lie one behind the other, and two products of one shape are
+// one launch.
+void directions_forward(std::vector<Direction>& dirs, const Tensor& xz, int64_t R, int64_t N, bool grad) {
+  const auto dt = xz.scalar_type();
+  const int64_t n = int64_t(dirs.size()), B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N;
+  const Tensor xc = empty({n, T, W}, dt, xz), delta = empty({n, T, W}, dt, xz), dbc = empty({n, T, cols}, dt, xz);
+  for (int64_t i = 0; i < n; ++i) {
+    Direction& d = dirs[i];
+    d.xc = alias(xc, i * T * W, {B, L, W});
+    d.delta = alias(delta, i * T * W, {B, L, W});
+    d.dbc = alias(dbc, i * T * cols, {B, L, cols});
+    conv_forward(columns(xz, 0, W), d.cw, d.cb, d.xc, d.reverse);
+  }
+  const Tensor xc0 = alias(xc, 0, {T, W}), dbc0 = alias(dbc, 0, {T, cols});
+  Products mm;
+  mm.each(n, dbc0, T * cols, xc0, T * W, transposed(dirs[0].Wx), cols * W, 1.f, 0.f);
+  mm.run();
+  mm.each(n, alias(delta, 0, {T, W}), T * W, columns(dbc0, 0, Rp), T * cols, transposed(dirs[0].Wdt), W * Rp, 1.f, 0.f);
+  mm.run();                                                                  // bias and softplus happen in the kernel
+  for (Direction& d : dirs) d.scan(xz, Rp, N, grad);
+}
+
+// d(xz) of direction i into dxz[i]; out and kt hold kDirParams entries per direction.
+void directions_backward(const std::vector<Direction>& dirs, const Tensor& xz, const Tensor& dy, const std::vector<Tensor>& dxz, int64_t R, int64_t N,
+                         const at::ScalarType* kt, const std::vector<std::vector<int64_t>>& cw_shape, Tensor* out, Convert& finish,
+                         std::vector<Tensor>& alive) {
+  const auto dt = xz.scalar_type();
+  const int64_t n = int64_t(dirs.size()), B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N;
+  const Tensor dx = empty({n, T, W}, dt, xz), dd = empty({n, T, W}, dt, xz), d_dbc = empty({n, T, cols}, dt, xz);
+  std::vector<ScanGrads> g;
+  Convert acc;
+  for (int64_t i = 0; i < n; ++i) {
+    const ScanSinks to{columns(dxz[i], W, W), alias(dx, i * T * W, {B, L, W}), alias(dd, i * T * W, {B, L, W}), W * dirs[i].cw.size(1) + W};
+    g.push_back(dirs[i].scan_back(xz, dy, to, Rp, N));
+    char* row = static_cast<char*>(d_dbc.data_ptr()) + i * T * cols * d_dbc.element_size();
+    acc.add(ptr(g[i].dB), at::kFloat, row + Rp * d_dbc.element_size(), dt, T, N, N, N, cols);   // float32 accumulators -> activation dtype
+    acc.add(ptr(g[i].dC), at::kFloat, row + (Rp + N) * d_dbc.element_size(), dt, T, N, N, N, cols);
+  }
+  acc.run();
+  const Tensor d0 = alias(d_dbc, 0, {T, cols}), dd0 = alias(dd, 0, {T, W}), dx0 = alias(dx, 0, {T, W}), xc0 = alias(dirs[0].xc, 0, {T, W}),
+               dbc0 = alias(dirs[0].dbc, 0, {T, cols});
+  Products mm;
+  mm.each(n, columns(d0, 0, Rp), T * cols, dd0, T * W, dirs[0].Wdt, W * Rp, 1.f, 0.f);          // through dt_proj
+  const auto dWdt = mm.tall(n, dd0, T * W, columns(dbc0, 0, Rp), T * cols, kt[kDtW], 1.f);      // (W, Rp)
+  mm.run();
+  const auto dWx = mm.tall(n, d0, T * cols, xc0, T * W, kt[kXproj], 1.f);                       // (Rp + 2 N, W)
+  mm.each(n, dx0, T * W, d0, T * cols, dirs[0].Wx, cols * W, 1.f, 1.f);      // + the gradient through x_proj, in the GEMM's epilogue
+  mm.run();
+  for (int64_t i = 0; i < n; ++i)
+    dirs[i].finish_back(xz, g[i], dWx[i], dWdt[i], dxz[i], R, N, kt + i * kDirParams, cw_shape[i], out + i * kDirParams, finish, alive);
+}
 
 enum { kX, kInW, kOutW, kBlockInputs };                     // then kDirParams per direction
 
@@ -246,13 +276,17 @@ struct BlockBackward : public torch::autograd::Node {
       }
       mm.run();
     }
-    const Tensor dxz = empty({B, L, 2 * W}, dt, xz_);
-    for (size_t i = 0; i < dirs.size(); ++i) {
-      const Tensor d = i == 0 ? dxz : empty({B, L, 2 * W}, dt, xz_);
-      const int first = kBlockInputs + int(i) * kDirParams;
-      dirs[i].get().backward(xz_, dy, d, R, N, kt.data() + first, dirs[i].cw_shape, out.data() + first, finish, alive);
-      if (i > 0) dxz.add_(d);
+    std::vector<Direction> ds;
+    std::vector<Tensor> each;
+    std::vector<std::vector<int64_t>> cw_shape;
+    for (const SavedDirection& d : dirs) {
+      ds.push_back(d.get());
+      each.push_back(empty({B, L, 2 * W}, dt, xz_));
+      cw_shape.push_back(d.cw_shape);
     }
+    directions_backward(ds, xz_, dy, each, R, N, kt.data() + kBlockInputs, cw_shape, out.data() + kBlockInputs, finish, alive);
+    const Tensor dxz = each[0];
+    if (each.size() > 1) dxz.add_(each[1]);
     if (in_w.defined) {
       const Tensor w = in_w.get(), x2 = x.get(), d2 = alias(dxz, 0, {T, 2 * W});
       if (task_should_compute_output(kInW)) {
@@ -314,15 +348,19 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
       if ((nd > 1 || reverse) && !tensor_map_ok(xz)) xz = xz.contiguous();
     }
     wo = conv.cast(po, dt);
+    const int64_t Rp = padded_rank(R, dt), cols = Rp + 2 * N;
+    const Tensor wx = nd > 1 ? empty({int64_t(nd), cols, W}, dt, x) : Tensor(), wdt = nd > 1 ? empty({int64_t(nd), W, Rp}, dt, x) : Tensor();
     for (size_t i = 0; i < nd; ++i) {
       dirs[i].reverse = reverse || i == 1;
-      dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N);
+      dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N, nd > 1 ? alias(wx, i * cols * W, {cols, W}) : Tensor(),
+                      nd > 1 ? alias(wdt, i * W * Rp, {W, Rp}) : Tensor());
     }
     conv.run();
     Products mm;
     if (wi.defined()) xz = alias(mm.of(x2, transposed(wi)), 0, {B, L, 2 * W});
     mm.run();
-    for (auto& d : dirs) d.forward(xz, R, N, grad);
+    for (auto& d : dirs) d.release();
+    directions_forward(dirs, xz, R, N, grad);
     s = nd == 1 ? dirs[0].y : dirs[0].y + dirs[1].y;
     if (wo.defined()) {
       const Tensor o = empty({T, wo.size(0)}, dt, xz);

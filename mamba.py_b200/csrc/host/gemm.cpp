@@ -106,54 +106,74 @@ void Products::run() {
 // 64 x 32 and walks all tokens in each, 17.7 us for 11 MB.  Cutting the tokens so that about every SM has a tile, with float32 partial
 // sums that the conversion of the gradients adds up on its way, puts the whole chip on it.  At most 16 cuts (the sum reads them all)
 // of at least 512 tokens (below that a product is a launch's latency anyway).
-Partials Products::tall(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha) {
+std::vector<Partials> Products::tall(int64_t n, const Tensor& a, int64_t sa, const Tensor& b, int64_t sb, at::ScalarType out, float alpha) {
   const auto dt = a.scalar_type();
   const int64_t T = a.size(0), M = a.size(1), N = b.size(1);
-  if (small(M, N, T, dt) && convertible(out)) {
-    const Tensor o = empty({M, N}, out, a);
-    if (add(o, transposed(a), b, alpha, 0.f)) return {o, 1, M, N};
-  }
   const Operand A(a), B(b);
-  if (!A.ok || !B.ok || A.trans || B.trans || b.size(0) != T || b.scalar_type() != dt || !convertible(dt) || !convertible(out) || !plain_settings()) {
-    const Tensor o = empty({M, N}, dt, a);
-    product_into(o, transposed(a), b, alpha, 0.f);
-    return {o, 1, M, N};
+  const bool own = small(M, N, T, dt) && convertible(dt) && convertible(out);
+  const bool ours = A.ok && B.ok && !A.trans && !B.trans && b.size(0) == T && b.scalar_type() == dt && convertible(dt) && convertible(out) && plain_settings();
+  std::vector<Partials> res;
+  const int64_t tiles = (M + 63) / 64 * ((N + 63) / 64) * n;
+  int64_t S = std::max<int64_t>(1, std::min<int64_t>({16, 148 / tiles, T / 512}));
+  if (own || !ours || (S == 1 && n == 1 && dt == at::kFloat)) {
+    for (int64_t i = 0; i < n; ++i) {
+      const Tensor o = empty({M, N}, own ? out : dt, a);
+      into(o, transposed(item(a, i, sa)), item(b, i, sb), alpha, 0.f);
+      res.push_back({o, 1, M, N});
+    }
+    return res;
   }
-  const int64_t tiles = ((M + 63) / 64) * ((N + 63) / 64);
-  int64_t S = std::min<int64_t>({16, 148 / tiles, T / 512});
-  S = std::max<int64_t>(S, 1);
   for (int64_t s = S; 2 * s > S && S > 1; --s)
     if (T % s == 0) {                                            // equal cuts where the number of tokens has a divisor nearby
       S = s;
       break;
     }
-  if (S == 1 && dt == at::kFloat) {
-    const Tensor o = empty({M, N}, dt, a);
-    product_into(o, transposed(a), b, alpha, 0.f);
-    return {o, 1, M, N};
-  }
   const int64_t len = T / S, rest = T - len * S;
   const int slices = int(S + (rest > 0));
   const auto ot = slices > 1 ? at::kFloat : out;
-  const Tensor o = slices > 1 ? empty({slices, M, N}, ot, a) : empty({M, N}, ot, a);
+  const Tensor o = empty({n * slices * M, N}, ot, a);
   const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
   const cudaDataType_t in_t = dt == at::kFloat ? CUDA_R_32F : CUDA_R_16BF, out_t = ot == at::kFloat ? CUDA_R_32F : CUDA_R_16BF;
   const float beta = 0.f;
-  auto run = [&](int64_t first, int64_t k, int64_t count, int64_t slice) {
-    const char *pa = static_cast<const char*>(a.data_ptr()) + first * A.ld * a.element_size(),
-               *pb = static_cast<const char*>(b.data_ptr()) + first * B.ld * b.element_size();
+  // `count` products of k tokens from element offsets oa, ob on, da and db apart, into slices from `slice` on
+  auto run = [&](int64_t oa, int64_t da, int64_t ob, int64_t db, int64_t k, int64_t count, int64_t slice) {
+    const char *pa = static_cast<const char*>(a.data_ptr()) + oa * a.element_size(), *pb = static_cast<const char*>(b.data_ptr()) + ob * b.element_size();
     char* po = static_cast<char*>(o.data_ptr()) + slice * M * N * o.element_size();
     const cublasStatus_t rc =
         count == 1 ? cublasGemmEx(handle, CUBLAS_OP_N, CUBLAS_OP_T, int(N), int(M), int(k), &alpha, pb, in_t, int(B.ld), pa, in_t, int(A.ld), &beta,
                                   po, out_t, int(N), CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT)
-                   : cublasGemmStridedBatchedEx(handle, CUBLAS_OP_N, CUBLAS_OP_T, int(N), int(M), int(k), &alpha, pb, in_t, int(B.ld), k * B.ld, pa, in_t,
-                                                int(A.ld), k * A.ld, &beta, po, out_t, int(N), M * N, int(count), CUBLAS_COMPUTE_32F,
-                                                CUBLAS_GEMM_DEFAULT);
+                   : cublasGemmStridedBatchedEx(handle, CUBLAS_OP_N, CUBLAS_OP_T, int(N), int(M), int(k), &alpha, pb, in_t, int(B.ld), db, pa, in_t,
+                                                int(A.ld), da, &beta, po, out_t, int(N), M * N, int(count), CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT);
     TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "mamba_b200: matrix product failed, cuBLAS status ", int(rc));
   };
-  run(0, len, S, 0);
-  if (rest) run(len * S, rest, 1, S);
-  return {o, slices, M, N};
+  if (rest == 0 && (n == 1 || (sa == T * A.ld && sb == T * B.ld))) {
+    run(0, len * A.ld, 0, len * B.ld, len, n * S, 0);            // cuts of all items are evenly spaced
+  } else {
+    for (int64_t i = 0; i < n; ++i) {
+      run(i * sa, len * A.ld, i * sb, len * B.ld, len, S, i * slices);
+      if (rest) run(i * sa + len * S * A.ld, 0, i * sb + len * S * B.ld, 0, rest, 1, i * slices + S);
+    }
+  }
+  for (int64_t i = 0; i < n; ++i)
+    res.push_back({slices == 1 ? alias(o, i * M * N, {M, N}) : alias(o, i * slices * M * N, {slices, M, N}), slices, M, N});
+  return res;
+}
+
+void Products::each(int64_t n, const Tensor& out, int64_t so, const Tensor& a, int64_t sa, const Tensor& b, int64_t sb, float alpha, float beta) {
+  const auto dt = out.scalar_type();
+  const Operand A(a), B(b), O(out);
+  const int64_t M = a.size(0), N = b.size(1), K = a.size(1);
+  if (n == 1 || small(M, N, K, dt) || !A.ok || !B.ok || !O.ok || O.trans || b.size(0) != K || out.size(0) != M || out.size(1) != N ||
+      a.scalar_type() != dt || b.scalar_type() != dt || !convertible(dt) || !plain_settings()) {
+    for (int64_t i = 0; i < n; ++i) into(item(out, i, so), item(a, i, sa), item(b, i, sb), alpha, beta);
+    return;
+  }
+  const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
+  const cudaDataType_t t = dt == at::kFloat ? CUDA_R_32F : CUDA_R_16BF;
+  const cublasStatus_t rc = cublasGemmStridedBatchedEx(handle, B.op(), A.op(), int(N), int(M), int(K), &alpha, ptr(b), t, int(B.ld), sb, ptr(a), t,
+                                                       int(A.ld), sa, &beta, ptr(out), t, int(O.ld), so, int(n), CUBLAS_COMPUTE_32F,
+                                                       CUBLAS_GEMM_DEFAULT);
+  TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "mamba_b200: matrix product failed, cuBLAS status ", int(rc));
 }
 
 }  // namespace mb200_host

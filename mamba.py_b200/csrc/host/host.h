@@ -93,6 +93,8 @@ inline Tensor columns(const Tensor& t, int64_t first, int64_t n) {
   return strided(t, first * t.stride(-1), shape, t.strides());
 }
 inline Tensor transposed(const Tensor& t) { return strided(t, 0, {t.size(1), t.size(0)}, {t.stride(1), t.stride(0)}); }
+// Item i of matrices that lie s elements apart.
+inline Tensor item(const Tensor& t, int64_t i, int64_t s) { return i ? strided(t, i * s, t.sizes(), t.strides()) : t; }
 inline void zero_fill(const Tensor& t) {
   C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), at::cuda::getCurrentCUDAStream()));
 }
@@ -141,7 +143,10 @@ struct Products {
   bool add(const Tensor& out, const Tensor& a, const Tensor& b, float alpha, float beta);       // false: not a small one
   void into(const Tensor& out, const Tensor& a, const Tensor& b, float alpha, float beta);      // out = alpha * a b + beta * out
   Tensor of(const Tensor& a, const Tensor& b);
-  Partials tall(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha);
+  // n products of one shape; item i of an operand lies s* elements behind item i - 1
+  void each(int64_t n, const Tensor& out, int64_t so, const Tensor& a, int64_t sa, const Tensor& b, int64_t sb, float alpha, float beta);
+  std::vector<Partials> tall(int64_t n, const Tensor& a, int64_t sa, const Tensor& b, int64_t sb, at::ScalarType out, float alpha);
+  Partials tall(const Tensor& a, const Tensor& b, at::ScalarType out, float alpha) { return tall(1, a, 0, b, 0, out, alpha)[0]; }
   void run();
 };
 

@@ -55,14 +55,16 @@ bool split_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carri
   return true;
 }
 
-ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out, const Tensor& dz,
-                          int64_t extra, int64_t pieces = 1, int64_t piece_len = 0) {
+ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& carries, const Tensor& g_in, bool want_g_out, const ScanSinks& to,
+                          int64_t pieces = 1, int64_t piece_len = 0) {
   const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states();
   ScanGrads g;
   const auto dt = a.x.scalar_type();
-  g.dx = empty({B, L, W}, dt, a.x);
-  g.dd = empty({B, L, W}, dt, a.x);
-  if (a.z.defined()) g.dz = dz.defined() ? dz : empty({B, L, W}, dt, a.x);
+  auto sink = [&](const Tensor& t) { return t.defined() ? t : empty({B, L, W}, dt, a.x); };
+  const int64_t extra = to.extra;
+  g.dx = sink(to.dx);
+  g.dd = sink(to.dd);
+  if (a.z.defined()) g.dz = sink(to.dz);
   // every buffer the kernel accumulates into comes out of ONE zero-filled allocation
   const int64_t nBC = B * L * N, nA = W * N;
   const Tensor acc = empty({2 * nBC + nA + 2 * W + extra}, at::kFloat, a.x);
@@ -85,7 +87,7 @@ ScanGrads launch_backward(const ScanArgs& a, const Tensor& dy, const Tensor& car
 }
 
 ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
-                         const Tensor& dz, int64_t extra) {
+                         const ScanSinks& to) {
   const int64_t B = a.batch(), L = a.length(), W = a.width(), N = a.states(), len = piece_length(L, S);
   const Tensor G = empty({B, S, W, N}, at::kFloat, a.x), g_in = empty({B, S, W, N}, at::kFloat, a.x);
   check(mb200_sscan_bwd_carry_pieces(ptr(a.delta), ptr(a.z), ptr(dy), ptr(a.C), fptr(a.A), fptr(a.bias), fptr(G), B, L, W, int(N),
@@ -94,7 +96,7 @@ ScanGrads split_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const T
         "mb200_sscan_bwd_carry");
   check_status("mb200_sscan_bwd_carry");
   check(mb200_carry_fold_range(fptr(P), fptr(G), nullptr, fptr(g_in), B, S, W * N, 0, int(S), 1, cuda_stream()), "mb200_carry_fold_range");
-  return launch_backward(a, dy, carries, g_in, want_g_out, dz, extra, S, len);
+  return launch_backward(a, dy, carries, g_in, want_g_out, to, S, len);
 }
 
 }  // namespace
@@ -123,8 +125,8 @@ bool scan_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carrie
   return S > 1 ? split_forward(a, S, want_last, want_carries, o) : launch_forward(a, o, want_last, want_carries) == MB200_OK;
 }
 ScanGrads scan_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
-                        const Tensor& dz, int64_t extra) {
-  return S > 1 ? split_backward(a, S, dy, carries, P, want_g_out, dz, extra) : launch_backward(a, dy, carries, Tensor(), want_g_out, dz, extra);
+                        const ScanSinks& to) {
+  return S > 1 ? split_backward(a, S, dy, carries, P, want_g_out, to) : launch_backward(a, dy, carries, Tensor(), want_g_out, to);
 }
 
 namespace {

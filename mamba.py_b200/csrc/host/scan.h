@@ -34,8 +34,12 @@ int64_t cuttable(const ScanArgs& a, int64_t S, bool grad, bool want_last);
 // S consecutive pieces per row; S = 1 is the single launch.  False (S = 1 only) when the kernels cannot scan these tensors
 // in reverse.
 bool scan_forward(const ScanArgs& a, int64_t S, bool want_last, bool want_carries, ScanOut& o);
-// dz may be written straight into a caller's (strided) view.
+// Where a caller wants gradients written (dz may be a strided view), and how many zeroed floats behind the accumulators.
+struct ScanSinks {
+  Tensor dz, dx, dd;
+  int64_t extra = 0;
+};
 ScanGrads scan_backward(const ScanArgs& a, int64_t S, const Tensor& dy, const Tensor& carries, const Tensor& P, bool want_g_out,
-                        const Tensor& dz = Tensor(), int64_t extra = 0);
+                        const ScanSinks& to = {});
 
 }  // namespace mb200_host
