@@ -161,30 +161,44 @@ struct Direction {
   std::vector<Tensor> keep;                                 // sources of the queued conversions
 };
 
-// Both directions go through every projection together: their operands lie one behind the other, and two products of one shape are
-// one launch.
-void directions_forward(std::vector<Direction>& dirs, const Tensor& xz, int64_t R, int64_t N, bool grad) {
-  const auto dt = xz.scalar_type();
-  const int64_t n = int64_t(dirs.size()), B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N;
-  const Tensor xc = empty({n, T, W}, dt, xz), delta = empty({n, T, W}, dt, xz), dbc = empty({n, T, cols}, dt, xz);
-  for (int64_t i = 0; i < n; ++i) {
-    Direction& d = dirs[i];
+// Both directions go through every projection together: their operands lie one behind the other in one tensor each, and two products
+// of one shape are one launch.  Whatever walks from one direction to the next does so inside these tensors, which the backward keeps
+// whole: two tensors saved apart need not come back side by side (saved-tensor hooks hand out copies).
+struct Joint {
+  Tensor xc, delta, dbc;                                    // (n, B * L, W), (n, B * L, W), (n, B * L, cols)
+  Tensor Wx, Wdt;                                           // (n, cols, W), (n, W, Rp), without the n for one direction
+
+  // A direction's part of the activations.
+  void share(Direction& d, int64_t i, int64_t B, int64_t L) const {
+    const int64_t T = B * L, W = xc.size(2), cols = dbc.size(2);
     d.xc = alias(xc, i * T * W, {B, L, W});
     d.delta = alias(delta, i * T * W, {B, L, W});
     d.dbc = alias(dbc, i * T * cols, {B, L, cols});
+  }
+};
+
+void directions_forward(std::vector<Direction>& dirs, Joint& j, const Tensor& xz, int64_t R, int64_t N, bool grad) {
+  const auto dt = xz.scalar_type();
+  const int64_t n = int64_t(dirs.size()), B = xz.size(0), L = xz.size(1), W = xz.size(2) / 2, T = B * L, Rp = padded_rank(R, dt), cols = Rp + 2 * N;
+  j.xc = empty({n, T, W}, dt, xz);
+  j.delta = empty({n, T, W}, dt, xz);
+  j.dbc = empty({n, T, cols}, dt, xz);
+  for (int64_t i = 0; i < n; ++i) {
+    Direction& d = dirs[i];
+    j.share(d, i, B, L);
     conv_forward(columns(xz, 0, W), d.cw, d.cb, d.xc, d.reverse);
   }
-  const Tensor xc0 = alias(xc, 0, {T, W}), dbc0 = alias(dbc, 0, {T, cols});
+  const Tensor xc0 = alias(j.xc, 0, {T, W}), dbc0 = alias(j.dbc, 0, {T, cols});
   Products mm;
-  mm.each(n, dbc0, T * cols, xc0, T * W, transposed(dirs[0].Wx), cols * W, 1.f, 0.f);
+  mm.each(n, dbc0, T * cols, xc0, T * W, transposed(alias(j.Wx, 0, {cols, W})), cols * W, 1.f, 0.f);
   mm.run();
-  mm.each(n, alias(delta, 0, {T, W}), T * W, columns(dbc0, 0, Rp), T * cols, transposed(dirs[0].Wdt), W * Rp, 1.f, 0.f);
+  mm.each(n, alias(j.delta, 0, {T, W}), T * W, columns(dbc0, 0, Rp), T * cols, transposed(alias(j.Wdt, 0, {W, Rp})), W * Rp, 1.f, 0.f);
   mm.run();                                                                  // bias and softplus happen in the kernel
   for (Direction& d : dirs) d.scan(xz, Rp, N, grad);
 }
 
 // d(xz) of direction i into dxz[i]; out and kt hold kDirParams entries per direction.
-void directions_backward(const std::vector<Direction>& dirs, const Tensor& xz, const Tensor& dy, const std::vector<Tensor>& dxz, int64_t R, int64_t N,
+void directions_backward(const std::vector<Direction>& dirs, const Joint& j, const Tensor& xz, const Tensor& dy, const std::vector<Tensor>& dxz, int64_t R, int64_t N,
                          const at::ScalarType* kt, const std::vector<std::vector<int64_t>>& cw_shape, Tensor* out, Convert& finish,
                          std::vector<Tensor>& alive) {
   const auto dt = xz.scalar_type();
@@ -200,14 +214,14 @@ void directions_backward(const std::vector<Direction>& dirs, const Tensor& xz, c
     acc.add(ptr(g[i].dC), at::kFloat, row + (Rp + N) * d_dbc.element_size(), dt, T, N, N, N, cols);
   }
   acc.run();
-  const Tensor d0 = alias(d_dbc, 0, {T, cols}), dd0 = alias(dd, 0, {T, W}), dx0 = alias(dx, 0, {T, W}), xc0 = alias(dirs[0].xc, 0, {T, W}),
-               dbc0 = alias(dirs[0].dbc, 0, {T, cols});
+  const Tensor d0 = alias(d_dbc, 0, {T, cols}), dd0 = alias(dd, 0, {T, W}), dx0 = alias(dx, 0, {T, W}), xc0 = alias(j.xc, 0, {T, W}),
+               dbc0 = alias(j.dbc, 0, {T, cols}), Wx0 = alias(j.Wx, 0, {cols, W}), Wdt0 = alias(j.Wdt, 0, {W, Rp});
   Products mm;
-  mm.each(n, columns(d0, 0, Rp), T * cols, dd0, T * W, dirs[0].Wdt, W * Rp, 1.f, 0.f);          // through dt_proj
+  mm.each(n, columns(d0, 0, Rp), T * cols, dd0, T * W, Wdt0, W * Rp, 1.f, 0.f);          // through dt_proj
   const auto dWdt = mm.tall(n, dd0, T * W, columns(dbc0, 0, Rp), T * cols, kt[kDtW], 1.f);      // (W, Rp)
   mm.run();
   const auto dWx = mm.tall(n, d0, T * cols, xc0, T * W, kt[kXproj], 1.f);                       // (Rp + 2 N, W)
-  mm.each(n, dx0, T * W, d0, T * cols, dirs[0].Wx, cols * W, 1.f, 1.f);      // + the gradient through x_proj, in the GEMM's epilogue
+  mm.each(n, dx0, T * W, d0, T * cols, Wx0, cols * W, 1.f, 1.f);      // + the gradient through x_proj, in the GEMM's epilogue
   mm.run();
   for (int64_t i = 0; i < n; ++i)
     dirs[i].finish_back(xz, g[i], dWx[i], dWdt[i], dxz[i], R, N, kt + i * kDirParams, cw_shape[i], out + i * kDirParams, finish, alive);
@@ -217,27 +231,25 @@ enum { kX, kInW, kOutW, kBlockInputs };                     // then kDirParams p
 
 struct BlockBackward : public torch::autograd::Node {
   struct SavedDirection {
-    Saved xc, dbc, delta, carries, P, A, D, bias, cw, cb, Wx, Wdt;
+    Saved carries, P, A, D, bias, cw, cb;
     bool reverse;
     int64_t S;
     std::vector<int64_t> cw_shape;
     template <typename F> void each(F f) {
-      for (Saved* s : {&xc, &dbc, &delta, &carries, &P, &A, &D, &bias, &cw, &cb, &Wx, &Wdt}) f(*s);
+      for (Saved* s : {&carries, &P, &A, &D, &bias, &cw, &cb}) f(*s);
     }
     void save(const Direction& d) {
-      xc.save(d.xc); dbc.save(d.dbc); delta.save(d.delta); carries.save(d.carries); P.save(d.P); A.save(d.A); D.save(d.D); bias.save(d.bias);
-      cw.save(d.cw); cb.save(d.cb); Wx.save(d.Wx); Wdt.save(d.Wdt);
+      carries.save(d.carries); P.save(d.P); A.save(d.A); D.save(d.D); bias.save(d.bias); cw.save(d.cw); cb.save(d.cb);
       reverse = d.reverse; S = d.S;
     }
     Direction get() const {
       Direction d;
       d.reverse = reverse; d.S = S;
-      d.xc = xc.get(); d.dbc = dbc.get(); d.delta = delta.get(); d.carries = carries.get(); d.P = P.get(); d.A = A.get(); d.D = D.get();
-      d.bias = bias.get(); d.cw = cw.get(); d.cb = cb.get(); d.Wx = Wx.get(); d.Wdt = Wdt.get();
+      d.carries = carries.get(); d.P = P.get(); d.A = A.get(); d.D = D.get(); d.bias = bias.get(); d.cw = cw.get(); d.cb = cb.get();
       return d;
     }
   };
-  Saved x, in_w, out_w, xz, y;
+  Saved x, in_w, out_w, xz, y, xc, delta, dbc, Wx, Wdt;
   std::vector<SavedDirection> dirs;
   std::vector<at::ScalarType> types;
   std::vector<int64_t> x_shape;
@@ -246,7 +258,7 @@ struct BlockBackward : public torch::autograd::Node {
 
   std::string name() const override { return "MambaBlockBackward"; }
   void release_variables() override {
-    for (Saved* s : {&x, &in_w, &out_w, &xz, &y}) s->reset();
+    for (Saved* s : {&x, &in_w, &out_w, &xz, &y, &xc, &delta, &dbc, &Wx, &Wdt}) s->reset();
     for (auto& d : dirs) d.each([](Saved& s) { s.reset(); });
   }
   variable_list apply(variable_list&& grads) override {
@@ -265,7 +277,7 @@ struct BlockBackward : public torch::autograd::Node {
     std::vector<Tensor> alive;
     Tensor dy = rows(grads[0], dt);
     if (out_w.defined) {
-      const Tensor w = out_w.get(), s2 = alias(y.get(), 0, {T, W}), d2 = dy.reshape({T, w.size(0)});
+      const Tensor w = out_w.get(), s2 = alias(y.get().contiguous(), 0, {T, W}), d2 = dy.reshape({T, w.size(0)});
       const Tensor ds = empty({T, W}, dt, xz_);
       mm.into(ds, d2, w, scale, 0.f);
       dy = alias(ds, 0, {B, L, W});
@@ -279,12 +291,14 @@ struct BlockBackward : public torch::autograd::Node {
     std::vector<Direction> ds;
     std::vector<Tensor> each;
     std::vector<std::vector<int64_t>> cw_shape;
+    const Joint joint{xc.get().contiguous(), delta.get().contiguous(), dbc.get().contiguous(), Wx.get().contiguous(), Wdt.get().contiguous()};
     for (const SavedDirection& d : dirs) {
       ds.push_back(d.get());
+      joint.share(ds.back(), int64_t(ds.size()) - 1, B, L);
       each.push_back(empty({B, L, 2 * W}, dt, xz_));
       cw_shape.push_back(d.cw_shape);
     }
-    directions_backward(ds, xz_, dy, each, R, N, kt.data() + kBlockInputs, cw_shape, out.data() + kBlockInputs, finish, alive);
+    directions_backward(ds, joint, xz_, dy, each, R, N, kt.data() + kBlockInputs, cw_shape, out.data() + kBlockInputs, finish, alive);
     const Tensor dxz = each[0];
     if (each.size() > 1) dxz.add_(each[1]);
     if (in_w.defined) {
@@ -328,6 +342,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
   const c10::cuda::CUDAGuard guard(x.device());
   const size_t nd = params.size() / kDirParams;
   std::vector<Direction> dirs(nd);
+  Joint joint;
   Tensor x2, wi, wo, xz, s, out;
   const float scale = halve ? 0.5f : 1.f;
   {
@@ -349,18 +364,25 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
     }
     wo = conv.cast(po, dt);
     const int64_t Rp = padded_rank(R, dt), cols = Rp + 2 * N;
-    const Tensor wx = nd > 1 ? empty({int64_t(nd), cols, W}, dt, x) : Tensor(), wdt = nd > 1 ? empty({int64_t(nd), W, Rp}, dt, x) : Tensor();
+    if (nd > 1) {
+      joint.Wx = empty({int64_t(nd), cols, W}, dt, x);
+      joint.Wdt = empty({int64_t(nd), W, Rp}, dt, x);
+    }
     for (size_t i = 0; i < nd; ++i) {
       dirs[i].reverse = reverse || i == 1;
-      dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N, nd > 1 ? alias(wx, i * cols * W, {cols, W}) : Tensor(),
-                      nd > 1 ? alias(wdt, i * W * Rp, {W, Rp}) : Tensor());
+      dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N, nd > 1 ? alias(joint.Wx, i * cols * W, {cols, W}) : Tensor(),
+                      nd > 1 ? alias(joint.Wdt, i * W * Rp, {W, Rp}) : Tensor());
+    }
+    if (nd == 1) {
+      joint.Wx = dirs[0].Wx;
+      joint.Wdt = dirs[0].Wdt;
     }
     conv.run();
     Products mm;
     if (wi.defined()) xz = alias(mm.of(x2, transposed(wi)), 0, {B, L, 2 * W});
     mm.run();
     for (auto& d : dirs) d.release();
-    directions_forward(dirs, xz, R, N, grad);
+    directions_forward(dirs, joint, xz, R, N, grad);
     s = nd == 1 ? dirs[0].y : dirs[0].y + dirs[1].y;
     if (wo.defined()) {
       const Tensor o = empty({T, wo.size(0)}, dt, xz);
@@ -382,6 +404,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
     if (wi.defined()) { node->x.save(x2); node->in_w.save(wi); }
     if (wo.defined()) { node->out_w.save(wo); node->y.save(s); }
     node->xz.save(xz);
+    node->xc.save(joint.xc); node->delta.save(joint.delta); node->dbc.save(joint.dbc); node->Wx.save(joint.Wx); node->Wdt.save(joint.Wdt);
     node->dirs.resize(nd);
     for (size_t i = 0; i < nd; ++i) {
       node->dirs[i].save(dirs[i]);

@@ -87,3 +87,24 @@ def test_block_against_float64(d_model, d_state, both, variant, amp):
         assert a.dtype == t.dtype and a.shape == b.shape
         err = ((a.double() - b).norm() / b.norm().clamp_min(1e-12)).item()
         assert err < tol and math.isfinite(err), (tuple(b.shape), err)
+
+
+@pytest.mark.parametrize("both", [False, True])
+@pytest.mark.parametrize("keep", ["clones", "host", "checkpoint"])
+def test_saved_tensors_may_come_back_as_copies(both, keep):
+    """Saved-tensor hooks and checkpointing hand the backward other tensors than the forward saved, each with storage of its own."""
+    from torch.utils.checkpoint import checkpoint
+    from mamba_b200 import mamba, vim
+    m = _build(40, 16, both)
+    run = vim.forward if both else mamba.forward
+    x, dy = torch.randn(3, 37, 40, device=DEV, requires_grad=True), torch.randn(3, 37, 40, device=DEV)
+    wanted = [x, *m.parameters()]
+    want = torch.autograd.grad(run(m, x), wanted, dy)
+    if keep == "checkpoint":
+        y = checkpoint(run, m, x, use_reentrant=False)
+    else:
+        hooks = torch.autograd.graph.save_on_cpu() if keep == "host" else torch.autograd.graph.saved_tensors_hooks(torch.clone, lambda t: t)
+        with hooks:
+            y = run(m, x)
+    for a, b in zip(torch.autograd.grad(y, wanted, dy), want):
+        assert ((a - b).norm() / b.norm().clamp_min(1e-12)).item() < 1e-5      # sums over atomics, in any order
