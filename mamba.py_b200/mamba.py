@@ -153,11 +153,22 @@ def step(self, x, cache):
     return self.out_proj(y), (h, inputs)
 
 
+_linear_forward = nn.Linear.forward
+
+
 def _plain_linear(m):
-    """(weight, bias) of a projection that is an ordinary nn.Linear and nothing else (no hooks, no subclass)."""
-    if type(m) is not nn.Linear or m._forward_hooks or m._forward_pre_hooks:
+    """(weight, bias) of a projection that is an ordinary nn.Linear and nothing else, so that calling it is the matrix product: no
+    subclass, no hook of any kind, no `forward` of its own (offload and dispatch wrappers put theirs on the instance), not compiled
+    by itself, and an ordinary tensor as its weight (quantised and distributed ones dispatch for themselves)."""
+    if type(m) is not nn.Linear or nn.Linear.forward is not _linear_forward:
         return None
-    p = m._parameters
+    d = m.__dict__
+    if (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d
+            or d.get("_compiled_call_impl") is not None):
+        return None
+    p = d["_parameters"]
+    if type(p["weight"]) not in (nn.Parameter, torch.Tensor):
+        return None
     return p["weight"], p["bias"]
 
 

@@ -102,3 +102,27 @@ def test_install_rebinds_reference_names_and_uninstall_restores():
         assert y.shape == (1, 8, 16)
     finally:
         sys.path.remove(REF)
+
+
+def _intercepted(how):
+    m = torch.nn.Linear(4, 4)
+    if how.startswith("register"):
+        getattr(m, how)(lambda *a: None)
+    elif how == "forward":
+        m.forward = lambda x: x
+    elif how == "compile":
+        m.compile(backend="eager")
+    elif how == "subclass":
+        m.__class__ = type("Mine", (torch.nn.Linear,), {})
+    elif how == "weight":
+        m.weight = torch.nn.Parameter(torch.zeros(4, 4).as_subclass(type("Packed", (torch.Tensor,), {})))
+    return m
+
+
+@pytest.mark.parametrize("how", ["register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook",
+                                 "register_full_backward_pre_hook", "forward", "compile", "subclass", "weight"])
+def test_projections_that_have_to_be_called(how):
+    """Only a projection whose call is the matrix product and nothing else goes straight to the native code."""
+    from mamba_b200.mamba import _plain_linear
+    assert _plain_linear(torch.nn.Linear(4, 4)) is not None
+    assert _plain_linear(_intercepted(how)) is None
