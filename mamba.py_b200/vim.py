@@ -12,7 +12,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import host as _host
-from .mamba import causal_conv1d_silu, run_block, selective_scan_fn
+from .mamba import _native_linear, causal_conv1d_silu, run_block, selective_scan_fn
 
 
 def _conv_silu(conv, xs, L):
@@ -42,6 +42,10 @@ def forward(self, x):
         second = [self.conv1d_b.weight, self.conv1d_b.bias, self.x_proj_b.weight, self.dt_proj_b.weight, self.dt_proj_b.bias,
                   self.A_log_b, self.D_b]
         native = self.conv1d_b.weight.shape[-1] == 4
+    # this block calls its x_proj as modules, so the native one is for those whose call is the matrix product; and without a bias
+    # of dt_proj the scan takes delta as it is
+    for s in ("", "_b") if cfg.bidirectional else ("",):
+        native = native and _native_linear(getattr(self, "x_proj" + s), dtype) is not None and getattr(self, "dt_proj" + s).bias is not None
     if native:
         out, xz = run_block(self, x, [first, second] if cfg.bidirectional else [first], cfg.bidirectional and cfg.divide_output)
         if out is not None:

@@ -108,3 +108,60 @@ def test_saved_tensors_may_come_back_as_copies(both, keep):
             y = run(m, x)
     for a, b in zip(torch.autograd.grad(y, wanted, dy), want):
         assert ((a - b).norm() / b.norm().clamp_min(1e-12)).item() < 1e-5      # sums over atomics, in any order
+
+
+def _count(m, seen, kind):
+    """Has `m` report its calls into `seen`, one way or another."""
+    call = m.forward
+
+    def forward(*a):
+        seen.append(kind)
+        return call(*a)
+    if kind == "forward":
+        m.forward = forward
+    else:
+        getattr(m, f"register_{kind}")(lambda *a: seen.append(kind))
+
+
+@pytest.mark.parametrize("kind", ["forward_hook", "forward_pre_hook", "full_backward_hook", "full_backward_pre_hook", "forward"])
+@pytest.mark.parametrize("name,both", [("in_proj", False), ("out_proj", False), ("in_proj", True), ("x_proj", True), ("x_proj_b", True), ("out_proj", True)])
+def test_intercepted_projections_are_called(name, both, kind):
+    """A projection that somebody listens to or has replaced is called as the module it is, with the same results."""
+    from mamba_b200 import mamba, step, vim
+    m, seen = _build(32, 16, both), []
+    run = vim.forward if both else mamba.forward
+    x, dy = torch.randn(2, 20, 32, device=DEV, requires_grad=True), torch.randn(2, 20, 32, device=DEV)
+    token, cache = torch.randn(2, 32, device=DEV), (None, torch.zeros(2, 64, 3, device=DEV))
+    want = [y := run(m, x), *torch.autograd.grad(y, [x, *m.parameters()], dy)]
+    with torch.no_grad():
+        want_step = step(m, token, cache)[0]
+    _count(getattr(m, name), seen, kind)
+    got = [y := run(m, x), *torch.autograd.grad(y, [x, *m.parameters()], dy)]
+    assert seen == [kind]
+    for a, b in zip(got, want):
+        assert ((a - b).norm() / b.norm().clamp_min(1e-12)).item() < 1e-5
+    with torch.no_grad():
+        got_step = step(m, token, cache)[0]
+    assert len(seen) == 1 + (name != "x_proj_b" and "backward" not in kind)
+    assert ((got_step - want_step).norm() / want_step.norm()).item() < 1e-5
+
+
+def test_bidirectional_block_with_biases_where_none_are_usual():
+    """x_proj with a bias, dt_proj without one: accepted, and the biases count."""
+    from mamba_b200 import vim
+    m = _build(32, 16, True)
+    x = torch.randn(2, 20, 32, device=DEV)
+    with torch.no_grad():
+        want = vim.forward(m, x)
+        for s in ("", "_b"):
+            old = getattr(m, "x_proj" + s)
+            new = nn.Linear(64, 34, device=DEV)
+            new.weight.copy_(old.weight)
+            new.bias.zero_()
+            setattr(m, "x_proj" + s, new)
+        assert (vim.forward(m, x) - want).norm() / want.norm() < 1e-5
+        m.x_proj_b.bias.fill_(0.5)
+        assert (vim.forward(m, x) - want).norm() / want.norm() > 1e-3
+        m.dt_proj.bias = None
+        m.dt_proj.weight.abs_()
+        assert torch.isfinite(vim.forward(m, 0.01 * x)).all()
