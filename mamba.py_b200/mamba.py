@@ -159,7 +159,8 @@ _linear_forward = nn.Linear.forward
 def _plain_linear(m):
     """(weight, bias) of a projection that is an ordinary nn.Linear and nothing else, so that calling it is the matrix product: no
     subclass, no hook of any kind, no `forward` of its own (offload and dispatch wrappers put theirs on the instance), not compiled
-    by itself, and an ordinary tensor as its weight (quantised and distributed ones dispatch for themselves)."""
+    by itself, and an ordinary tensor as its weight (quantised and distributed ones dispatch for themselves) among its parameters
+    (replicas and pruning keep theirs as plain attributes)."""
     if type(m) is not nn.Linear or nn.Linear.forward is not _linear_forward:
         return None
     d = m.__dict__
@@ -167,7 +168,7 @@ def _plain_linear(m):
             or d.get("_compiled_call_impl") is not None):
         return None
     p = d["_parameters"]
-    if type(p["weight"]) not in (nn.Parameter, torch.Tensor):
+    if type(p.get("weight")) not in (nn.Parameter, torch.Tensor) or "bias" not in p:
         return None
     return p["weight"], p["bias"]
 
@@ -186,7 +187,9 @@ def _plain_block(self):
     if self.config.d_state not in (8, 16, 32, 64):
         return None
     conv = conv._parameters
-    return (*lin[0], conv.get("weight"), conv.get("bias"), lin[1][0], *lin[2], A_log, D, *lin[3]) if "weight" in conv else None
+    if conv.get("weight") is None or "bias" not in conv:
+        return None
+    return *lin[0], conv["weight"], conv["bias"], lin[1][0], *lin[2], A_log, D, *lin[3]
 
 
 def _fusable(self, x, dtype):

@@ -126,3 +126,16 @@ def test_projections_that_have_to_be_called(how):
     from mamba_b200.mamba import _plain_linear
     assert _plain_linear(torch.nn.Linear(4, 4)) is not None
     assert _plain_linear(_intercepted(how)) is None
+
+
+@pytest.mark.parametrize("gone", ["in_proj.weight", "in_proj.bias", "conv1d.weight", "conv1d.bias", "out_proj.weight", "dt_proj.bias", "A_log"])
+def test_parameters_that_are_plain_attributes(gone):
+    """Replicas, pruning and wrappers take parameters out of `_parameters` and leave attributes: the block is then not a plain one."""
+    from mamba_b200.mamba import _plain_block
+    from tests.helpers import RefShapedBlock
+    m = RefShapedBlock(16)
+    assert _plain_block(m) is not None
+    owner, name = (m.get_submodule(gone.split(".")[0]), gone.split(".")[1]) if "." in gone else (m, gone)
+    value = owner._parameters.pop(name)
+    owner.__dict__[name] = value
+    assert _plain_block(m) is None

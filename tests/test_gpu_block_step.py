@@ -56,3 +56,27 @@ def test_block_step_first_token_and_graph():
             g.replay()
     torch.cuda.synchronize()
     assert torch.equal(o0, o1) and torch.equal(c0[0], c1[0]) and torch.equal(c0[1], c1[1])
+
+
+def test_replicas_and_pruned_modules():
+    """Blocks whose parameters are plain attributes run through their modules and give what the block itself gives."""
+    import torch.nn.utils.prune as prune
+    from mamba_b200 import mamba, step
+    torch.manual_seed(5)
+    blk = RefShapedBlock(32).to(DEV)
+    x, token, cache = torch.randn(2, 20, 32, device=DEV), torch.randn(2, 32, device=DEV), (None, torch.zeros(2, 64, 3, device=DEV))
+    replica = blk._replicate_for_data_parallel()
+    for part, source in [(replica, blk)] + [(c._replicate_for_data_parallel(), c) for c in blk.children()]:
+        for name, p in source._parameters.items():
+            setattr(part, name, p)
+        if part is not replica:
+            replica._modules[next(k for k, v in blk._modules.items() if v is source)] = part
+    with torch.no_grad():
+        want = mamba.forward(blk, x), step(blk, token, cache)[0]
+        got = [(mamba.forward(replica, x), step(replica, token, cache)[0])]
+        for name, p in (("conv1d", "bias"), ("in_proj", "weight"), ("out_proj", "weight")):
+            prune.identity(getattr(blk, name), p)
+        got.append((mamba.forward(blk, x), step(blk, token, cache)[0]))
+    for pair in got:
+        for a, b in zip(pair, want):
+            assert_close(a, b, 1e-4, 1e-5)
