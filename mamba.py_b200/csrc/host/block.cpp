@@ -341,6 +341,22 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
   }
   const c10::cuda::CUDAGuard guard(x.device());
   const size_t nd = params.size() / kDirParams;
+  const int64_t width = in[kBlockInputs + kDtW].defined() && in[kBlockInputs + kDtW].dim() == 2 ? in[kBlockInputs + kDtW].size(0) : -1;
+  TORCH_CHECK(x.dim() == 3, "mamba_b200: a block takes (B, L, width) activations, got ", x.sizes());
+  if (in_w.defined()) shape_is(in_w, {2 * width, x.size(2)}, "in_proj.weight");
+  else shape_is(x, {x.size(0), x.size(1), 2 * width}, "the in_proj output");
+  if (out_w.defined()) TORCH_CHECK(out_w.dim() == 2 && out_w.size(1) == width, "mamba_b200: out_proj.weight should take ", width, " features, got ", out_w.sizes());
+  for (size_t i = 0; i < nd; ++i) {
+    const Tensor* p = in.data() + kBlockInputs + i * kDirParams;
+    for (int k : {kConvW, kXproj, kDtW, kDtB, kALog, kD}) TORCH_CHECK(p[k].defined(), "mamba_b200: a block needs every parameter but the conv bias");
+    numel_is(p[kConvW], width * p[kConvW].size(-1), "conv1d.weight");
+    numel_is(p[kConvB], width, "conv1d.bias");
+    shape_is(p[kXproj], {R + 2 * N, width}, "x_proj.weight");
+    shape_is(p[kDtW], {width, R}, "dt_proj.weight");
+    numel_is(p[kDtB], width, "dt_proj.bias");
+    shape_is(p[kALog], {width, N}, "A_log");
+    numel_is(p[kD], width, "D");
+  }
   std::vector<Direction> dirs(nd);
   Joint joint;
   Tensor x2, wi, wo, xz, s, out;

@@ -34,6 +34,14 @@ template <typename... Ts> void require_cuda(const Ts&... ts) {
     TORCH_CHECK(!t->defined() || t->is_cuda(), "mamba_b200 runs on CUDA tensors only (there is no CPU path)");
 }
 
+// Kernels and GEMMs take sizes from one tensor for all: what calling the modules one by one would compare is compared here.
+inline void shape_is(const Tensor& t, at::IntArrayRef want, const char* what) {
+  TORCH_CHECK(t.sizes() == want, "mamba_b200: ", what, " should be ", want, ", got ", t.sizes());
+}
+inline void numel_is(const Tensor& t, int64_t want, const char* what) {
+  TORCH_CHECK(!t.defined() || t.numel() == want, "mamba_b200: ", what, " should have ", want, " elements, got ", t.numel());
+}
+
 inline void check(int rc, const char* what) {
   TORCH_CHECK(rc == MB200_OK, what, " failed: ", mb200_strerror(rc), " (code ", rc, ")");
 }

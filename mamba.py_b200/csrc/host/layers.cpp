@@ -5,7 +5,11 @@
 namespace mb200_host {
 namespace {
 
-Tensor filter(const Tensor& weight) { return f32(weight).view({weight.size(0), weight.size(-1)}); }
+// The filter of `width` channels, (width, d_conv).
+Tensor filter(const Tensor& weight, int64_t width) {
+  numel_is(weight, width * weight.size(-1), "the filter");
+  return f32(weight).view({width, weight.size(-1)});
+}
 
 struct ConvBackward : public torch::autograd::Node {
   Saved x, w, b;
@@ -44,8 +48,9 @@ Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias_
   {
     const BelowAutograd guard_ad;
     xs = rows(x, act_dtype(x));
-    w32 = filter(weight);
+    w32 = filter(weight, xs.size(2));
     b32 = f32(bias);
+    numel_is(b32, xs.size(2), "the bias");
     const int64_t B = xs.size(0), L = xs.size(1), W = xs.size(2), K = w32.size(1);
     y = empty({B, L, W}, xs.scalar_type(), xs);
     check(mb200_conv1d_silu_fwd(ptr(xs), fptr(w32), fptr(b32), ptr(y), B, L, W, int(K), st(xs, 0), st(xs, 1), st(y, 0), st(y, 1),

@@ -50,6 +50,9 @@ WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weig
   const auto dt = act_dtype(x);
   const Tensor xs = rows(x, dt), win = inputs.to(dt).contiguous(), w = small_param(weight), bias = small_param(bias_);
   const int64_t n = xs.size(0), W = xs.size(1);
+  numel_is(w, W * w.size(-1), "the filter");
+  numel_is(bias, W, "the bias");
+  TORCH_CHECK(win.numel() >= n * W * (w.size(-1) - 1), "mamba_b200: the window holds fewer than ", n, " rows of ", W, " channels");
   WindowStep o;
   o.xc = empty({n, W}, dt, xs);
   if (inplace) {
@@ -120,8 +123,22 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
   require_cuda(x, h, inputs, in_w, in_b, conv_w, conv_b, xproj_w, dt_w, dt_b, A_log, D, out_w, out_b);
   const c10::cuda::CUDAGuard guard(x.device());
   const auto dt = x.scalar_type();
-  const int64_t B = x.size(0), Dm = x.size(1), W = dt_w.size(0);
-  bool one = B >= 1 && B <= 8 && (dt == at::kFloat || dt == at::kBFloat16) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+  TORCH_CHECK(x.dim() == 2 && dt_w.dim() == 2 && out_w.dim() == 2, "mamba_b200: a step takes (B, d_model) activations and matrices as weights");
+  const int64_t B = x.size(0), Dm = x.size(1), W = dt_w.size(0), K = conv_w.size(-1);
+  shape_is(in_w, {2 * W, Dm}, "in_proj.weight");
+  numel_is(in_b, 2 * W, "in_proj.bias");
+  numel_is(conv_w, W * K, "conv1d.weight");
+  numel_is(conv_b, W, "conv1d.bias");
+  shape_is(xproj_w, {R + 2 * N, W}, "x_proj.weight");
+  shape_is(dt_w, {W, R}, "dt_proj.weight");
+  numel_is(dt_b, W, "dt_proj.bias");
+  shape_is(A_log, {W, N}, "A_log");
+  numel_is(D, W, "D");
+  shape_is(out_w, {out_w.size(0), W}, "out_proj.weight");
+  numel_is(out_b, out_w.size(0), "out_proj.bias");
+  TORCH_CHECK(inputs.numel() >= B * W * (K - 1) && (!h.defined() || h.numel() >= B * W * N), "mamba_b200: the caches hold fewer than ", B,
+              " rows of ", W, " channels");
+  bool one = out_w.size(0) == Dm && B >= 1 && B <= 8 && (dt == at::kFloat || dt == at::kBFloat16) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
              !wants_grad(x, in_w, in_b, out_w, out_b);
   for (const Tensor* t : {&in_w, &in_b, &xproj_w, &dt_w, &out_w, &out_b})
     one = one && (!t->defined() || (t->scalar_type() == dt && t->is_contiguous()));

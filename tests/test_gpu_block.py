@@ -165,3 +165,35 @@ def test_bidirectional_block_with_biases_where_none_are_usual():
         m.dt_proj.bias = None
         m.dt_proj.weight.abs_()
         assert torch.isfinite(vim.forward(m, 0.01 * x)).all()
+
+
+@pytest.mark.parametrize("name,shape", [("in_proj", (96, 32)), ("in_proj", (128, 40)), ("conv1d", (48, 1, 4)), ("x_proj", (33, 64)), ("x_proj", (34, 48)),
+                                        ("dt_proj", (64, 3)), ("dt_proj", (48, 2)), ("out_proj", (32, 48)), ("A_log", (48, 16)), ("A_log", (64, 8)),
+                                        ("D", (48,))])
+@pytest.mark.parametrize("both", [False, True])
+def test_parameters_of_other_sizes_are_refused(name, shape, both):
+    """What no longer is compared by calling the modules one by one is compared by the native block and step."""
+    from mamba_b200 import mamba, step, vim
+    m = _build(32, 16, both)
+    p = nn.Parameter(torch.zeros(shape, device=DEV))
+    if name in ("A_log", "D"):
+        setattr(m, name, p)
+    else:
+        getattr(m, name).weight = p
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        (vim.forward if both else mamba.forward)(m, torch.zeros(2, 20, 32, device=DEV))
+    for rows in (2, 9):
+        with torch.no_grad(), pytest.raises(RuntimeError):
+            step(m, torch.zeros(rows, 32, device=DEV), (None, torch.zeros(rows, 64, 3, device=DEV)))
+
+
+def test_activations_and_caches_of_other_sizes_are_refused():
+    from mamba_b200 import mamba, step
+    m = _build(32, 16, False)
+    z = lambda *s: torch.zeros(*s, device=DEV)
+    with torch.no_grad():
+        for bad in (lambda: mamba.forward(m, z(2, 20, 40)), lambda: step(m, z(2, 40), (None, z(2, 64, 3))), lambda: step(m, z(2, 32), (None, z(1, 64, 3))),
+                    lambda: step(m, z(2, 32), (z(1, 64, 16), z(2, 64, 3))), lambda: mamba.causal_conv1d_silu(z(2, 20, 32), z(16, 1, 4)),
+                    lambda: mamba.conv_step_fn(z(2, 32), z(2, 32, 3), z(16, 1, 4), None)):
+            with pytest.raises(RuntimeError):
+                bad()
