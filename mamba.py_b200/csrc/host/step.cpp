@@ -192,6 +192,8 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
   StateStep s;
   {
     const BelowAutograd guard_ad;
+    // the kernel reads A in 16-byte vectors; a parameter may lie anywhere (one piece of a flat buffer)
+    if (!once && reinterpret_cast<uintptr_t>(A.data_ptr()) % 16) A = A.clone(at::MemoryFormat::Contiguous);
     s = state_step(w.xc, h, delta, A, !once, columns(dbc, R, N), columns(dbc, R + N, N), Df, columns(xz, W, W), bf, false);
   }
   return {project(s.y, out_w, out_b_), s.h, w.window};

@@ -80,3 +80,26 @@ def test_replicas_and_pruned_modules():
     for pair in got:
         for a, b in zip(pair, want):
             assert_close(a, b, 1e-4, 1e-5)
+
+
+@pytest.mark.parametrize("Bsz", [2, 9, 31, 40])
+@pytest.mark.parametrize("d_model", [32, 33])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_parameters_off_the_16_byte_grid(Bsz, d_model, dtype):
+    """Every parameter one element into a flat buffer gives what parameters of their own give, on each path of a step."""
+    from mamba_b200 import step
+    torch.manual_seed(Bsz)
+    blk = RefShapedBlock(d_model).to(dtype).to(DEV)
+    x, h, win = (torch.randn(*s, device=DEV) for s in ((Bsz, d_model), (Bsz, 2 * d_model, 16), (Bsz, 2 * d_model, 3)))
+    x, win = x.to(dtype), win.to(dtype)
+    with torch.no_grad():
+        want, (want_h, _) = step(blk, x, (h, win))
+        for p in blk.parameters():
+            flat = torch.zeros(p.numel() + 8, dtype=dtype, device=DEV)
+            flat[1:1 + p.numel()] = p.flatten()
+            p.data = flat[1:1 + p.numel()].view(p.shape)
+            assert p.data_ptr() % 16
+        got, (got_h, _) = step(blk, x, (h, win))
+    rt, at = (1e-4, 1e-5) if dtype == torch.float32 else (3e-2, 3e-2)
+    assert_close(got, want, rt, at)
+    assert_close(got_h, want_h, rt, at)
