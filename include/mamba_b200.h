@@ -423,6 +423,12 @@ typedef struct {
 } mb200_block_step_args;
 int64_t mb200_block_step_scratch_floats(int64_t B, int64_t W, int64_t R, int N);
 int mb200_block_step_barrier_bytes(void);
+/* How many reads of the status word (mb200_device_status) have found that a step gave up at one of its barriers.  Such a launch
+ * leaves its counters unusable, and later launches on them return at once and report the same: whoever keeps counters between
+ * launches replaces them by zeroed ones when this number has changed. */
+unsigned mb200_block_step_give_ups(void);
+/* Self-test of that (no counterpart in the reference): marks `barriers` as a launch that gave up leaves them. */
+int mb200_selftest_block_step_give_up(void* barriers, void* stream);
 int mb200_block_step(const mb200_block_step_args* args, float* scratch, void* barriers, void* stream);
 
 #ifdef __cplusplus

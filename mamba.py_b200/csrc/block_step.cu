@@ -11,6 +11,8 @@
 //   3  delta = dt_proj(dbc), state update, C-contraction, D skip, gate: a group of lanes per (token, channel)
 //   4  out = out_proj(y), one warp per row
 // Values between phases are rounded to the activation type, as the separate kernels round them.
+#include <atomic>
+#include <cstddef>
 #include "common.cuh"
 
 namespace mb200 {
@@ -277,12 +279,23 @@ int block_step_states(StepParams& p, cudaStream_t st) {
 
 using namespace mb200;
 
+static std::atomic<unsigned> g_block_step_give_ups{0};
+
 // Reads and clears the status word of the step kernel.  Synchronises the device.
 int mb200_block_step_device_status() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_block_step_status, sizeof(int)) != cudaSuccess) return -1;
-  if (v) cudaMemcpyToSymbol(g_block_step_status, &zero, sizeof(int));
+  if (v) {
+    cudaMemcpyToSymbol(g_block_step_status, &zero, sizeof(int));
+    g_block_step_give_ups.fetch_add(1);
+  }
   return v;
+}
+extern "C" unsigned mb200_block_step_give_ups(void) { return g_block_step_give_ups.load(); }
+extern "C" int mb200_selftest_block_step_give_up(void* barriers, void* stream) {
+  if (!barriers) return MB200_EINVAL;
+  char* word = static_cast<char*>(barriers) + offsetof(StepBarriers, poisoned);
+  return cudaMemsetAsync(word, 1, sizeof(unsigned), static_cast<cudaStream_t>(stream)) == cudaSuccess ? MB200_OK : MB200_ELAUNCH;
 }
 
 extern "C" int64_t mb200_block_step_scratch_floats(int64_t B, int64_t W, int64_t R, int N) { return B * (3 * W + R + 2 * N); }

@@ -108,8 +108,9 @@ inline void zero_fill(const Tensor& t) {
 }
 inline void* cuda_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
-// With MB200_CHECK_STATUS=1 in the environment every fused-scan launch is followed by a device synchronisation and a
-// read of the kernels' status word; a bounded wait that gave up then raises.
+// With MB200_CHECK_STATUS=1 in the environment every launch of a kernel with bounded waits (the fused scans, the one-launch step)
+// is followed by a device synchronisation and a read of the kernels' status word; a wait that gave up then raises.  A stream that
+// is being captured into a graph launches nothing yet and is left alone.
 void check_status(const char* what);
 
 // The library's own tensor operations record nothing: autograd sees the nodes below only.
@@ -224,6 +225,9 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
                                               const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w,
                                               const Tensor& dt_b, const Tensor& A_log, const Tensor& D, const Tensor& out_w,
                                               const OptTensor& out_b, int64_t dt_rank, int64_t d_state);
+
+// Spoils the barrier counters that the current stream keeps for the one-launch step on `on`'s device, as a launch that gave up does.
+void selftest_block_step_give_up(const Tensor& on);
 
 int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad);
 

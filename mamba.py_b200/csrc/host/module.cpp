@@ -23,4 +23,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("reversible", &reversible);
   m.def("block_step", &block_step, NoGil());
   m.def("pick_pieces", &pick_pieces);
+  m.def("selftest_block_step_give_up", &selftest_block_step_give_up);
 }

@@ -11,6 +11,9 @@ void check_status(const char* what) {
     return v && *v && std::string(v) != "0";
   }();
   if (!on) return;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(at::cuda::getCurrentCUDAStream(), &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return;
   const int s = mb200_device_status();
   TORCH_CHECK(s == 0, what, ": a bounded wait inside the kernel gave up (device status ", s, "); its outputs are invalid");
 }

@@ -70,17 +70,23 @@ WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weig
 // ---- barrier counters of the one-launch step -----------------------------------------------------------------------
 // A launch leaves its counters zero for the next one on the same stream, so a stream keeps its own.  At most kMaxStreams are
 // kept; a stream beyond them, and a stream that is being captured into a graph (whose replays may run anywhere), gets
-// counters of its own for the one call, cleared on the stream.
+// counters of its own for the one call, cleared on the stream.  A launch that gave up at a barrier spoils its counters; once
+// somebody has read its status word, none from before are used again.
 constexpr size_t kMaxStreams = 64;
 
 Tensor barrier_counters(const Tensor& on) {
   static std::mutex mutex;
   static std::unordered_map<uint64_t, Tensor> kept;
+  static unsigned give_ups = 0;
   const auto s = at::cuda::getCurrentCUDAStream();
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   C10_CUDA_CHECK(cudaStreamIsCapturing(s, &capturing));
   const uint64_t key = (uint64_t(s.device_index()) << 56) ^ uint64_t(s.id());
   std::lock_guard<std::mutex> lock(mutex);
+  if (const unsigned now = mb200_block_step_give_ups(); now != give_ups) {
+    kept.clear();
+    give_ups = now;
+  }
   const bool keep = capturing == cudaStreamCaptureStatusNone;
   if (keep) {
     const auto it = kept.find(key);
@@ -93,6 +99,11 @@ Tensor barrier_counters(const Tensor& on) {
 }
 
 }  // namespace
+
+void selftest_block_step_give_up(const Tensor& on) {
+  const c10::cuda::CUDAGuard guard(on.device());
+  check(mb200_selftest_block_step_give_up(ptr(barrier_counters(on)), cuda_stream()), "mb200_selftest_block_step_give_up");
+}
 
 std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const Tensor& delta, const Tensor& A, const Tensor& B,
                                     const Tensor& C, const OptTensor& D, const OptTensor& z, const OptTensor& bias, bool inplace) {
@@ -158,6 +169,7 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
     const int rc = mb200_block_step(&a, fptr(scratch), ptr(bars), cuda_stream());
     if (rc != MB200_EUNSUPPORTED && rc != MB200_ETOOBIG) {
       check(rc, "mb200_block_step");
+      check_status("mb200_block_step");
       return {out, h_new, fresh};
     }
   }

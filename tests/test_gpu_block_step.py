@@ -103,3 +103,39 @@ def test_parameters_off_the_16_byte_grid(Bsz, d_model, dtype):
     rt, at = (1e-4, 1e-5) if dtype == torch.float32 else (3e-2, 3e-2)
     assert_close(got, want, rt, at)
     assert_close(got_h, want_h, rt, at)
+
+
+@pytest.mark.expects_wait_timeout
+def test_a_step_that_gave_up_is_reported_and_not_for_good():
+    """Counters marked as a launch that gave up leaves them: later steps on them report it, and once that has been read the stream works
+    again.  With MB200_CHECK_STATUS=1 the step itself raises."""
+    import os
+    import subprocess
+    import sys
+    from mamba_b200 import _lib, step
+    from tests.helpers import ROOT
+    torch.manual_seed(1)
+    blk, x, cache = RefShapedBlock(64).to(DEV), torch.randn(2, 64, device=DEV), (None, torch.zeros(2, 128, 3, device=DEV))
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        for stream in (torch.cuda.current_stream(), side):
+            with torch.cuda.stream(stream):
+                want = step(blk, x, cache)[0]
+                _lib.host().selftest_block_step_give_up(x)
+                step(blk, x, cache)
+                stream.synchronize()
+                assert _lib.device_status(0) == 1 and _lib.device_status(0) == 0
+                for _ in range(2):
+                    assert torch.equal(step(blk, x, cache)[0], want)
+                stream.synchronize()
+                assert _lib.device_status(0) == 0
+    code = ("import torch; from mamba_b200 import _lib, step; from tests.helpers import RefShapedBlock\n"
+            "b, x = RefShapedBlock(64).cuda(), torch.zeros(2, 64, device='cuda'); c = (None, torch.zeros(2, 128, 3, device='cuda'))\n"
+            "with torch.no_grad():\n"
+            "    step(b, x, c); _lib.host().selftest_block_step_give_up(x)\n"
+            "    try: step(b, x, c); print('silent')\n"
+            "    except RuntimeError as e: print('raised', 'gave up' in str(e))\n"
+            "    step(b, x, c); g = torch.cuda.CUDAGraph()\n"
+            "    with torch.cuda.graph(g): step(b, x, c)\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, MB200_CHECK_STATUS="1"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "raised True" in r.stdout, r.stdout + r.stderr
