@@ -494,6 +494,8 @@ extern "C" int mb200_selftest_wait_timeout(int polls, void* stream) {
 }
 
 extern "C" int mb200_device_status(void) {
+  // reading a symbol waits for the default stream only, not for streams created apart from it
+  if (cudaDeviceSynchronize() != cudaSuccess) return -1;
   const int f = mb200_fwd_device_status(), b = mb200_bwd_device_status(), k = mb200_block_step_device_status();
   int s = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&s, g_selftest_status, sizeof(int)) != cudaSuccess) return -1;

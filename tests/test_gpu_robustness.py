@@ -119,3 +119,14 @@ def test_reverse_backward_with_a_misaligned_upstream_gradient():
     for k in ("x", "delta", "z", "B", "C", "A", "D"):
         scale = max(1.0, go[k].abs().max().item())
         assert_close(lv[k].grad, go[k].float(), 1e-4, 1e-5 * scale * 4, k)
+
+
+@pytest.mark.expects_wait_timeout
+def test_status_waits_for_every_stream():
+    """Reading the status word waits for launches on streams that do not synchronise with the default one."""
+    from mamba_b200 import _lib
+    side = torch.cuda.Stream()
+    for _ in range(2):
+        assert _lib.load().mb200_selftest_wait_timeout(1 << 19, side.cuda_stream) == 0      # some 50 ms
+        assert _lib.device_status(0) == 1
+    assert _lib.device_status(0) == 0
