@@ -309,7 +309,7 @@ int mb200_add_rmsnorm_bwd(const void* s, const float* weight, const float* rstd,
                           int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, int dtype_res,
                           int dtype_y, void* stream);
 
-/* Element-wise jobs, up to 24 in one launch.  Job: dst[r, c] = op(src[r, c]) for r < rows, c < cols, both with unit
+/* Element-wise jobs, up to MB200_CONVERT_MAX_JOBS in one launch.  Job: dst[r, c] = op(src[r, c]) for r < rows, c < cols, both with unit
  * stride along c and their own row strides; columns src_cols .. cols-1 (all of them if src is NULL) count as zero.
  * MB200_CONVERT_NEG_EXP: dst = -exp(src).  MB200_CONVERT_MUL, _ADD: dst = src * factor, src + factor; factor is dense float32
  * (rows, cols). */
@@ -323,6 +323,7 @@ typedef struct {
   int slices;             /* > 1: src is the sum of that many matrices, slice_stride elements apart */
   int64_t slice_stride;
 } mb200_convert_job;
+enum { MB200_CONVERT_MAX_JOBS = 24 };
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
 /* mb200_conv_step_params with up to 3 conversions in the same launch. */

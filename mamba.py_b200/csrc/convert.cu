@@ -7,7 +7,7 @@
 namespace mb200 {
 namespace {
 
-constexpr int kMaxJobs = 24;
+constexpr int kMaxJobs = MB200_CONVERT_MAX_JOBS;
 
 __global__ void __launch_bounds__(kConvertThreads) convert_kernel(const __grid_constant__ Jobs<kMaxJobs> jobs) {
   convert_block(jobs, int(blockIdx.x));

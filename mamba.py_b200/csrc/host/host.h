@@ -159,12 +159,14 @@ struct Products {
   void run();
 };
 
-// Up to 24 element-wise jobs in one launch (mb200_convert).
+// Element-wise jobs of one launch (mb200_convert).
 struct Convert {
-  mb200_convert_job jobs[24];
+  mb200_convert_job jobs[MB200_CONVERT_MAX_JOBS];
   int n = 0;
   mb200_convert_job& add(const void* src, at::ScalarType st, void* dst, at::ScalarType dt, int64_t rows, int64_t cols, int64_t src_cols,
                          int64_t src_stride, int64_t dst_stride, int op = MB200_CONVERT_COPY) {
+    // (not launched when full: a job's source may be a product that has yet to run)
+    TORCH_CHECK(n < MB200_CONVERT_MAX_JOBS, "mamba_b200: more than ", int(MB200_CONVERT_MAX_JOBS), " conversions for one launch");
     mb200_convert_job& j = jobs[n++];
     j = mb200_convert_job{src, dst, nullptr, rows, cols, src_cols, src_stride, dst_stride, dtype_code(st), dtype_code(dt), op, 1, 0};
     return j;
@@ -226,6 +228,8 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
                                               const Tensor& dt_b, const Tensor& A_log, const Tensor& D, const Tensor& out_w,
                                               const OptTensor& out_b, int64_t dt_rank, int64_t d_state);
 
+// Queues `n` empty conversions for one launch, without launching them.
+void selftest_queue_conversions(int64_t n);
 // Spoils the barrier counters that the current stream keeps for the one-launch step on `on`'s device, as a launch that gave up does.
 void selftest_block_step_give_up(const Tensor& on);
 

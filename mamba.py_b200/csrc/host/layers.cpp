@@ -232,6 +232,11 @@ std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residu
   return {y, s};
 }
 
+void selftest_queue_conversions(int64_t n) {
+  Convert conv;
+  for (int64_t i = 0; i < n; ++i) conv.add(nullptr, at::kFloat, nullptr, at::kFloat, 0, 0, 0, 0, 0);
+}
+
 // ---------------------------------------------------------------------------------------------- the last residual add
 namespace {
 

@@ -139,3 +139,11 @@ def test_parameters_that_are_plain_attributes(gone):
     value = owner._parameters.pop(name)
     owner.__dict__[name] = value
     assert _plain_block(m) is None
+
+
+def test_conversions_of_one_launch_are_bounded():
+    """One more conversion than a launch takes is an error, not a write past the queue."""
+    from mamba_b200 import _lib
+    _lib.host().selftest_queue_conversions(24)
+    with pytest.raises(RuntimeError, match="more than 24 conversions"):
+        _lib.host().selftest_queue_conversions(25)
