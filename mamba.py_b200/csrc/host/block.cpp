@@ -337,6 +337,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
   bool grad = false;
   for (const Tensor& t : in) {
     require_cuda(t);
+    refuse_tangents(t);
     grad = grad || wants_grad(t);
   }
   const c10::cuda::CUDAGuard guard(x.device());

@@ -3,6 +3,7 @@
 // libmamba_b200.so (include/mamba_b200.h) only.
 #pragma once
 #include <torch/extension.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -122,6 +123,13 @@ template <typename... Ts> bool wants_grad(const Ts&... ts) {
   for (const Tensor* t : {&ts...})
     if (t->defined() && t->requires_grad()) return true;
   return false;
+}
+// The nodes have no forward-mode derivative.  A tangent that a call would lose is an error, with gradients recorded or not.
+inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
+template <typename... Ts> void refuse_tangents(const Ts&... ts) {
+  if (!torch::autograd::ForwardADLevel::try_get_by_idx(0)) return;
+  for (const Tensor* t : {&ts...})
+    TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(*t), "mamba_b200: forward-mode automatic differentiation is not implemented");
 }
 template <typename N> std::shared_ptr<N> new_node() { return std::shared_ptr<N>(new N(), torch::autograd::deleteNode); }
 

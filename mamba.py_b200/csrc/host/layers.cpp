@@ -43,6 +43,7 @@ struct ConvBackward : public torch::autograd::Node {
 Tensor conv1d_silu(const Tensor& x, const Tensor& weight, const OptTensor& bias_) {
   const Tensor& bias = value(bias_);
   require_cuda(x, weight, bias);
+  refuse_tangents(x, weight, bias);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor y, xs, w32, b32;
   {
@@ -166,6 +167,7 @@ constexpr const char* kNeedCuda = "mamba_b200 kernels need CUDA tensors; there i
 Tensor rms_norm(const Tensor& x, const OptTensor& weight_, double eps) {
   const Tensor& weight = value(weight_);
   TORCH_CHECK(x.is_cuda(), kNeedCuda);
+  refuse_tangents(x, weight);
   const c10::cuda::CUDAGuard guard(x.device());
   const bool grad = wants_grad(x, weight);
   Tensor y, x2, w32, rstd;
@@ -199,6 +201,7 @@ Tensor rms_norm(const Tensor& x, const OptTensor& weight_, double eps) {
 std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const OptTensor& residual_, const OptTensor& weight_, double eps) {
   const Tensor &residual = value(residual_), &weight = value(weight_);
   TORCH_CHECK(x.is_cuda(), kNeedCuda);
+  refuse_tangents(x, residual, weight);
   const c10::cuda::CUDAGuard guard(x.device());
   // the sum has the type `x + residual` would give; under autocast y comes out in the autocast dtype, which is what the
   // projection that consumes it would cast it to anyway
@@ -260,7 +263,7 @@ struct AddResidualBackward : public torch::autograd::Node {
 // x + residual at the end of a stack: a bfloat16 mixer output on a float32 stream in one vectorised pass.
 Tensor add_residual(const Tensor& x, const Tensor& residual) {
   const bool ours = x.is_cuda() && residual.is_cuda() && x.sizes() == residual.sizes() && x.is_contiguous() && residual.is_contiguous() &&
-                    x.scalar_type() == at::kBFloat16 && residual.scalar_type() == at::kFloat;
+                    x.scalar_type() == at::kBFloat16 && residual.scalar_type() == at::kFloat && !has_tangent(x) && !has_tangent(residual);
   if (!ours) return at::add(x, residual);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor s;

@@ -227,6 +227,7 @@ py::object selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A,
   {
     py::gil_scoped_release no_gil;
     require_cuda(x, delta, A, B, C, D, z, bias, h0);
+    refuse_tangents(x, delta, A, B, C, D, z, bias, h0);
     const c10::cuda::CUDAGuard guard(x.device());
     const auto dt = act_dtype(x, delta, z, B, C);
     const bool grad = wants_grad(x, delta, A, B, C, D, z, bias, h0);
@@ -316,6 +317,7 @@ struct PScanBackward : public torch::autograd::Node {
 
 Tensor pscan(const Tensor& A, const Tensor& X) {
   require_cuda(A, X);
+  refuse_tangents(A, X);
   TORCH_CHECK_VALUE(A.dim() == 4 && A.sizes() == X.sizes(), "pscan expects two (B, L, D, N) tensors, got ", A.sizes(), " and ", X.sizes());
   TORCH_CHECK_TYPE(A.scalar_type() == X.scalar_type(), "A_in and X_in must have the same dtype");
   act_dtype(X);

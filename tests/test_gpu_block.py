@@ -197,3 +197,29 @@ def test_activations_and_caches_of_other_sizes_are_refused():
                     lambda: mamba.conv_step_fn(z(2, 32), z(2, 32, 3), z(16, 1, 4), None)):
             with pytest.raises(RuntimeError):
                 bad()
+
+
+@pytest.mark.parametrize("what", ["block", "both", "rms_norm", "add_rms_norm", "conv", "scan", "pscan"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_tangents_are_refused(what, grad):
+    """None of these has a forward-mode derivative: a tangent is an error and not lost."""
+    import torch.autograd.forward_ad as fw
+    import mamba_b200
+    from mamba_b200 import mamba, vim
+    r = lambda *s: torch.randn(*s, device=DEV)
+    block, both, B = _build(32, 16, False), _build(32, 16, True), r(2, 20, 16)
+    call = {"block": lambda x: mamba.forward(block, x), "both": lambda x: vim.forward(both, x), "rms_norm": lambda x: mamba.rms_norm(x, r(32)),
+            "add_rms_norm": lambda x: mamba.add_rms_norm(r(2, 20, 32), x, r(32)), "conv": lambda x: mamba.causal_conv1d_silu(x, r(32, 1, 4)),
+            "scan": lambda x: mamba_b200.selective_scan_fn(r(2, 20, 32), x, -torch.ones(32, 16, device=DEV), B, B),
+            "pscan": lambda x: mamba_b200.pscan(x[..., None], x[..., None])}[what]
+    call(r(2, 20, 32))
+    with fw.dual_level(), torch.set_grad_enabled(grad), pytest.raises(NotImplementedError):
+        call(fw.make_dual(r(2, 20, 32), r(2, 20, 32)))
+
+
+def test_last_residual_add_keeps_a_tangent():
+    import torch.autograd.forward_ad as fw
+    from mamba_b200 import _lib
+    x, s, t = (torch.randn(2, 20, 32, device=DEV) for _ in range(3))
+    with fw.dual_level():
+        assert torch.equal(fw.unpack_dual(_lib.host().add_residual(x.bfloat16(), fw.make_dual(s, t))).tangent, t)
