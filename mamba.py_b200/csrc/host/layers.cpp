@@ -153,6 +153,10 @@ struct AddRmsNormBackward : public torch::autograd::Node {
     } else {
       ds = grads[1];                                                       // only the sum was used further on
       if (!ds.defined()) return out;
+      if (w32.defined() && task_should_compute_output(2)) {                // which the weight has no part in
+        out[2] = empty(w32.sizes(), tw, s2);
+        zero_fill(out[2]);
+      }
     }
     if (!out[0].defined()) out[0] = like(ds, tx);
     if (has_residual) out[1] = like(ds, tr);

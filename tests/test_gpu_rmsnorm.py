@@ -87,3 +87,12 @@ def test_residual_add_fused_with_rms_norm(shape, dx, dres):
     if rc is not None:
         assert_close(rc.grad, rr.grad.float(), tol[0], tol[1] * 4, "dres")
     assert_close(wc.grad, wr.grad.float(), tol[0] * 10, tol[1] * max(1.0, wr.grad.abs().max().item()) * 4, "dweight")
+
+
+def test_add_rms_norm_with_one_output_used():
+    """Where only the sum is used further on, the weight's gradient is zero, not missing."""
+    import mamba_b200
+    x, r, w = (torch.randn(*s, device=DEV, requires_grad=True) for s in ((3, 5, 32), (3, 5, 32), (32,)))
+    _, s = mamba_b200.add_rms_norm(x, r, w, 1e-5)
+    dx, dr, dw = torch.autograd.grad(s.sum(), (x, r, w))
+    assert torch.equal(dx, torch.ones_like(x)) and torch.equal(dr, dx) and not dw.any() and dw.shape == w.shape
