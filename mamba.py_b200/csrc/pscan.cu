@@ -279,6 +279,10 @@ pscan_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* __re
 // these pairs by shuffles, the warps' totals go through shared memory, and the thread walks its steps again from the state
 // that enters them, out of registers.  Longer rows are a loop that carries the state.  Inputs are read once (the segmented
 // passes read them twice) and nothing is allocated.
+// Nothing is multiplied by a state that is not there (zero times infinity is not zero): a span's state begins with its first step's
+// input, and before any state has entered the row a product of A, which may have overflowed, has no part in the result.
+// Spans of up to 64 steps are still combined by their products: a state of zero behind steps whose product is beyond float32's range
+// comes out as NaN, and an infinite one may, as both do in the reference's tree (mambapy/pscan.py:35-110).
 // Forward / backward, us, segmented passes before: 1 x 1000 x 2048 channels float32 26.4 / 28.9 -> 8.8 / 12.8, bfloat16 33 / 38 -> 8.8 / 8.8;
 // 4 x 1000 x 8192 float32 122 / 175 -> 76 / 121 (bytes 61 / 102); 1 x 16384 x 24576 1340 / 1850 -> 953 / 1609; 64 steps of 512 channels
 // 8.1 / 12.9 -> 4.7 / 4.7 (one serial thread per vector before).
@@ -349,19 +353,21 @@ __device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total) {
 }
 
 // The state entering this thread's segment, from the state `carry` entering the CTA's timesteps, which becomes the one leaving them.
+// none: no state enters, `carry` is zero.
 template <typename T, int V, bool kReverse>
-__device__ __forceinline__ void enter(const Span<V>& before, const Span<V>* totals, float (&carry)[V], float (&h)[V]) {
+__device__ __forceinline__ void enter(const Span<V>& before, const Span<V>* totals, bool none, float (&carry)[V], float (&h)[V]) {
   constexpr int kVecs = CtaTile<T, V>::kVecs;
   const int warps = blockDim.x / 32, warp = threadIdx.x / 32, mine = kReverse ? warps - 1 - warp : warp, v = threadIdx.x % kVecs;
 #pragma unroll 1
   for (int k = 0; k < warps; ++k) {
     if (k == mine) {
 #pragma unroll
-      for (int i = 0; i < V; ++i) h[i] = fmaf(before.P[i], carry[i], before.S[i]);
+      for (int i = 0; i < V; ++i) h[i] = none ? before.S[i] : fmaf(before.P[i], carry[i], before.S[i]);
     }
     const Span<V>& t = totals[(kReverse ? warps - 1 - k : k) * kVecs + v];
 #pragma unroll
-    for (int i = 0; i < V; ++i) carry[i] = fmaf(t.P[i], carry[i], t.S[i]);
+    for (int i = 0; i < V; ++i) carry[i] = none ? t.S[i] : fmaf(t.P[i], carry[i], t.S[i]);
+    none = false;
   }
 }
 
@@ -401,12 +407,12 @@ pscan_cta_fwd_kernel(const T* __restrict__ A, const T* __restrict__ X, T* __rest
 #pragma unroll
         for (int i = 0; i < V; ++i) {
           const float af = av[u].f(i);
-          w.S[i] = fmaf(af, w.S[i], xv[u].f(i));
+          w.S[i] = u || t0 == 0 ? fmaf(af, w.S[i], xv[u].f(i)) : xv[u].f(i);   // step 0 as the walk below has it
           w.P[i] *= af;
         }
     warp_exclusive<T, V, false>(w, totals[buf] + threadIdx.x / 32 * kVecs);
     __syncthreads();                                     // one per chunk: the next one writes the other buffer
-    enter<T, V, false>(w, totals[buf], carry, h);
+    enter<T, V, false>(w, totals[buf], first == 0 && !h0, carry, h);
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (u < n) {
@@ -469,7 +475,7 @@ pscan_cta_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* 
         }
     warp_exclusive<T, V, true>(w, totals[buf] + threadIdx.x / 32 * kVecs);
     __syncthreads();
-    enter<T, V, true>(w, totals[buf], carry, cy);
+    enter<T, V, true>(w, totals[buf], first + chunk >= L, carry, cy);
 #pragma unroll
     for (int u = U - 1; u >= 0; --u)
       if (u < n) {
