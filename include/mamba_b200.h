@@ -412,7 +412,7 @@ int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, 
  * (2W, D_model), xproj_w (R+2N, W), dt_w (W, R), out_w (D_model, W) and in_b, out_b (or NULL) have type `dtype`, the small
  * parameters conv_w (W, d_conv), conv_b (W, or NULL), dt_b (W), A_log (W, N), D (W) a type each.  conv_out may be conv_in, h_out
  * may be h_in.  scratch: mb200_block_step_scratch_floats floats; barriers: mb200_block_step_barrier_bytes bytes that are zero
- * before the first launch, left zero by every launch for the next, and used by one launch at a time.
+ * before the first launch, left fit for the next one by every launch, and used by one launch at a time.
  * MB200_EUNSUPPORTED: weight rows off the 16-byte grid.  MB200_ETOOBIG: more than 8 tokens, or activations beyond 200 KB. */
 typedef struct {
   const void *x, *in_w, *in_b, *conv_in, *conv_w, *conv_b, *xproj_w, *dt_w, *dt_b, *A_log, *D, *out_w, *out_b;

@@ -24,7 +24,8 @@ constexpr int kBarrierSpins = 1 << 22;                 // polls at least 32 ns a
 
 __device__ int g_block_step_status = MB200_DEV_OK;
 
-// Counters of the three barriers, zero between launches; [3] marks a workspace whose launch gave up.
+// Counters of the three barriers, zero when a launch comes to them (the third is cleared behind the next launch's first barrier);
+// `poisoned` marks a workspace whose launch gave up.
 struct StepBarriers {
   unsigned count[3];
   unsigned poisoned;

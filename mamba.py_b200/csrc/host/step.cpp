@@ -68,9 +68,10 @@ WindowStep window_step(const Tensor& x, const Tensor& inputs, const Tensor& weig
 }
 
 // ---- barrier counters of the one-launch step -----------------------------------------------------------------------
-// A launch leaves its counters zero for the next one on the same stream, so a stream keeps its own.  At most kMaxStreams are
-// kept; a stream beyond them, and a stream that is being captured into a graph (whose replays may run anywhere), gets
-// counters of its own for the one call, cleared on the stream.  A launch that gave up at a barrier spoils its counters; once
+// A launch leaves its counters fit for the next one on the same stream, so a stream keeps its own.  At most kMaxStreams are
+// kept; a stream beyond them, a stream that is being captured into a graph (whose replays may run anywhere), and a stream that
+// torch did not make (destroyed, its handle may come back for another stream while its last launch still runs) gets counters of its
+// own for the one call, cleared on the stream.  A launch that gave up at a barrier spoils its counters; once
 // somebody has read its status word, none from before are used again.
 constexpr size_t kMaxStreams = 64;
 
@@ -87,7 +88,8 @@ Tensor barrier_counters(const Tensor& on) {
     kept.clear();
     give_ups = now;
   }
-  const bool keep = capturing == cudaStreamCaptureStatusNone;
+  const bool foreign = s.stream() && reinterpret_cast<intptr_t>(s.stream()) == s.id();        // torch's own have numbers for ids
+  const bool keep = capturing == cudaStreamCaptureStatusNone && !foreign;
   if (keep) {
     const auto it = kept.find(key);
     if (it != kept.end()) return it->second;

@@ -139,3 +139,23 @@ def test_a_step_that_gave_up_is_reported_and_not_for_good():
             "    with torch.cuda.graph(g): step(b, x, c)\n")
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, MB200_CHECK_STATUS="1"), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "raised True" in r.stdout, r.stdout + r.stderr
+
+
+def test_streams_of_others_keep_nothing():
+    """A stream that torch did not make may be destroyed and its handle used again: it has counters for each call."""
+    import ctypes
+    from mamba_b200 import _lib, step
+    torch.manual_seed(2)
+    blk, x, cache = RefShapedBlock(64).to(DEV), torch.randn(2, 64, device=DEV), (None, torch.zeros(2, 128, 3, device=DEV))
+    rt = ctypes.CDLL("libcudart.so.12")
+    handle = ctypes.c_void_p()
+    with torch.no_grad():
+        want = step(blk, x, cache)[0]
+        torch.cuda.synchronize()
+        assert rt.cudaStreamCreateWithFlags(ctypes.byref(handle), 1) == 0
+        with torch.cuda.stream(torch.cuda.ExternalStream(handle.value)):
+            for _ in range(3):
+                assert torch.equal(step(blk, x, cache)[0], want)
+                _lib.host().selftest_block_step_give_up(x)
+        torch.cuda.synchronize()
+        assert rt.cudaStreamDestroy(handle) == 0
