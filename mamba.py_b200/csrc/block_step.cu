@@ -249,12 +249,14 @@ int block_step_launch(StepParams& p, cudaStream_t st) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return MB200_ELAUNCH;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return MB200_ELAUNCH;
+  // 48 KB are there without asking, for the kernel's own few static bytes (a barrier's answer) as well
+  if (smem > 47 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return MB200_ELAUNCH;
   void* args[] = {&p};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(unsigned(sms)), dim3(kStepThreads), args, size_t(smem), st) ==
-                 cudaSuccess
-             ? MB200_OK
-             : MB200_ELAUNCH;
+  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(unsigned(sms)), dim3(kStepThreads), args, size_t(smem), st) ==
+      cudaSuccess)
+    return MB200_OK;
+  (void)cudaGetLastError();                              // not for the next launch to find
+  return MB200_ELAUNCH;
 }
 
 template <typename T, int N>
