@@ -114,7 +114,8 @@ std::vector<Partials> Products::tall(int64_t n, const Tensor& a, int64_t sa, con
   const bool ours = A.ok && B.ok && !A.trans && !B.trans && b.size(0) == T && b.scalar_type() == dt && convertible(dt) && convertible(out) && plain_settings();
   std::vector<Partials> res;
   const int64_t tiles = (M + 63) / 64 * ((N + 63) / 64) * n;
-  int64_t S = std::max<int64_t>(1, std::min<int64_t>({16, 148 / tiles, T / 512}));
+  const int64_t sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  int64_t S = tiles ? std::max<int64_t>(1, std::min<int64_t>({16, sms / tiles, T / 512})) : 1;
   if (own || !ours || (S == 1 && n == 1 && dt == at::kFloat)) {
     for (int64_t i = 0; i < n; ++i) {
       const Tensor o = empty({M, N}, own ? out : dt, a);
