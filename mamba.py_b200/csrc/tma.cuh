@@ -54,10 +54,20 @@ inline bool tma_encode(CUtensorMap* map, const void* base, bool bf16, int64_t B,
   cuuint64_t strides[2] = {cuuint64_t(sl) * es, cuuint64_t(sb_eff) * es};
   cuuint32_t box[3] = {cuuint32_t(box_c), cuuint32_t(box_l), 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  return enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-             const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  auto encode = [&] {
+    return enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+               const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult rc = encode();
+  if (rc == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread that has made no runtime call yet (autograd's, in front of its first kernel) has no current context, and this may be
+    // its first call of all.  Selecting the device it is on binds that device's.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) rc = encode();
+  }
+  return rc == CUDA_SUCCESS;
 }
 
 #ifdef __CUDACC__

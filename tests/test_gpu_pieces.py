@@ -92,3 +92,25 @@ def test_carries_that_were_not_written_do_not_enter():
     y = mamba_b200.selective_scan_fn(a[0], a[1], A, *BC, delta_bias=torch.zeros(1536, device=DEV))
     for g in torch.autograd.grad(y, a, torch.ones_like(y)):
         assert torch.isfinite(g).all()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+def test_first_call_of_a_thread(reverse):
+    """A scan's backward as the first CUDA call that autograd's thread makes, and a forward as the first of a new thread: tensor maps are
+    encoded there as everywhere (rows of any length are cut, and scanned in reverse, on the tensor-map path only)."""
+    import os
+    import subprocess
+    import sys
+    from tests.helpers import ROOT
+    code = ("import threading, torch, mamba_b200\n"
+            "torch.manual_seed(0); r = lambda *s: torch.randn(*s, device='cuda')\n"
+            "leaves = [t.requires_grad_() for t in (r(1, 1003, 256), 0.1 * r(1, 1003, 256).abs(), -r(256, 16).exp(), r(1, 1003, 16), r(1, 1003, 16))]\n"
+            f"run = lambda: mamba_b200.selective_scan_fn(*leaves, reverse={reverse})\n"
+            "dy, first = r(1, 1003, 256), []\n"
+            "t = threading.Thread(target=lambda: first.append(run().detach())); t.start(); t.join()\n"
+            "y = run(); a = torch.autograd.grad(y, leaves, dy); b = torch.autograd.grad(run(), leaves, dy)\n"
+            "assert torch.equal(first[0], y)\n"
+            "for p, q in zip(a, b): assert (p - q).norm() <= 1e-5 * q.norm()\n"
+            "print('done')\n")
+    p = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and "done" in p.stdout, p.stdout + p.stderr
