@@ -197,15 +197,15 @@ struct ScanBackward : public torch::autograd::Node {
 // work items a piece (a CTA owns one, three fit an SM), and one CTA alone on an SM runs much faster than one of three.
 // Measured, us for 2048 timesteps with 1 / 2 / 3 CTAs on every SM of 148, means of both types and of A as initialised and as trained:
 // forward 85 / 127 / 185 (80 / 119 / 166 without saved states and with A as initialised, 90 / 138 / 206 the other way round), backward
-// 315 / 456 / 636, forward carry pass 65 / 96 / 134, reverse one 71 / 104 / 146.  Launches and the fold cost about 6 us a pass.  Fewer
-// pieces win unless more are 3 % better.  Over 140 rows of 960 to 7680 steps (1 to 32 rows 64 to 5120 wide, both types, training and
-// inference) the count picked takes 0.8 % longer than the best one on average and 7.4 % at most; the model is 6 % off (one sigma).
+// 315 / 456 / 636, forward carry pass 65 / 96 / 134, reverse one 71 / 104 / 146; of these, filling the pipeline takes as long as some
+// 20 timesteps.  The launches of a carry pass and a fold add about 4 us.  Over 140 cases of 960 to 7680 steps (1 to 32 rows 64 to 5120
+// wide, both types, training and inference) the count picked takes 0.4 % longer than the best one on average and 5.4 % at most.
 int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
-  constexpr double kFwd[] = {0, 85. / 2048, 127. / 2048, 185. / 2048}, kBwd[] = {0, 315. / 2048, 456. / 2048, 636. / 2048},
-                   kFwdCarry[] = {0, 65. / 2048, 96. / 2048, 134. / 2048}, kBwdCarry[] = {0, 71. / 2048, 104. / 2048, 146. / 2048};
+  constexpr double kFill = 20, kFwd[] = {0, 85, 127, 185}, kBwd[] = {0, 315, 456, 636}, kFwdCarry[] = {0, 65, 96, 134},
+                   kBwdCarry[] = {0, 71, 104, 146};
   const double items = double(batch) * double((width + 31) / 32);
   const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  auto passes = [&](double ctas, const double (&t)[4]) {                 // us per timestep of the longest SM
+  auto passes = [&](double ctas, const double (&t)[4]) {                 // of 2048 timesteps on the longest SM
     const int per_sm = int(std::ceil(ctas / sms)), full = per_sm / 3, rest = per_sm % 3;
     return full * t[3] + t[rest];
   };
@@ -214,9 +214,10 @@ int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
   for (int64_t S = 1; S <= 24 && (S == 1 || length / S >= 64); ++S) {
     const double len = double(S == 1 ? length : (length + 16 * S - 1) / (16 * S) * 16);
     if (S > 1 && (S - 1) * len >= length) continue;
-    double us = len * (passes(items * S, kFwd) + (grad ? passes(items * S, kBwd) : 0));
-    if (S > 1) us += len * passes(items * (S - 1), kFwdCarry) + 12 + (grad ? len * passes(items * (S - 1), kBwdCarry) + 12 : 0);
-    if (S == 1 || us < 0.97 * best_us) {
+    double all = passes(items * S, kFwd) + (grad ? passes(items * S, kBwd) : 0);
+    if (S > 1) all += passes(items * (S - 1), kFwdCarry) + (grad ? passes(items * (S - 1), kBwdCarry) : 0);
+    const double us = all * (len + kFill) / (2048 + kFill) + (S > 1 ? (grad ? 8 : 4) : 0);
+    if (S == 1 || us < best_us) {
       best = S;
       best_us = us;
     }
