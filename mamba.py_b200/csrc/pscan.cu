@@ -326,8 +326,9 @@ template <int V> struct Span {                                   // a run of tim
 
 // On entry `w` is the thread's own span.  On return it is the span of everything before the thread's segment in scan order
 // inside its warp, and the warp's total is in `total` of shared memory.  kReverse: scan order runs from the last segment to the first.
+// fresh: no state enters the warp, so that whatever the products hold is left out.
 template <typename T, int V, bool kReverse>
-__device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total) {
+__device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total, bool fresh) {
   constexpr int kVecs = CtaTile<T, V>::kVecs, kSegs = CtaTile<T, V>::kSegs;
   const int lane = threadIdx.x & 31, seg = kReverse ? kSegs - 1 - lane / kVecs : lane / kVecs;
 #pragma unroll
@@ -342,6 +343,9 @@ __device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total) {
       }
     }
   }
+  if (fresh)
+#pragma unroll
+    for (int i = 0; i < V; ++i) w.P[i] = 0.f;
   if (seg == kSegs - 1) total[lane % kVecs] = w;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
@@ -353,21 +357,19 @@ __device__ __forceinline__ void warp_exclusive(Span<V>& w, Span<V>* total) {
 }
 
 // The state entering this thread's segment, from the state `carry` entering the CTA's timesteps, which becomes the one leaving them.
-// none: no state enters, `carry` is zero.
 template <typename T, int V, bool kReverse>
-__device__ __forceinline__ void enter(const Span<V>& before, const Span<V>* totals, bool none, float (&carry)[V], float (&h)[V]) {
+__device__ __forceinline__ void enter(const Span<V>& before, const Span<V>* totals, float (&carry)[V], float (&h)[V]) {
   constexpr int kVecs = CtaTile<T, V>::kVecs;
   const int warps = blockDim.x / 32, warp = threadIdx.x / 32, mine = kReverse ? warps - 1 - warp : warp, v = threadIdx.x % kVecs;
 #pragma unroll 1
   for (int k = 0; k < warps; ++k) {
     if (k == mine) {
 #pragma unroll
-      for (int i = 0; i < V; ++i) h[i] = none ? before.S[i] : fmaf(before.P[i], carry[i], before.S[i]);
+      for (int i = 0; i < V; ++i) h[i] = fmaf(before.P[i], carry[i], before.S[i]);
     }
     const Span<V>& t = totals[(kReverse ? warps - 1 - k : k) * kVecs + v];
 #pragma unroll
-    for (int i = 0; i < V; ++i) carry[i] = none ? t.S[i] : fmaf(t.P[i], carry[i], t.S[i]);
-    none = false;
+    for (int i = 0; i < V; ++i) carry[i] = fmaf(t.P[i], carry[i], t.S[i]);
   }
 }
 
@@ -407,12 +409,16 @@ pscan_cta_fwd_kernel(const T* __restrict__ A, const T* __restrict__ X, T* __rest
 #pragma unroll
         for (int i = 0; i < V; ++i) {
           const float af = av[u].f(i);
-          w.S[i] = u || t0 == 0 ? fmaf(af, w.S[i], xv[u].f(i)) : xv[u].f(i);   // step 0 as the walk below has it
+          w.S[i] = u ? fmaf(af, w.S[i], xv[u].f(i)) : xv[u].f(i);
           w.P[i] *= af;
         }
-    warp_exclusive<T, V, false>(w, totals[buf] + threadIdx.x / 32 * kVecs);
+    const bool fresh = first == 0 && !h0 && threadIdx.x < 32;
+    if (fresh && t0 == 0 && n > 0)
+#pragma unroll
+      for (int i = 0; i < V; ++i) w.S[i] = fmaf(av[0].f(i), 0.f, w.S[i]);  // step 0 as the walk below has it
+    warp_exclusive<T, V, false>(w, totals[buf] + threadIdx.x / 32 * kVecs, fresh);
     __syncthreads();                                     // one per chunk: the next one writes the other buffer
-    enter<T, V, false>(w, totals[buf], first == 0 && !h0, carry, h);
+    enter<T, V, false>(w, totals[buf], carry, h);
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (u < n) {
@@ -473,9 +479,9 @@ pscan_cta_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* 
           w.S[i] = af * (gv[u].f(i) + w.S[i]);
           w.P[i] *= af;
         }
-    warp_exclusive<T, V, true>(w, totals[buf] + threadIdx.x / 32 * kVecs);
+    warp_exclusive<T, V, true>(w, totals[buf] + threadIdx.x / 32 * kVecs, first + chunk >= L && threadIdx.x + 32 >= blockDim.x);
     __syncthreads();
-    enter<T, V, true>(w, totals[buf], first + chunk >= L, carry, cy);
+    enter<T, V, true>(w, totals[buf], carry, cy);
 #pragma unroll
     for (int u = U - 1; u >= 0; --u)
       if (u < n) {
