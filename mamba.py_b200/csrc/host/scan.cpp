@@ -198,10 +198,11 @@ struct ScanBackward : public torch::autograd::Node {
 // Measured, us for 2048 timesteps with 1 / 2 / 3 CTAs on every SM of 148, means of both types and of A as initialised and as trained:
 // forward 85 / 127 / 185 (80 / 119 / 166 without saved states and with A as initialised, 90 / 138 / 206 the other way round), backward
 // 315 / 456 / 636, forward carry pass 65 / 96 / 134, reverse one 71 / 104 / 146; of these, filling the pipeline takes as long as some
-// 20 timesteps.  The launches of a carry pass and a fold add about 4 us.  Over 140 cases of 960 to 7680 steps (1 to 32 rows 64 to 5120
-// wide, both types, training and inference) the count picked takes 0.4 % longer than the best one on average and 5.4 % at most.
+// 10 timesteps.  A carry pass and a fold add 4 us of launches on the GPU and 12 of host time, which is what short calls wait for.  Over
+// 140 cases of 960 to 7680 steps (1 to 32 rows 64 to 5120 wide, both types, training and inference) the count picked takes 0.4 % longer
+// than the best one on average and 5.8 % at most.
 int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
-  constexpr double kFill = 20, kFwd[] = {0, 85, 127, 185}, kBwd[] = {0, 315, 456, 636}, kFwdCarry[] = {0, 65, 96, 134},
+  constexpr double kFill = 10, kFwd[] = {0, 85, 127, 185}, kBwd[] = {0, 315, 456, 636}, kFwdCarry[] = {0, 65, 96, 134},
                    kBwdCarry[] = {0, 71, 104, 146};
   const double items = double(batch) * double((width + 31) / 32);
   const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
@@ -216,7 +217,7 @@ int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
     if (S > 1 && (S - 1) * len >= length) continue;
     double all = passes(items * S, kFwd) + (grad ? passes(items * S, kBwd) : 0);
     if (S > 1) all += passes(items * (S - 1), kFwdCarry) + (grad ? passes(items * (S - 1), kBwdCarry) : 0);
-    const double us = all * (len + kFill) / (2048 + kFill) + (S > 1 ? (grad ? 8 : 4) : 0);
+    const double us = all * (len + kFill) / (2048 + kFill) + (S > 1 ? (grad ? 24 : 12) : 0);
     if (S == 1 || us < best_us) {
       best = S;
       best_us = us;
