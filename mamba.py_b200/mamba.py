@@ -153,7 +153,7 @@ def step(self, x, cache):
     return self.out_proj(y), (h, inputs)
 
 
-_linear_forward = nn.Linear.forward
+_Linear, _linear_forward = nn.Linear, nn.Linear.forward
 
 
 def _plain_linear(m):
@@ -161,16 +161,17 @@ def _plain_linear(m):
     subclass, no hook of any kind, no `forward` of its own (offload and dispatch wrappers put theirs on the instance), not compiled
     by itself, and an ordinary tensor as its weight (quantised and distributed ones dispatch for themselves) among its parameters
     (replicas and pruning keep theirs as plain attributes)."""
-    if type(m) is not nn.Linear or nn.Linear.forward is not _linear_forward:
+    if type(m) is not _Linear or _Linear.forward is not _linear_forward:
         return None
     d = m.__dict__
     if (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d
             or d.get("_compiled_call_impl") is not None):
         return None
     p = d["_parameters"]
-    if type(p.get("weight")) not in (nn.Parameter, torch.Tensor) or "bias" not in p:
+    w = p.get("weight")
+    if not (type(w) is nn.Parameter or type(w) is torch.Tensor) or "bias" not in p:
         return None
-    return p["weight"], p["bias"]
+    return w, p["bias"]
 
 
 def _plain_block(self):
@@ -178,7 +179,7 @@ def _plain_block(self):
     extended (layer norms on dt, B, C) and has to be called as the module it is."""
     d = self.__dict__
     mods, pars = d.get("_modules"), d.get("_parameters")
-    if not mods or _has_any_global_hook() or any(mods.get(k) is not None for k in ("dt_layernorm", "B_layernorm", "C_layernorm")):
+    if not mods or _has_any_global_hook() or not (mods.get("dt_layernorm") is mods.get("B_layernorm") is mods.get("C_layernorm") is None):
         return None
     lin = [_plain_linear(mods.get(k)) for k in ("in_proj", "x_proj", "dt_proj", "out_proj")]
     conv, A_log, D = mods.get("conv1d"), pars.get("A_log"), pars.get("D")
@@ -200,30 +201,36 @@ def _fusable(self, x, dtype):
             and getattr(self, "C_layernorm", None) is None and cfg.d_state in (8, 16, 32, 64))
 
 
-def _native_linear(m, dtype):
+def _native_linear(m, dtype, amp):
     """The weight of a projection the native block can run itself on activations of `dtype`: an ordinary nn.Linear without
     a bias, of the activations' type or cast to it by autocast.  None for any other, which is called as the module it is."""
     p = _plain_linear(m)
-    if p is None or p[1] is not None or _has_any_global_hook():
+    if p is None or p[1] is not None:
         return None
-    ours = p[0].is_cuda and (p[0].dtype == dtype or (torch.is_autocast_enabled("cuda") and p[0].dtype in (torch.float32, torch.bfloat16)))
-    return p[0] if ours else None
+    w = p[0]
+    return w if w.is_cuda and (w.dtype == dtype or (amp and w.dtype in (torch.float32, torch.bfloat16))) else None
 
 
-def run_block(self, x, directions, halve=False):
+def run_block(self, x, directions, halve=False, called=()):
     """in_proj, the scans of `directions` (lists of seven parameters) and out_proj as one native call, with those projections
-    called as modules that are not ordinary ones.  None if the block does not take the native path; the second value is
-    in_proj(x) if that has been computed on the way."""
-    dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
-    in_w = _native_linear(self.in_proj, dtype) if x.dim() == 3 and x.dtype in (torch.float32, torch.bfloat16) else None
+    called as modules that are not ordinary ones.  None if the block does not take the native path, as it does not when one of
+    `called`, projections whose weights are among the parameters, has to be called; the second value is in_proj(x) if that has been
+    computed on the way."""
+    amp = torch.is_autocast_enabled("cuda")
+    dtype = torch.get_autocast_dtype("cuda") if amp else x.dtype
+    own = not _has_any_global_hook()
+    in_w = _native_linear(self.in_proj, dtype, amp) if own and x.dim() == 3 and x.dtype in (torch.float32, torch.bfloat16) else None
     if in_w is None or not _fusable(self, x, dtype):
         x, in_w = self.in_proj(x), None
         dtype = x.dtype
         if not _fusable(self, x, dtype):
             return None, x
+    for m in called:
+        if not own or _native_linear(m, dtype, amp) is None:
+            return None, x if in_w is None else self.in_proj(x)
     cfg = self.config
     params = [p for d in directions for p in d]
-    out_w = _native_linear(self.out_proj, dtype)
+    out_w = _native_linear(self.out_proj, dtype, amp) if own else None
     if out_w is not None:
         return _host().block(x, in_w, out_w, params, cfg.dt_rank, cfg.d_state, False, halve), None
     y = _host().block(x, in_w, None, params, cfg.dt_rank, cfg.d_state, False, False)

@@ -12,7 +12,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import host as _host
-from .mamba import _native_linear, causal_conv1d_silu, run_block, selective_scan_fn
+from .mamba import causal_conv1d_silu, run_block, selective_scan_fn
 
 
 def _conv_silu(conv, xs, L):
@@ -35,19 +35,19 @@ def forward(self, x):
     """mambapy/vim.py:205-261; x: (B, L, D) -> (B, L, D)."""
     _, L, _ = x.shape
     cfg = self.config
-    first = [self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight, self.dt_proj.bias, self.A_log, self.D]
-    dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
-    native = not cfg.bidirectional
-    if cfg.bidirectional and _host().reversible(self.D.shape[0], cfg.d_state, dtype):
-        second = [self.conv1d_b.weight, self.conv1d_b.bias, self.x_proj_b.weight, self.dt_proj_b.weight, self.dt_proj_b.bias,
-                  self.A_log_b, self.D_b]
-        native = self.conv1d_b.weight.shape[-1] == 4
-    # this block calls its x_proj as modules, so the native one is for those whose call is the matrix product; and without a bias
-    # of dt_proj the scan takes delta as it is
-    for s in ("", "_b") if cfg.bidirectional else ("",):
-        native = native and _native_linear(getattr(self, "x_proj" + s), dtype) is not None and getattr(self, "dt_proj" + s).bias is not None
-    if native:
-        out, xz = run_block(self, x, [first, second] if cfg.bidirectional else [first], cfg.bidirectional and cfg.divide_output)
+    conv, x_proj, dt_proj = self.conv1d, self.x_proj, self.dt_proj
+    directions = [[conv.weight, conv.bias, x_proj.weight, dt_proj.weight, dt_proj.bias, self.A_log, self.D]]
+    called = [x_proj]                                     # as modules, unless calling them is no more than the product
+    native = True
+    if cfg.bidirectional:
+        dtype = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        conv, x_proj, dt_proj = self.conv1d_b, self.x_proj_b, self.dt_proj_b
+        directions.append([conv.weight, conv.bias, x_proj.weight, dt_proj.weight, dt_proj.bias, self.A_log_b, self.D_b])
+        called.append(x_proj)
+        native = _host().reversible(directions[1][6].shape[0], cfg.d_state, dtype) and conv.weight.shape[-1] == 4
+    # without a bias of dt_proj the scan takes delta as it is
+    if native and all(d[4] is not None for d in directions):
+        out, xz = run_block(self, x, directions, cfg.bidirectional and cfg.divide_output, called)
         if out is not None:
             return out
     else:
