@@ -1,4 +1,5 @@
 // Decode steps: the state update, the conv window, and the whole block.
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include "host.h"
@@ -124,10 +125,30 @@ std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, cons
   return {o.xc, o.window};
 }
 
+// Whether so few tokens that the one launch is the better way.  It reads the activations of all tokens from shared memory again for
+// every output row, where the library's bfloat16 kernels use the tensor cores; the float32 ones take longer nearly everywhere.  us a
+// layer, weights from HBM, called from Python / inside a CUDA graph, one launch : library:
+//               256 wide             768 wide             1536 wide             2560 wide
+//   float32  1  15/17 : 39/16        21/23 : 39/28        32/33 : 52/39         59/59 : 68/54
+//            2  16/17 : 40/25        23/24 : 58/47        36/37 : 102/91        71/72 : 146/138
+//            4  17/18 : 40/28        27/29 : 65/53        45/46 : 112/97        92/93 : 129/117
+//            8  21/22 : 43/34        38/40 : 80/69        67/67 : 105/92        140/141 : 161/146
+//   bfloat16 1  15/16 : 47/16        21/23 : 48/24        30/31 : 51/31         51/52 : 54/43
+//            2  18/19 : 48/15        27/29 : 49/24        39/40 : 52/30         72/72 : 53/43
+//            4  23/25 : 48/16        41/44 : 49/23        60/61 : 52/30         122/121 : 54/43
+//            8  35/37 : 49/16        73/75 : 49/23        103/104 : 52/30       217/216 : 54/44
+// So up to 8 tokens in float32, and in bfloat16 as long as the tokens the kernel is built for (1, 2, 4, 8) times the inner width are
+// at most 8192 values.
+static constexpr int64_t kOneLaunchTokens = 8, kOneLaunchValuesBf16 = 8192;
+static bool takes_one_launch(int64_t tokens, int64_t d_model, int64_t width, at::ScalarType dt) {
+  if (tokens < 1 || tokens > kOneLaunchTokens) return false;
+  const int64_t built = tokens <= 2 ? tokens : tokens <= 4 ? 4 : 8;
+  return dt == at::kFloat || (dt == at::kBFloat16 && built * std::max(d_model, width) <= kOneLaunchValuesBf16);
+}
+
 // One decode step of a block (mambapy/mamba.py:351-414) -> (output (B, D), state, window), with fresh cache tensors.
-// Up to 8 tokens go through one cooperative launch (block_step.cu) when every weight has the activations' type and nothing wants
-// a gradient; otherwise the projections are library GEMMs with the two step kernels between them.  Beyond 8 tokens the
-// projections are real matrix products and the library's kernels are the better ones.
+// A few tokens go through one cooperative launch (block_step.cu) when every weight has the activations' type and nothing wants
+// a gradient; otherwise the projections are library GEMMs with the two step kernels between them.
 std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& h_, const Tensor& inputs, const Tensor& in_w,
                                               const OptTensor& in_b_, const Tensor& conv_w, const OptTensor& conv_b_, const Tensor& xproj_w,
                                               const Tensor& dt_w, const Tensor& dt_b, const Tensor& A_log, const Tensor& D,
@@ -151,7 +172,7 @@ std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& 
   numel_is(out_b, out_w.size(0), "out_proj.bias");
   TORCH_CHECK(inputs.numel() >= B * W * (K - 1) && (!h.defined() || h.numel() >= B * W * N), "mamba_b200: the caches hold fewer than ", B,
               " rows of ", W, " channels");
-  bool one = out_w.size(0) == Dm && B >= 1 && B <= 8 && (dt == at::kFloat || dt == at::kBFloat16) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+  bool one = out_w.size(0) == Dm && takes_one_launch(B, Dm, W, dt) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
              !wants_grad(x, in_w, in_b, out_w, out_b);
   for (const Tensor* t : {&in_w, &in_b, &xproj_w, &dt_w, &out_w, &out_b})
     one = one && (!t->defined() || (t->scalar_type() == dt && t->is_contiguous()));

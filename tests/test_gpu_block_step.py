@@ -11,7 +11,8 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("Bsz,d_model,N", [(1, 16, 16), (1, 768, 16), (2, 20, 8), (3, 136, 16), (5, 64, 32), (8, 200, 64), (8, 1024, 16), (9, 64, 16),
-                                           (8, 752, 16), (5, 768, 16), (3, 1536, 8), (2, 3072, 8)])       # activations of just under and of 48 KB
+                                           (8, 752, 16), (5, 768, 16), (3, 1536, 8), (2, 3072, 8),        # activations of just under and of 48 KB
+                                           (4, 1024, 16), (4, 1032, 16), (8, 512, 8), (2, 2056, 8), (8, 2560, 16)])  # and around bfloat16's limit
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_block_step_vs_oracle(Bsz, d_model, N, dtype):
     from mamba_b200 import step
