@@ -36,10 +36,16 @@ bool plain_settings() {
          ctx.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK;
 }
 
-// Tiles of 32 x 32 and terms up to which one launch for two products beats the library's two.  Device time of one, ours / library, us:
-// float32 (122, 256, 64) 6.3 / 6.3, (64, 64, 256) 10.4 / 8.3, (500, 500, 128) 8.4 / 6.6, (512, 512, 256) 14.5 / 9.2; bfloat16, where the
-// library has tensor cores, (122, 256, 64) 6.3 / 4.3, (122, 64, 128) 10.4 / 4.3, (512, 512, 64) 8.4 / 4.3.  A launch and its host work are
-// worth 5 to 9 us: two layers of 64 channels went from 665 to 525 us a training step.
+// Tiles of 32 x 32 and terms up to which a product goes through our own kernel.  What that saves is host time, for a product that shares
+// a launch and for one alone (a library call takes the host longer than a launch); on the GPU it is never ahead.  Device time of one,
+// ours / library, us: float32 (122, 256, 64) 6.3 / 6.3, (64, 64, 256) 10.4 / 8.3, (500, 500, 128) 8.4 / 6.6, (512, 512, 256) 14.5 / 9.2;
+// bfloat16, where the library has tensor cores, (122, 256, 64) 6.3 / 4.3, (122, 64, 128) 10.4 / 4.3, (512, 512, 64) 8.4 / 4.3.
+// Calls that fall under the rule wait for the host.  us, two layers of 64 channels, 122 tokens, ours / ours where shared / library:
+//                            called from Python     inside a CUDA graph, where there is no host work
+//   training    float32      506 / 549 / 643        178 / 172 / 197
+//               bfloat16     665 / 693 / 691        178 / 156 / 156
+//   inference   float32      117 / 156 / 152         68 /  64 /  62
+//               bfloat16     159 / 174 / 174         62 /  53 /  51
 bool small(int64_t M, int64_t N, int64_t K, at::ScalarType dt) {
   const int64_t tiles = (M + 31) / 32 * ((N + 31) / 32);
   if (dt == at::kFloat) return tiles <= 64 ? K <= 256 : tiles <= 296 && K <= 128;

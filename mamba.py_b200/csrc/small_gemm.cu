@@ -2,10 +2,11 @@
 //
 // A training step of a small layer has twelve products of a few hundred by a few hundred.  The library takes about 4.6 us of GPU and
 // more than that of host time for each; what they compute is under a microsecond.  Here the products that do not depend on one
-// another (a projection's input gradient and its weight gradient) share a launch.  Bound by latency: a CTA owns a 32 x 32 tile and
-// walks K in slabs of 32 through shared memory, the next slab's loads in flight while one is multiplied; any strides, so that
-// transposes cost nothing.  float32 multiply-adds for either input type.  Two layers of 64 channels, 122 tokens, a training step:
-// 665 -> 525 us with 8 launches a layer for 12.
+// another (a projection's input gradient and its weight gradient) share a launch, and a launch is all the host does.  Bound by
+// latency: a CTA owns a 32 x 32 tile and walks K in slabs of 32 through shared memory, the next slab's loads in flight while one is
+// multiplied; any strides, so that transposes cost nothing.  float32 multiply-adds for either input type.  Two layers of 64 channels,
+// 122 tokens, a training step called from Python: 643 us with the library's products, 506 with these, 8 launches a layer for 12 (inside
+// a CUDA graph 197 and 178).
 #include "common.cuh"
 
 namespace mb200 {
