@@ -326,7 +326,7 @@ typedef struct {
 enum { MB200_CONVERT_MAX_JOBS = 24 };
 int mb200_convert(const mb200_convert_job* jobs, int n, void* stream);
 
-/* mb200_conv_step_params with up to 3 conversions in the same launch. */
+/* mb200_conv_step with the filter and bias in the model's own types (float32 or bfloat16 each) and up to 3 conversions in the same launch. */
 int mb200_conv_step_convert(const void* xin, const void* conv_in, const void* w, int w_dtype, const void* bias, int bias_dtype, void* xc,
                             void* conv_out, int64_t B, int64_t ED, int K, int64_t x_sb, int dtype, const mb200_convert_job* jobs, int n_jobs,
                             void* stream);
@@ -396,15 +396,13 @@ int mb200_add_rmsnorm_bwd_both(const void* s, const float* weight, const float* 
 int mb200_rmsnorm_fwd_typed(const void* x, const void* weight, int w_dtype, void* y, float* rstd, int64_t rows, int64_t D,
                             int64_t x_rs, int64_t y_rs, float eps, int dtype, void* stream);
 
-/* mb200_ssm_step and mb200_conv_step with the small parameters in the model's own types (float32 or bfloat16 each); with A_is_log
+/* mb200_ssm_step with the small parameters in the model's own types (float32 or bfloat16 each); with A_is_log
  * A holds A_log and the decay rate is -exp(A_log). */
 int mb200_ssm_step_params(const void* x, const void* delta, const void* z, const void* A, int A_dtype, int A_is_log,
                           const void* Bm, const void* Cm, const void* D, int D_dtype, const void* delta_bias, int bias_dtype,
                           const float* h_in, float* h_out, void* y, int64_t B, int64_t ED, int N,
                           int64_t x_sb, int64_t d_sb, int64_t z_sb, int64_t b_sb, int64_t c_sb, int64_t y_sb,
                           int dtype, int flags, void* stream);
-int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype, const void* bias, int bias_dtype,
-                           void* xc, void* conv_out, int64_t B, int64_t ED, int K, int64_t x_sb, int dtype, void* stream);
 
 /* One decode step of a whole block for up to 8 tokens in one cooperative launch: in_proj, conv window and SiLU, x_proj,
  * dt_proj, state update with softplus(delta + dt_b), gate, out_proj (mambapy/mamba.py:351-414).  x (B, D_model) with row stride

@@ -329,7 +329,7 @@ struct BlockBackward : public torch::autograd::Node {
 // dt_proj weight and bias, A_log, D of one direction or of both.  Returns out_proj of the (summed, with `halve` averaged) scans, or
 // with out_w undefined the scan itself.
 Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, const std::vector<OptTensor>& params, int64_t R, int64_t N,
-             bool reverse, bool halve) {
+             bool halve) {
   const Tensor &in_w = value(in_w_), &out_w = value(out_w_);
   TORCH_CHECK_VALUE(params.size() == kDirParams || params.size() == 2 * kDirParams, "a block has 7 parameters per direction");
   std::vector<Tensor> in{x, in_w, out_w};
@@ -377,7 +377,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
       wi = conv.cast(pi, dt);
     } else {
       xz = rows(px, dt);
-      if ((nd > 1 || reverse) && !tensor_map_ok(xz)) xz = xz.contiguous();
+      if (nd > 1 && !tensor_map_ok(xz)) xz = xz.contiguous();
     }
     wo = conv.cast(po, dt);
     const int64_t Rp = padded_rank(R, dt), cols = Rp + 2 * N;
@@ -386,7 +386,7 @@ Tensor block(const Tensor& x, const OptTensor& in_w_, const OptTensor& out_w_, c
       joint.Wdt = empty({int64_t(nd), W, Rp}, dt, x);
     }
     for (size_t i = 0; i < nd; ++i) {
-      dirs[i].reverse = reverse || i == 1;
+      dirs[i].reverse = i == 1;
       dirs[i].prepare(conv, in.data() + kBlockInputs + i * kDirParams, dt, W, R, N, nd > 1 ? alias(joint.Wx, i * cols * W, {cols, W}) : Tensor(),
                       nd > 1 ? alias(joint.Wdt, i * W * Rp, {W, Rp}) : Tensor());
     }

@@ -229,7 +229,7 @@ std::tuple<Tensor, Tensor> ssm_step(const Tensor& x, const OptTensor& h, const T
 std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, const Tensor& weight, const OptTensor& bias, bool inplace);
 
 Tensor block(const Tensor& x, const OptTensor& in_w, const OptTensor& out_w, const std::vector<OptTensor>& params, int64_t dt_rank,
-             int64_t d_state, bool reverse, bool halve);
+             int64_t d_state, bool halve);
 bool reversible(int64_t width, int64_t d_state, at::ScalarType dt);
 std::tuple<Tensor, Tensor, Tensor> block_step(const Tensor& x, const OptTensor& h, const Tensor& inputs, const Tensor& in_w, const OptTensor& in_b,
                                               const Tensor& conv_w, const OptTensor& conv_b, const Tensor& xproj_w, const Tensor& dt_w,

@@ -22,7 +22,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("block", &block, NoGil());
   m.def("reversible", &reversible);
   m.def("block_step", &block_step, NoGil());
-  m.def("pick_pieces", &pick_pieces);
   m.def("selftest_queue_conversions", &selftest_queue_conversions);
   m.def("selftest_block_step_give_up", &selftest_block_step_give_up);
 }

@@ -389,16 +389,10 @@ extern "C" int mb200_conv_step_convert(const void* xin, const void* conv_in, con
   return check_launch();
 }
 
-extern "C" int mb200_conv_step_params(const void* xin, const void* conv_in, const void* w, int w_dtype,
-                                      const void* bias, int bias_dtype, void* xc, void* conv_out, int64_t B, int64_t ED,
-                                      int K, int64_t x_sb, int dtype, void* stream) {
-  return mb200_conv_step_convert(xin, conv_in, w, w_dtype, bias, bias_dtype, xc, conv_out, B, ED, K, x_sb, dtype, nullptr, 0, stream);
-}
-
 extern "C" int mb200_conv_step(const void* xin, const void* conv_in, const float* w,
                                const float* bias, void* xc, void* conv_out, int64_t B, int64_t ED,
                                int K, int64_t x_sb, int dtype, void* stream) {
-  return mb200_conv_step_params(xin, conv_in, w, MB200_F32, bias, MB200_F32, xc, conv_out, B, ED, K, x_sb, dtype, stream);
+  return mb200_conv_step_convert(xin, conv_in, w, MB200_F32, bias, MB200_F32, xc, conv_out, B, ED, K, x_sb, dtype, nullptr, 0, stream);
 }
 
 extern "C" int mb200_carry_fold(const float* P, const float* S, float* out, int64_t R, int64_t M,

@@ -232,8 +232,8 @@ def run_block(self, x, directions, halve=False, called=()):
     params = [p for d in directions for p in d]
     out_w = _native_linear(self.out_proj, dtype, amp) if own else None
     if out_w is not None:
-        return _host().block(x, in_w, out_w, params, cfg.dt_rank, cfg.d_state, False, halve), None
-    y = _host().block(x, in_w, None, params, cfg.dt_rank, cfg.d_state, False, False)
+        return _host().block(x, in_w, out_w, params, cfg.dt_rank, cfg.d_state, halve), None
+    y = _host().block(x, in_w, None, params, cfg.dt_rank, cfg.d_state, False)
     return self.out_proj(y / 2 if halve else y), None
 
 
