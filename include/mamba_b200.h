@@ -64,9 +64,9 @@ const char* mb200_strerror(int code);
 int mb200_version(void);
 
 /* Device-side status of the kernels launched so far on the current device: 0, or 1 when a
- * bounded wait between the producer and consumer warps of the fused scan gave up (the launch's
- * outputs are then invalid).  Reads and clears the word; SYNCHRONISES the device, so it is for
- * tests and diagnostics, not for the hot path.  Returns -1 if the word cannot be read. */
+ * bounded wait between the producer and consumer warps of the fused scan, or at a grid barrier of
+ * mb200_block_step, gave up (the launch's outputs are then invalid).  Reads and clears the word;
+ * SYNCHRONISES the device, every stream of it, so it is for tests and diagnostics, not for the hot path.  Returns -1 if the word cannot be read. */
 int mb200_device_status(void);
 
 /* Self-test of that mechanism (no counterpart in the reference): launches one warp that waits, with

@@ -112,8 +112,8 @@ CHECK_STATUS = os.environ.get("MB200_CHECK_STATUS", "0") not in ("", "0")
 
 
 def check_status(device, what: str) -> None:
-    """With MB200_CHECK_STATUS=1 in the environment every fused-scan launch is followed by a device
-    synchronisation and a read of the status word, and a give-up raises.  Off by default (it
+    """With MB200_CHECK_STATUS=1 in the environment every launch of a kernel with bounded waits is followed by a
+    device synchronisation and a read of the status word, and a give-up raises.  Off by default (it
     serialises host and device); meant for debugging a suspected hang."""
     if CHECK_STATUS:
         st = device_status(device)
