@@ -66,7 +66,8 @@ int mb200_version(void);
 /* Device-side status of the kernels launched so far on the current device: 0, or 1 when a
  * bounded wait between the producer and consumer warps of the fused scan, or at a grid barrier of
  * mb200_block_step, gave up (the launch's outputs are then invalid).  Reads and clears the word;
- * SYNCHRONISES the device, every stream of it, so it is for tests and diagnostics, not for the hot path.  Returns -1 if the word cannot be read. */
+ * SYNCHRONISES the device, every stream of it, so it is for tests and diagnostics, not for the hot
+ * path.  Returns -1 if the word cannot be read. */
 int mb200_device_status(void);
 
 /* Self-test of that mechanism (no counterpart in the reference): launches one warp that waits, with
@@ -411,7 +412,8 @@ int mb200_ssm_step_params(const void* x, const void* delta, const void* z, const
  * parameters conv_w (W, d_conv), conv_b (W, or NULL), dt_b (W), A_log (W, N), D (W) a type each.  conv_out may be conv_in, h_out
  * may be h_in.  scratch: mb200_block_step_scratch_floats floats; barriers: mb200_block_step_barrier_bytes bytes that are zero
  * before the first launch, left fit for the next one by every launch, and used by one launch at a time.
- * MB200_EUNSUPPORTED: weight rows off the 16-byte grid.  MB200_ETOOBIG: more than 8 tokens, or activations beyond 200 KB. */
+ * MB200_EUNSUPPORTED: weight rows off the 16-byte grid.  MB200_ETOOBIG: more than 8 tokens, d_conv
+ * above 8, or activations beyond 200 KB. */
 typedef struct {
   const void *x, *in_w, *in_b, *conv_in, *conv_w, *conv_b, *xproj_w, *dt_w, *dt_b, *A_log, *D, *out_w, *out_b;
   const float* h_in;

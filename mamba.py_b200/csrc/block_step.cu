@@ -316,7 +316,7 @@ extern "C" int mb200_block_step(const mb200_block_step_args* args, float* scratc
     return MB200_EINVAL;
   // 16-byte weight rows; the activations of all tokens fit shared memory
   const int64_t v = a.dtype == MB200_F32 ? 4 : 8, len = a.D_model > a.W ? a.D_model : a.W, slots = a.B <= 2 ? a.B : a.B <= 4 ? 4 : 8;
-  if (a.B > 8 || slots * len * 4 > 200 * 1024) return MB200_ETOOBIG;
+  if (a.B > 8 || a.d_conv > 8 || slots * len * 4 > 200 * 1024) return MB200_ETOOBIG;       // the filter as in mb200_conv_step
   if (a.D_model % v || a.W % v || !aligned16(a.in_w) || !aligned16(a.xproj_w) || !aligned16(a.out_w)) return MB200_EUNSUPPORTED;
   StepParams p;
   p.a = a;

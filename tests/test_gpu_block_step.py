@@ -60,6 +60,23 @@ def test_block_step_first_token_and_graph():
     assert torch.equal(o0, o1) and torch.equal(c0[0], c1[0]) and torch.equal(c0[1], c1[1])
 
 
+@pytest.mark.parametrize("Bsz", [2, 9])
+def test_longest_filter(Bsz):
+    """A filter of 8 steps runs, one of 9 is refused, on each path of a step."""
+    from mamba_b200 import step
+    for K in (8, 9):
+        blk, x, win = RefShapedBlock(32, d_conv=K).to(DEV), torch.randn(Bsz, 32, device=DEV), torch.randn(Bsz, 64, K - 1, device=DEV)
+        with torch.no_grad():
+            if K == 9:
+                with pytest.raises(RuntimeError):
+                    step(blk, x, (None, win))
+                continue
+            got, (_, new) = step(blk, x, (None, win))
+            want, (_, w2) = O.block_step(x.cpu(), (None, win.cpu()), {k: v.detach().cpu() for k, v in blk.weights().items()})
+        assert_close(got, want, 1e-4, 1e-5)
+        assert_close(new, w2, 1e-4, 1e-5)
+
+
 def test_replicas_and_pruned_modules():
     """Blocks whose parameters are plain attributes run through their modules and give what the block itself gives."""
     import torch.nn.utils.prune as prune
