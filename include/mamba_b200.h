@@ -50,6 +50,9 @@ enum {
                                relative (the reference's initialisation, mambapy/mamba.py:168-169) and
                                then form the four decays of a state quad from two ex2 and three
                                multiplies; any other A takes the general path on its own.            */
+  MB200_PAIRED_STATES = 8,  /* `carries` holds entry c of row b as (N/2, ED, 2) instead of (ED, N): the two states 2k, 2k+1 of
+                               all channels side by side, which warps of neighbouring channels write and read in whole
+                               lines.  The forward and the backward of a scan must agree on it.  */
   MB200_REVERSE = 2         /* scan from t = L-1 down to 0 (h[t] = a[t] h[t+1] + ...): what the
                                reference's bidirectional model gets by flipping the sequence,
                                scanning and flipping back (mambapy/vim.py:228-261).  h0 is then the
@@ -146,7 +149,7 @@ int mb200_pscan_bwd(const void* A, const void* H, const void* gradH,
  * A: (ED, N) float32 dense.  D: (ED) float32 or NULL (treated as 0).
  * h0 / hT: optional (B, ED, N) float32 incoming / outgoing state.
  * carries: optional (B, ceil(L/chunk), ED, N) float32; entry c receives the state that
- *          enters timestep c*chunk.  Needed by mb200_sscan_bwd. */
+ *          enters timestep c*chunk.  Needed by mb200_sscan_bwd.  (MB200_PAIRED_STATES: another order inside an entry.) */
 int mb200_sscan_fwd(const void* x, const void* delta, const void* z,
                     const float* A, const void* Bm, const void* Cm, const float* D,
                     const float* delta_bias, const float* h0,

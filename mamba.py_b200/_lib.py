@@ -16,6 +16,7 @@ F32, BF16 = 0, 1
 DELTA_SOFTPLUS = 1
 REVERSE = 2
 GENERAL_DECAY = 4
+PAIRED_STATES = 8
 EUNSUPPORTED = -8
 
 _i64, _int, _ptr = C.c_int64, C.c_int, C.c_void_p

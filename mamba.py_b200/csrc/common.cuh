@@ -98,6 +98,22 @@ __device__ __forceinline__ float2 softplus_fast2(float2 x) {
   r.y = x.y > 20.f ? x.y : (e.y < 1e-2f ? poly.y : lg.y);
   return r;
 }
+// softplus_fast2 and its derivative, the sigmoid, which shares the exponential.
+__device__ __forceinline__ float2 softplus_sigmoid_fast2(float2 x, float2& sig) {
+  const float2 m = __fmul2_rn(x, make_float2(kLog2e, kLog2e));
+  const float2 e = make_float2(ex2f(fminf(m.x, 80.f)), ex2f(fminf(m.y, 80.f)));       // e / (1 + e) must not become inf * 0
+  const float2 third = make_float2(-1.f / 3.f, -1.f / 3.f), half = make_float2(0.5f, 0.5f), one = make_float2(1.f, 1.f);
+  const float2 nh = make_float2(-1.f, -1.f);
+  const float2 inner = __ffma2_rn(e, third, half);
+  const float2 poly = __fmul2_rn(e, __ffma2_rn(__fmul2_rn(e, inner), nh, one));
+  const float2 s = __fadd2_rn(e, one);
+  const float2 lg = __fmul2_rn(make_float2(lg2f(s.x), lg2f(s.y)), make_float2(kLn2, kLn2));
+  sig = __fmul2_rn(e, make_float2(rcpf(s.x), rcpf(s.y)));
+  float2 r;
+  r.x = x.x > 20.f ? x.x : (e.x < 1e-2f ? poly.x : lg.x);
+  r.y = x.y > 20.f ? x.y : (e.y < 1e-2f ? poly.y : lg.y);
+  return r;
+}
 __device__ __forceinline__ float2 sigmoid_fast2(float2 x) {
   const float2 m = __fmul2_rn(x, make_float2(-kLog2e, -kLog2e));
   const float2 d = __fadd2_rn(make_float2(ex2f(m.x), ex2f(m.y)), make_float2(1.f, 1.f));

@@ -8,7 +8,7 @@ namespace mb200_host {
 struct ScanArgs {
   Tensor x, delta, A, B, C, D, z, bias, h0;
   bool reverse = false;
-  int flags() const { return (bias.defined() ? MB200_DELTA_SOFTPLUS : 0) | (reverse ? MB200_REVERSE : 0); }
+  int flags() const { return (bias.defined() ? MB200_DELTA_SOFTPLUS : 0) | (reverse ? MB200_REVERSE : 0) | MB200_PAIRED_STATES; }
   int code() const { return dtype_code(x.scalar_type()); }
   int64_t batch() const { return x.size(0); }
   int64_t length() const { return x.size(1); }

@@ -84,6 +84,27 @@ __device__ __forceinline__ void commit_bc(const Regs& rB, const Regs& rC, float*
   }
 }
 
+// Where the saved state {2k, 2k+1} of channel e lies inside an entry of ED x N floats: next to the channel's other states, or
+// (MB200_PAIRED_STATES) next to the same pair of the neighbouring channels.
+__host__ __device__ __forceinline__ int64_t state_pair(bool paired, int64_t ED, int N, int64_t e, int k) {
+  return paired ? (k * ED + e) * 2 : e * N + 2 * k;
+}
+// Four consecutive states from 4q on.
+__device__ __forceinline__ void store_states(float* entry, bool paired, int64_t ED, int N, int64_t e, int q, float4 h) {
+  if (paired) {
+    *reinterpret_cast<float2*>(entry + state_pair(true, ED, N, e, 2 * q)) = make_float2(h.x, h.y);
+    *reinterpret_cast<float2*>(entry + state_pair(true, ED, N, e, 2 * q + 1)) = make_float2(h.z, h.w);
+  } else {
+    *reinterpret_cast<float4*>(entry + e * N + 4 * q) = h;
+  }
+}
+__device__ __forceinline__ float4 load_states(const float* entry, bool paired, int64_t ED, int N, int64_t e, int q) {
+  if (!paired) return *reinterpret_cast<const float4*>(entry + e * N + 4 * q);
+  const float2 lo = *reinterpret_cast<const float2*>(entry + state_pair(true, ED, N, e, 2 * q));
+  const float2 hi = *reinterpret_cast<const float2*>(entry + state_pair(true, ED, N, e, 2 * q + 1));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
 struct SscanFwdParams {
   const void *x, *delta, *z, *Bm, *Cm;
   const float *A, *D, *delta_bias, *h0;

@@ -10,16 +10,23 @@
 // (two saved states per tile):
 //   - warp 4 issues TMA loads of the raw x, delta, z, dy, B, C boxes a few tiles ahead into a
 //     shared-memory ring and converts each landed tile into float32 operands
-//     ({softplus(delta+bias), delta*x}, dy*silu(z), B, C; double-buffered).
-//   - warps 0-3 (consumers; a thread owns 4 states of one channel) recompute the 8 states of a
+//     ({softplus(delta+bias), delta*x}, its derivative, dy*silu(z), that of silu, B, C; double-buffered).
+//   - warps 0-3 (consumers; a thread owns 2 states of 2 neighbouring channels) recompute the 8 states of a
 //     chunk forwards from its saved state into registers and walk them backwards:
 //     g[t] = dy'[t] C[t] + a[t+1] g[t+1],  da = g h[t-1].  Operands of the walk are fetched two
-//     timesteps ahead.  Per timestep a thread leaves three partial sums over its 4 states (for y,
-//     dx, ddelta) and its 8 products for dB, dC in shared memory, in windows of 2 timesteps.
+//     timesteps ahead.  Per timestep a thread leaves its partial sums over states (for y, dx, ddelta; two
+//     lanes add theirs first) and its products for dB, dC, already added over its two channels, in shared
+//     memory, in windows of 2 timesteps.
+//     Why 2 x 2: what goes through shared memory is what bounds the kernel.  Of its 4 elements a thread hands
+//     over 8 products and 3 sums (4 states of a channel), 4 and 3 (2 x 2, with three shuffles) or 2 and 12; and
+//     B and C are then 8-byte loads of two addresses, delta and delta*x 16-byte loads that two lanes share.
+//     44.6 -> 33.9 wavefronts per 128 elements and 610 -> 544 us on 8 x 2048 x 1536 in bfloat16, together with
+//     what follows; without the shuffles (twice the sums to write and to read) 587.
 //   - warps 5 and 7 finish alternate windows: sum the 4 partials of each channel, form dx, ddelta,
-//     dz (and the running sums for dD and d(delta_bias)), store them.  delta and dy' come from the
-//     operand tile, so only sigmoid(z) and 1 - exp(-delta) are evaluated here.
-//   - warp 6 sums the dB, dC products of each window over the CTA's 32 channels and adds the
+//     dz (and the running sums for dD and d(delta_bias)), store them.  delta, dy' and the derivatives of
+//     softplus and silu come from the operand tile: the converter has their exponentials in hand, and these
+//     two warps were what the consumers waited for (614 us with the derivatives evaluated here).
+//   - warp 6 sums the dB, dC products of each window over the CTA's 16 channel pairs and adds the
 //     result to global memory with vector atomics.
 //   - Hand-off through CTA-local mbarriers; every wait is bounded (see mbar_wait).  A barrier's
 //     round trip through the busy shared-memory pipe costs a few hundred cycles, so the consumers
@@ -38,7 +45,9 @@ constexpr int kHalf = kChunk;                // states kept in registers at a ti
 constexpr int kBWin = 2;                     // timesteps per reduction window
 constexpr int kWinsPerTile = kBTile / kBWin;
 constexpr int kBwdThreads = 256;
-constexpr int kEpStride = 34;                // float4 per (t, which, q) row of the dB/dC products
+constexpr int kNpPlane = kBN / 4 * kBTE;     // one kind of partial sum of a timestep: floats [state quad][channel]
+constexpr int kNpStep = 3 * kNpPlane;        // for y, dx, ddelta
+constexpr int kEpStep = kBN / 2 * kBTE / 2;  // dB, dC products of a timestep: float4 [state pair][channel pair]
 
 __device__ int g_bwd_status = MB200_DEV_OK;
 
@@ -56,23 +65,18 @@ template <typename T> struct TmaBwdSmem {
   static constexpr int kBcBytes = kBTile * kBN * int(sizeof(T));
   static constexpr int kStageBytes = 4 * kActBytes + 2 * kBcBytes;       // x, delta, z, dy, B, C
   static constexpr int kRaw = 0;
-  static constexpr int kOp = kRaw + kStages * kStageBytes;                // float2 [2][16][32]
-  static constexpr int kDyp = kOp + 2 * kBTile * kBTE * 8;                // float  [2][16][32]
+  static constexpr int kOp = kRaw + kStages * kStageBytes;                // float4 [2][16][16]
+  static constexpr int kAux = kOp + 2 * kBTile * kBTE * 8;                // float4 [2][16][16]
+  static constexpr int kDyp = kAux + 2 * kBTile * kBTE * 8;               // float  [2][16][32]
   static constexpr int kB = kDyp + 2 * kBTile * kBTE * 4;                 // float  [2][16][16]
   static constexpr int kC = kB + 2 * kBTile * kBN * 4;
-  static constexpr int kNp = kC + 2 * kBTile * kBN * 4;                   // float  [2][kBWin][3][128]
-  static constexpr int kEp = kNp + 2 * kBWin * 3 * 128 * 4;                  // float4 [2][kBWin][2][4][kEpStride]
-  static constexpr int kD = kEp + 2 * kBWin * 2 * 4 * kEpStride * 16;     // float [32]
+  static constexpr int kNp = kC + 2 * kBTile * kBN * 4;                   // float  [2][kBWin][3][4][32]
+  static constexpr int kEp = kNp + 2 * kBWin * kNpStep * 4;                  // float4 [2][kBWin][8][16]
+  static constexpr int kD = kEp + 2 * kBWin * kEpStep * 16;               // float [32]
   static constexpr int kBias = kD + kBTE * 4;
   static constexpr int kBars = kBias + kBTE * 4;                          // 2*kStages + 8 mbarriers
   static constexpr int kBytes = kBars + (2 * kStages + 8) * 8;
 };
-
-// The partial sums over a thread's 4 states (for y, dx, ddelta) go to three planes of 128 floats per
-// timestep; the 4 lanes of a channel are neighbours, so a finishing thread fetches one sum of one
-// channel with a single 16-byte load.  np_chan(c) is the float4 position of channel c in a plane: the
-// XOR keeps the finishing warps' loads (channels 2l, 2l+1 per lane) free of bank conflicts.
-__device__ __forceinline__ int np_chan(int c) { return c ^ ((c >> 3) & 1); }
 
 __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -88,7 +92,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
   constexpr int N = kBN;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  float2* s_op = reinterpret_cast<float2*>(smem_raw + S::kOp);
+  float4* s_op = reinterpret_cast<float4*>(smem_raw + S::kOp);      // {delta, delta, delta*x, delta*x} of a channel pair
+  float4* s_aux = reinterpret_cast<float4*>(smem_raw + S::kAux);    // {d softplus x 2, dy d(silu z)/dz x 2} of a channel pair
   float* s_dyp = reinterpret_cast<float*>(smem_raw + S::kDyp);
   float* s_B = reinterpret_cast<float*>(smem_raw + S::kB);
   float* s_C = reinterpret_cast<float*>(smem_raw + S::kC);
@@ -148,145 +153,155 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
   }
   if (warp < 4) {
     // ================================================================== consumers
-    const int e_l = tid >> 2, q = tid & 3;
-    const int64_t e = e0 + e_l;
-    const bool e_ok = e < p.ED;
-    float2 A2[2], gc[2], dAacc[2];
+    // A thread owns the states n0, n0 + 1 of the channels c0, c0 + 1; the two lanes of a channel pair are neighbours.
+    const int sp = 2 * warp + (lane & 1), cp = lane >> 1;             // state pair 0..7, channel pair 0..15
+    const int n0 = 2 * sp, c0 = 2 * cp;
+    const int64_t e = e0 + c0;
+    const bool ok0 = e < p.ED, ok1 = e + 1 < p.ED;
+    float2 A2[2], gc[2], dAacc[2];                                    // [state]{channel}
     {
-      float a4[4], g4[4];
+      const float* A0 = p.A + e * N + n0;
+      const float* g0 = p.g_in ? p.g_in + ((b * p.pieces + pc) * p.ED + e) * N + n0 : nullptr;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        a4[j] = e_ok ? p.A[e * N + 4 * q + j] * kLog2e : 0.f;
-        g4[j] = (e_ok && p.g_in) ? p.g_in[((b * p.pieces + pc) * p.ED + e) * N + 4 * q + j] : 0.f;
+      for (int k = 0; k < 2; ++k) {
+        A2[k] = make_float2(ok0 ? A0[k] * kLog2e : 0.f, ok1 ? A0[N + k] * kLog2e : 0.f);
+        gc[k] = make_float2(ok0 && g0 ? g0[k] : 0.f, ok1 && g0 ? g0[N + k] : 0.f);
+        dAacc[k] = make_float2(0.f, 0.f);
       }
-      A2[0] = make_float2(a4[0], a4[1]); A2[1] = make_float2(a4[2], a4[3]);
-      gc[0] = make_float2(g4[0], g4[1]); gc[1] = make_float2(g4[2], g4[3]);
-      dAacc[0] = dAacc[1] = make_float2(0.f, 0.f);
     }
-    const int op_off0 = op_index(0, e_l, kBTE), op_off1 = op_index(1, e_l, kBTE) - kBTE;
-    const int npo = np_chan(e_l) * 4 + q;
-    const int nchunks = int((p.L + kHalf - 1) / kHalf);
-    const float* carry_base = p.carries + (b * nchunks * p.ED + e) * N + 4 * q;
-    auto load_carry = [&](int c) {
-      return (e_ok && c < nchunks) ? *reinterpret_cast<const float4*>(carry_base + c * p.ED * N)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+    // slot of this channel pair in the rows of the operand tile (even and odd rows are swizzled differently)
+    const int op_off0 = swz(0, cp), op_off1 = swz(1, cp);
+    const int npo = warp * kBTE + lane;
+    // sum over the 4 states of both lanes of a channel pair: the even lane gets the first channel's, the odd one the second's
+    auto lanes_sum = [&](float2 v) {
+      const float give = (lane & 1) ? v.x : v.y, keep = (lane & 1) ? v.y : v.x;
+      return keep + __shfl_xor_sync(0xffffffffu, give, 1);
     };
-    // states entering the first / second half (in scan order) of iteration j's tile
-    // (time chunk 2*tile + 1 is the first half in scan order when reversed, chunk 2*tile otherwise)
-    const int c_lo = t_lo / kHalf;
-    float4 carry_next = load_carry(c_lo + (rev ? 1 : 2 * (ntiles - 1))), carry_next_mid = load_carry(c_lo + (rev ? 0 : 2 * (ntiles - 1) + 1));
-
-    for (int j = 0; j < ntiles; ++j) {
-      const int buf = int(j & 1);
-      const float4 cv = carry_next, cm = carry_next_mid;
-      if (j + 1 < ntiles) {                               // the next tile's two states, a tile ahead
-        const int c = c_lo + (rev ? 2 * j + 2 : 2 * (ntiles - 2 - j));
-        carry_next = load_carry(rev ? c + 1 : c);
-        carry_next_mid = load_carry(rev ? c : c + 1);
+    float4* const epo = s_ep + sp * 16 + (cp ^ ((sp & 1) * 4));
+    const int nchunks = int((p.L + kHalf - 1) / kHalf);
+    // saved states of a chunk as [state]{channel}
+    struct Pair { float2 v[2]; };
+    const bool paired = (p.flags & MB200_PAIRED_STATES) != 0, wide = paired && ok1 && !(p.ED & 1);
+    const float* carry_base = p.carries + b * nchunks * p.ED * N + state_pair(paired, p.ED, N, e, sp);
+    auto load_carry = [&](int c) {
+      Pair r;
+      r.v[0] = r.v[1] = make_float2(0.f, 0.f);
+      const float* src = carry_base + c * p.ED * N;
+      if (c < nchunks) {
+        if (wide) {
+          const float4 q = *reinterpret_cast<const float4*>(src);
+          r.v[0] = make_float2(q.x, q.z); r.v[1] = make_float2(q.y, q.w);
+        } else {
+          if (ok0) { const float2 q = *reinterpret_cast<const float2*>(src); r.v[0].x = q.x; r.v[1].x = q.y; }
+          if (ok1) { const float2 q = *reinterpret_cast<const float2*>(src + (paired ? 2 : N)); r.v[0].y = q.x; r.v[1].y = q.y; }
+        }
       }
-      if (!mbar_wait(&op_full[buf], int((j >> 1) & 1))) { fail(); return; }
-      const float2* op = s_op + buf * kBTile * kBTE;
-      const float* dyp = s_dyp + buf * kBTile * kBTE + e_l;
-      const float* sB = s_B + buf * kBTile * N + 4 * q;
-      const float* sC = s_C + buf * kBTile * N + 4 * q;
-      const float2 hp[2] = {make_float2(cv.x, cv.y), make_float2(cv.z, cv.w)};   // state entering the tile
-
-      // one forward step of the recurrence from operands in shared memory
-      auto step = [&](int s, float2 (&h)[2]) {
-        const int t = row(s);
-        const float2 o = op[t * kBTE + ((t & 1) ? op_off1 : op_off0)];
-        const float4 Bq = *reinterpret_cast<const float4*>(sB + t * N);
-        const float2 dd = make_float2(o.x, o.x), dxx = make_float2(o.y, o.y);
-        const float2 e0v = __fmul2_rn(dd, A2[0]), e1v = __fmul2_rn(dd, A2[1]);
-        const float2 a0 = make_float2(ex2f(e0v.x), ex2f(e0v.y)), a1 = make_float2(ex2f(e1v.x), ex2f(e1v.y));
-        h[0] = __ffma2_rn(a0, h[0], __fmul2_rn(dxx, make_float2(Bq.x, Bq.y)));
-        h[1] = __ffma2_rn(a1, h[1], __fmul2_rn(dxx, make_float2(Bq.z, Bq.w)));
-      };
-      const float2 hmid[2] = {make_float2(cm.x, cm.y), make_float2(cm.z, cm.w)};   // state entering the second half
+      return r;
+    };
+    // Chunks are taken from the end of the scan to its start; the state entering the next one is fetched a chunk ahead.
+    const int c_lo = t_lo / kHalf, nch = 2 * ntiles;
+    auto chunk_at = [&](int k) { return c_lo + (rev ? k : nch - 1 - k); };
+    Pair carry_next = load_carry(chunk_at(0));
 
 #pragma unroll 1
-      for (int half = 1; half >= 0; --half) {
-        // states after each step of this half, in registers
-        float2 hh[kHalf][2];
-        {
-          float2 h[2] = {half ? hmid[0] : hp[0], half ? hmid[1] : hp[1]};
+    for (int k8 = 0; k8 < nch; ++k8) {
+      const int j = k8 >> 1, buf = j & 1, second = k8 & 1;   // tile, its operand buffer, second chunk taken from it
+      const Pair hin = carry_next;                           // state entering the chunk
+      if (k8 + 1 < nch) carry_next = load_carry(chunk_at(k8 + 1));
+      if (!second && !mbar_wait(&op_full[buf], (j >> 1) & 1)) { fail(); return; }
+      // rows of the chunk: step i of the scan is row `rw(i)`
+      const int r0 = buf * kBTile + ((second != 0) == rev ? kHalf : 0);
+      auto rw = [](int i) { return rev ? kHalf - 1 - i : i; };
+      const float4* op0 = s_op + r0 * (kBTE / 2) + op_off0;
+      const float4* op1 = s_op + r0 * (kBTE / 2) + op_off1;
+      const float* dyp = s_dyp + r0 * kBTE + c0;
+      const float* sB = s_B + r0 * N + n0;
+      constexpr int kBtoC = (S::kC - S::kB) / 4;
+
+      // states after each step of the chunk, in registers
+      float2 hh[kHalf][2];
+      {
+        float2 h[2] = {hin.v[0], hin.v[1]};
 #pragma unroll
-          for (int i = 0; i < kHalf; ++i) {
-            step(half * kHalf + i, h);
-            hh[i][0] = h[0]; hh[i][1] = h[1];
-          }
-        }
-        // operands of the reverse walk are fetched one timestep ahead, so that their trip through the
-        // shared-memory pipe overlaps the previous timestep's arithmetic, stores and barrier traffic
-        struct Opnd { float2 o; float dy; float4 B, C; };
-        auto fetch = [&](int s) {
-          const int t = row(s);
-          Opnd r;
-          r.o = op[t * kBTE + ((t & 1) ? op_off1 : op_off0)];
-          r.dy = dyp[t * kBTE];
-          r.B = *reinterpret_cast<const float4*>(sB + t * N);
-          r.C = *reinterpret_cast<const float4*>(sC + t * N);
-          return r;
-        };
-        Opnd nx = fetch(half * kHalf + kHalf - 1), nx2 = fetch(half * kHalf + kHalf - 2);
-#pragma unroll
-        for (int wi = kHalf / kBWin - 1; wi >= 0; --wi) {
-          // window sequence number: tiles in processing order, windows from the tile's end
-          const int wseq = j * kWinsPerTile + (1 - half) * (kHalf / kBWin) + (kHalf / kBWin - 1 - wi);
-          const int wb = int(wseq & 1);
-          // asked now, needed only before the first store of the window
-          const bool slot_free = wseq < 2 || mbar_test(&win_empty[wb], int(((wseq - 2) >> 1) & 1));
-          float* np = s_np + wb * kBWin * 3 * 128;
-          float4* ep = s_ep + wb * kBWin * 2 * 4 * kEpStride;
-#pragma unroll
-          for (int ti = kBWin - 1; ti >= 0; --ti) {
-            const int i = wi * kBWin + ti;                    // index inside the half
-            const int t = half * kHalf + i;                   // index inside the tile
-            const Opnd cu = nx;
-            nx = nx2;
-            if (i > 1) nx2 = fetch(t - 2);
-            const float2 o = cu.o;
-            const float dyv = cu.dy;
-            const float4 Bq = cu.B, Cq = cu.C;
-            const float2 dd = make_float2(o.x, o.x), dxx = make_float2(o.y, o.y), dy2 = make_float2(dyv, dyv);
-            const float2 Bv[2] = {make_float2(Bq.x, Bq.y), make_float2(Bq.z, Bq.w)};
-            const float2 Cv[2] = {make_float2(Cq.x, Cq.y), make_float2(Cq.z, Cq.w)};
-            float2 ysum = make_float2(0.f, 0.f), gBs = ysum, wAs = ysum;
-            float2 dBp[2], dCp[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const float2 hcur = hh[i][k];
-              const float2 hprev = i ? hh[i - 1][k] : (half ? hmid[k] : hp[k]);
-              const float2 g = __ffma2_rn(dy2, Cv[k], gc[k]);
-              ysum = __ffma2_rn(hcur, Cv[k], ysum);
-              dCp[k] = __fmul2_rn(dy2, hcur);
-              dBp[k] = __fmul2_rn(g, dxx);
-              gBs = __ffma2_rn(g, Bv[k], gBs);
-              const float2 ev = __fmul2_rn(dd, A2[k]);
-              gc[k] = __fmul2_rn(make_float2(ex2f(ev.x), ex2f(ev.y)), g);
-              const float2 w = __fmul2_rn(gc[k], hprev);
-              dAacc[k] = __ffma2_rn(w, dd, dAacc[k]);
-              wAs = __ffma2_rn(w, A2[k], wAs);
-            }
-            if (ti == kBWin - 1 && !slot_free && !mbar_wait(&win_empty[wb], int(((wseq - 2) >> 1) & 1))) { fail(); return; }
-            np[(ti * 3 + 0) * 128 + npo] = ysum.x + ysum.y;
-            np[(ti * 3 + 1) * 128 + npo] = gBs.x + gBs.y;
-            np[(ti * 3 + 2) * 128 + npo] = wAs.x + wAs.y;
-            ep[((ti * 2 + 0) * 4 + q) * kEpStride + e_l] = make_float4(dBp[0].x, dBp[0].y, dBp[1].x, dBp[1].y);
-            ep[((ti * 2 + 1) * 4 + q) * kEpStride + e_l] = make_float4(dCp[0].x, dCp[0].y, dCp[1].x, dCp[1].y);
-          }
-          mbar_arrive(&win_full[wb]);
+        for (int i = 0; i < kHalf; ++i) {
+          const int r = rw(i);
+          const float4 o = ((r & 1) ? op1 : op0)[r * (kBTE / 2)];
+          const float2 Bp = *reinterpret_cast<const float2*>(sB + r * N);
+          const float2 dt = make_float2(o.x, o.y), dtx = make_float2(o.z, o.w);
+          const float2 e0v = __fmul2_rn(dt, A2[0]), e1v = __fmul2_rn(dt, A2[1]);
+          const float2 a0 = make_float2(ex2f(e0v.x), ex2f(e0v.y)), a1 = make_float2(ex2f(e1v.x), ex2f(e1v.y));
+          h[0] = __ffma2_rn(a0, h[0], __fmul2_rn(dtx, make_float2(Bp.x, Bp.x)));
+          h[1] = __ffma2_rn(a1, h[1], __fmul2_rn(dtx, make_float2(Bp.y, Bp.y)));
+          hh[i][0] = h[0]; hh[i][1] = h[1];
         }
       }
-      mbar_arrive(&op_empty[buf]);
+      // operands of the reverse walk are fetched two timesteps ahead, so that their trip through the
+      // shared-memory pipe overlaps the previous timestep's arithmetic, stores and barrier traffic
+      struct Opnd { float4 o; float2 dy, B, C; };
+      auto fetch = [&](int i) {
+        const int rr = rw(i);
+        Opnd r;
+        r.o = ((rr & 1) ? op1 : op0)[rr * (kBTE / 2)];
+        r.dy = *reinterpret_cast<const float2*>(dyp + rr * kBTE);
+        r.B = *reinterpret_cast<const float2*>(sB + rr * N);
+        r.C = *reinterpret_cast<const float2*>(sB + kBtoC + rr * N);
+        return r;
+      };
+      Opnd nx = fetch(kHalf - 1), nx2 = fetch(kHalf - 2);
+#pragma unroll
+      for (int wi = kHalf / kBWin - 1; wi >= 0; --wi) {
+        // window sequence number: chunks in processing order, windows from the chunk's end; a chunk has an even number of them
+        const int wseq = k8 * (kHalf / kBWin) + (kHalf / kBWin - 1 - wi);
+        const int wb = (kHalf / kBWin - 1 - wi) & 1;
+        // asked now, needed only before the first store of the window
+        const bool slot_free = wseq < 2 || mbar_test(&win_empty[wb], int(((wseq - 2) >> 1) & 1));
+        float* np = s_np + wb * kBWin * kNpStep;
+        float4* ep = epo + wb * kBWin * kEpStep;
+#pragma unroll
+        for (int ti = kBWin - 1; ti >= 0; --ti) {
+          const int i = wi * kBWin + ti;                    // index inside the chunk
+          const Opnd cu = nx;
+          nx = nx2;
+          if (i > 1) nx2 = fetch(i - 2);
+          const float2 dt = make_float2(cu.o.x, cu.o.y), dtx = make_float2(cu.o.z, cu.o.w), dy2 = cu.dy;
+          const float2 Bv[2] = {make_float2(cu.B.x, cu.B.x), make_float2(cu.B.y, cu.B.y)};
+          const float2 Cv[2] = {make_float2(cu.C.x, cu.C.x), make_float2(cu.C.y, cu.C.y)};
+          float2 ysum, gBs, wAs;                                            // {channel}
+          float dB[2], dC[2];                                               // [state], over the two channels
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float2 hcur = hh[i][k], hprev = i ? hh[i - 1][k] : hin.v[k];
+            const float2 g = __ffma2_rn(dy2, Cv[k], gc[k]);
+            ysum = k ? __ffma2_rn(hcur, Cv[k], ysum) : __fmul2_rn(hcur, Cv[k]);
+            dC[k] = fmaf(dy2.y, hcur.y, dy2.x * hcur.x);
+            dB[k] = fmaf(g.y, dtx.y, g.x * dtx.x);
+            gBs = k ? __ffma2_rn(g, Bv[k], gBs) : __fmul2_rn(g, Bv[k]);
+            const float2 ev = __fmul2_rn(dt, A2[k]);
+            gc[k] = __fmul2_rn(make_float2(ex2f(ev.x), ex2f(ev.y)), g);
+            const float2 w = __fmul2_rn(gc[k], hprev);
+            dAacc[k] = __ffma2_rn(w, dt, dAacc[k]);
+            wAs = k ? __ffma2_rn(w, A2[k], wAs) : __fmul2_rn(w, A2[k]);
+          }
+          const float s0 = lanes_sum(ysum), s1 = lanes_sum(gBs), s2 = lanes_sum(wAs);
+          if (ti == kBWin - 1 && !slot_free && !mbar_wait(&win_empty[wb], int(((wseq - 2) >> 1) & 1))) { fail(); return; }
+          np[ti * kNpStep + npo] = s0;
+          np[ti * kNpStep + kNpPlane + npo] = s1;
+          np[ti * kNpStep + 2 * kNpPlane + npo] = s2;
+          ep[ti * kEpStep] = make_float4(dB[0], dB[1], dC[0], dC[1]);
+        }
+        mbar_arrive(&win_full[wb]);
+      }
+      if (second) mbar_arrive(&op_empty[buf]);
     }
-    if (e_ok) {
-      float* dA = p.dA + e * N + 4 * q;
-      atomicAdd(dA + 0, dAacc[0].x); atomicAdd(dA + 1, dAacc[0].y);
-      atomicAdd(dA + 2, dAacc[1].x); atomicAdd(dA + 3, dAacc[1].y);
-      if (p.g_out && pc == (rev ? p.pieces - 1 : 0))       // the carry that leaves the scan's first timestep
-        *reinterpret_cast<float4*>(p.g_out + (b * p.ED + e) * N + 4 * q) =
-            make_float4(gc[0].x, gc[0].y, gc[1].x, gc[1].y);
+    const bool leaves = p.g_out && pc == (rev ? p.pieces - 1 : 0);   // the carry that leaves the scan's first timestep
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (!(c ? ok1 : ok0)) continue;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        atomicAdd(p.dA + (e + c) * N + n0 + k, c ? dAacc[k].y : dAacc[k].x);
+        if (leaves) p.g_out[(b * p.ED + e + c) * N + n0 + k] = c ? gc[k].y : gc[k].x;
+      }
     }
     return;
   }
@@ -325,7 +340,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       const T* rd = reinterpret_cast<const T*>(st + S::kActBytes);
       const T* rz = reinterpret_cast<const T*>(st + 2 * S::kActBytes);
       const T* rdy = reinterpret_cast<const T*>(st + 3 * S::kActBytes);
-      float2* tile = s_op + buf * kBTile * kBTE;
+      float4* tile = s_op + buf * kBTile * (kBTE / 2);
+      float4* auxt = s_aux + buf * kBTile * (kBTE / 2);
       float* dyt = s_dyp + buf * kBTile * kBTE;
       const float4 bq = *reinterpret_cast<const float4*>(s_bias + (lane & 7) * 4);   // this lane's 4 channels
       const float bias4[4] = {bq.x, bq.y, bq.z, bq.w};
@@ -338,26 +354,35 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         const Vec4<T> yv4 = *reinterpret_cast<const Vec4<T>*>(rdy + rr * kBTE + cc);
         Vec4<T> zv4 = yv4;
         if (has_z) zv4 = *reinterpret_cast<const Vec4<T>*>(rz + rr * kBTE + cc);
-        float2 o[4];
+        float2 o[4], sg[2], dq[2];
         float dyo[4];
 #pragma unroll
         for (int k = 0; k < 4; k += 2) {                   // two channels at a time (packed arithmetic)
           float2 dv = pair_f(&dv4.v[k]);
-          if (softplus) dv = softplus_fast2(__fadd2_rn(dv, make_float2(bias4[k], bias4[k + 1])));
+          sg[k / 2] = dq[k / 2] = make_float2(0.f, 0.f);
+          if (softplus) dv = softplus_sigmoid_fast2(__fadd2_rn(dv, make_float2(bias4[k], bias4[k + 1])), sg[k / 2]);
           if (rr >= rows_ok) dv = make_float2(0.f, 0.f);
           const float2 dx2 = __fmul2_rn(dv, pair_f(&xv.v[k]));
-          o[k] = make_float2(dv.x, dx2.x);
-          o[k + 1] = make_float2(dv.y, dx2.y);
+          o[k] = dv;
+          o[k + 1] = dx2;
           float2 g = pair_f(&yv4.v[k]);
           if (has_z) {
-            const float2 zf = pair_f(&zv4.v[k]);
-            g = __fmul2_rn(g, __fmul2_rn(zf, sigmoid_fast2(zf)));
+            // silu(z) = z s, its derivative s (1 + z (1 - s))
+            const float2 zf = pair_f(&zv4.v[k]), s = sigmoid_fast2(zf);
+            const float2 one = make_float2(1.f, 1.f), mone = make_float2(-1.f, -1.f);
+            const float2 gs = __fmul2_rn(g, s);
+            dq[k / 2] = __fmul2_rn(gs, __ffma2_rn(zf, __ffma2_rn(s, mone, one), one));
+            g = __fmul2_rn(gs, zf);
           }
           dyo[k] = g.x;
           dyo[k + 1] = g.y;
         }
-        *reinterpret_cast<float4*>(tile + op_index(rr, cc, kBTE)) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
-        *reinterpret_cast<float4*>(tile + op_index(rr, cc + 2, kBTE)) = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
+        tile[rr * (kBTE / 2) + swz(rr, cc >> 1)] = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+        tile[rr * (kBTE / 2) + swz(rr, (cc >> 1) + 1)] = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
+        if (softplus || has_z) {
+          auxt[rr * (kBTE / 2) + swz(rr, cc >> 1)] = make_float4(sg[0].x, sg[0].y, dq[0].x, dq[0].y);
+          auxt[rr * (kBTE / 2) + swz(rr, (cc >> 1) + 1)] = make_float4(sg[1].x, sg[1].y, dq[1].x, dq[1].y);
+        }
         *reinterpret_cast<float4*>(dyt + rr * kBTE + cc) = make_float4(dyo[0], dyo[1], dyo[2], dyo[3]);
       }
       const T* rB = reinterpret_cast<const T*>(st + 4 * S::kActBytes);      // B box then C box
@@ -381,14 +406,12 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
 
   if (warp == 6) {
     // ================================================================== dB, dC: sums over channels
-    // A lane owns one row of products (timestep of the window, dB | dC, state quad: 16 rows) and one half
-    // of the CTA's 32 channels; it adds its 16 float4 and sends the four sums to global memory with one
-    // vector atomic.  Rows are kEpStride = 34 float4 apart, which puts rows r and r + 4 into the same
-    // banks: the lanes of rows 4..7 and 12..15 therefore take each pair of neighbouring channels in the
-    // opposite order (index c ^ 1), through two base pointers, so that no index is computed in the loop.
-    const int hf = lane >> 4, r = lane & 15;
-    const int ti = r >> 3, which = (r >> 2) & 1, qq = r & 3;       // r = (ti * 2 + which) * 4 + qq
-    float* gbase = (which ? p.dC : p.dB) + b * p.L * N + 4 * qq;
+    // A lane owns one row of products (timestep of the window, state pair) and one half of the CTA's 16 channel pairs: it adds
+    // its 8 float4 {dB, dB, dC, dC}.  The lanes of a quarter-warp start at different channel pairs, which keeps their loads out of
+    // each other's banks.  Neighbouring lanes then swap halves, so that each holds four consecutive states of dB or of dC and
+    // sends them to global memory with one vector atomic.
+    const int hf = lane >> 4, r = lane & 15, ti = r >> 3, which = r & 1;
+    float* gbase = (which ? p.dC : p.dB) + b * p.L * N + 4 * ((r & 7) >> 1);
     for (int j = 0; j < ntiles; ++j) {
       const int t0 = tile_t0(j);
 #pragma unroll 1
@@ -396,19 +419,20 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         const int wseq = j * kWinsPerTile + wl;
         const int wb = wseq & 1;
         if (!mbar_wait(&win_full[wb], (wseq >> 1) & 1)) { fail(); return; }
-        const float4* rowp = s_ep + wb * kBWin * 2 * 4 * kEpStride + r * kEpStride + hf * 16;
-        const float4* pe = rowp + which;                          // even channels: c ^ which = c + which
-        const float4* po = rowp - which;                          // odd channels:  c ^ which = c - which
+        const float4* rowp = s_ep + wb * kBWin * kEpStep + r * 16 + hf * 8;
         float2 acc0 = make_float2(0.f, 0.f), acc1 = acc0;
 #pragma unroll
-        for (int c = 0; c < kBTE / 2; ++c) {
-          const float4 v = (c & 1) ? po[c] : pe[c];
+        for (int c = 0; c < 8; ++c) {
+          const float4 v = rowp[c ^ (r & 7)];
           acc0 = __fadd2_rn(acc0, make_float2(v.x, v.y));
           acc1 = __fadd2_rn(acc1, make_float2(v.z, v.w));
         }
         mbar_arrive(&win_empty[wb]);
+        const float2 give = which ? acc0 : acc1;
+        const float2 got = make_float2(__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1));
+        const float2 lo = which ? got : acc0, hi = which ? acc1 : got;
         const int t = t0 + row(win_t(wl) + ti);
-        if (t < t_hi) red_add_v4(gbase + int64_t(t) * N, acc0.x, acc0.y, acc1.x, acc1.y);
+        if (t < t_hi) red_add_v4(gbase + int64_t(t) * N, lo.x, lo.y, hi.x, hi.y);
       }
     }
     return;
@@ -428,56 +452,44 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       if (!mbar_wait(&raw_full[j % kStages], int((j / kStages) & 1))) { fail(); return; }
       const unsigned char* st = stage_ptr(j);
       const T* rx = reinterpret_cast<const T*>(st);
-      const T* rz = reinterpret_cast<const T*>(st + 2 * S::kActBytes);
-      const T* rdy = reinterpret_cast<const T*>(st + 3 * S::kActBytes);
-      // delta and dy' come from the operand tile the consumers are reading (still held: this warp
+      // delta, dy' and the derivatives come from the operand tile the consumers are reading (still held: this warp
       // is one of the arrivals the converter waits for before it reuses the buffer)
       const int buf = int(j & 1);
-      const float2* opt = s_op + buf * kBTile * kBTE;
+      const float4* opt = s_op + buf * kBTile * (kBTE / 2);
+      const float4* auxt = s_aux + buf * kBTile * (kBTE / 2);
       const float* dyt = s_dyp + buf * kBTile * kBTE;
 #pragma unroll 1
       for (int wl = par; wl < kWinsPerTile; wl += 2) {
         const int wseq = j * kWinsPerTile + wl;
         if (!mbar_wait(&win_full[par], int((wseq >> 1) & 1))) { fail(); return; }
-        const float4* np = reinterpret_cast<const float4*>(s_np + (par * kBWin + ti) * 3 * 128);
-        float ys[2], gBs[2], wAs[2];
+        const float* np = s_np + (par * kBWin + ti) * kNpStep;
+        float2 sums[3];                                  // of y, dx, ddelta, over the 4 state quads of both channels
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const int cs = np_chan(c0 + k);
-          const float4 v0 = np[cs], v1 = np[32 + cs], v2 = np[64 + cs];
-          ys[k] = (v0.x + v0.y) + (v0.z + v0.w);
-          gBs[k] = (v1.x + v1.y) + (v1.z + v1.w);
-          wAs[k] = (v2.x + v2.y) + (v2.z + v2.w);
+        for (int v = 0; v < 3; ++v) {
+          float2 q[kBN / 4];
+#pragma unroll
+          for (int k = 0; k < kBN / 4; ++k) q[k] = *reinterpret_cast<const float2*>(np + v * kNpPlane + k * kBTE + c0);
+#pragma unroll
+          for (int w = kBN / 8; w > 0; w /= 2)
+#pragma unroll
+            for (int k = 0; k < w; ++k) q[k] = __fadd2_rn(q[k], q[k + w]);
+          sums[v] = q[0];
         }
         mbar_arrive(&win_empty[par]);
         const int tt = row(win_t(wl) + ti);              // row inside the tile
         const int t = t0 + tt;
         if (t < t_hi && c0 < cols_ok) {
           const Vec2<T> xv = *reinterpret_cast<const Vec2<T>*>(rx + tt * kBTE + c0);
-          const float4 o4 = *reinterpret_cast<const float4*>(opt + op_index(tt, c0, kBTE));   // {delta, delta*x} x 2
+          const float2 dv = *reinterpret_cast<const float2*>(opt + tt * (kBTE / 2) + swz(tt, c0 >> 1));
           const float2 dyg2 = *reinterpret_cast<const float2*>(dyt + tt * kBTE + c0);
-          const Vec2<T> yv2 = *reinterpret_cast<const Vec2<T>*>(rdy + tt * kBTE + c0);
-          Vec2<T> zv2 = yv2;
-          if (has_z) zv2 = *reinterpret_cast<const Vec2<T>*>(rz + tt * kBTE + c0);
+          float4 aux = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (softplus || has_z) aux = auxt[tt * (kBTE / 2) + swz(tt, c0 >> 1)];
           Vec2<T> ox, od, oz;
-          const float2 xf = pair_f(&xv.v[0]), dv = make_float2(o4.x, o4.z), gB = make_float2(gBs[0], gBs[1]);
-          const float2 one = make_float2(1.f, 1.f), mone = make_float2(-1.f, -1.f);
-          if (has_z) {
-            // dz = dy (y + D x) sg (1 + z (1 - sg))
-            const float2 zf = pair_f(&zv2.v[0]), sg = sigmoid_fast2(zf);
-            const float2 yd = __fmul2_rn(pair_f(&yv2.v[0]), __ffma2_rn(Dv, xf, make_float2(ys[0], ys[1])));
-            pair_to(&oz.v[0], __fmul2_rn(__fmul2_rn(yd, sg), __ffma2_rn(zf, __ffma2_rn(sg, mone, one), one)));
-          }
+          const float2 xf = pair_f(&xv.v[0]), gB = sums[1];
+          if (has_z) pair_to(&oz.v[0], __fmul2_rn(make_float2(aux.z, aux.w), __ffma2_rn(Dv, xf, sums[0])));
           pair_to(&ox.v[0], __ffma2_rn(dyg2, Dv, __fmul2_rn(dv, gB)));
-          float2 dd = __ffma2_rn(xf, gB, __fmul2_rn(make_float2(wAs[0], wAs[1]), make_float2(1.f / kLog2e, 1.f / kLog2e)));
-          if (softplus) {
-            // d softplus = sigmoid(raw) = 1 - exp(-softplus(raw)); series where the difference cancels
-            const float2 m = __fmul2_rn(dv, make_float2(-kLog2e, -kLog2e));
-            const float2 far = __ffma2_rn(make_float2(ex2f(m.x), ex2f(m.y)), mone, one);
-            const float2 inner = __ffma2_rn(dv, make_float2(-1.f / 6.f, -1.f / 6.f), make_float2(0.5f, 0.5f));
-            const float2 near = __fmul2_rn(dv, __ffma2_rn(__fmul2_rn(dv, inner), mone, one));
-            dd = __fmul2_rn(dd, make_float2(dv.x < 1e-2f ? near.x : far.x, dv.y < 1e-2f ? near.y : far.y));
-          }
+          float2 dd = __ffma2_rn(xf, gB, __fmul2_rn(sums[2], make_float2(1.f / kLog2e, 1.f / kLog2e)));
+          if (softplus) dd = __fmul2_rn(dd, make_float2(aux.x, aux.y));
           dDacc = __ffma2_rn(dyg2, xf, dDacc);               // of channels past the end: never added up
           dbacc = __fadd2_rn(dbacc, dd);
           pair_to(&od.v[0], dd);

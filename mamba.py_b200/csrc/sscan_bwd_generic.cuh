@@ -146,8 +146,7 @@ sscan_bwd_generic_kernel(const SscanBwdParams p) {
   };
   auto load_carry = [&](int64_t c, float (&hp)[4]) {
     if (e_ok) {
-      const float4 v = *reinterpret_cast<const float4*>(
-          p.carries + ((b * nchunks + c) * p.ED + e) * N + 4 * q);
+      const float4 v = load_states(p.carries + (b * nchunks + c) * p.ED * N, (p.flags & MB200_PAIRED_STATES) != 0, p.ED, N, e, q);
       hp[0] = v.x; hp[1] = v.y; hp[2] = v.z; hp[3] = v.w;
     } else {
       hp[0] = hp[1] = hp[2] = hp[3] = 0.f;

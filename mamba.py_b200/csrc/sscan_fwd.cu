@@ -148,8 +148,9 @@ __device__ __forceinline__ bool s4d_structured(const float* a4, float a0, int q)
 // (gc <- a[t] * (dy'[t] * C[t] + gc), t = L-1 ... 0): the caller passes dy as `x` and C as `Bm`, the
 // converter forms dy' = dy * silu(z) instead of delta * x, and the recurrence multiplies by the decay
 // after adding the input.  It has no y and saves no states; the result leaves through hT.
-// kHasY = false is the pass that only wants states (no C-contraction, no epilogue).
-template <typename T, int N, bool kRev, bool kCarry, bool kHasY>
+// kHasY = false is the pass that only wants states (no C-contraction, no epilogue).  kSave: the states entering the chunks go to
+// p.carries (a template parameter because the test alone costs the recurrence warps 2 % of a prompt).
+template <typename T, int N, bool kRev, bool kCarry, bool kHasY, bool kSave>
 __global__ void __launch_bounds__(FwdGeom<N>::kThreads, FwdGeom<N>::kOcc)
 sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams p) {
   using G = FwdGeom<N>;
@@ -238,7 +239,8 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
       yp_off0 = yp_off1 = ((e_l >> 2) * 4 + q) * 4 + (e_l & 3);   // [channel quad][q][channel in quad]
     }
     const int64_t nchunks = (p.L + kChunk - 1) / kChunk;
-    float* carry_base = p.carries ? p.carries + (b * nchunks * p.ED + e0 + e_l) * N + 4 * q : nullptr;
+    const bool paired = (p.flags & MB200_PAIRED_STATES) != 0;
+    float* carry_base = p.carries + b * nchunks * p.ED * N;
     // row of processing step t is rb0 + t * rstep (in operand-tile rows); odd rows use the other swizzle offset
     constexpr int rb0 = rev ? kTile - 1 : 0, rstep = rev ? -1 : 1;
     const int off_even = rev ? op_off1 : op_off0, off_odd = rev ? op_off0 : op_off1;
@@ -305,14 +307,14 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
         for (int t = 0; t < kDecayAhead; ++t) rd[t] = prepare(ld[t]);
 #pragma unroll
         for (int t = 0; t < kTile; ++t) {
-          if (t % kChunk == 0 && carry_base) {                              // state entering this chunk
+          if (kSave && t % kChunk == 0) {                                   // state entering this chunk
             const int64_t c = t0a / kChunk + (rev ? 1 - t / kChunk : t / kChunk);
             if (c < nchunks) {
 #pragma unroll
               for (int i = 0; i < kCPT; ++i)
                 if (e_ok[i])
-                  *reinterpret_cast<float4*>(carry_base + (c * p.ED + i) * N) =
-                      make_float4(hlo[i].x, hlo[i].y, hhi[i].x, hhi[i].y);
+                  store_states(carry_base + c * p.ED * N, paired, p.ED, N, e0 + e_l + i, q,
+                               make_float4(hlo[i].x, hlo[i].y, hhi[i].x, hhi[i].y));
             }
           }
           if (t + kLoadAhead < kTile) ld[t + kLoadAhead] = load(t + kLoadAhead);
@@ -563,9 +565,12 @@ int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
   else if (ok) m.z = m.x;
   if (!ok) return 1;                                   // caller falls back to the generic path
   const bool rv = (p.flags & MB200_REVERSE) != 0, hy = p.y != nullptr;
-  auto k = (p.flags & kFlagCarryPass) ? sscan_fwd_tma_kernel<T, N, true, true, false>
-           : rv ? (hy ? sscan_fwd_tma_kernel<T, N, true, false, true> : sscan_fwd_tma_kernel<T, N, true, false, false>)
-                : (hy ? sscan_fwd_tma_kernel<T, N, false, false, true> : sscan_fwd_tma_kernel<T, N, false, false, false>);
+  const bool sv = p.carries != nullptr;
+  auto k = (p.flags & kFlagCarryPass) ? sscan_fwd_tma_kernel<T, N, true, true, false, false> : sscan_fwd_tma_kernel<T, N, false, false, false, false>;
+#define MB200_FWD_PICK(R, Y, S) if (!(p.flags & kFlagCarryPass) && rv == R && hy == Y && sv == S) k = sscan_fwd_tma_kernel<T, N, R, false, Y, S>;
+  MB200_FWD_PICK(false, true, true) MB200_FWD_PICK(true, true, true) MB200_FWD_PICK(false, true, false) MB200_FWD_PICK(true, true, false)
+  MB200_FWD_PICK(false, false, true) MB200_FWD_PICK(true, false, true) MB200_FWD_PICK(true, false, false)
+#undef MB200_FWD_PICK
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes) != cudaSuccess)
     return MB200_ELAUNCH;
   dim3 grid(unsigned((p.ED + G::kTE - 1) / G::kTE), unsigned(p.B), unsigned(p.launch_pieces));

@@ -136,9 +136,8 @@ sscan_fwd_generic_kernel(const SscanFwdParams p) {
 #pragma unroll
       for (int t = 0; t < kTT; ++t) {
         if ((t % kChunk) == 0 && p.carries && e_ok && t0 + t < p.L) {
-          float4* dst = reinterpret_cast<float4*>(
-              p.carries + ((b * nchunks + (t0 + t) / kChunk) * p.ED + e) * N + 4 * q);
-          *dst = make_float4(hlo.x, hlo.y, hhi.x, hhi.y);
+          store_states(p.carries + (b * nchunks + (t0 + t) / kChunk) * p.ED * N, (p.flags & MB200_PAIRED_STATES) != 0, p.ED, N, e, q,
+                       make_float4(hlo.x, hlo.y, hhi.x, hhi.y));
         }
         const float2 o = op[t * kTE + ((t & 1) ? op_off1 : op_off0)];   // {delta, delta*x}
         const float4 Bq = *reinterpret_cast<const float4*>(sB + t * N);
