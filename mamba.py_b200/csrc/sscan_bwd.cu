@@ -250,11 +250,12 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       Opnd nx = fetch(kHalf - 1), nx2 = fetch(kHalf - 2);
 #pragma unroll
       for (int wi = kHalf / kBWin - 1; wi >= 0; --wi) {
-        // window sequence number: chunks in processing order, windows from the chunk's end; a chunk has an even number of them
-        const int wseq = k8 * (kHalf / kBWin) + (kHalf / kBWin - 1 - wi);
-        const int wb = (kHalf / kBWin - 1 - wi) & 1;
+        // Windows are taken from the chunk's end, the two buffers in turn.  A chunk has four, so that buffer and parity are
+        // known here (the first wait for each buffer, parity 1 of a new barrier, returns at once).
+        const int wb = (kHalf / kBWin - 1 - wi) & 1, wpar = ((kHalf / kBWin - 1 - wi) >> 1) ^ 1;
+        static_assert(kHalf / kBWin == 4, "buffers and parities repeat every chunk");
         // asked now, needed only before the first store of the window
-        const bool slot_free = wseq < 2 || mbar_test(&win_empty[wb], int(((wseq - 2) >> 1) & 1));
+        const bool slot_free = mbar_test(&win_empty[wb], wpar);
         float* np = s_np + wb * kBWin * kNpStep;
         float4* ep = epo + wb * kBWin * kEpStep;
 #pragma unroll
@@ -283,7 +284,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
             wAs = k ? __ffma2_rn(w, A2[k], wAs) : __fmul2_rn(w, A2[k]);
           }
           const float s0 = lanes_sum(ysum), s1 = lanes_sum(gBs), s2 = lanes_sum(wAs);
-          if (ti == kBWin - 1 && !slot_free && !mbar_wait(&win_empty[wb], int(((wseq - 2) >> 1) & 1))) { fail(); return; }
+          if (ti == kBWin - 1 && !slot_free && !mbar_wait(&win_empty[wb], wpar)) { fail(); return; }
           np[ti * kNpStep + npo] = s0;
           np[ti * kNpStep + kNpPlane + npo] = s1;
           np[ti * kNpStep + 2 * kNpPlane + npo] = s2;
