@@ -15,6 +15,7 @@
 // pre-activation; the 4 warps of a CTA take 4 consecutive chunks of the same channels and add their
 // sums for dw and dbias in shared memory first, so global memory sees one atomic per CTA and value.
 #include <initializer_list>
+#include <type_traits>
 #include "common.cuh"
 
 namespace mb200 {
@@ -22,14 +23,16 @@ namespace {
 
 constexpr int kConvK = 4;
 constexpr int kConvThreads = 256;
-constexpr int kConvChunkFwd = 32;             // forward chunk (compile time: its loop is fully unrolled)
+// Forward chunks (compile time: the loop over one is fully unrolled), the one whose waves of CTAs are shorter: 8 x 2048 x 1536 in
+// bfloat16 is one wave of 64 steps (22.9 us) or two of 32 (25.4), 64 x 197 x 384 one of either (9.2 / 9.0).
+constexpr int kConvChunkFwd[2] = {32, 64};
 // Timesteps whose loads are in flight together.  Forward 8 (with 3 CTAs of 256 threads per SM): 29.5 us on the 130m layer
 // against 33.8 for 4.  Backward 4 (with 4 CTAs of 128 threads): 60 us; 6 and 8 need more registers than 16 warps per SM leave
 // and measured 71 and 75, walking backwards with CTAs of 256 threads 69.
 constexpr int kConvGroup = 8, kConvGroupBwd = 4;
 constexpr int kConvBwdThreads = 128;
 
-static_assert(kConvChunkFwd % kConvGroup == 0, "a chunk is a whole number of groups");
+static_assert(kConvChunkFwd[0] % kConvGroup == 0 && kConvChunkFwd[1] % kConvGroup == 0, "a chunk is a whole number of groups");
 
 template <typename T, int V> struct alignas(sizeof(T) * V) CVec {
   T v[V];
@@ -109,14 +112,14 @@ __device__ __forceinline__ CVec<T, V> pack(const Pk<W> (&o)[V / W]) {
 }
 
 // grid: x = ceil(nvec / 32) channel groups, y = ceil(nchunk / 8), z = batch; warp w of a CTA takes chunk 8*y + w
-template <typename T, int V>
+template <typename T, int V, int kChunkLen>
 __global__ void __launch_bounds__(kConvThreads, 3)
 conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                        T* __restrict__ y, int64_t L, int64_t ED, int64_t x_sb, int64_t x_sl,
                        int64_t y_sb, int64_t y_sl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t e = (int64_t(blockIdx.x) * 32 + lane) * V;
-  const int64_t t0 = (int64_t(blockIdx.y) * (kConvThreads / 32) + warp) * kConvChunkFwd;
+  const int64_t t0 = (int64_t(blockIdx.y) * (kConvThreads / 32) + warp) * kChunkLen;
   if (e >= ED || t0 >= L) return;
   const int64_t b = blockIdx.z;
   constexpr int W = (V % 2 == 0) ? 2 : 1, P = V / W;
@@ -128,28 +131,26 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
 #pragma unroll
     for (int k = 0; k < kConvK; ++k) wk[i][k] = F::load(w + (e + W * i) * kConvK + k, kConvK);
   }
-  const T* xp = x + b * x_sb + e;
-  T* yp = y + b * y_sb + e;
+  const T* xp = x + b * x_sb + e + t0 * x_sl;
+  T* yp = y + b * y_sb + e + t0 * y_sl;
 #pragma unroll
   for (int k = 0; k < kConvK - 1; ++k) {                  // x[t0-3 .. t0-1]
-    const int64_t t = t0 - (kConvK - 1) + k;
     F xv[P];
-    unpack<T, V, W>(cload<T, V>(xp + t * x_sl, t >= 0), xv);
+    unpack<T, V, W>(cload<T, V>(xp + (k - (kConvK - 1)) * x_sl, t0 > 0), xv);
 #pragma unroll
     for (int i = 0; i < P; ++i) win[i][k] = xv[i];
   }
-  // fully unrolled: the compiler hoists the loads of later groups over the arithmetic of earlier ones
-#pragma unroll
-  for (int g = 0; g < kConvChunkFwd / kConvGroup; ++g) {
+  // Whole chunks (all but a row's last) test nothing (28.1 -> 25.4 us, see above, together with moving pointers); their loop is fully unrolled, so that the compiler hoists the loads of later
+  // groups over the arithmetic of earlier ones.
+  auto group = [&](auto whole, int left) {
     CVec<T, V> v[kConvGroup];
 #pragma unroll
     for (int j = 0; j < kConvGroup; ++j) {
-      const int64_t t = t0 + g * kConvGroup + j;
-      v[j] = cload<T, V>(xp + t * x_sl, t < L);
+      v[j] = cload<T, V>(xp, decltype(whole)::value || j < left);
+      xp += x_sl;
     }
 #pragma unroll
     for (int j = 0; j < kConvGroup; ++j) {
-      const int64_t t = t0 + g * kConvGroup + j;
       F xn[P], o[P];
       unpack<T, V, W>(v[j], xn);
 #pragma unroll
@@ -161,8 +162,17 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
         win[i][0] = win[i][1]; win[i][1] = win[i][2]; win[i][2] = xn[i];
         o[i] = pmul(acc, psigmoid(acc));
       }
-      if (t < L) cstore<T, V>(yp + t * y_sl, pack<T, V, W>(o));
+      if (decltype(whole)::value || j < left) cstore<T, V>(yp, pack<T, V, W>(o));
+      yp += y_sl;
     }
+  };
+  const int left = int(min64(L - t0, kChunkLen));
+  if (left == kChunkLen) {
+#pragma unroll
+    for (int g = 0; g < kChunkLen / kConvGroup; ++g) group(std::true_type{}, 0);
+  } else {
+#pragma unroll 1
+    for (int g = 0; g < left; g += kConvGroup) group(std::false_type{}, left - g);
   }
 }
 
@@ -193,93 +203,106 @@ conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
 #pragma unroll
       for (int k = 0; k < kConvK; ++k) wk[i][k] = F::load(w + (e + W * i) * kConvK + k, kConvK);
     }
-    const T* xp = x + b * x_sb + e;
-    const T* gp = dy + b * dy_sb + e;
-    T* op = dx + b * dx_sb + e;
+    // Two and a half times the instructions of the arithmetic went into bounds, row addresses and shifting the windows: 47 -> 42 us on
+    // 8 x 2048 x 1536 in bfloat16, 16.2 -> 14.6 on 64 x 197 x 384.
     // Time is walked forwards in groups of kConvGroupBwd steps whose loads go out together; dx trails by three steps, because
-    // dx[t-3] needs dpre[t-3 .. t].  Slots 0..2 of the two windows are the last three steps of the group before.
+    // dx[t-3] needs dpre[t-3 .. t].  The windows hold four steps, as many as a group, so that every slot is known at compile time.
     constexpr int kG = kConvGroupBwd, kH = kConvK - 1;
-    F xw[P][kG + kH], dw_[P][kG + kH], dwacc[P][kConvK], dbacc[P];
+    static_assert(kG == kConvK, "window slots repeat with the groups");
+    F xw[P][kG], dw_[P][kG], dwacc[P][kConvK], dbacc[P];
 #pragma unroll
     for (int i = 0; i < P; ++i) {
       dbacc[i] = F::splat(0.f);
 #pragma unroll
       for (int k = 0; k < kConvK; ++k) dwacc[i][k] = F::splat(0.f);
 #pragma unroll
-      for (int k = 0; k < kH; ++k) dw_[i][k] = F::splat(0.f);
+      for (int k = 0; k < kG; ++k) dw_[i][k] = F::splat(0.f);
     }
+    const T* xg = x + b * x_sb + e + t0 * x_sl;
+    const T* gg = dy + b * dy_sb + e + t0 * dy_sl;
+    T* og = dx + b * dx_sb + e + (t0 - kH) * dx_sl;
 #pragma unroll
     for (int k = 0; k < kH; ++k) {                         // x[t0-3 .. t0-1]
-      const int64_t t = t0 - kH + k;
       F xv[P];
-      unpack<T, V, W>(cload<T, V>(xp + t * x_sl, t >= 0), xv);
+      unpack<T, V, W>(cload<T, V>(xg + (k - kH) * x_sl, t0 > 0), xv);
 #pragma unroll
-      for (int i = 0; i < P; ++i) xw[i][k] = xv[i];
+      for (int i = 0; i < P; ++i) xw[i][k + 1] = xv[i];
     }
-    // steps t1 .. t1+2 only produce dpre for the chunk's last outputs: their own dx, dw belong to the next chunk
     const F one = F::splat(1.f), mone = F::splat(-1.f);
-    CVec<T, V> gv[kG], xv[kG], gn[kG], xq[kG];
-    const int64_t t_end = min64(L, t1 + kH);
-    auto fetch = [&](int64_t tg, CVec<T, V> (&xq)[kG], CVec<T, V> (&gn)[kG]) {
-      const T* xg = xp + tg * x_sl;
-      const T* gg = gp + tg * dy_sl;
+    struct Group { CVec<T, V> x[kG], g[kG]; };
+    // Steps counted from t0: `own` of them belong to the chunk.  The three behind them only produce dpre for the chunk's last
+    // outputs: their own dx, dw belong to the next chunk.  (x, dy read as 0 past the end of the row.)
+    const int own = int(t1 - t0), end = int(min64(L, t1 + kH) - t0);
+    auto fetch = [&](int s0, Group& q) {
+      if (s0 + kG <= end) {
 #pragma unroll
-      for (int j = 0; j < kG; ++j) {
-        const bool ok = tg + j < t_end;
-        xq[j] = cload<T, V>(xg, ok);
-        gn[j] = cload<T, V>(gg, ok);
-        xg += x_sl; gg += dy_sl;
+        for (int j = 0; j < kG; ++j) {
+          q.x[j] = cload<T, V>(xg, true);
+          q.g[j] = cload<T, V>(gg, true);
+          xg += x_sl; gg += dy_sl;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kG; ++j) {
+          q.x[j] = cload<T, V>(xg, s0 + j < end);
+          q.g[j] = cload<T, V>(gg, s0 + j < end);
+          xg += x_sl; gg += dy_sl;
+        }
       }
     };
-    if constexpr (kAhead) fetch(t0, xq, gn);
-#pragma unroll 1
-    for (int64_t tg = t0; tg < t1 + kH; tg += kG) {
-      if constexpr (kAhead) {
-#pragma unroll
-        for (int j = 0; j < kG; ++j) { gv[j] = gn[j]; xv[j] = xq[j]; }
-        fetch(tg + kG, xq, gn);
-      } else {
-        fetch(tg, xv, gv);
-      }
-      T* og = op + (tg - kH) * dx_sl;
+    auto group = [&](auto inside, int s0, const Group& q) {
+      constexpr bool kIn = decltype(inside)::value;        // every step and every output of the group belongs to the chunk
 #pragma unroll
       for (int j = 0; j < kG; ++j) {
-        const int64_t t = tg + j;
-        const bool own = t < t1;
         F g[P], xn[P], o[P];
-        unpack<T, V, W>(gv[j], g);
-        unpack<T, V, W>(xv[j], xn);
+        unpack<T, V, W>(q.g[j], g);
+        unpack<T, V, W>(q.x[j], xn);
 #pragma unroll
         for (int i = 0; i < P; ++i) {
-          xw[i][j + kH] = xn[i];
+          xw[i][j] = xn[i];
           F pre = bv[i];
 #pragma unroll
-          for (int k = 0; k < kConvK; ++k) pre = pfma(wk[i][k], xw[i][j + k], pre);
+          for (int k = 0; k < kConvK; ++k) pre = pfma(wk[i][k], xw[i][(j + 1 + k) % kG], pre);
           const F sg = psigmoid(pre);
           // dpre = dy * s * (1 + pre * (1 - s));  dy is 0 past the end
           const F dp = pmul(pmul(g[i], sg), pfma(pre, pfma(sg, mone, one), one));
-          dw_[i][j + kH] = dp;
+          dw_[i][j] = dp;
           // dx[t-3] = w3*dpre[t-3] + w2*dpre[t-2] + w1*dpre[t-1] + w0*dpre[t]
           F acc = pmul(wk[i][0], dp);
 #pragma unroll
-          for (int k = 1; k < kConvK; ++k) acc = pfma(wk[i][k], dw_[i][j + kH - k], acc);
+          for (int k = 1; k < kConvK; ++k) acc = pfma(wk[i][k], dw_[i][(j + kG - k) % kG], acc);
           o[i] = acc;
-          if (own) {
+          if (kIn || s0 + j < own) {
             dbacc[i] = padd(dbacc[i], dp);
 #pragma unroll
-            for (int k = 0; k < kConvK; ++k) dwacc[i][k] = pfma(dp, xw[i][j + k], dwacc[i][k]);
+            for (int k = 0; k < kConvK; ++k) dwacc[i][k] = pfma(dp, xw[i][(j + 1 + k) % kG], dwacc[i][k]);
           }
         }
-        if (t - kH >= t0 && t - kH < t1) cstore<T, V>(og, pack<T, V, W>(o));
+        if (kIn || (s0 + j >= kH && s0 + j - kH < own)) cstore<T, V>(og, pack<T, V, W>(o));
         og += dx_sl;
       }
-#pragma unroll
-      for (int i = 0; i < P; ++i)
-#pragma unroll
-        for (int k = 0; k < kH; ++k) {
-          xw[i][k] = xw[i][kG + k];
-          dw_[i][k] = dw_[i][kG + k];
-        }
+    };
+    auto run = [&](int s0, const Group& q) {
+      if (s0 >= kH && s0 + kG <= own) group(std::true_type{}, s0, q);
+      else group(std::false_type{}, s0, q);
+    };
+    if constexpr (kAhead) {                                // two groups of loads in turn, one of them in flight
+      Group q0, q1;
+      fetch(0, q0);
+#pragma unroll 1
+      for (int s0 = 0; s0 < own + kH; s0 += 2 * kG) {
+        fetch(s0 + kG, q1);
+        run(s0, q0);
+        fetch(s0 + 2 * kG, q0);
+        run(s0 + kG, q1);
+      }
+    } else {
+#pragma unroll 1
+      for (int s0 = 0; s0 < own + kH; s0 += kG) {
+        Group q;
+        fetch(s0, q);
+        run(s0, q);
+      }
     }
 #pragma unroll
     for (int i = 0; i < P; ++i) {
@@ -353,13 +376,22 @@ extern "C" int mb200_conv1d_silu_fwd(const void* x, const float* w, const float*
   const bool vec = conv_vec_ok(ED, kv, {x, y}, {x_sb, x_sl, y_sb, y_sl});
   const int v = vec ? kv : 1;
   const int64_t cols = (ED + 32 * int64_t(v) - 1) / (32 * int64_t(v));
-  const int chunk = kConvChunkFwd;
-  const int64_t nchunk = (L + chunk - 1) / chunk;
-  const int64_t ngroup = (nchunk + kConvThreads / 32 - 1) / (kConvThreads / 32);
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int64_t ngroup = 0, best = 0;
+  bool longer = false;
+  for (int k = 0; k < 2; ++k) {
+    const int chunk = kConvChunkFwd[k];
+    const int64_t groups = ((L + chunk - 1) / chunk + kConvThreads / 32 - 1) / (kConvThreads / 32);
+    const int64_t waves = (cols * groups * B + 3 * sms - 1) / (3 * sms), cost = waves * (chunk + kConvK - 1);
+    if (k == 0 || cost < best) { best = cost; ngroup = groups; longer = k == 1; }
+  }
   if (B > 65535 || ngroup > 65535) return MB200_ETOOBIG;
   const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(ngroup), static_cast<unsigned>(B));
-#define MB200_CONV_FWD(TT, VV) \
-  conv1d_silu_fwd_kernel<TT, VV><<<grid, kConvThreads, 0, st>>>((const TT*)x, w, bias, (TT*)y, L, ED, x_sb, x_sl, y_sb, y_sl)
+#define MB200_CONV_FWD(TT, VV) do { \
+    if (longer) conv1d_silu_fwd_kernel<TT, VV, kConvChunkFwd[1]><<<grid, kConvThreads, 0, st>>>((const TT*)x, w, bias, (TT*)y, L, ED, x_sb, x_sl, y_sb, y_sl); \
+    else conv1d_silu_fwd_kernel<TT, VV, kConvChunkFwd[0]><<<grid, kConvThreads, 0, st>>>((const TT*)x, w, bias, (TT*)y, L, ED, x_sb, x_sl, y_sb, y_sl); \
+  } while (0)
   if (dtype == MB200_F32) { if (vec) MB200_CONV_FWD(float, 4); else MB200_CONV_FWD(float, 1); }
   else { if (vec) MB200_CONV_FWD(__nv_bfloat16, 4); else MB200_CONV_FWD(__nv_bfloat16, 1); }
 #undef MB200_CONV_FWD

@@ -64,3 +64,17 @@ def test_wide_bfloat16_backward(Bsz, L, ED):
     y = F.silu(F.conv1d(x32.transpose(1, 2), w, b, groups=ED, padding=3)[..., :L].transpose(1, 2))
     for a, r in zip(got, torch.autograd.grad(y, (x32, w, b), dy.float())):
         assert ((a.float() - r).norm() / r.norm()).item() < 5e-3
+
+
+@pytest.mark.parametrize("Bsz,L,ED", [(8, 2048, 1536), (8, 2041, 1536), (8, 1985, 1540), (4, 31, 2052)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_forward_chunks(Bsz, L, ED, dtype):
+    """Chunks of 64 (one wave of CTAs), whole, a step short, one step in the last; chunks of 32, a step short."""
+    import mamba_b200
+    g = torch.Generator(device="cuda").manual_seed(L)
+    new = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, b = new(Bsz, L, ED).to(dtype), new(ED, 1, 4), new(ED)
+    y = mamba_b200.mamba.causal_conv1d_silu(x, w, b)
+    xp = F.pad(x.float(), (0, 0, 3, 0))
+    r = F.silu(sum(xp[:, k:k + L] * w[:, 0, k] for k in range(4)) + b)
+    assert ((y.float() - r).norm() / r.norm()).item() < (3e-3 if dtype == torch.bfloat16 else 1e-5)
