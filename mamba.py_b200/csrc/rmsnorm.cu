@@ -311,8 +311,13 @@ norm_rows_fwd_kernel(const TX* __restrict__ x, const TR* __restrict__ res_in, co
 
 // ds = (g - shat * mean(g * shat)) * rstd (+ dres), g = dy * w, shat = s * rstd;  dw = sum over rows of dy * shat.  ds_bf16, when
 // given, is ds once more, dense and rounded: the gradient of a bfloat16 mixer output beside that of the float32 stream.
+// The grid is one wave of CTAs, so that the rows they walk are few and the dweight atomics too: as many as fit by registers, 3 per SM
+// with up to 3 chunks a thread (compiled for that: 88 registers instead of 80 let only two in, and a grid for three then ran in two
+// waves), 2 with 4 and 1 with 8.  us before / after, 12.6 M elements in float32: 53 / 40 at 768 wide, 46 / 38 at 192, 46 / 34 at 2048,
+// 54 / 46 at 5120 (with 3 CTAs per SM forced on 4 chunks 46 and 60 at 2048 and 2560, for 34 and 47).
+constexpr int norm_bwd_ctas(int chunks) { return chunks <= 3 ? 3 : chunks == 4 ? 2 : 1; }
 template <typename TR, typename TY, int kTPR, int kC>
-__global__ void __launch_bounds__(kNormThreads)
+__global__ void __launch_bounds__(kNormThreads, norm_bwd_ctas(kC))
 norm_rows_bwd_kernel(const TR* __restrict__ s, const float* __restrict__ w, const float* __restrict__ rstd,
                      const TY* __restrict__ dy, const TR* __restrict__ dres, TR* __restrict__ ds,
                      __nv_bfloat16* __restrict__ ds_bf16, float* __restrict__ dw,
@@ -436,8 +441,7 @@ bool rows_bwd(const void* s, const float* w, const float* rstd, const void* dy, 
               int64_t s_rs, int64_t dy_rs, int64_t dr_rs, int64_t ds_rs, cudaStream_t st) {
   return with_row_layout(D, [&]<int kTPR, int kC>(RowLayout<kTPR, kC>) {
     constexpr int kRows = kNormThreads / kTPR;
-    // 3 CTAs per SM keep enough rows in flight; more would only add dweight atomics
-    const int64_t want = (rows + kRows - 1) / kRows, cap = int64_t(sm_count()) * 3;
+    const int64_t want = (rows + kRows - 1) / kRows, cap = int64_t(sm_count()) * norm_bwd_ctas(kC);
     norm_rows_bwd_kernel<TR, TY, kTPR, kC><<<unsigned(want < cap ? want : cap), kNormThreads, 0, st>>>(
         (const TR*)s, w, rstd, (const TY*)dy, (const TR*)dres, (TR*)ds, (__nv_bfloat16*)ds_bf16, dw, rows, D, s_rs, dy_rs, dr_rs, ds_rs);
   });
