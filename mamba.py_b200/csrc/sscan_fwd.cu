@@ -71,16 +71,21 @@ constexpr int kTile = 2 * kChunk;          // timesteps per tile (two saved stat
 #endif
 constexpr int kLoadAhead = MB200_FWD_LA, kDecayAhead = MB200_FWD_EA;   // software-pipeline depths of the recurrence warps
 constexpr int kDefer = MB200_FWD_DEFER;     // timesteps of partial sums a recurrence thread holds before storing them
-template <int N> struct FwdGeom {
+// kWide: 6 + 6 warps and 48 channels, alone on its SM.  For a scan whose 32-channel tiles are a few more than the SMs, so that some SMs
+// hold two and the rest wait for them: us per 2048 steps with one such CTA 98-106 on every SM, with two of 32 channels 112-125 (with one
+// 77-83).  With more CTAs than SMs the narrow tile is the better one (two of 48 channels 169-191, three of 32 157-175); 40 channels
+// (5 + 5 warps) straddle state quads and took 95-104.
+template <int N, bool kWide = false> struct FwdGeom {
   static constexpr int kCPT = (N == 16) ? MB200_FWD_CPT : 1;
-  static constexpr int kCW = (N == 16) ? MB200_FWD_CW : 4;
-  static constexpr int kPW = (N == 16) ? MB200_FWD_PW : 4;
-  static constexpr int kOcc = (N == 16) ? MB200_FWD_OCC : 3;          // CTAs per SM the kernel is compiled for
+  static constexpr int kCW = kWide ? 6 : (N == 16) ? MB200_FWD_CW : 4;
+  static constexpr int kPW = kWide ? 6 : (N == 16) ? MB200_FWD_PW : 4;
+  static constexpr int kOcc = kWide ? 1 : (N == 16) ? MB200_FWD_OCC : 3;          // CTAs per SM the kernel is compiled for
   static constexpr int kLPE = N / 4;                                   // lanes per channel group
   static constexpr int kConsumers = 32 * kCW;
   static constexpr int kProducers = 32 * kPW;
   static constexpr int kThreads = kConsumers + kProducers + 32;      // + the warp that issues the TMA copies
   static constexpr int kTE = kConsumers / kLPE * kCPT;                 // channels per CTA
+  static_assert(!kWide || (N == 16 && kCPT == 1), "the wide tile is laid out for d_state 16, one channel per thread");
   static_assert(kCPT == 1 || (kCPT == 2 && N == 16), "two channels per thread are laid out for d_state 16");
   static_assert(kTE % 8 == 0, "a tile row is a whole number of 16-byte vectors in bf16");
 };
@@ -89,8 +94,8 @@ struct FwdMaps {
   CUtensorMap x, d, z, B, C;
 };
 
-template <typename T, int N> struct TmaFwdSmem {
-  using G = FwdGeom<N>;
+template <typename T, int N, bool kWide = false> struct TmaFwdSmem {
+  using G = FwdGeom<N, kWide>;
   static constexpr int kStages = Ring<T>::kStages;
   static constexpr int kTE = G::kTE;
   static constexpr int kYpRow = kTE * G::kLPE;                          // partial sums per timestep
@@ -150,11 +155,11 @@ __device__ __forceinline__ bool s4d_structured(const float* a4, float a0, int q)
 // after adding the input.  It has no y and saves no states; the result leaves through hT.
 // kHasY = false is the pass that only wants states (no C-contraction, no epilogue).  kSave: the states entering the chunks go to
 // p.carries (a template parameter because the test alone costs the recurrence warps 2 % of a prompt).
-template <typename T, int N, bool kRev, bool kCarry, bool kHasY, bool kSave>
-__global__ void __launch_bounds__(FwdGeom<N>::kThreads, FwdGeom<N>::kOcc)
+template <typename T, int N, bool kRev, bool kCarry, bool kHasY, bool kSave, bool kWide = false>
+__global__ void __launch_bounds__(FwdGeom<N, kWide>::kThreads, FwdGeom<N, kWide>::kOcc)
 sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams p) {
-  using G = FwdGeom<N>;
-  using S = TmaFwdSmem<T, N>;
+  using G = FwdGeom<N, kWide>;
+  using S = TmaFwdSmem<T, N, kWide>;
   constexpr int kLPE = G::kLPE, kTE = G::kTE, kStages = S::kStages;
   constexpr int kCPT = G::kCPT, kNC = G::kConsumers, kNP = G::kProducers, kYpRow = S::kYpRow;
 
@@ -578,10 +583,10 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
   }
 }
 
-template <typename T, int N>
-int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
-  using G = FwdGeom<N>;
-  using S = TmaFwdSmem<T, N>;
+template <typename T, int N, bool kWide>
+int tma_launch_tile(const SscanFwdParams& p, cudaStream_t st) {
+  using G = FwdGeom<N, kWide>;
+  using S = TmaFwdSmem<T, N, kWide>;
   constexpr bool bf = sizeof(T) == 2;
   FwdMaps m;
   bool ok = tma_encode(&m.x, p.x, bf, p.B, p.L, p.ED, p.x_sb, p.x_sl, G::kTE, kTile) &&
@@ -593,16 +598,32 @@ int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
   if (!ok) return 1;                                   // caller falls back to the generic path
   const bool rv = (p.flags & MB200_REVERSE) != 0, hy = p.y != nullptr;
   const bool sv = p.carries != nullptr;
-  auto k = (p.flags & kFlagCarryPass) ? sscan_fwd_tma_kernel<T, N, true, true, false, false> : sscan_fwd_tma_kernel<T, N, false, false, false, false>;
-#define MB200_FWD_PICK(R, Y, S) if (!(p.flags & kFlagCarryPass) && rv == R && hy == Y && sv == S) k = sscan_fwd_tma_kernel<T, N, R, false, Y, S>;
-  MB200_FWD_PICK(false, true, true) MB200_FWD_PICK(true, true, true) MB200_FWD_PICK(false, true, false) MB200_FWD_PICK(true, true, false)
-  MB200_FWD_PICK(false, false, true) MB200_FWD_PICK(true, false, true) MB200_FWD_PICK(true, false, false)
-#undef MB200_FWD_PICK
+  void (*k)(const FwdMaps, const SscanFwdParams) = nullptr;
+  if constexpr (!kWide) {
+    if (p.flags & kFlagCarryPass) k = sscan_fwd_tma_kernel<T, N, true, true, false, false>;
+    else if (!hy) k = rv ? (sv ? sscan_fwd_tma_kernel<T, N, true, false, false, true> : sscan_fwd_tma_kernel<T, N, true, false, false, false>)
+                         : (sv ? sscan_fwd_tma_kernel<T, N, false, false, false, true> : sscan_fwd_tma_kernel<T, N, false, false, false, false>);
+  }
+  if (!k) k = rv ? (sv ? sscan_fwd_tma_kernel<T, N, true, false, true, true, kWide> : sscan_fwd_tma_kernel<T, N, true, false, true, false, kWide>)
+                 : (sv ? sscan_fwd_tma_kernel<T, N, false, false, true, true, kWide> : sscan_fwd_tma_kernel<T, N, false, false, true, false, kWide>);
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes) != cudaSuccess)
     return MB200_ELAUNCH;
   dim3 grid(unsigned((p.ED + G::kTE - 1) / G::kTE), unsigned(p.B), unsigned(p.launch_pieces));
   k<<<grid, G::kThreads, S::kBytes, st>>>(m, p);
   return check_launch();
+}
+
+template <typename T, int N>
+int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
+  if constexpr (N == 16) {
+    int dev = 0, sms = 0;
+    if (p.y && !(p.flags & kFlagCarryPass) && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
+      const int64_t rows = p.B * p.launch_pieces, narrow = FwdGeom<N>::kTE, wide = FwdGeom<N, true>::kTE;
+      if (rows * ((p.ED + narrow - 1) / narrow) > sms && rows * ((p.ED + wide - 1) / wide) <= sms) return tma_launch_tile<T, N, true>(p, st);
+    }
+  }
+  return tma_launch_tile<T, N, false>(p, st);
 }
 
 template <typename T>

@@ -244,3 +244,25 @@ def test_rows_cut_into_pieces_bf16_long():
     for k in ("x", "delta", "z", "B", "C", "A", "D"):
         scale = max(1.0, go[k].abs().max().item())
         assert_close(gk[k], go[k].float(), BF_RTOL, BF_ATOL * scale, f"grad {k}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("ED, L", [(32 * 148 + 8, 45), (48 * 148, 16)])
+def test_wide_tiles(dtype, reverse, ED, L):
+    """One CTA of 48 channels per SM (more 32-channel tiles than the 148 SMs, ragged last tile) against the same channels in two
+    launches of 32-channel tiles: the same operations in the same order."""
+    from mamba_b200.mamba import sscan_fwd_raw
+    g = torch.Generator(device="cuda").manual_seed(ED)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x, z = r(1, L, ED).to(dtype), r(1, L, ED).to(dtype)
+    delta = torch.nn.functional.softplus(r(1, L, ED) - 3).to(dtype)
+    A, Bm, Cm, D, h0 = -torch.exp(r(ED, 16)), r(1, L, 16).to(dtype), r(1, L, 16).to(dtype), r(ED), r(1, ED, 16)
+    run = lambda a, b, want: sscan_fwd_raw(x[..., a:b], delta[..., a:b], A[a:b], Bm, Cm, D[a:b], z[..., a:b], h0=h0[:, a:b].contiguous(),
+                                           want_last=True, want_carries=want, reverse=reverse)
+    for want in (False, True):
+        whole, parts = run(0, ED, want), [run(a, b, want) for a, b in ((0, 2560), (2560, ED))]
+        assert torch.equal(whole[0], torch.cat([p[0] for p in parts], 2))
+        assert torch.equal(whole[1], torch.cat([p[1] for p in parts], 1))
+        if want:
+            assert torch.equal(whole[2], torch.cat([p[2] for p in parts], 3))
