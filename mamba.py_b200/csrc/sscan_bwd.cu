@@ -19,7 +19,8 @@
 //     memory, in windows of 2 timesteps.
 //     Why 2 x 2: what goes through shared memory is what bounds the kernel.  Of its 4 elements a thread hands
 //     over 8 products and 3 sums (4 states of a channel), 4 and 3 (2 x 2, with three shuffles) or 2 and 12; and
-//     B and C are then 8-byte loads of two addresses, delta and delta*x 16-byte loads that two lanes share.
+//     B and C of a state pair are then short loads of two addresses (side by side, so that the reverse walk takes one),
+//     delta and delta*x 16-byte loads that two lanes share.
 //     44.6 -> 33.9 wavefronts per 128 elements and 610 -> 544 us on 8 x 2048 x 1536 in bfloat16, together with
 //     what follows; without the shuffles (twice the sums to write and to read) 587.
 //   - warps 5 and 7 finish alternate windows: sum the 4 partials of each channel, form dx, ddelta,
@@ -68,9 +69,8 @@ template <typename T> struct TmaBwdSmem {
   static constexpr int kOp = kRaw + kStages * kStageBytes;                // float4 [2][16][16]
   static constexpr int kAux = kOp + 2 * kBTile * kBTE * 8;                // float4 [2][16][16]
   static constexpr int kDyp = kAux + 2 * kBTile * kBTE * 8;               // float  [2][16][32]
-  static constexpr int kB = kDyp + 2 * kBTile * kBTE * 4;                 // float  [2][16][16]
-  static constexpr int kC = kB + 2 * kBTile * kBN * 4;
-  static constexpr int kNp = kC + 2 * kBTile * kBN * 4;                   // float  [2][kBWin][3][4][32]
+  static constexpr int kBC = kDyp + 2 * kBTile * kBTE * 4;                // float4 [2][16][8]
+  static constexpr int kNp = kBC + 4 * kBTile * kBN * 4;                   // float  [2][kBWin][3][4][32]
   static constexpr int kEp = kNp + 2 * kBWin * kNpStep * 4;                  // float4 [2][kBWin][8][16]
   static constexpr int kD = kEp + 2 * kBWin * kEpStep * 16;               // float [32]
   static constexpr int kBias = kD + kBTE * 4;
@@ -95,8 +95,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
   float4* s_op = reinterpret_cast<float4*>(smem_raw + S::kOp);      // {delta, delta, delta*x, delta*x} of a channel pair
   float4* s_aux = reinterpret_cast<float4*>(smem_raw + S::kAux);    // {d softplus x 2, dy d(silu z)/dz x 2} of a channel pair
   float* s_dyp = reinterpret_cast<float*>(smem_raw + S::kDyp);
-  float* s_B = reinterpret_cast<float*>(smem_raw + S::kB);
-  float* s_C = reinterpret_cast<float*>(smem_raw + S::kC);
+  float4* s_BC = reinterpret_cast<float4*>(smem_raw + S::kBC);      // {B, B, C, C} of a state pair
   float* s_np = reinterpret_cast<float*>(smem_raw + S::kNp);
   float4* s_ep = reinterpret_cast<float4*>(smem_raw + S::kEp);
   float* s_D = reinterpret_cast<float*>(smem_raw + S::kD);
@@ -144,12 +143,13 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
   __syncthreads();
   auto fail = [&]() { atomicExch(&g_bwd_status, MB200_DEV_WAIT_TIMEOUT); };
 
-  // The recurrence warps need far more registers than the others: hand 32 registers per thread of
-  // warps 4-7 over to warps 0-3 (the kernel is compiled for 80; 128 * 48 + 128 * 112 = 256 * 80).
+  // The recurrence warps need far more registers than the others: hand 24 registers per thread of
+  // warps 4-7 over to warps 0-3 (the kernel is compiled for 80; 128 * 56 + 128 * 104 = 256 * 80).  112 / 48: 524 us
+  // for 523, and 292 for 280 where an SM holds one CTA; 120 / 40 spills.
   if (warp < 4) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   }
   if (warp < 4) {
     // ================================================================== consumers
@@ -215,8 +215,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       const float4* op0 = s_op + r0 * (kBTE / 2) + op_off0;
       const float4* op1 = s_op + r0 * (kBTE / 2) + op_off1;
       const float* dyp = s_dyp + r0 * kBTE + c0;
-      const float* sB = s_B + r0 * N + n0;
-      constexpr int kBtoC = (S::kC - S::kB) / 4;
+      const float4* sBC = s_BC + r0 * (N / 2) + sp;
 
       // states after each step of the chunk, in registers
       float2 hh[kHalf][2];
@@ -226,7 +225,7 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         for (int i = 0; i < kHalf; ++i) {
           const int r = rw(i);
           const float4 o = ((r & 1) ? op1 : op0)[r * (kBTE / 2)];
-          const float2 Bp = *reinterpret_cast<const float2*>(sB + r * N);
+          const float2 Bp = *reinterpret_cast<const float2*>(sBC + r * (N / 2));
           const float2 dt = make_float2(o.x, o.y), dtx = make_float2(o.z, o.w);
           const float2 e0v = __fmul2_rn(dt, A2[0]), e1v = __fmul2_rn(dt, A2[1]);
           const float2 a0 = make_float2(ex2f(e0v.x), ex2f(e0v.y)), a1 = make_float2(ex2f(e1v.x), ex2f(e1v.y));
@@ -237,14 +236,13 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
       }
       // operands of the reverse walk are fetched two timesteps ahead, so that their trip through the
       // shared-memory pipe overlaps the previous timestep's arithmetic, stores and barrier traffic
-      struct Opnd { float4 o; float2 dy, B, C; };
+      struct Opnd { float4 o; float2 dy; float4 bc; };
       auto fetch = [&](int i) {
         const int rr = rw(i);
         Opnd r;
         r.o = ((rr & 1) ? op1 : op0)[rr * (kBTE / 2)];
         r.dy = *reinterpret_cast<const float2*>(dyp + rr * kBTE);
-        r.B = *reinterpret_cast<const float2*>(sB + rr * N);
-        r.C = *reinterpret_cast<const float2*>(sB + kBtoC + rr * N);
+        r.bc = sBC[rr * (N / 2)];
         return r;
       };
       Opnd nx = fetch(kHalf - 1), nx2 = fetch(kHalf - 2);
@@ -265,8 +263,8 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
           nx = nx2;
           if (i > 1) nx2 = fetch(i - 2);
           const float2 dt = make_float2(cu.o.x, cu.o.y), dtx = make_float2(cu.o.z, cu.o.w), dy2 = cu.dy;
-          const float2 Bv[2] = {make_float2(cu.B.x, cu.B.x), make_float2(cu.B.y, cu.B.y)};
-          const float2 Cv[2] = {make_float2(cu.C.x, cu.C.x), make_float2(cu.C.y, cu.C.y)};
+          const float2 Bv[2] = {make_float2(cu.bc.x, cu.bc.x), make_float2(cu.bc.y, cu.bc.y)};
+          const float2 Cv[2] = {make_float2(cu.bc.z, cu.bc.z), make_float2(cu.bc.w, cu.bc.w)};
           float2 ysum, gBs, wAs;                                            // {channel}
           float dB[2], dC[2];                                               // [state], over the two channels
 #pragma unroll
@@ -389,16 +387,14 @@ sscan_bwd_tma_kernel(const __grid_constant__ BwdMaps maps, const SscanBwdParams 
         *reinterpret_cast<float4*>(dyt + rr * kBTE + cc) = make_float4(dyo[0], dyo[1], dyo[2], dyo[3]);
       }
       const T* rB = reinterpret_cast<const T*>(st + 4 * S::kActBytes);      // B box then C box
-      float* dstB = s_B + buf * kBTile * N;
-      float* dstC = s_C + buf * kBTile * N;
+      float2* dst = reinterpret_cast<float2*>(s_BC + buf * kBTile * (N / 2));
       constexpr int kBcVecs = kBTile * N / 4;                                // 64
 #pragma unroll
       for (int i = 0; i < 2 * kBcVecs / 32; ++i) {
-        const int v = lane + 32 * i;
+        const int v = lane + 32 * i, q = v % kBcVecs;                        // four states of one row of B, then of C
         const Vec4<T> r4 = *reinterpret_cast<const Vec4<T>*>(rB + v * 4);
-        float* dst = (v < kBcVecs) ? dstB + v * 4 : dstC + (v - kBcVecs) * 4;
-        *reinterpret_cast<float4*>(dst) = make_float4(Elem<T>::to_f(r4.v[0]), Elem<T>::to_f(r4.v[1]),
-                                                      Elem<T>::to_f(r4.v[2]), Elem<T>::to_f(r4.v[3]));
+        dst[4 * q + (v >= kBcVecs)] = make_float2(Elem<T>::to_f(r4.v[0]), Elem<T>::to_f(r4.v[1]));
+        dst[4 * q + 2 + (v >= kBcVecs)] = make_float2(Elem<T>::to_f(r4.v[2]), Elem<T>::to_f(r4.v[3]));
       }
       mbar_arrive(&op_full[buf]);
       mbar_arrive(&raw_free[j % kStages]);
