@@ -112,7 +112,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) block_step_kernel(const StepP
   extern __shared__ __align__(16) float s_x[];            // (kB, max(D, W)) float32
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t B = a.B, D = a.D_model, W = a.W, R = a.R, cols = R + 2 * N;
-  const int64_t gwarp = int64_t(blockIdx.x) * kStepWarps + warp, nwarps = int64_t(gridDim.x) * kStepWarps;
+  // Neighbouring rows go to different SMs: a phase with fewer rows than warps, or a few more, then loads all SMs alike, and not the first
+  // third of them.  us a launch, rows in blocks / spread: 76 / 61 at 6 tokens 1024 wide in float32, 20.6 / 13.4 at 3 x 256 in bfloat16,
+  // 172 / 153 at 8 x 2048, 191 / 180 at 1 x 2560 (four layers, bfloat16), 16.1 / 15.2 at 1 x 768.
+  const int64_t gwarp = int64_t(warp) * gridDim.x + blockIdx.x, nwarps = int64_t(gridDim.x) * kStepWarps;
   if (*reinterpret_cast<volatile unsigned*>(&p.bar->poisoned)) {
     if (threadIdx.x == 0) atomicExch(&g_block_step_status, MB200_DEV_WAIT_TIMEOUT);
     return;
@@ -128,7 +131,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) block_step_kernel(const StepP
     s_x[i] = b < B ? Elem<T>::to_f(static_cast<const T*>(a.x)[b * a.x_sb + d]) : 0.f;
   }
   __syncthreads();
-  for (int64_t r = gwarp; r < 2 * W; r += nwarps) {
+  // (with four rows a warp and more every SM is busy, and rows that follow each other in memory stream better: 108.5 / 109.8 at 1 x 2560, float32)
+  const bool many = 2 * W >= 4 * nwarps;
+  for (int64_t r = many ? int64_t(blockIdx.x) * kStepWarps + warp : gwarp; r < 2 * W; r += nwarps) {
     float acc[kB];
 #pragma unroll
     for (int b = 0; b < kB; ++b) acc[b] = 0.f;
@@ -167,7 +172,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) block_step_kernel(const StepP
   if (blockIdx.x == 0 && threadIdx.x == 0) p.bar->count[2] = 0;        // nobody is near the third barrier yet
 
   // ---- 2: x_proj
-  if (int64_t(blockIdx.x) * kStepWarps < cols) stage(p.xc, W);            // CTAs without a row go straight to the barrier
+  if (int64_t(blockIdx.x) < cols) stage(p.xc, W);            // CTAs without a row go straight to the barrier
   for (int64_t r = gwarp; r < cols; r += nwarps) {
     float acc[kB];
 #pragma unroll
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) block_step_kernel(const StepP
   if (blockIdx.x == 0 && threadIdx.x == 0) p.bar->count[0] = p.bar->count[1] = 0;
 
   // ---- 4: out_proj
-  if (int64_t(blockIdx.x) * kStepWarps >= D) return;
+  if (int64_t(blockIdx.x) >= D) return;
   stage(p.y, W);
   for (int64_t r = gwarp; r < D; r += nwarps) {
     float acc[kB];
