@@ -98,10 +98,15 @@ __device__ __forceinline__ float2 softplus_fast2(float2 x) {
   r.y = x.y > 20.f ? x.y : (e.y < 1e-2f ? poly.y : lg.y);
   return r;
 }
+__device__ __forceinline__ float min_nan(float a, float b) {       // a NaN stays one
+  float y;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
 // softplus_fast2 and its derivative, the sigmoid, which shares the exponential.
 __device__ __forceinline__ float2 softplus_sigmoid_fast2(float2 x, float2& sig) {
   const float2 m = __fmul2_rn(x, make_float2(kLog2e, kLog2e));
-  const float2 e = make_float2(ex2f(fminf(m.x, 80.f)), ex2f(fminf(m.y, 80.f)));       // e / (1 + e) must not become inf * 0
+  const float2 e = make_float2(ex2f(min_nan(m.x, 80.f)), ex2f(min_nan(m.y, 80.f)));   // e / (1 + e) must not become inf * 0
   const float2 third = make_float2(-1.f / 3.f, -1.f / 3.f), half = make_float2(0.5f, 0.5f), one = make_float2(1.f, 1.f);
   const float2 nh = make_float2(-1.f, -1.f);
   const float2 inner = __ffma2_rn(e, third, half);

@@ -384,9 +384,10 @@ extern "C" int mb200_conv1d_silu_fwd(const void* x, const float* w, const float*
     const int chunk = kConvChunkFwd[k];
     const int64_t groups = ((L + chunk - 1) / chunk + kConvThreads / 32 - 1) / (kConvThreads / 32);
     const int64_t waves = (cols * groups * B + 3 * sms - 1) / (3 * sms), cost = waves * (chunk + kConvK - 1);
+    if (k == 0 && groups > 65535) return MB200_ETOOBIG;
     if (k == 0 || cost < best) { best = cost; ngroup = groups; longer = k == 1; }
   }
-  if (B > 65535 || ngroup > 65535) return MB200_ETOOBIG;
+  if (B > 65535) return MB200_ETOOBIG;
   const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(ngroup), static_cast<unsigned>(B));
 #define MB200_CONV_FWD(TT, VV) do { \
     if (longer) conv1d_silu_fwd_kernel<TT, VV, kConvChunkFwd[1]><<<grid, kConvThreads, 0, st>>>((const TT*)x, w, bias, (TT*)y, L, ED, x_sb, x_sl, y_sb, y_sl); \

@@ -266,3 +266,31 @@ def test_wide_tiles(dtype, reverse, ED, L):
         assert torch.equal(whole[1], torch.cat([p[1] for p in parts], 1))
         if want:
             assert torch.equal(whole[2], torch.cat([p[2] for p in parts], 3))
+
+
+def test_extreme_delta_in_the_backward():
+    """delta + bias of NaN, -inf, and values whose exponential overflows: the channel with the NaN, and only it, comes out as NaN (from
+    its gradients' first affected timestep on); the others match the derivative of softplus there (0 and 1)."""
+    import mamba_b200
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    L, E = 24, 32
+    x, z, B, C, dy = r(1, L, E), r(1, L, E), r(1, L, 16), r(1, L, 16), r(1, L, E)
+    A, D, bias = -torch.exp(0.1 * r(E, 16)), r(E), r(E) - 4
+    delta = r(1, L, E)
+    delta[0, 10, 3], delta[0, 11, 5], delta[0, 12, 7], delta[0, 13, 9] = float("nan"), -float("inf"), 200.0, 60.0
+    p = [t.requires_grad_() for t in (x, delta)]
+    y = mamba_b200.selective_scan_fn(x, delta, A, B, C, D, z=z, delta_bias=bias)
+    dx, dd = torch.autograd.grad(y, p, dy)
+    others = [e for e in range(E) if e != 3]
+    assert torch.isnan(y[0, 10:, 3]).all() and torch.isfinite(y[0, :, others]).all() and torch.isfinite(y[0, :10, 3]).all()
+    assert torch.isnan(dd[0, :11, 3]).all() and torch.isfinite(dd[0, :, others]).all() and torch.isfinite(dx[0, :, others]).all()
+    assert dd[0, 11, 5] == 0
+    # the derivative of softplus is 1 at 60: an undiscretised delta has the same gradient
+    dt = torch.nn.functional.softplus(delta.detach() + bias)
+    keep = dt.clone()
+    keep[0, 10, 3] = 0.01
+    q = [t.detach().clone().requires_grad_() for t in (x, keep)]
+    y2 = mamba_b200.selective_scan_fn(q[0], q[1], A, B, C, D, z=z)
+    dx2, dd2 = torch.autograd.grad(y2, q, dy)
+    assert torch.allclose(dd[0, 13, 9], dd2[0, 13, 9], rtol=1e-4, atol=1e-5) and torch.allclose(dd[0, 12, 7], dd2[0, 12, 7], rtol=1e-4, atol=1e-5)
