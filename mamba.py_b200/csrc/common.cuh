@@ -55,7 +55,7 @@ __device__ __forceinline__ float ex2f(float x) {       // 2^x on the MUFU pipe
 }
 // Reciprocal and base-2 logarithm straight from the MUFU pipe: __fdividef and __log2f add scaling for results below 2^-126 and
 // arguments below 2^-126, which 1 + e^x never has.  With the packed forms below in the element-wise warps of the fused scans this
-// took their backward from 652 to 619 us (8 x 2048 x 1536, bfloat16; forward now 193 with saved states, 164 without): those warps
+// took their backward from 652 to 619 us (8 x 2048 x 1536, bfloat16): those warps
 // share the issue slots with the recurrences.  (A softplus_fast without its early return costs ssm_step_kernel registers and 4 us of 30.)
 __device__ __forceinline__ float rcpf(float x) {
   float y;

@@ -21,8 +21,8 @@
 //     over 8 products and 3 sums (4 states of a channel), 4 and 3 (2 x 2, with three shuffles) or 2 and 12; and
 //     B and C of a state pair are then short loads of two addresses (side by side, so that the reverse walk takes one),
 //     delta and delta*x 16-byte loads that two lanes share.
-//     44.6 -> 33.9 wavefronts per 128 elements and 610 -> 544 us on 8 x 2048 x 1536 in bfloat16, together with
-//     what follows; without the shuffles (twice the sums to write and to read) 587.
+//     44.6 -> 34.8 wavefronts per 128 elements and 610 -> 544 us on 8 x 2048 x 1536 in bfloat16, together with
+//     what follows (526 with index arithmetic out of the loops); without the shuffles (twice the sums) 587.
 //   - warps 5 and 7 finish alternate windows: sum the 4 partials of each channel, form dx, ddelta,
 //     dz (and the running sums for dD and d(delta_bias)), store them.  delta, dy' and the derivatives of
 //     softplus and silu come from the operand tile: the converter has their exponentials in hand, and these

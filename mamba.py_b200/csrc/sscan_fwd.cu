@@ -4,8 +4,8 @@
 //
 // What bounds it.  Per (b, t, e, n) element the kernel needs one ex2 (16/clk/SM on the MUFU
 // pipe), four FP32 operations, and its B and C operands out of shared memory; HBM traffic is
-// 0.5 byte per element.  Measured on B200 no single unit is the limit (shared-memory pipe ~75 %, issue
-// ~65 %, FMA ~40 %, MUFU ~38 %, DRAM ~20 %): the time is that of the in-order recurrence warps, whose
+// 0.5 byte per element.  Measured on B200 no single unit is the limit (shared-memory pipe 82 %, issue
+// 65 %, FMA 46 %, MUFU 46 %, DRAM ~24 %; the first two above 90 % and 75 % on SMs with three CTAs): the time is that of the in-order recurrence warps, whose
 // dependent chain only overlaps with the other resident warps.  So: no redundant arithmetic (every
 // recurrence is walked serially along L by exactly one thread), everything that is not the recurrence
 // (softplus, delta*x, D skip, gate, conversions: 70 % as many instructions again) runs on other warps,
