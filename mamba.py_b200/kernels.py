@@ -86,6 +86,18 @@ def sscan_fwd_raw(x, delta, A, Bm, Cm, D, z=None, delta_bias=None, h0=None,
     return y, hT, carries
 
 
+def _states_order(carries, Bsz, chunks, ED, N):
+    """Flag for the order of the saved states, which their shape tells: two by two, as `sscan_fwd_raw` saves them, or the
+    (ED, N) entries of the C ABI's default."""
+    if carries.dtype == torch.float32 and carries.is_contiguous():
+        if carries.shape == (Bsz, chunks, N // 2, ED, 2):
+            return _lib.PAIRED_STATES
+        if carries.shape == (Bsz, chunks, ED, N):
+            return 0
+    raise ValueError(f"saved states must be contiguous float32 of shape {(Bsz, chunks, N // 2, ED, 2)} or {(Bsz, chunks, ED, N)}, "
+                     f"got {carries.dtype} {tuple(carries.shape)}")
+
+
 def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None, want_g_out=False,
                   reverse=False, general_decay=False, out_dz=None):
     """Launch the fused backward.  Returns (dx, ddelta, dz, dB, dC, dA, dD, dbias, g_out).
@@ -94,6 +106,8 @@ def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None,
     lib = _lib.load()
     Bsz, L, ED = x.shape
     N = A.shape[1]
+    chunk = lib.mb200_sscan_chunk()
+    order = _states_order(carries, Bsz, (L + chunk - 1) // chunk, ED, N)
     dev = x.device
     dx = torch.empty((Bsz, L, ED), dtype=x.dtype, device=dev)
     dd = torch.empty_like(dx)
@@ -109,7 +123,7 @@ def sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, delta_bias, dy, carries, g_in=None,
     dbias = acc[2 * nBC + nA + ED:] if delta_bias is not None else None
     g_out = torch.empty((Bsz, ED, N), dtype=torch.float32, device=dev) if want_g_out else None
     flags = ((_lib.DELTA_SOFTPLUS if delta_bias is not None else 0) | (_lib.REVERSE if reverse else 0)
-             | (_lib.GENERAL_DECAY if general_decay else 0) | _lib.PAIRED_STATES)
+             | (_lib.GENERAL_DECAY if general_decay else 0) | order)
     zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
     dzs = (dz.stride(0), dz.stride(1)) if dz is not None else (0, 0)
     with torch.cuda.device(dev):

@@ -147,3 +147,12 @@ def test_conversions_of_one_launch_are_bounded():
     _lib.host().selftest_queue_conversions(24)
     with pytest.raises(RuntimeError, match="more than 24 conversions"):
         _lib.host().selftest_queue_conversions(25)
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 8, 8, 2), (1, 1, 16, 16), (1, 2, 16, 8), (2, 2, 16, 16)])
+def test_saved_states_of_another_shape_are_refused(shape):
+    """Neither (B, chunks, N/2, ED, 2) nor (B, chunks, ED, N), here (1, 2, 8, 16, 2) and (1, 2, 16, 16): refused before anything else."""
+    from mamba_b200.kernels import sscan_bwd_raw
+    t, s = torch.zeros(1, 9, 16), torch.zeros(1, 9, 16)
+    with pytest.raises(ValueError, match="saved states"):
+        sscan_bwd_raw(t, t, torch.zeros(16, 16), s, s, None, None, None, t, torch.zeros(shape))

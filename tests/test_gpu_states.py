@@ -58,3 +58,24 @@ def test_both_orders_agree(E, stride, N, reverse, L):
             assert torch.equal(a, b), name
         else:                       # float atomics: at most 90 terms in another order, each sum good to 90 * 2^-24 of its largest
             assert_close(a, b, 1e-5, 1e-5 * max(1.0, b.abs().max().item()))
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+def test_raw_backward_takes_both_orders(reverse):
+    """States of either order, told apart by their shape, give the same gradients through the raw launchers."""
+    from mamba_b200.kernels import sscan_bwd_raw, sscan_fwd_raw
+    g = torch.Generator().manual_seed(2)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    B, L, E, N = 2, 37, 40, 16
+    x, z, dy, Bm, Cm, D = r(B, L, E), r(B, L, E), r(B, L, E), r(B, L, N), r(B, L, N), r(E)
+    delta, A = torch.nn.functional.softplus(r(B, L, E) - 3), -torch.exp(r(E, N))
+    paired = sscan_fwd_raw(x, delta, A, Bm, Cm, D, z, want_carries=True, reverse=reverse)[2]
+    plain = paired.permute(0, 1, 3, 2, 4).reshape(B, -1, E, N).contiguous()
+    want, got = (sscan_bwd_raw(x, delta, A, Bm, Cm, D, z, None, dy, c, reverse=reverse) for c in (paired, plain))
+    for i, (a, b) in enumerate(zip(got, want)):
+        if a is None:
+            continue
+        if i < 3:
+            assert torch.equal(a, b)
+        else:                       # float atomics, as above: at most 2 * 37 terms in another order
+            assert_close(a, b, 1e-5, 1e-5 * max(1.0, b.abs().max().item()))
