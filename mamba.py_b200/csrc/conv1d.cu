@@ -140,8 +140,8 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
 #pragma unroll
     for (int i = 0; i < P; ++i) win[i][k] = xv[i];
   }
-  // Whole chunks (all but a row's last) test nothing (28.1 -> 25.4 us, see above, together with moving pointers); their loop is fully unrolled, so that the compiler hoists the loads of later
-  // groups over the arithmetic of earlier ones.
+  // Whole chunks (all but a row's last) test nothing; their loop is fully unrolled, so that the compiler hoists the loads of later
+  // groups over the arithmetic of earlier ones (28.1 -> 25.4 us, see above, together with moving pointers).
   auto group = [&](auto whole, int left) {
     CVec<T, V> v[kConvGroup];
 #pragma unroll
@@ -167,13 +167,19 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     }
   };
   const int left = int(min64(L - t0, kChunkLen));
-  if (left == kChunkLen) {
+  // A row's last chunk takes 1, 2, 4 or (of 64 steps) 8 groups with bounds, unrolled as well.  One group at a time leaves 8 rows in
+  // flight and always all of them issues loads that read nothing; us so / so / by what is left, bfloat16: 64 x 31 x 1536
+  // 10.1 / 6.5 / 6.2, 64 x 7 x 1536 4.3 / 6.0 / 3.5, 64 x 127 x 768 9.1 / 7.6 / 7.5, 8 x 2041 x 1536 27.0 / 23.6 / 22.3.
+  auto groups = [&](auto count, auto whole) {
 #pragma unroll
-    for (int g = 0; g < kChunkLen / kConvGroup; ++g) group(std::true_type{}, 0);
-  } else {
-#pragma unroll 1
-    for (int g = 0; g < left; g += kConvGroup) group(std::false_type{}, left - g);
-  }
+    for (int g = 0; g < decltype(count)::value; ++g) group(whole, left - g * kConvGroup);
+  };
+  using All = std::integral_constant<int, kChunkLen / kConvGroup>;
+  if (left == kChunkLen) groups(All{}, std::true_type{});
+  else if (left <= kConvGroup) groups(std::integral_constant<int, 1>{}, std::false_type{});
+  else if (left <= 2 * kConvGroup) groups(std::integral_constant<int, 2>{}, std::false_type{});
+  else if (kChunkLen == 4 * kConvGroup || left <= 4 * kConvGroup) groups(std::integral_constant<int, 4>{}, std::false_type{});
+  else groups(All{}, std::false_type{});
 }
 
 // dx[t] = sum_k w[k] * dpre[t+3-k];  dw[k] = sum_{b,t} dpre[t] * x[t-3+k];  dbias = sum dpre;
