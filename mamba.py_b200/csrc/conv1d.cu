@@ -167,9 +167,10 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     }
   };
   const int left = int(min64(L - t0, kChunkLen));
-  // A row's last chunk takes 1, 2, 4 or (of 64 steps) 8 groups with bounds, unrolled as well.  One group at a time leaves 8 rows in
+  // A row's last chunk takes 1, 2, 4 or (of 64 steps) 6 or 8 groups with bounds, unrolled as well.  One group at a time leaves 8 rows in
   // flight and always all of them issues loads that read nothing; us so / so / by what is left, bfloat16: 64 x 31 x 1536
-  // 10.1 / 6.5 / 6.2, 64 x 7 x 1536 4.3 / 6.0 / 3.5, 64 x 127 x 768 9.1 / 7.6 / 7.5, 8 x 2041 x 1536 27.0 / 23.6 / 22.3.
+  // 10.1 / 6.5 / 6.2, 64 x 7 x 1536 4.3 / 6.0 / 3.5, 64 x 127 x 768 9.1 / 7.6 / 7.5, 8 x 2041 x 1536 27.0 / 23.6 / 22.3.  (33 to 48 steps in 8 groups
+  // instead of 6: 23 x 289 x 378 5.1 us for 4.3.)
   auto groups = [&](auto count, auto whole) {
 #pragma unroll
     for (int g = 0; g < decltype(count)::value; ++g) group(whole, left - g * kConvGroup);
@@ -179,6 +180,7 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
   else if (left <= kConvGroup) groups(std::integral_constant<int, 1>{}, std::false_type{});
   else if (left <= 2 * kConvGroup) groups(std::integral_constant<int, 2>{}, std::false_type{});
   else if (kChunkLen == 4 * kConvGroup || left <= 4 * kConvGroup) groups(std::integral_constant<int, 4>{}, std::false_type{});
+  else if (left <= 6 * kConvGroup) groups(std::integral_constant<int, 6>{}, std::false_type{});
   else groups(All{}, std::false_type{});
 }
 
