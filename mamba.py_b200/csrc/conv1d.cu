@@ -23,8 +23,12 @@ namespace {
 
 constexpr int kConvK = 4;
 constexpr int kConvThreads = 256;
-// Forward chunks (compile time: the loop over one is fully unrolled), the one whose waves of CTAs are shorter: 8 x 2048 x 1536 in
-// bfloat16 is one wave of 64 steps (22.9 us) or two of 32 (25.4), 64 x 197 x 384 one of either (9.2 / 9.0).
+// Forward chunks (compile time: the loop over one is fully unrolled).  The longer one saves halo and CTAs, the shorter one has half
+// the latency, so 64 steps are taken where they put fewer CTAs on the busiest SM (beyond the three that an SM holds, in whole waves)
+// and fewer steps, added over its warps that have a chunk.  us with 32 / 64 steps, bfloat16: 8 x 300 x 1536 (2 CTAs or 1, which has 5
+// warps with work) 8.9 / 7.5, 42 x 265 x 512 (3 / 2) 12.7 / 9.1, 4 x 777 x 2048 (2 / 1) 9.1 / 8.2, 8 x 2048 x 1536 (6 / 3) 23.4 / 22.5, but
+// 8 x 1003 x 1536 (3 / 2) 12.8 / 14.0, 64 x 197 x 384 (2 / 2) 8.8 / 8.3, 1 x 98 x 512 (1 / 1) 3.8 / 5.4.  Over 100 shapes of 33 to 8192
+// steps, both types, this takes 0.3 % longer than the better one on average and 10 % at most (by waves of CTAs alone 2.3 and 43).
 constexpr int kConvChunkFwd[2] = {32, 64};
 // Timesteps whose loads are in flight together.  Forward 8 (with 3 CTAs of 256 threads per SM): 29.5 us on the 130m layer
 // against 33.8 for 4.  Backward 4 (with 4 CTAs of 128 threads): 60 us; 6 and 8 need more registers than 16 warps per SM leave
@@ -386,14 +390,18 @@ extern "C" int mb200_conv1d_silu_fwd(const void* x, const float* w, const float*
   const int64_t cols = (ED + 32 * int64_t(v) - 1) / (32 * int64_t(v));
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t ngroup = 0, best = 0;
+  int64_t ngroup = 0, best = 0, best_rounds = 0;
   bool longer = false;
   for (int k = 0; k < 2; ++k) {
-    const int chunk = kConvChunkFwd[k];
-    const int64_t groups = ((L + chunk - 1) / chunk + kConvThreads / 32 - 1) / (kConvThreads / 32);
-    const int64_t waves = (cols * groups * B + 3 * sms - 1) / (3 * sms), cost = waves * (chunk + kConvK - 1);
+    constexpr int64_t kWarps = kConvThreads / 32, kResident = 3;
+    const int64_t chunk = kConvChunkFwd[k], chunks = (L + chunk - 1) / chunk, groups = (chunks + kWarps - 1) / kWarps;
     if (k == 0 && groups > 65535) return MB200_ETOOBIG;
-    if (k == 0 || cost < best) { best = cost; ngroup = groups; longer = k == 1; }
+    const int64_t ctas = cols * groups * B, per_sm = (ctas + sms - 1) / sms, full = min64(chunks, kWarps);
+    const int64_t rounds = per_sm <= kResident ? per_sm : (per_sm + kResident - 1) / kResident * kResident;
+    // in a last round of no more than `cols` CTAs all are a row's last
+    const int64_t last = rounds == per_sm && ctas - (rounds - 1) * sms <= cols ? chunks - (groups - 1) * kWarps : full;
+    const int64_t cost = ((rounds - 1) * full + last) * (chunk + kConvK - 1);
+    if (k == 0 || (rounds < best_rounds && cost < best)) { best = cost; best_rounds = rounds; ngroup = groups; longer = k == 1; }
   }
   if (B > 65535) return MB200_ETOOBIG;
   const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(ngroup), static_cast<unsigned>(B));

@@ -68,11 +68,11 @@ def test_wide_bfloat16_backward(Bsz, L, ED):
 
 @pytest.mark.parametrize("Bsz,L,ED", [(8, 2048, 1536), (8, 2041, 1536), (8, 1985, 1540), (4, 31, 2052)]
                          + [(8, 1984 + left, 1536) for left in (8, 9, 16, 17, 32, 33, 63)]
-                         + [(2, L, ED) for L in (1, 8, 9, 16, 17, 31, 32, 33, 41, 49, 63) for ED in (132, 33)])
+                         + [(2, L, ED) for L in (1, 8, 9, 16, 17, 31, 32, 33, 41, 49, 63) for ED in (132, 33)] + [(150, 300, 132), (150, 300, 33)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_forward_chunks(Bsz, L, ED, dtype):
     """Chunks of 64 (one wave of CTAs), whole, a step short, and with last ones at both ends of every number of groups; chunks of 32
-    the same, four channels a thread and one."""
+    the same, four channels a thread and one.  (150 rows of 300 steps: 64-step chunks for five of a CTA's eight warps.)"""
     import mamba_b200
     g = torch.Generator(device="cuda").manual_seed(L)
     new = lambda *s: torch.randn(*s, generator=g, device="cuda")
