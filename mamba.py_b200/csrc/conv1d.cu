@@ -190,13 +190,19 @@ conv1d_silu_fwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
 
 // dx[t] = sum_k w[k] * dpre[t+3-k];  dw[k] = sum_{b,t} dpre[t] * x[t-3+k];  dbias = sum dpre;
 // dpre[t] = dy[t] * silu'(pre[t]),  pre recomputed from x.
-// kAhead: the next group's loads are in flight during a group's arithmetic.
-template <typename T, int V, bool kAhead>
+// kLong: chunks long enough to pay for code of their own, which short ones spend more time fetching than running.
+//   bfloat16, four channels: the next group's loads are in flight during a group's arithmetic (kAhead), and groups inside the chunk
+//   test nothing (kWhole): 8 x 2048 x 1536 41.8 -> 37.7 us, 64 x 1024 x 2048 207 -> 177 against neither; with the loop unrolled by two
+//   instead of handing the loaded group on, 72 bytes spilled and 41.6 and 202.  One channel a thread has kWhole alone (84.6 -> 83.2).
+//   float32, four channels, has no registers for loads ahead (70 us for 56) and no use for kWhole: whole loads without bounds alone.
+// Short ones without any of it: 64 x 31 x 1536 16.0 -> 15.0 us in bfloat16, 17.0 -> 15.4 in float32.
+template <typename T, int V, bool kLong>
 __global__ void __launch_bounds__(kConvBwdThreads, 4)
 conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                        const T* __restrict__ dy, T* __restrict__ dx, float* __restrict__ dw,
                        float* __restrict__ dbias, int64_t L, int64_t ED, int64_t x_sb, int64_t x_sl,
                        int64_t dy_sb, int64_t dy_sl, int64_t dx_sb, int64_t dx_sl, int chunk) {
+  constexpr bool kAhead = kLong && sizeof(T) == 2 && V > 1, kWhole = kLong && (sizeof(T) == 2 || V == 1);
   __shared__ float s_acc[32 * V * (kConvK + 1)];          // per channel of the CTA: dw[0..3], dbias
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < 32 * V * (kConvK + 1); i += kConvBwdThreads) s_acc[i] = 0.f;
@@ -246,7 +252,7 @@ conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
     // outputs: their own dx, dw belong to the next chunk.  (x, dy read as 0 past the end of the row.)
     const int own = int(t1 - t0), end = int(min64(L, t1 + kH) - t0);
     auto fetch = [&](int s0, Group& q) {
-      if (s0 + kG <= end) {
+      if (kLong && !kAhead && s0 + kG <= end) {
 #pragma unroll
         for (int j = 0; j < kG; ++j) {
           q.x[j] = cload<T, V>(xg, true);
@@ -295,18 +301,17 @@ conv1d_silu_bwd_kernel(const T* __restrict__ x, const float* __restrict__ w, con
       }
     };
     auto run = [&](int s0, const Group& q) {
-      if (s0 >= kH && s0 + kG <= own) group(std::true_type{}, s0, q);
+      if (kWhole && s0 >= kH && s0 + kG <= own) group(std::true_type{}, s0, q);
       else group(std::false_type{}, s0, q);
     };
-    if constexpr (kAhead) {                                // two groups of loads in turn, one of them in flight
-      Group q0, q1;
-      fetch(0, q0);
+    if constexpr (kAhead) {
+      Group q, next;
+      fetch(0, q);
 #pragma unroll 1
-      for (int s0 = 0; s0 < own + kH; s0 += 2 * kG) {
-        fetch(s0 + kG, q1);
-        run(s0, q0);
-        fetch(s0 + 2 * kG, q0);
-        run(s0 + kG, q1);
+      for (int s0 = 0; s0 < own + kH; s0 += kG) {
+        fetch(s0 + kG, next);
+        run(s0, q);
+        q = next;
       }
     } else {
 #pragma unroll 1
@@ -434,14 +439,15 @@ extern "C" int mb200_conv1d_silu_bwd(const void* x, const float* w, const float*
   const int64_t ngroup = (nchunk + kConvBwdThreads / 32 - 1) / (kConvBwdThreads / 32);
   if (B > 65535 || ngroup > 65535) return MB200_ETOOBIG;
   const dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>(ngroup), static_cast<unsigned>(B));
-#define MB200_CONV_BWD(TT, VV, AHEAD)                                                                          \
-  conv1d_silu_bwd_kernel<TT, VV, AHEAD><<<grid, kConvBwdThreads, 0, st>>>((const TT*)x, w, bias, (const TT*)dy, \
-      (TT*)dx, dw, dbias, L, ED, x_sb, x_sl, dy_sb, dy_sl, dx_sb, dx_sl, chunk)
-  if (dtype == MB200_F32) { if (vec) MB200_CONV_BWD(float, 4, false); else MB200_CONV_BWD(float, 1, false); }
-  // Long chunks gain from loads a group ahead: 56 -> 49.5 us at 8 x 2048 x 1536 (chunks of 88), 103 -> 83.5 at 4 x 2048 x 5120.  Short
-  // ones are over too soon: 16.7 -> 18.7 us at 64 x 197 x 384 (chunks of 20).  float32 has no registers for it (70 us with 3 CTAs per SM, 63 without).
-  else if (vec && chunk >= 48) MB200_CONV_BWD(__nv_bfloat16, 4, true);
-  else { if (vec) MB200_CONV_BWD(__nv_bfloat16, 4, false); else MB200_CONV_BWD(__nv_bfloat16, 1, false); }
+#define MB200_CONV_BWD(TT, VV) do { \
+    if (longer) conv1d_silu_bwd_kernel<TT, VV, true><<<grid, kConvBwdThreads, 0, st>>>((const TT*)x, w, bias, (const TT*)dy, (TT*)dx, dw, dbias, L, ED, x_sb, x_sl, dy_sb, dy_sl, dx_sb, dx_sl, chunk); \
+    else conv1d_silu_bwd_kernel<TT, VV, false><<<grid, kConvBwdThreads, 0, st>>>((const TT*)x, w, bias, (const TT*)dy, (TT*)dx, dw, dbias, L, ED, x_sb, x_sl, dy_sb, dy_sl, dx_sb, dx_sl, chunk); \
+  } while (0)
+  // us as a short / long chunk: bfloat16 20.0 / 20.9 at 8 x 900 x 1536 (chunks of 40), 21.9 / 22.1 at 8 x 1003 x 1536 (44), 26.4 / 25.1 at
+  // 8 x 1200 x 1536 (52); float32 24.0 / 25.2 at 64 x 127 x 768 (24), 24.8 / 23.4 at 1 x 1777 x 5120 (32), 34.6 / 31.4 at 8 x 1003 x 1536 (44).
+  const bool longer = chunk >= (dtype == MB200_F32 ? 32 : 48);
+  if (dtype == MB200_F32) { if (vec) MB200_CONV_BWD(float, 4); else MB200_CONV_BWD(float, 1); }
+  else { if (vec) MB200_CONV_BWD(__nv_bfloat16, 4); else MB200_CONV_BWD(__nv_bfloat16, 1); }
 #undef MB200_CONV_BWD
   return check_launch();
 }

@@ -66,6 +66,23 @@ def test_wide_bfloat16_backward(Bsz, L, ED):
         assert ((a.float() - r).norm() / r.norm()).item() < 5e-3
 
 
+@pytest.mark.parametrize("Bsz,L,ED", [(64, 301, 772), (64, 301, 195), (64, 197, 772), (64, 31, 132), (64, 31, 131), (3, 1003, 516)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_backward_chunks(Bsz, L, ED, dtype):
+    """Long chunks (64 steps in the first two) and short ones, four channels a thread and one, against float64.  float32: two factors of every term come from a
+    sigmoid good to 1e-5; bfloat16: dx is rounded to 2^-9."""
+    import mamba_b200
+    g = torch.Generator(device="cuda").manual_seed(L + ED)
+    new = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, dy, w, b = new(Bsz, L, ED).to(dtype).requires_grad_(), new(Bsz, L, ED).to(dtype), new(ED, 1, 4).requires_grad_(), new(ED).requires_grad_()
+    got = torch.autograd.grad(mamba_b200.mamba.causal_conv1d_silu(x, w, b), (x, w, b), dy)
+    x64, w64, b64 = (t.detach().double().requires_grad_() for t in (x, w, b))
+    xp = F.pad(x64, (0, 0, 3, 0))
+    y = F.silu(sum(xp[:, k:k + L] * w64[:, 0, k] for k in range(4)) + b64)
+    for a, r in zip(got, torch.autograd.grad(y, (x64, w64, b64), dy.double())):
+        assert ((a.double() - r).norm() / r.norm()).item() < (3e-3 if dtype == torch.bfloat16 else 2e-5)
+
+
 @pytest.mark.parametrize("Bsz,L,ED", [(8, 2048, 1536), (8, 2041, 1536), (8, 1985, 1540), (4, 31, 2052)]
                          + [(8, 1984 + left, 1536) for left in (8, 9, 16, 17, 32, 33, 63)]
                          + [(2, L, ED) for L in (1, 8, 9, 16, 17, 31, 32, 33, 41, 49, 63) for ED in (132, 33)] + [(150, 300, 132), (150, 300, 33)])
