@@ -154,7 +154,9 @@ __device__ __forceinline__ bool s4d_structured(const float* a4, float a0, int q)
 // converter forms dy' = dy * silu(z) instead of delta * x, and the recurrence multiplies by the decay
 // after adding the input.  It has no y and saves no states; the result leaves through hT.
 // kHasY = false is the pass that only wants states (no C-contraction, no epilogue).  kSave: the states entering the chunks go to
-// p.carries (a template parameter because the test alone costs the recurrence warps 2 % of a prompt).
+// p.carries (a template parameter because the test alone costs the recurrence warps 3 % of a prompt and 4 to 14 % of a carry pass:
+// 78.3 -> 80.9 us for 2048 steps of one CTA per SM, 52.7 -> 59.9 for 23 of 24 pieces of 53013 x 64).  Without y and kSave it is a carry pass,
+// which returns every piece's state; without y but with kSave a scan, which returns a row's last and saves states if there is p.carries.
 template <typename T, int N, bool kRev, bool kCarry, bool kHasY, bool kSave, bool kWide = false>
 __global__ void __launch_bounds__(FwdGeom<N, kWide>::kThreads, FwdGeom<N, kWide>::kOcc)
 sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams p) {
@@ -183,7 +185,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
   const int64_t slot = b * p.pieces + pc;
   const int cols_ok = int(min64(kTE, p.ED - e0));
   const bool softplus = (p.flags & MB200_DELTA_SOFTPLUS) != 0;
-  constexpr bool has_y = kHasY;
+  constexpr bool has_y = kHasY, kEvery = !kHasY && !kSave;
   const bool has_z = p.z != nullptr;
   const int ntiles = (t_hi - t_lo + kTile - 1) / kTile;
   // Direction.  With MB200_REVERSE time is walked from L-1 down to 0: processing tile kt is the
@@ -258,7 +260,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     // The pass that only wants states (the carry pass of a split sequence) also returns the decay product of
     // the whole span, exp(A * sum_t delta[t]): the sum costs one add per timestep here, and a pass of its own
     // over delta otherwise.
-    constexpr bool kWantP = !kHasY && !kCarry;
+    constexpr bool kWantP = kEvery && !kCarry;
     float dsum[kCPT], dcomp[kCPT];
 #pragma unroll
     for (int i = 0; i < kCPT; ++i) dsum[i] = dcomp[i] = 0.f;
@@ -317,7 +319,7 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
         for (int t = 0; t < kDecayAhead; ++t) rd[t] = prepare(ld[t]);
 #pragma unroll
         for (int t = 0; t < kTile; ++t) {
-          if (kSave && t % kChunk == 0) {                                   // state entering this chunk
+          if (kSave && t % kChunk == 0 && (kHasY || p.carries)) {            // state entering this chunk
             if (t0a + (rev ? kChunk - t : t) < p.L) {
 #pragma unroll
               for (int i = 0; i < kCPT; ++i) {
@@ -391,11 +393,11 @@ sscan_fwd_tma_kernel(const __grid_constant__ FwdMaps maps, const SscanFwdParams 
     const bool ok = structured ? run_tiles(std::true_type{}) : run_tiles(std::false_type{});
     if (!ok) return;
     // the scan itself returns the state that leaves its last piece, the carry passes every piece's
-    if (p.hT && (!kHasY || pc == (rev ? 0 : p.pieces - 1))) {
+    if (p.hT && (kEvery || pc == (rev ? 0 : p.pieces - 1))) {
 #pragma unroll
       for (int i = 0; i < kCPT; ++i)
         if (e_ok[i])
-          *reinterpret_cast<float4*>(p.hT + ((kHasY ? b : slot) * p.ED + e0 + e_l + i) * N + 4 * q) =
+          *reinterpret_cast<float4*>(p.hT + ((kEvery ? slot : b) * p.ED + e0 + e_l + i) * N + 4 * q) =
               make_float4(hlo[i].x, hlo[i].y, hhi[i].x, hhi[i].y);
     }
     if constexpr (kWantP) {
@@ -605,7 +607,7 @@ int tma_launch_tile(const SscanFwdParams& p, cudaStream_t st) {
   else if (ok) m.z = m.x;
   if (!ok) return 1;                                   // caller falls back to the generic path
   const bool rv = (p.flags & MB200_REVERSE) != 0, hy = p.y != nullptr;
-  const bool sv = p.carries != nullptr;
+  const bool sv = p.carries != nullptr || (!hy && !p.pT && p.pieces > 1);
   void (*k)(const FwdMaps, const SscanFwdParams) = nullptr;
   if constexpr (!kWide) {
     if (p.flags & kFlagCarryPass) k = sscan_fwd_tma_kernel<T, N, true, true, false, false>;

@@ -43,6 +43,10 @@ def test_uneven_pieces_vs_oracle(Bsz, L, ED, pieces, dtype, monkeypatch):
     fold = lambda a, b, o, rev: lib.mb200_carry_fold_range(p(a), p(b), None, p(o), Bsz, pieces, ED * 16, 0, pieces, rev, st)
     assert fold(P, S, h_in, 0) == 0
     call("mb200_sscan_fwd_pieces", [x, d, z, A, Bm, Cm, D, None, h_in, y, hT, car], ss(x, d, z, Bm, Cm, y))
+    for saved in (None, torch.zeros_like(car)):                         # without y too: one state a row, and nothing behind them
+        last = torch.full((Bsz * pieces, ED, 16), 7.0, device=DEV)
+        call("mb200_sscan_fwd_pieces", [x, d, z, A, Bm, Cm, D, None, h_in, None, last, saved], ss(x, d, z, Bm, Cm, y))
+        assert torch.equal(last[:Bsz], hT) and (last[Bsz:] == 7.0).all() and (saved is None or torch.equal(saved, car))
     call("mb200_sscan_bwd_carry_pieces", [d, z, gy, Cm, A, None, G], ss(d, z, gy, Cm))
     assert fold(P, G, g_in, 1) == 0
     dx, dd, dz = (new(Bsz, L, ED, dt=dtype) for _ in range(3))
