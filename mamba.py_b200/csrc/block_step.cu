@@ -251,13 +251,10 @@ int block_step_launch(StepParams& p, cudaStream_t st) {
   auto k = block_step_kernel<T, N, kB>;
   const int64_t len = p.a.D_model > p.a.W ? p.a.D_model : p.a.W;
   const int smem = int(kB * len * 4);
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return MB200_ELAUNCH;
   // 48 KB are there without asking, for the kernel's own few static bytes (a barrier's answer) as well
   if (smem > 47 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return MB200_ELAUNCH;
   void* args[] = {&p};
-  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(unsigned(sms)), dim3(kStepThreads), args, size_t(smem), st) ==
+  if (cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k), dim3(unsigned(sm_count())), dim3(kStepThreads), args, size_t(smem), st) ==
       cudaSuccess)
     return MB200_OK;
   (void)cudaGetLastError();                              // not for the next launch to find

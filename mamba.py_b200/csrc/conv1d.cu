@@ -356,9 +356,7 @@ using namespace mb200;
 // Chunk length (multiple of 4 in [16, 256]) that minimises waves x (chunk + halo): `cols` warps per
 // (row, chunk), `warps_per_sm` resident warps per SM.
 static int pick_conv_chunk(int64_t B, int64_t L, int64_t cols, int warps_per_sm) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const double cap = double(sms) * warps_per_sm;
+  const double cap = double(sm_count()) * warps_per_sm;
   int best = 32;
   double best_cost = 1e300;
   for (int c = 16; c <= 256; c += 4) {
@@ -393,8 +391,7 @@ extern "C" int mb200_conv1d_silu_fwd(const void* x, const float* w, const float*
   const bool vec = conv_vec_ok(ED, kv, {x, y}, {x_sb, x_sl, y_sb, y_sl});
   const int v = vec ? kv : 1;
   const int64_t cols = (ED + 32 * int64_t(v) - 1) / (32 * int64_t(v));
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t sms = sm_count();
   int64_t ngroup = 0, best = 0, best_rounds = 0;
   bool longer = false;
   for (int k = 0; k < 2; ++k) {

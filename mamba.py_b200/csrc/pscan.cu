@@ -502,13 +502,6 @@ pscan_cta_bwd_kernel(const T* __restrict__ A, const T* __restrict__ H, const T* 
   }
 }
 
-int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Serial threads when they fill the GPU by themselves (256 per SM: enough loads in flight).  Otherwise a CTA per 16 channels of a row,
 // as long as a row is a few rounds of such a CTA or there are CTAs enough for several on every SM (at 2 per SM, 1 x 8192 x 5120,
 // the backward lost 213 -> 230 us to the second wave); what is left, few channels and a long row, is cut into segments.

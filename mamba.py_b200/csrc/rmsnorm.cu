@@ -406,12 +406,6 @@ norm_rows_bwd_kernel(const TR* __restrict__ s, const float* __restrict__ w, cons
   }
 }
 
-int sm_count() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Runs go(threads per row, chunks) with the smallest row layout that holds D columns; false: D needs the row-by-row kernels.
 template <int kTPR, int kC> struct RowLayout {};
 template <typename F> bool with_row_layout(int64_t D, F&& go) {

@@ -628,10 +628,8 @@ int tma_launch_tile(const SscanFwdParams& p, cudaStream_t st) {
 template <typename T, int N>
 int tma_launch_n(const SscanFwdParams& p, cudaStream_t st) {
   if constexpr (N == 16) {
-    int dev = 0, sms = 0;
-    if (p.y && !(p.flags & kFlagCarryPass) && cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
-      const int64_t rows = p.B * p.launch_pieces, narrow = FwdGeom<N>::kTE, wide = FwdGeom<N, true>::kTE;
+    if (p.y && !(p.flags & kFlagCarryPass)) {
+      const int64_t sms = sm_count(), rows = p.B * p.launch_pieces, narrow = FwdGeom<N>::kTE, wide = FwdGeom<N, true>::kTE;
       if (rows * ((p.ED + narrow - 1) / narrow) > sms && rows * ((p.ED + wide - 1) / wide) <= sms) return tma_launch_tile<T, N, true>(p, st);
     }
   }
