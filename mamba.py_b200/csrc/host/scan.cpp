@@ -195,17 +195,17 @@ struct ScanBackward : public torch::autograd::Node {
 
 // How many pieces to cut each row into, from a model of the time: the fused kernels have batch * ceil(width / 32) independent
 // work items a piece (a CTA owns one, three fit an SM), and one CTA alone on an SM runs much faster than one of three.
-// Measured with the kernels of the time, us for 2048 timesteps with 1 / 2 / 3 CTAs on every SM of 148, means of both types and of A as initialised and as trained:
-// forward 85 / 127 / 185 (80 / 119 / 166 without saved states and with A as initialised, 90 / 138 / 206 the other way round), backward
-// 315 / 456 / 636, forward carry pass 65 / 96 / 134, reverse one 71 / 104 / 146; of these, filling the pipeline takes as long as some
-// 10 timesteps.  A carry pass and a fold add 4 us of launches on the GPU and 12 of host time, which is what short calls wait for.  Over
-// 140 cases of 960 to 7680 steps (1 to 32 rows 64 to 5120 wide, both types, training and inference) the count picked takes 0.4 % longer
-// than the best one on average and 5.8 % at most.  The kernels have become faster since (forward 84 / 125 / 175, 107 with one 48-channel
-// CTA on every SM; backward 287 / 387 / 530; carry passes 57 / 88 / 126 and 64 / 95 / 136), nearly in proportion: over 44 cases of 3840
-// steps the picks cost 1.5 % with the old times and 1.7 % with these, so the old ones stay.
+// Measured, us for 2048 timesteps with 1 / 2 / 3 CTAs on every SM of 148, means of both types and of A as initialised and as trained:
+// forward 82 / 123 / 174 with saved states, 79 / 121 / 170 without (81 / 119 / 169 and 79 / 116 / 164 for A as initialised, 82 / 126 / 179 and
+// 80 / 125 / 177 as trained), 112 and 105 with one 48-channel CTA on every SM; backward 279 / 378 / 538; forward carry pass 55 / 87 / 125
+// (49 / 78 / 110, 60 / 96 / 140), reverse one 62 / 94 / 135.  Of these, filling the pipeline takes as long as some 10 timesteps.  A carry pass and
+// a fold add 4 us of launches on the GPU and 12 of host time, which is what short calls wait for (with 12 for a training step's two of them
+// the picks lost 10 to 40 % below 256 steps).  Over 44 cases of 3840 steps (1 to 16 rows 64 to 5120 wide, both types, training and inference) the count picked takes
+// 1.9 % longer than the best one on average and 8.8 % at most; where it differs from what the times of earlier kernels picked (2.4 % of
+// shapes) it is 0.7 % faster on average, between 17 % faster and 13 % slower.
 int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
-  constexpr double kFill = 10, kFwdWide = 107, kFwd[] = {0, 85, 127, 185}, kBwd[] = {0, 315, 456, 636}, kFwdCarry[] = {0, 65, 96, 134},
-                   kBwdCarry[] = {0, 71, 104, 146};
+  constexpr double kFill = 10, kFwdSaving[] = {0, 82, 123, 174}, kFwd[] = {0, 79, 121, 170}, kBwd[] = {0, 279, 378, 538},
+                   kFwdCarry[] = {0, 55, 87, 125}, kBwdCarry[] = {0, 62, 94, 135}, kFwdWide[] = {105, 112};
   const double items = double(batch) * double((width + 31) / 32);
   const double sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   auto passes = [&](double ctas, const double (&t)[4]) {                 // of 2048 timesteps on the longest SM
@@ -218,7 +218,7 @@ int64_t pick_pieces(int64_t batch, int64_t length, int64_t width, bool grad) {
     const double len = double(S == 1 ? length : (length + 16 * S - 1) / (16 * S) * 16);
     if (S > 1 && (S - 1) * len >= length) continue;
     const bool wide = items * S > sms && double(batch) * double((width + 47) / 48) * S <= sms;      // one 48-channel CTA per SM instead
-    double all = (wide ? kFwdWide : passes(items * S, kFwd)) + (grad ? passes(items * S, kBwd) : 0);
+    double all = (wide ? kFwdWide[grad] : passes(items * S, grad ? kFwdSaving : kFwd)) + (grad ? passes(items * S, kBwd) : 0);
     if (S > 1) all += passes(items * (S - 1), kFwdCarry) + (grad ? passes(items * (S - 1), kBwdCarry) : 0);
     const double us = all * (len + kFill) / (2048 + kFill) + (S > 1 ? (grad ? 24 : 12) : 0);
     if (S == 1 || us < best_us) {
