@@ -246,26 +246,83 @@ def test_rows_cut_into_pieces_bf16_long():
         assert_close(gk[k], go[k].float(), BF_RTOL, BF_ATOL * scale, f"grad {k}")
 
 
+def _wide(rows, ED):
+    """Whether such a forward takes one 48-channel CTA per SM."""
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    return rows * -(-ED // 32) > sms >= rows * -(-ED // 48)
+
+
+# A of channels 0, 1, ... of a tile of 48: as initialised, any, or by turns (a warp with both takes the general path, and the warps
+# 1 and 4 of a wide tile hold two state quads, which no warp of a narrow one does)
+def _some_A(kind, r, ED):
+    fresh, other = -torch.arange(1, 17, device=DEV, dtype=torch.float32).repeat(ED, 1), -torch.exp(r(ED, 16))
+    if kind == "mixed":
+        other = torch.where((torch.arange(ED, device=DEV) % 48 < 20)[:, None], fresh, other)
+    return fresh if kind == "fresh" else other
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("reverse", [False, True])
-@pytest.mark.parametrize("ED, L", [(32 * 148 + 8, 45), (48 * 148, 16)])
-def test_wide_tiles(dtype, reverse, ED, L):
-    """One CTA of 48 channels per SM (more 32-channel tiles than the 148 SMs, ragged last tile) against the same channels in two
-    launches of 32-channel tiles: the same operations in the same order."""
+@pytest.mark.parametrize("rows, L, full", [(1, 45, False), (1, 16, True), (3, 40, True), (3, 29, False)])
+@pytest.mark.parametrize("A_kind", ["any", "fresh", "mixed"])
+@pytest.mark.parametrize("softplus", [False, True])
+def test_wide_tiles(dtype, reverse, rows, L, full, A_kind, softplus):
+    """One CTA of 48 channels per SM (more 32-channel tiles than SMs; as many wide tiles as SMs, or a ragged last one) against the same
+    channels in two launches of 32-channel tiles: the same operations in the same order, but for warps whose channels and quads take
+    the two paths of the decay by turns."""
     from mamba_b200.mamba import sscan_fwd_raw
+    per_row = torch.cuda.get_device_properties(DEV).multi_processor_count // rows
+    ED = 48 * per_row if full else 32 * per_row + 40
+    cut = ED // 16 * 8
+    assert _wide(rows, ED) and not _wide(rows, cut) and not _wide(rows, ED - cut)
     g = torch.Generator(device="cuda").manual_seed(ED)
     r = lambda *s: torch.randn(*s, generator=g, device=DEV)
-    x, z = r(1, L, ED).to(dtype), r(1, L, ED).to(dtype)
-    delta = torch.nn.functional.softplus(r(1, L, ED) - 3).to(dtype)
-    A, Bm, Cm, D, h0 = -torch.exp(r(ED, 16)), r(1, L, 16).to(dtype), r(1, L, 16).to(dtype), r(ED), r(1, ED, 16)
+    x, z = r(rows, L, ED).to(dtype), r(rows, L, ED).to(dtype)
+    delta, bias = r(rows, L, ED), r(ED) - 3 if softplus else None
+    delta = (delta if softplus else torch.nn.functional.softplus(delta - 3)).to(dtype)
+    A, Bm, Cm, D, h0 = _some_A(A_kind, r, ED), r(rows, L, 16).to(dtype), r(rows, L, 16).to(dtype), r(ED), r(rows, ED, 16)
     run = lambda a, b, want: sscan_fwd_raw(x[..., a:b], delta[..., a:b], A[a:b], Bm, Cm, D[a:b], z[..., a:b], h0=h0[:, a:b].contiguous(),
-                                           want_last=True, want_carries=want, reverse=reverse)
+                                           delta_bias=bias[a:b] if softplus else None, want_last=True, want_carries=want, reverse=reverse)
+
+    def same(a, b, name):
+        if A_kind != "mixed":
+            assert torch.equal(a, b), name
+        else:                                          # decays good to 2^-20 of their rate either way: the contract of either path
+            rt, at = (RTOL, ATOL) if a.dtype == torch.float32 else (BF_RTOL, BF_ATOL)
+            assert_close(a, b, rt, at * max(1.0, b.abs().max().item()), name)
+
     for want in (False, True):
-        whole, parts = run(0, ED, want), [run(a, b, want) for a, b in ((0, 2560), (2560, ED))]
-        assert torch.equal(whole[0], torch.cat([p[0] for p in parts], 2))
-        assert torch.equal(whole[1], torch.cat([p[1] for p in parts], 1))
+        whole, parts = run(0, ED, want), [run(a, b, want) for a, b in ((0, cut), (cut, ED))]
+        same(whole[0], torch.cat([p[0] for p in parts], 2), "y")
+        same(whole[1], torch.cat([p[1] for p in parts], 1), "state")
         if want:
-            assert torch.equal(whole[2], torch.cat([p[2] for p in parts], 3))
+            same(whole[2], torch.cat([p[2] for p in parts], 3), "saved states")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("A_kind", ["any", "fresh"])
+@pytest.mark.parametrize("rows, S", [(1, 4), (2, 3)])
+def test_wide_tiles_of_pieces(dtype, A_kind, rows, S):
+    """Rows cut into as many pieces as give every SM one 48-channel CTA, against the whole rows in 32-channel tiles: outputs, the
+    outgoing state and every gradient, with an incoming state."""
+    import mamba_b200
+    per_row = torch.cuda.get_device_properties(DEV).multi_processor_count // (rows * S)
+    ED, L = 48 * per_row - 8, 16 * 5 * S
+    assert _wide(rows * S, ED) and not _wide(rows, ED)
+    g = torch.Generator(device="cuda").manual_seed(ED)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    act = [t.to(dtype).requires_grad_() for t in (r(rows, L, ED), r(rows, L, ED), r(rows, L, 16), r(rows, L, 16), r(rows, L, ED))]
+    par = [t.requires_grad_() for t in (_some_A(A_kind, r, ED), r(ED), r(ED) - 3, r(rows, ED, 16))]
+    (x, delta, Bm, Cm, z), (A, D, bias, h0), dy = act, par, r(rows, L, ED).to(dtype)
+
+    def run(pieces):
+        y, hT = mamba_b200.selective_scan_fn(x, delta, A, Bm, Cm, D, z=z, delta_bias=bias, h0=h0, return_last_state=True, subshards=pieces)
+        return (y, hT) + torch.autograd.grad(y, act + par, dy)
+
+    names = "y hT x delta B C z A D bias h0".split()
+    for name, a, b in zip(names, run(S), run(1)):
+        rt, at = (RTOL, ATOL) if dtype == torch.float32 else (BF_RTOL, BF_ATOL)
+        assert_close(a, b, rt, at * 4 * max(1.0, b.float().abs().max().item()), name)
 
 
 def test_extreme_delta_in_the_backward():
