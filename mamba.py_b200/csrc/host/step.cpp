@@ -128,18 +128,19 @@ std::tuple<Tensor, Tensor> conv_step(const Tensor& x, const Tensor& inputs, cons
 // Whether so few tokens that the one launch is the better way.  It reads the activations of all tokens from shared memory again for
 // every output row, where the library's bfloat16 kernels use the tensor cores; the float32 ones take longer nearly everywhere.  us a
 // layer, weights from HBM, called from Python / inside a CUDA graph, one launch : library:
-//               256 wide             768 wide             1536 wide             2560 wide
-//   float32  1  15/17 : 39/16        21/23 : 39/28        32/33 : 52/39         59/59 : 68/54
-//            2  16/17 : 40/25        23/24 : 58/47        36/37 : 102/91        71/72 : 146/138
-//            4  17/18 : 40/28        27/29 : 65/53        45/46 : 112/97        92/93 : 129/117
-//            8  21/22 : 43/34        38/40 : 80/69        67/67 : 105/92        140/141 : 161/146
-//   bfloat16 1  15/16 : 47/16        21/23 : 48/24        30/31 : 51/31         51/52 : 54/43
-//            2  18/19 : 48/15        27/29 : 49/24        39/40 : 52/30         72/72 : 53/43
-//            4  23/25 : 48/16        41/44 : 49/23        60/61 : 52/30         122/121 : 54/43
-//            8  35/37 : 49/16        73/75 : 49/23        103/104 : 52/30       217/216 : 54/44
-// (Before the rows of a phase were spread over all SMs, which took 5 to 35 % off the one launch and nothing off the library.)
+//               256 wide             768 wide             1536 wide            2560 wide
+//   float32  1  14/16 : 40/16        21/23 : 42/29        32/31 : 55/39         61/59 : 71/55
+//            2  15/16 : 40/22        22/23 : 59/47        38/37 : 105/92        73/72 : 149/139
+//            4  15/17 : 40/28        25/27 : 65/54        43/42 : 114/101       90/88 : 131/117
+//            8  17/19 : 43/34        33/33 : 81/69        61/59 : 109/92        128/126 : 164/146
+//   bfloat16 1  15/17 : 49/19        21/22 : 50/24        28/28 : 52/31         51/50 : 58/44
+//            2  16/18 : 49/16        23/25 : 51/24        35/35 : 53/30         67/66 : 58/43
+//            4  17/19 : 50/16        31/33 : 51/23        51/50 : 53/30         107/105 : 56/43
+//            8  21/22 : 50/19        47/48 : 51/23        84/84 : 52/30         184/183 : 57/44
+// One token 4096 wide 106/104 : 113/96 in float32, 77/79 : 86/71 in bfloat16.
 // So up to 8 tokens in float32, and in bfloat16 as long as the tokens the kernel is built for (1, 2, 4, 8) times the inner width are
-// at most 8192 values.
+// at most 8192 values.  Beyond that a call from Python still gains a little here and there (4 x 1536 51 : 53, 8 x 768 47 : 51, 8 x 1024 42 : 51),
+// but only host time: the GPU is busy for twice as long (8 x 1024 in a graph 43 : 26).
 static constexpr int64_t kOneLaunchTokens = 8, kOneLaunchValuesBf16 = 8192;
 static bool takes_one_launch(int64_t tokens, int64_t d_model, int64_t width, at::ScalarType dt) {
   if (tokens < 1 || tokens > kOneLaunchTokens) return false;

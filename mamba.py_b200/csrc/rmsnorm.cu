@@ -313,7 +313,9 @@ norm_rows_fwd_kernel(const TX* __restrict__ x, const TR* __restrict__ res_in, co
 // given, is ds once more, dense and rounded: the gradient of a bfloat16 mixer output beside that of the float32 stream.
 // The grid is one wave of CTAs, so that the rows they walk are few and the dweight atomics too: as many as fit by registers, 3 per SM
 // with up to 3 chunks a thread (compiled for that: 88 registers instead of 80 let only two in, and a grid for three then ran in two
-// waves), 2 with 4 and 1 with 8.  us before / after, 12.6 M elements in float32: 53 / 40 at 768 wide, 46 / 38 at 192, 46 / 34 at 2048,
+// waves), 2 with 4 and 1 with 8.  Some of these spill 8 to 24 bytes for it (3 chunks of float32: 116 us with the spill against 123 for
+// two CTAs per SM at 60000 x 768 with a residual gradient, 30.9 / 28.9 at 16384 x 768 without one, 7.4 / 5.5 at 2048; 4 chunks: 36 against
+// 51 for one CTA at 16384 x 1024).  us before / after, 12.6 M elements in float32: 53 / 40 at 768 wide, 46 / 38 at 192, 46 / 34 at 2048,
 // 54 / 46 at 5120 (with 3 CTAs per SM forced on 4 chunks 46 and 60 at 2048 and 2560, for 34 and 47).
 constexpr int norm_bwd_ctas(int chunks) { return chunks <= 3 ? 3 : chunks == 4 ? 2 : 1; }
 template <typename TR, typename TY, int kTPR, int kC>

@@ -72,9 +72,10 @@ constexpr int kTile = 2 * kChunk;          // timesteps per tile (two saved stat
 constexpr int kLoadAhead = MB200_FWD_LA, kDecayAhead = MB200_FWD_EA;   // software-pipeline depths of the recurrence warps
 constexpr int kDefer = MB200_FWD_DEFER;     // timesteps of partial sums a recurrence thread holds before storing them
 // kWide: 6 + 6 warps and 48 channels, alone on its SM.  For a scan whose 32-channel tiles are a few more than the SMs, so that some SMs
-// hold two and the rest wait for them: us per 2048 steps with one such CTA 98-106 on every SM, with two of 32 channels 112-125 (with one
-// 77-83).  With more CTAs than SMs the narrow tile is the better one (two of 48 channels 169-191, three of 32 157-175); 40 channels
-// (5 + 5 warps) straddle state quads and took 95-104.
+// hold two and the rest wait for them: us per 2048 steps without saved states with one such CTA on every SM 102-109, with two of 32 channels
+// 116-126 (with one 79-80).  With more CTAs than SMs two of 48 channels (163-177) are as fast as three of 32 (164-177), so there is nothing
+// to gain.  40 channels (5 + 5 warps) took 95-104 when 48 took 98-106: where 40 are few enough for one CTA per SM (4737 to 5920 channels
+// over all rows, a 5120-wide prompt among them) they would be some 2 % faster, for another eight kernels; not built.
 template <int N, bool kWide = false> struct FwdGeom {
   static constexpr int kCPT = (N == 16) ? MB200_FWD_CPT : 1;
   static constexpr int kCW = kWide ? 6 : (N == 16) ? MB200_FWD_CW : 4;
